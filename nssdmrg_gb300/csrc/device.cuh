@@ -115,7 +115,7 @@ struct DevLanczos {
     float *slot32 = nullptr;     // [3][n] H*psi parts of the persistent chunk kernel
     size_t chunk_smem = 0;
     bool chunk_ok = false;       // the chunk kernel fits (one CTA per SM)
-    int chunk_vc = 0;            // basis vectors in its shared-memory row cache (0: no cache)
+    int chunk_vc = 0;            // basis vectors in its shared-memory row cache (2, or 0: no cache)
     int chunk_cs = 0;            // cached floats per vector (rows of one CTA)
     size_t chunk_smem_vc = 0;    // its dynamic shared memory with the row cache
     float *pitem = nullptr;      // per-item alpha partials of the batched kernel
@@ -126,6 +126,7 @@ struct DevLanczos {
     // of CHECK iterations with the key it was captured for
     void *vcur = nullptr;        // [n] doubles' room
     int *jdev = nullptr;
+    float *pro = nullptr;        // omega estimates of the partial reorthogonalisation (see k_lanczos.cu)
     cudaGraphExec_t gx = nullptr;
     uint64_t gx_gen = 0;
     int gx_prec = -1, gx_mmax = 0, gx_ndefl = -1, gx_launches = 0;

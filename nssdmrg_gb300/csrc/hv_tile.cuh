@@ -351,6 +351,15 @@ __device__ __forceinline__ void item_store(Item32Smem &sm, int ph, int k0, int k
     }
 }
 
+// The anchored refinement's vectors whose products with H v are wanted: u
+// and nd deflation vectors y[k*n..] (u null: none)
+struct AncCols {
+    const float *u, *y;
+    int nd;
+    int64_t n;
+};
+constexpr int ANC_MAX = 5;              // u and up to four y
+
 // One item by 256 threads (lt = thread index in the group): each thread owns
 // rows {ty, ty+16} x columns {2tx, 2tx+1}, so a K step of four costs two
 // float4 and four float2 shared-memory reads for sixteen FMAs.  The staged
@@ -359,11 +368,13 @@ __device__ __forceinline__ void item_store(Item32Smem &sm, int ph, int k0, int k
 // part in columns 0..63, H_R part in 64..127), a LEFT / RIGHT item its K
 // range (<= HV_KMAX) in one round per 128.  The A x B tables (and the
 // per-term offsets) are read in the same round.  The outputs times `scale`
-// go to the item's slot; returns this thread's share of sum_i (v[i] scale)
-// (out[i] scale) over its outputs.
-template <class Sync>
-__device__ __forceinline__ float hv32_item(const ItemRec &it, const float *__restrict__ v, float *const *slots,
-                                           const Hv32Ops &op, Item32Smem &sm, int lt, Sync sync, float scale) {
+// go to the item's slot; this thread's share of sum_i (v[i] scale)
+// (out[i] scale) over its outputs is added to p[0], those of u.out and
+// y_k.out to p[1..NA].
+template <int NA, class Sync>
+__device__ __forceinline__ void hv32_item(const ItemRec &it, const float *__restrict__ v, float *const *slots,
+                                          const Hv32Ops &op, Item32Smem &sm, int lt, Sync sync, float scale,
+                                          const AncCols &ac, float (&p)[1 + NA]) {
     const int row0 = it.a.y, col0 = it.a.z, part = it.a.w;
     const int dl = it.b.x, dr = it.b.y, t0 = it.b.z, t1 = it.b.w;
     const int64_t o = lohi(it.c.x, it.c.y);
@@ -486,18 +497,24 @@ __device__ __forceinline__ float hv32_item(const ItemRec &it, const float *__res
         }
     }
     float *out = slots[part == HV_LEFT ? 1 : (part == HV_RIGHT ? 2 : 0)] + o;
-    float p = 0.f;
+#pragma unroll
     for (int rr = 0; rr < 2; ++rr)
+#pragma unroll
         for (int cc = 0; cc < 2; ++cc) {
             const int il = row0 + ty + 16 * rr, ir = col0 + 2 * tx + cc;
             if (il < dl && ir < dr) {
                 const int64_t idx2 = (int64_t)il * dr + ir;
                 const float y = acc[rr][cc] * scale;
                 out[idx2] = y;
-                p = fmaf(W[idx2] * scale, y, p);
+                p[0] = fmaf(W[idx2] * scale, y, p[0]);
+                if constexpr (NA > 0) {
+                    if (ac.u) p[1] = fmaf(ac.u[o + idx2], y, p[1]);
+#pragma unroll
+                    for (int k = 0; k < NA - 1; ++k)
+                        if (k < ac.nd) p[2 + k] = fmaf(ac.y[(int64_t)k * ac.n + o + idx2], y, p[2 + k]);
+                }
             }
         }
-    return p;
 }
 
 }  // namespace nss

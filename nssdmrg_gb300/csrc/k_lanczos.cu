@@ -2,28 +2,41 @@
 // small tridiagonal problem on the host.
 //
 // Replaces SciFortran sp_eigh (ARPACK, called at src/DMRG_SUPERBLOCK.f90:
-// 394-425) for the direct mode.  Algorithm: Lanczos with full
-// reorthogonalisation -- the three-term recurrence first, then one classical
-// Gram-Schmidt projection of the (small) residual against the whole basis,
-// and a second projection only when that one removes more than half of the
-// residual -- the whole Krylov basis kept resident in HBM (no restarts), and a
-// convergence test every CHECK steps on the tridiagonal matrix T_m:
+// 394-425) for the direct mode.  Algorithm: Lanczos with partial
+// reorthogonalisation, the whole Krylov basis kept resident in HBM (no
+// restarts), and a convergence test every CHECK steps on the tridiagonal matrix T_m:
 // residual beta_m |s_m| <= tol |theta| for each wanted Ritz pair, the ARPACK
 // criterion.  Breakdown (beta ~ 0, invariant subspace) restarts with a fresh
 // random vector orthogonal to the basis.  Eigenvectors are gauge-dependent,
 // so parity with the reference is on eigenvalues and on what the RDM derives
 // from them.
 //
+// Orthogonality is kept by partial reorthogonalisation (H. D. Simon, "The
+// Lanczos algorithm with partial reorthogonalization", Math. Comp. 42
+// (1984)): a recurrence on the inner products omega_{j,k} = v_j . v_k, driven
+// by alpha, beta and rounding terms, estimates the loss, and the projection
+// against the whole basis (classical Gram-Schmidt, repeated when it removes
+// more than half of the residual) runs only at a step where an estimate
+// exceeds a threshold, and at the step after it.  A basis orthogonal to
+// sqrt(eps) gives a tridiagonal matrix within eps ||H|| of the projection of
+// H on its span, so Ritz values are as accurate as with a projection at every
+// step; the threshold lies lower (struct Pro) so that the vectors are too.  On
+// the measured superblocks 4 to 12 of 50 to 100 steps project.  A projection
+// reads the basis twice (2 N m sizeof(T) bytes) and costs two more grid
+// barriers.  Against projecting at every step, solves went from 5.6 to 3.3 ms
+// (FP64, N = 3 958), 13.1 to 10.1 ms (FP64, 66 600), 2.72 to 2.52 ms (mixed,
+// 66 600), 13.9 to 10.8 ms (mixed, 398 000), and 16 batched solves of up to
+// 9 500 states from 10.9 to 10.1 ms.
+//
 // Per iteration j (m = j+1 basis vectors) two kinds of launch:
 //   sector H*psi   w = H v_j                      (k_hv_* kernels)
 //   k_orth         one cooperative launch, one CTA per SM, each CTA owning a
 //                  contiguous slice of the rows; grid barriers separate
 //                    alpha = v_j . w
-//                    w -= alpha v_j + beta_{j-1} v_{j-1};  h = V_m^T w, ww = w.w
-//                    w -= V_m h, beta^2 = w.w  (again if beta^2 < ww/2)
+//                    w -= alpha v_j + beta_{j-1} v_{j-1};  beta^2 = w.w
+//                    (at a projecting step: h = V_m^T w; w -= V_m h, beta^2 =
+//                    w.w, again if it fell by more than half)
 //                    v_{j+1} = w / beta, or the breakdown flag
-// Projecting the raw H v_j instead (one pass) lets the orthogonality error
-// grow by ||H||/beta per step; the recurrence-first order keeps it at 1e-15.
 // Every grid-level sum is reduced by every CTA in the same fixed order, so
 // all CTAs hold bitwise identical scalars and take the same branches.
 //
@@ -335,7 +348,69 @@ struct OrthArgs {
     // fixed input of the next H*psi (null: step a.j, no copy)
     int *jdev;
     void *vcur;
+    // omega estimates: [pstride] of v_j, [pstride] of v_{j-1}, then one int
+    // (the next step projects whatever its estimates say) and, anchored, the
+    // products of u and y_k with v_j and with v_{j-1}
+    float *pro;
 };
+
+// The omega recurrence's constants per basis type: level after a projection,
+// rounding term per (beta_k + beta_j + |alpha_j|: H v_j is rounded at the size
+// of its largest part), and the threshold.  sqrt(eps) would do
+// for Ritz values; what a projection takes off a vector (up to beta times the
+// threshold, mostly along a converged Ritz vector) is not in the tridiagonal
+// matrix, though, and enters a wanted vector that has not converged yet.  At
+// 5e-13 that stays below the solver's tolerance (at 1e-8 a 96-state
+// superblock's residual was 1e-10 |theta|); it costs two to four more
+// projecting steps a solve.  The FP32 phase's vector is refined afterwards.
+template <class T>
+struct Pro;
+template <>
+struct Pro<double> {
+    static constexpr float EPS1 = 4.4e-16f, NOISE = 2.2e-16f, DELTA = 5e-13f;
+};
+template <>
+struct Pro<float> {
+    static constexpr float EPS1 = 2.4e-7f, NOISE = 1.2e-7f, DELTA = 5e-5f;
+};
+
+constexpr int PRO_TAIL = 16;     // floats after the estimates: the int, then two rows of ANC_MAX products
+
+// The start of a Lanczos run (or of a restart from a vector orthogonal to
+// the basis): every estimate at the level of a projection
+__global__ void k_pro_reset(float *pro, int ps, float eps1) {
+    for (int k = threadIdx.x; k < 2 * ps; k += blockDim.x) pro[k] = eps1;
+    if (threadIdx.x < PRO_TAIL) pro[2 * ps + threadIdx.x] = 0.f;
+}
+
+// The estimates of v_{j+1} from those of v_j (so) and v_{j-1} (sp) into sn,
+// for the tridiagonal coefficients sa, sb (sa[j], sb[j] included); returns
+// whether one exceeds the threshold (same value in every thread and CTA).
+// Called by all threads; m = j + 1.  FP32 is enough for estimates, and an
+// FP64 chain would take as long as the rest of a small step.
+template <class T>
+__device__ __forceinline__ bool pro_step(const float *so, const float *sp, const float *sa, const float *sb, float *sn,
+                                         int j, float delta = Pro<T>::DELTA) {
+    const float bj = sb[j], aj = sa[j], bp = j > 0 ? sb[j - 1] : 0.f, ib = 1.f / bj;
+    int over = 0;
+    for (int k = threadIdx.x; k <= j; k += blockDim.x) {
+        float t;
+        if (k < j) {
+            const float bk = sb[k];
+            const float up = k + 1 == j ? 1.f : so[k + 1];
+            const float old = k + 1 == j ? 1.f : sp[k];
+            t = bk * up + (sa[k] - aj) * so[k] - bp * old;
+            if (k > 0) t += sb[k - 1] * so[k - 1];
+            t += copysignf(Pro<T>::NOISE * (bk + bj + fabsf(aj)), t);
+            t *= ib;
+        } else {
+            t = fmaxf(Pro<T>::EPS1, Pro<T>::NOISE * fabsf(aj) * ib);
+        }
+        sn[k] = t;
+        if (!(fabsf(t) <= delta)) over = 1;
+    }
+    return __syncthreads_or(over) != 0;
+}
 
 constexpr int PA_COLS = 8;       // per-CTA values of the first phase (alpha, u.w, r.v, y_k.w)
 
@@ -392,21 +467,30 @@ __device__ __forceinline__ void fail_exit(unsigned *bar, int *h_flags) {
     grid_exit(bar);
 }
 
-// CTA sums of NV values at once (512 threads), valid in thread 0
+// CTA sums of NV values at once, valid in thread 0; only the first nw warps
+// hold values (uniform over the CTA).  An FP64 add takes a warp's share of the
+// FP64 pipe for 64 cycles, so a small superblock's CTA, whose few rows fill
+// one or two warps, must not run the tree on all sixteen.
 template <class R, int NV>
-__device__ __forceinline__ void block_sums(R (&v)[NV], R *scr) {
+__device__ __forceinline__ void block_sums(R (&v)[NV], R *scr, int nw = ORTH_WARPS) {
+    const int warp = threadIdx.x >> 5;
+    if (warp < nw) {
 #pragma unroll
-    for (int q = 0; q < NV; ++q) v[q] = warp_sum<R>(v[q]);
+        for (int q = 0; q < NV; ++q) v[q] = warp_sum<R>(v[q]);
+    }
+    if (nw == 1) return;
     __syncthreads();
-    if ((threadIdx.x & 31) == 0)
+    if (warp < nw && (threadIdx.x & 31) == 0)
 #pragma unroll
-        for (int q = 0; q < NV; ++q) scr[q * ORTH_WARPS + (threadIdx.x >> 5)] = v[q];
+        for (int q = 0; q < NV; ++q) scr[q * ORTH_WARPS + warp] = v[q];
     __syncthreads();
-    if (threadIdx.x < 32) {
+    if (warp == 0) {
 #pragma unroll
         for (int q = 0; q < NV; ++q) {
-            R t = threadIdx.x < ORTH_WARPS ? scr[q * ORTH_WARPS + threadIdx.x] : (R)0;
-            v[q] = warp_sum<R>(t);
+            R t = threadIdx.x < nw ? scr[q * ORTH_WARPS + threadIdx.x] : (R)0;
+#pragma unroll
+            for (int o = ORTH_WARPS / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+            v[q] = t;
         }
     }
 }
@@ -426,7 +510,8 @@ __device__ __forceinline__ R strided_sum(const R *p, int i0, int end, int stride
             v[q] = b < end ? __ldcg(p + b) : (R)0;
         }
 #pragma unroll
-        for (int q = 0; q < 8; ++q) t += v[q];
+        for (int q = 0; q < 8; ++q)
+            if (b0 + q * stride < end) t += v[q];
     }
     return t;
 }
@@ -572,9 +657,61 @@ __host__ __device__ inline int orth_redsz(int pstride, int cw) {
     return ORTH_WARPS * cw > pstride + cw ? ORTH_WARPS * cw : pstride + cw;
 }
 
-// shared memory of k_orth, in elements of T: hs, red, scratch
+// floats of the omega recurrence in shared memory: estimates of v_j, v_{j-1},
+// v_{j+1}, alpha, beta
+__host__ __device__ inline size_t pro_floats(int pstride) { return 5 * (size_t)((pstride + 3) & ~3); }
+
+// shared memory of k_orth in bytes: hs, red, scratch (T), the recurrence
 __host__ __device__ inline size_t orth_smem(int pstride, int cw, size_t tsize) {
-    return (size_t)(pstride + orth_redsz(pstride, cw) + 8 * ORTH_WARPS + 16) * tsize;
+    const size_t t = (size_t)(pstride + orth_redsz(pstride, cw) + 8 * ORTH_WARPS + 16) * tsize;
+    return ((t + 15) & ~(size_t)15) + pro_floats(pstride) * sizeof(float);
+}
+
+// The recurrence's shared arrays
+struct ProSmem {
+    float *so, *sp, *sn, *sa, *sb;
+    __device__ ProSmem(void *base, int ps) {
+        const int st = (ps + 3) & ~3;
+        so = (float *)base;
+        sp = so + st;
+        sn = sp + st;
+        sa = sn + st;
+        sb = sa + st;
+    }
+    // state of step j from global memory (estimates, alpha_k, beta_k, k < j)
+    __device__ __forceinline__ void load(const float *pro, int ps, const double *alpha, const double *beta, int j) {
+        for (int k = threadIdx.x; k < j; k += blockDim.x) {
+            so[k] = __ldcg(pro + k);
+            sp[k] = __ldcg(pro + ps + k);
+            sa[k] = (float)__ldcg(alpha + k);
+            sb[k] = (float)__ldcg(beta + k);
+        }
+    }
+    // after step j: the new estimates become v_{j+1}'s
+    __device__ __forceinline__ void advance() {
+        float *t = sp;
+        sp = so;
+        so = sn;
+        sn = t;
+    }
+    __device__ __forceinline__ void store(float *pro, int ps, int j, int force) const {
+        for (int k = threadIdx.x; k <= j; k += blockDim.x) {
+            pro[k] = so[k];
+            pro[ps + k] = sp[k];
+        }
+        if (threadIdx.x == 0) *(int *)(pro + 2 * ps) = force;
+    }
+};
+
+// FP64 superblocks of fewer states than this project at every step: the
+// truncation errors of small chains (1 - sum lambda, 1e-12) follow the last
+// bits of the ground state, so their arithmetic stays what it was.  An FP32
+// basis projects at every step once it fills an eighth of its space: close to
+// exhausting it the estimates' model no longer holds.
+constexpr int64_t PRO_MIN_N = 3072;
+template <class T>
+__device__ __forceinline__ bool pro_always(int m, int64_t n) {
+    return sizeof(T) == 8 ? n < PRO_MIN_N : 8 * (int64_t)m > n;
 }
 
 template <class T, int CW>
@@ -592,16 +729,18 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_orth(OrthArgs a) {
     T *red = hs + ps;
     T *scr = red + orth_redsz(ps, CW);               // [8 x 16] block sums, then [16] broadcasts
     T *bc = scr + 8 * ORTH_WARPS;
+    ProSmem pro(osm_raw + (orth_smem(ps, CW, sizeof(T)) - pro_floats(ps) * sizeof(float)), ps);
     const int G = gridDim.x, blk = blockIdx.x, tid = threadIdx.x;
     const int64_t n = a.n;
     const int64_t chunk = (n + G - 1) / G;
     const int64_t i0 = min(n, (int64_t)blk * chunk), i1 = min(n, i0 + chunk);
+    const int nw = (int)min((int64_t)ORTH_WARPS, max((int64_t)1, (chunk + 31) / 32));   // warps with rows
     T *V = (T *)a.V, *w = (T *)a.w;
     const int j = a.jdev ? *(volatile const int *)a.jdev : a.j, m = j + 1;
     const T *vj = V + (int64_t)j * n;
     const T *vjm = V + (int64_t)(j > 0 ? j - 1 : 0) * n;
     T *pA = (T *)a.part, *pH = pA + PA_COLS * G, *pB = pH + (int64_t)ps * G, *pH2 = pB + G,
-      *pB2 = pH2 + (int64_t)ps * G;
+      *pB2 = pH2 + (int64_t)ps * G, *pW = pB2 + G;
     int *err = flags + F_ERR;
     const T *au = (const T *)a.anc_u, *ar = (const T *)a.anc_r, *ay = (const T *)a.defl;
     const bool anc = au != nullptr;
@@ -626,14 +765,17 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_orth(OrthArgs a) {
                 if (k < nd) av[3 + k] += ay[(int64_t)k * n + i] * wi;
         }
     }
+    const T beta_m = j > 0 ? (T)__ldcg(a.beta + j - 1) : (T)0;
+    if (!pro_always<T>(m, n)) pro.load(a.pro, ps, a.alpha, a.beta, j);
+    int force = __ldcg((const int *)(a.pro + 2 * ps));
     if (anc) {
-        block_sums<T, PA_COLS>(av, scr);
+        block_sums<T, PA_COLS>(av, scr, nw);
         if (tid == 0)
 #pragma unroll
             for (int q = 0; q < PA_COLS; ++q) pA[q * G + blk] = av[q];
     } else {
         T a1[1] = {av[0]};
-        block_sums<T, 1>(a1, scr);
+        block_sums<T, 1>(a1, scr, nw);
         if (tid == 0) pA[blk] = a1[0];
     }
     if (blk == 0 && tid == 0) flags[F_HOST] = host_stop;
@@ -655,77 +797,149 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_orth(OrthArgs a) {
         tot[0] = t1[0];
     }
     const T alpha0 = tot[0];
-    {   // three-term step (and the anchor projections), then h = V_m^T w and ww = w.w
-        const T b3 = j > 0 ? (T)a.beta[j - 1] : (T)0;
-        for (int64_t i = i0 + tid; i < i1; i += ORTH_THREADS) {
-            T x = w[i] - alpha0 * vj[i];
-            if (j > 0) x -= b3 * vjm[i];
-            if (anc) {
-                x -= tot[1] * au[i];
+    const bool always = pro_always<T>(m, n);
+    // three-term step (and the anchor projections); ww = w.w, and what is left
+    // of w along u and y_k, taken off when w is normalised: alpha v_j and
+    // beta v_{j-1} bring back alpha and beta times the rounding-level products
+    // u.v_j and u.v_{j-1}, which would grow from step to step
+    T ew[1 + ANC_MAX];
 #pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    if (k < nd) x -= tot[3 + k] * ay[(int64_t)k * n + i];
-            }
-            w[i] = x;
+    for (int q = 0; q < 1 + ANC_MAX; ++q) ew[q] = (T)0;
+    for (int64_t i = i0 + tid; i < i1; i += ORTH_THREADS) {
+        T x = w[i] - alpha0 * vj[i];
+        if (j > 0) x -= beta_m * vjm[i];
+        if (anc) {
+            x -= tot[1] * au[i];
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (k < nd) x -= tot[3 + k] * ay[(int64_t)k * n + i];
+            ew[1] += au[i] * x;
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (k < nd) ew[2 + k] += ay[(int64_t)k * n + i] * x;
+        }
+        w[i] = x;
+        if (!always) ew[0] += x * x;
+    }
+    T bb[1] = {(T)0};
+    bool project = always;
+    if (!always || anc) {
+        if (anc) {
+            block_sums<T, 1 + ANC_MAX>(ew, scr, nw);
+            if (tid == 0)
+#pragma unroll
+                for (int q = 0; q < 1 + ANC_MAX; ++q) pW[q * G + blk] = ew[q];
+        } else {
+            T s1[1] = {ew[0]};
+            block_sums<T, 1>(s1, scr, nw);
+            if (tid == 0) pW[blk] = s1[0];
+        }
+        if (!grid_sync(a.bar, epoch, err, a.spin)) { fail_exit(a.bar, a.h_flags); return; }
+        if (anc) {
+            grid_totals<T, 1 + ANC_MAX>(pW, G, bc, ew);
+            bb[0] = ew[0];
+        } else {
+            grid_totals<T, 1>(pW, G, bc + 8, bb);
+        }
+    }
+    if (!always) {
+        // does this step project?  (same decision in every CTA; beta in FP32
+        // is enough for the estimates)
+        if (tid == 0) {
+            pro.sa[j] = (float)alpha0;
+            pro.sb[j] = sqrtf((float)bb[0]);
         }
         __syncthreads();
-        cta_dots<T, CW>(V, m, w, n, i0, i1, true, red, pH + blk, G);
+        const bool over = pro_step<T>(pro.so, pro.sp, pro.sa, pro.sb, pro.sn, j);
+        project = over || force;
+        if (project) {
+            force = over && !force;
+            for (int k = tid; k <= j; k += ORTH_THREADS) pro.sn[k] = Pro<T>::EPS1;
+        }
     }
-    if (!grid_sync(a.bar, epoch, err, a.spin)) { fail_exit(a.bar, a.h_flags); return; }
-    grid_columns<T>(pH, G, m + 1, hs);
-    __syncthreads();
-    const T ww = hs[m];
-    T hj = hs[j];
-    {
-        T s1[1] = {cta_update<T>(V, m, w, n, i0, i1, hs)};
-        block_sums<T, 1>(s1, scr);
-        if (tid == 0) pB[blk] = s1[0];
-    }
-    if (!grid_sync(a.bar, epoch, err, a.spin)) { fail_exit(a.bar, a.h_flags); return; }
-    T bb[1];
-    grid_totals<T, 1>(pB, G, bc + 8, bb);
-    if (bb[0] < (T)0.5 * ww) {   // second projection (same decision in every CTA)
-        cta_dots<T, CW>(V, m, w, n, i0, i1, false, red, pH2 + blk, G);
-        if (!grid_sync(a.bar, epoch, err, a.spin)) { fail_exit(a.bar, a.h_flags); return; }
-        grid_columns<T>(pH2, G, m, hs);
+    T hj = (T)0;
+    if (project) {
         __syncthreads();
-        hj += hs[j];
-        T s1[1] = {cta_update<T>(V, m, w, n, i0, i1, hs)};
-        block_sums<T, 1>(s1, scr);
-        if (tid == 0) pB2[blk] = s1[0];
+        cta_dots<T, CW>(V, m, w, n, i0, i1, true, red, pH + blk, G);
         if (!grid_sync(a.bar, epoch, err, a.spin)) { fail_exit(a.bar, a.h_flags); return; }
-        grid_totals<T, 1>(pB2, G, bc + 9, bb);
+        grid_columns<T>(pH, G, m + 1, hs);
+        __syncthreads();
+        const T ww = hs[m];
+        hj = hs[j];
+        {
+            T s1[1] = {cta_update<T>(V, m, w, n, i0, i1, hs)};
+            block_sums<T, 1>(s1, scr, nw);
+            if (tid == 0) pB[blk] = s1[0];
+        }
+        if (!grid_sync(a.bar, epoch, err, a.spin)) { fail_exit(a.bar, a.h_flags); return; }
+        grid_totals<T, 1>(pB, G, bc + 9, bb);
+        if (bb[0] < (T)0.5 * ww) {   // second projection (same decision in every CTA)
+            cta_dots<T, CW>(V, m, w, n, i0, i1, false, red, pH2 + blk, G);
+            if (!grid_sync(a.bar, epoch, err, a.spin)) { fail_exit(a.bar, a.h_flags); return; }
+            grid_columns<T>(pH2, G, m, hs);
+            __syncthreads();
+            hj += hs[j];
+            T s1[1] = {cta_update<T>(V, m, w, n, i0, i1, hs)};
+            block_sums<T, 1>(s1, scr, nw);
+            if (tid == 0) pB2[blk] = s1[0];
+            if (!grid_sync(a.bar, epoch, err, a.spin)) { fail_exit(a.bar, a.h_flags); return; }
+            grid_totals<T, 1>(pB2, G, bc + 10, bb);
+        }
     }
     const T alpha_j = alpha0 + hj;
-    const T beta_j = sqrt(bb[0]);
+    // one warp takes the root and the reciprocal: on all sixteen they would
+    // hold the FP64 pipe for over a microsecond
+    if (tid < 32) {
+        const T bt = sqrt(bb[0]);
+        const T iv = (T)1 / bt;
+        if (tid == 0) {
+            bc[11] = bt;
+            bc[12] = iv;
+        }
+    }
+    __syncthreads();
+    const T beta_j = bc[11];
     bool brk = false;
     if (m < a.mmax) {
-        const T scale = fmax(fabs(alpha_j), j > 0 ? (T)a.beta[j - 1] : (T)0);
+        const T scale = fmax(fabs(alpha_j), beta_m);
         brk = !(beta_j > (T)1e-13 * fmax(scale, (T)1e-30));
         if (!brk) {
-            const T inv = (T)1 / beta_j;
+            const T inv = bc[12];
             T *vn = V + (int64_t)m * n;
             T *vc = (T *)a.vcur;
             for (int64_t i = i0 + tid; i < i1; i += ORTH_THREADS) {
-                const T x = w[i] * inv;
+                T x = w[i];
+                if (anc) {
+                    x -= ew[1] * au[i];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        if (k < nd) x -= ew[2 + k] * ay[(int64_t)k * n + i];
+                }
+                x *= inv;
                 vn[i] = x;
                 if (vc) vc[i] = x;
             }
         }
     }
-    if (blk == 0 && tid == 0) {
-        if (a.jdev) *a.jdev = j + 1;   // every CTA read j before the first barrier
-        a.alpha[j] = (double)alpha_j;
-        a.beta[j] = (double)beta_j;
-        a.h_alpha[j] = (double)alpha_j;
-        a.h_beta[j] = (double)beta_j;
-        if (brk) {
-            flags[F_BREAK] = m;
-            flags[F_STOP] = 2;
-            a.h_flags[F_BREAK] = m;
-            a.h_flags[F_STOP] = 2;
+    if (blk == 0) {
+        if (!always) {
+            pro.advance();
+            pro.store(a.pro, ps, j, force);          // every CTA read its copy before the first barrier
         }
-        __threadfence_system();
+        if (tid == 0) {
+            if (a.jdev) *a.jdev = j + 1;             // every CTA read j before the first barrier
+            a.alpha[j] = (double)alpha_j;
+            a.beta[j] = (double)beta_j;
+            a.h_alpha[j] = (double)alpha_j;
+            a.h_beta[j] = (double)beta_j;
+            if (brk) {
+                flags[F_BREAK] = m;
+                flags[F_STOP] = 2;
+                a.h_flags[F_BREAK] = m;
+                a.h_flags[F_STOP] = 2;
+            }
+            __threadfence_system();
+        }
     }
     grid_exit(a.bar);
 }
@@ -741,12 +955,12 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_orth(OrthArgs a) {
 //                  previous w'' scaled by 1/beta, the alpha partials come out
 //                  of the item epilogues
 //   barrier
-//   three-term step on the CTA's rows (w = slot0 + slot1 - alpha v_j -
-//   beta v_{j-1}) and the CGS dots, with the anchored refinement's extra
-//   columns (u.w, r.v_j, y_k.w)
-//   barrier, column sums, update w -= V h, beta^2 partials
-//   barrier, (second projection when needed), next step
-// so an iteration costs three grid barriers and no launch.  V rows are only
+//   three-term step on the CTA's rows (w = slots - alpha v_j - beta v_{j-1},
+//   less the anchored refinement's components along u and y_k), beta^2 = w.w
+//   barrier; beta, the omega estimates; at a projecting step the CGS dots,
+//   a barrier, column sums, w -= V h, beta^2 partials, a barrier (and again
+//   when the projection removed more than half)
+// so an iteration costs two grid barriers and no launch.  V rows are only
 // touched by the CTA that owns them; the work vectors alternate between two
 // buffers so that the items reading w''_{j-1} (all rows) never race with the
 // writes of w''_j.  The normalisation v_j = w''_{j-1} / beta_{j-1} is written
@@ -762,12 +976,12 @@ struct ChunkArgs {
     const ItemRec *items;
     int nitems;
     Hv32Ops op;
-    // shared-memory copy of the CTA's rows: basis vectors V[l < vc] and the
-    // work vector, `cs` floats per vector (0: everything from global memory)
+    // shared-memory copy of the CTA's rows of the last two basis vectors and
+    // of the work vector (vc = 2; 0: everything from global memory), `cs`
+    // floats per vector
     int vc = 0, cs = 0;
 };
 
-constexpr int CHUNK_EXTRA = 8;   // extra partial columns of the anchored refinement
 constexpr int CHUNK_MAXIT = 16;  // iterations per launch (>= CHECK)
 
 __host__ __device__ inline size_t chunk_smem(int pstride) {
@@ -787,77 +1001,7 @@ inline bool chunk_cache_enabled() {
     return !(e && std::atoi(e) == 0);
 }
 
-__device__ __forceinline__ void cp_async4(float *dst, const float *src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
-                 : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
-// cta_dots on the row cache: the CTA's rows of V[l] (l < vc) at vs[l*cs + r]
-// and of w at ws[r] (r = row - i0).  Cached columns: one warp per column,
-// the lanes down the rows, one warp sum (shared-memory operands need no
-// loads in flight; the multi-column form below measured 3-5 us here against
-// 1.5 us).  Columns l >= vc stream from global memory in the multi-column
-// form of cta_dots (CW columns per lane, to keep enough loads in flight).
-template <int CW>
-__device__ __forceinline__ void cta_dots_vc(const float *__restrict__ vs, int vc, int cs, const float *__restrict__ V,
-                                            int m, const float *__restrict__ ws, int64_t n, int64_t i0, int64_t i1,
-                                            bool ww, float *red, float *out, int G) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int len = (int)(i1 - i0);
-    const int mc = min(m, vc);
-    const int n1 = mc + ((ww && m <= vc) ? 1 : 0);   // the w.w column here when nothing is left beyond the cache
-    for (int l = warp; l < n1; l += ORTH_WARPS) {
-        const float *src = l < mc ? vs + (int64_t)l * cs : ws;
-        float acc = 0.f;
-#pragma unroll 8
-        for (int r = lane; r < len; r += 32) acc += src[r] * ws[r];
-        acc = warp_sum<float>(acc);
-        if (lane == 0) out[(int64_t)l * G] = acc;
-    }
-    if (m <= vc) return;
-    const int ncol = m - vc + (ww ? 1 : 0);
-    const int ng = (ncol + CW - 1) / CW;
-    const int nq = ng >= ORTH_WARPS ? 1 : ORTH_WARPS / ng;
-    const int rs = ng * CW;
-    const int qlen = (len + nq - 1) / nq;
-    const float *Vg = V + i0;
-    for (int item = warp; item < ng * nq; item += ORTH_WARPS) {
-        const int g = item % ng, q = item / ng, l0 = vc + g * CW;
-        const int r0 = q * qlen, r1 = min(len, r0 + qlen);
-        float acc[CW];
-#pragma unroll
-        for (int c = 0; c < CW; ++c) acc[c] = 0.f;
-        if (l0 + CW <= m) {
-            const float *vr = Vg + (int64_t)l0 * n;
-            for (int r = r0 + lane; r < r1; r += 32) {
-                const float wv = ws[r];
-#pragma unroll
-                for (int c = 0; c < CW; ++c) acc[c] += vr[(int64_t)c * n + r] * wv;
-            }
-        } else {
-            for (int r = r0 + lane; r < r1; r += 32) {
-                const float wv = ws[r];
-#pragma unroll
-                for (int c = 0; c < CW; ++c) {
-                    const int l = l0 + c;
-                    if (l < m) acc[c] += Vg[(int64_t)l * n + r] * wv;
-                    else if (ww && l == m) acc[c] += wv * wv;
-                }
-            }
-        }
-        const float s = multi_reduce<float, CW>(acc, lane);
-        if (lane < CW && l0 - vc + lane < ncol) red[q * rs + l0 - vc + lane] = s;
-    }
-    __syncthreads();
-    for (int l = threadIdx.x; l < ncol; l += ORTH_THREADS) {
-        float s = 0.f;
-        for (int q = 0; q < nq; ++q) s += red[q * rs + l];
-        out[(int64_t)(vc + l) * G] = s;
-    }
-}
-
+template <bool ANC>
 __global__ void __launch_bounds__(ORTH_THREADS, 1) k_chunk32(ChunkArgs a) {
     constexpr int CW = OrthCW<float>::value;
     int *flags = a.o.flags;
@@ -875,43 +1019,52 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_chunk32(ChunkArgs a) {
     float *red = hs + ps;
     float *scr = red + orth_redsz(ps, CW);
     float *bc = scr + 8 * ORTH_WARPS;
+    ProSmem pro(chunk_raw + (chunk_smem(ps) - pro_floats(ps) * sizeof(float)), ps);
     const int G = gridDim.x, blk = blockIdx.x, tid = threadIdx.x, grp = tid >> 8, lt = tid & 255;
     const int64_t n = a.o.n;
     const int64_t chunk = (n + G - 1) / G;
     const int64_t i0 = min(n, (int64_t)blk * chunk), i1 = min(n, i0 + chunk);
+    const int nw = (int)min((int64_t)ORTH_WARPS, max((int64_t)1, (chunk + 31) / 32));   // warps with rows
     float *V = (float *)a.o.V;
     float *pA = (float *)a.o.part, *pH = pA + PA_COLS * G, *pB = pH + (int64_t)ps * G, *pH2 = pB + G,
-          *pB2 = pH2 + (int64_t)ps * G;
+          *pB2 = pH2 + (int64_t)ps * G, *pW = pB2 + G;
     int *err = flags + F_ERR;
-    const float *au = (const float *)a.o.anc_u, *ar = (const float *)a.o.anc_r, *ay = (const float *)a.o.defl;
-    const bool anc = au != nullptr;
-    const int nd = anc ? a.o.ndefl : 0;
-    const int nx = anc ? 3 + nd : 0;                 // extra columns: u.w, r.v_j, y_k.w
-    // row cache: the dots and updates of every iteration read the CTA's rows
-    // of V and of w from shared memory instead of L2 (a round of dependent
-    // loads less per phase); global V and w stay complete (other CTAs read
-    // w, the host-side steps read V).  The basis vectors of earlier launches
-    // are copied in asynchronously, behind the first H*psi items.
+    const float *ar = (const float *)a.o.anc_r;
+    const AncCols ac{(const float *)a.o.anc_u, (const float *)a.o.defl, a.o.ndefl, n};
+    // row cache: the three-term step reads the CTA's rows of v_{j-1} and of
+    // the previous w from shared memory instead of L2 (one round of loads
+    // less per step); global V and w stay complete
     const bool yc = a.vc > 0;
-    const int vc = a.vc, cs = a.cs;
-    float *vcache = (float *)(chunk_raw + chunk_cache_off(ps));
-    float *ycache = vcache + (size_t)vc * cs;
-    if (yc) {
-        const int rows = (int)(i1 - i0);
-        const int npre = min(vc, a.first_from_v ? a.j0 + 1 : a.j0);
-        for (int e = tid; e < npre * rows; e += ORTH_THREADS) {
-            const int l = e / rows, r = e - l * rows;
-            cp_async4(vcache + l * cs + r, V + (int64_t)l * n + i0 + r);
-        }
-        cp_async_commit();
-    }
+    const int cs = a.cs;
+    float *vcache = (float *)(chunk_raw + chunk_cache_off(ps));   // V[l] at slot l & 1
+    float *ycache = vcache + 2 * (size_t)cs;
     float beta_prev = a.j0 > 0 ? (float)a.o.beta[a.j0 - 1] : 0.f;
+    pro.load(a.o.pro, ps, a.o.alpha, a.o.beta, a.j0);
+    // u.v_j, y_k.v_j and u.v_{j-1}, y_k.v_{j-1}: rounding level, but alpha v_j
+    // and beta v_{j-1} in the three-term step would let them grow
+    constexpr int NA = ANC ? ANC_MAX : 0;            // anchor columns
+    float dc[NA + 1], dm[NA + 1];
+#pragma unroll
+    for (int q = 0; q < NA; ++q) {
+        dc[q] = __ldcg(a.o.pro + 2 * ps + 1 + q);
+        dm[q] = __ldcg(a.o.pro + 2 * ps + 1 + ANC_MAX + q);
+    }
+    int force = __ldcg((const int *)(a.o.pro + 2 * ps));
     int done = 0, brk_m = 0;
     // CTA 0 publishes the completed iterations (device arrays, host mirrors)
     auto publish = [&]() {
         if (tid == 0 && *(volatile int *)err) {
             a.o.h_flags[F_ERR] = 1;
             __threadfence_system();
+        }
+        if (blk == 0 && done > 0) {
+            pro.store(a.o.pro, ps, a.j0 + done - 1, force);
+            if (tid == 0)
+#pragma unroll
+                for (int q = 0; q < NA; ++q) {
+                    a.o.pro[2 * ps + 1 + q] = dc[q];
+                    a.o.pro[2 * ps + 1 + ANC_MAX + q] = dm[q];
+                }
         }
         if (blk == 0 && tid == 0) {
             for (int q = 0; q < done; ++q) {
@@ -920,7 +1073,7 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_chunk32(ChunkArgs a) {
                 a.o.beta[j] = (double)rec_b[q];
                 a.o.h_alpha[j] = (double)rec_a[q];
                 a.o.h_beta[j] = (double)rec_b[q];
-                if (anc) a.o.h_m[j] = (double)rec_m[q];
+                if constexpr (ANC) a.o.h_m[j] = (double)rec_m[q];
             }
             if (brk_m) {
                 flags[F_BREAK] = brk_m;
@@ -940,16 +1093,16 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_chunk32(ChunkArgs a) {
         float *y = a.buf[(jj + 1) & 1];
         int host_stop = 0;
         if (blk == 0 && tid == 0) host_stop = *(volatile const int *)(a.o.h_flags + F_NFLAGS);
-        // H v_j into the slots, alpha partials from the items
-        float ap = 0.f;
+        // H v_j into the slots; alpha, u.w and y_k.w partials from the items
+        float ap[1 + NA];
+#pragma unroll
+        for (int q = 0; q < 1 + NA; ++q) ap[q] = 0.f;
         for (int ti = 2 * blk + grp; ti < a.nitems; ti += 2 * G)
-            ap += hv32_item(a.items[ti], x, a.slot, a.op, ism[grp], lt, GroupSync{1 + grp}, sc);
-        if (yc && jj == a.j0) cp_async_wait_all();   // the row cache (published by the barriers below)
-        {
-            float a1[1] = {ap};
-            block_sums<float, 1>(a1, scr);
-            if (tid == 0) pA[blk] = a1[0];
-        }
+            hv32_item<NA>(a.items[ti], x, a.slot, a.op, ism[grp], lt, GroupSync{1 + grp}, sc, ac, ap);
+        block_sums<float, 1 + NA>(ap, scr);
+        if (tid == 0)
+#pragma unroll
+            for (int q = 0; q < 1 + NA; ++q) pA[q * G + blk] = ap[q];
         if (blk == 0 && tid == 0) flags[F_HOST] = host_stop;
         if (!grid_sync(a.o.bar, epoch, err, a.o.spin)) { publish(); return; }
         if (__ldcg(&flags[F_HOST])) {
@@ -963,125 +1116,120 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_chunk32(ChunkArgs a) {
         const int64_t if0 = i0 + tid;
         float hv0 = 0.f;
         if (if0 < i1) hv0 = s0[if0] + s1[if0] + s2[if0];
-        float alpha0;
-        {
-            float t1[1];
-            grid_totals<float, 1>(pA, G, bc, t1);
-            alpha0 = t1[0];
-        }
-        // v_j into V (own rows), three-term step, anchor extras
-        float ex[CHUNK_EXTRA];
+        float tot[1 + NA];
+        grid_totals<float, 1 + NA>(pA, G, bc, tot);
 #pragma unroll
-        for (int q = 0; q < CHUNK_EXTRA; ++q) ex[q] = 0.f;
+        for (int q = 0; q < NA; ++q) tot[1 + q] -= tot[0] * dc[q] + beta_prev * dm[q];
+        const float alpha0 = tot[0];
+        // v_j into V (own rows), three-term step, anchor projections; w.w,
+        // u.w, y_k.w and r.v_j
+        float sv[2 + NA];
+#pragma unroll
+        for (int q = 0; q < 2 + NA; ++q) sv[q] = 0.f;
         {
             float *vj = V + (int64_t)jj * n;
             const float *vjm = V + (int64_t)(jj > 0 ? jj - 1 : 0) * n;
             // own rows of x: the cached w of the previous iteration of this launch
             const bool xc = yc && jj > a.j0;
-            const bool jc = jj < vc, jmc = jj > 0 && jj - 1 < vc;
+            float *vcj = vcache + (jj & 1) * (size_t)cs;
+            const float *vcm = vcache + ((jj + 1) & 1) * (size_t)cs;
             for (int64_t i = if0; i < i1; i += ORTH_THREADS) {
                 const int r = (int)(i - i0);
                 const float v = (xc ? ycache[r] : x[i]) * sc;
                 if (!first) vj[i] = v;
-                if (jc) vcache[jj * cs + r] = v;
                 float w = (i == if0 ? hv0 : (s0[i] + s1[i] + s2[i])) - alpha0 * v;
-                if (jj > 0) w -= beta_prev * (jmc ? vcache[(jj - 1) * cs + r] : vjm[i]);
-                y[i] = w;
-                if (yc) ycache[r] = w;
-                if (anc) {
-                    ex[0] += au[i] * w;
-                    ex[1] += ar[i] * v;
+                if (jj > 0) w -= beta_prev * (xc ? vcm[r] : vjm[i]);
+                if constexpr (ANC) {
+                    sv[1] += ar[i] * v;
+                    w -= tot[1] * ac.u[i];
 #pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        if (k < nd) ex[2 + k] += ay[(int64_t)k * n + i] * w;
-                }
-            }
-        }
-        __syncthreads();
-        if (yc) cta_dots_vc<CW>(vcache, vc, cs, V, m, ycache, n, i0, i1, true, red, pH + blk, G);
-        else cta_dots<float, CW>(V, m, y, n, i0, i1, true, red, pH + blk, G);
-        if (anc) {
-            block_sums<float, CHUNK_EXTRA>(ex, scr);
-            if (tid == 0) {
-                pH[(int64_t)(m + 1) * G + blk] = ex[0];
-                pH[(int64_t)(m + 2) * G + blk] = ex[1];
+                    for (int k = 0; k < ANC_MAX - 1; ++k)
+                        if (k < ac.nd) w -= tot[2 + k] * ac.y[(int64_t)k * n + i];
+                    sv[2] += ac.u[i] * w;
 #pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    if (k < nd) pH[(int64_t)(m + 3 + k) * G + blk] = ex[2 + k];
-            }
-        }
-        if (!grid_sync(a.o.bar, epoch, err, a.o.spin)) { publish(); return; }
-        grid_columns<float>(pH, G, m + 1 + nx, hs);
-        __syncthreads();
-        const float ww = hs[m];
-        float hj = hs[jj];
-        const float mj = anc ? hs[m + 2] : 0.f;
-        // w -= V h (+ the anchor and deflation components)
-        auto update = [&](int xoff) -> float {
-            float ss = 0.f;
-            const int mc = min(m, vc);
-            for (int64_t i = i0 + tid; i < i1; i += ORTH_THREADS) {
-                const int r = (int)(i - i0);
-                float w = yc ? ycache[r] : y[i];
-#pragma unroll 8
-                for (int l = 0; l < mc; ++l) w -= vcache[l * cs + r] * hs[l];
-#pragma unroll 32
-                for (int l = mc; l < m; ++l) w -= V[(int64_t)l * n + i] * hs[l];
-                if (anc) {
-                    w -= hs[xoff] * au[i];
-                    for (int k = 0; k < nd; ++k) w -= hs[xoff + 2 + k] * ay[(int64_t)k * n + i];
+                    for (int k = 0; k < ANC_MAX - 1; ++k)
+                        if (k < ac.nd) sv[3 + k] += ac.y[(int64_t)k * n + i] * w;
                 }
                 y[i] = w;
-                if (yc) ycache[r] = w;
-                ss += w * w;
+                if (yc) {
+                    vcj[r] = v;
+                    ycache[r] = w;
+                }
+                sv[0] += w * w;
             }
-            return ss;
-        };
-        {
-            float s1[1] = {update(m + 1)};
-            block_sums<float, 1>(s1, scr);
-            if (tid == 0) pB[blk] = s1[0];
+        }
+        if constexpr (ANC) {
+            block_sums<float, 2 + NA>(sv, scr, nw);
+            if (tid == 0)
+#pragma unroll
+                for (int q = 0; q < 2 + NA; ++q) pW[q * G + blk] = sv[q];
+        } else {
+            float s1[1] = {sv[0]};
+            block_sums<float, 1>(s1, scr, nw);
+            if (tid == 0) pW[blk] = s1[0];
         }
         if (!grid_sync(a.o.bar, epoch, err, a.o.spin)) { publish(); return; }
-        float bb;
-        {
+        if constexpr (ANC) {
+            grid_totals<float, 2 + NA>(pW, G, bc + 8, sv);
+        } else {
             float t1[1];
-            grid_totals<float, 1>(pB, G, bc + 8, t1);
-            bb = t1[0];
+            grid_totals<float, 1>(pW, G, bc + 8, t1);
+            sv[0] = t1[0];
         }
-        if (bb < 0.5f * ww) {   // second projection (same decision in every CTA)
-            if (yc) cta_dots_vc<CW>(vcache, vc, cs, V, m, ycache, n, i0, i1, false, red, pH2 + blk, G);
-            else cta_dots<float, CW>(V, m, y, n, i0, i1, false, red, pH2 + blk, G);
-            if (anc) {
-#pragma unroll
-                for (int q = 0; q < CHUNK_EXTRA; ++q) ex[q] = 0.f;
+        float bb = sv[0];
+        const float mj = sv[1];
+        if (tid == 0) {
+            pro.sa[jj] = alpha0;
+            pro.sb[jj] = sqrtf(bb);
+        }
+        __syncthreads();
+        // does this step project?  (same decision in every CTA)
+        const bool over = pro_step<float>(pro.so, pro.sp, pro.sa, pro.sb, pro.sn, jj);
+        float hj = 0.f;
+        if (over || force || pro_always<float>(m, n)) {
+            force = over && !force;
+            for (int k = tid; k <= jj; k += ORTH_THREADS) pro.sn[k] = Pro<float>::EPS1;
+            // w -= V h
+            auto update = [&]() -> float {
+                float ss = 0.f;
                 for (int64_t i = i0 + tid; i < i1; i += ORTH_THREADS) {
-                    const float w = yc ? ycache[i - i0] : y[i];
-                    ex[0] += au[i] * w;
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        if (k < nd) ex[2 + k] += ay[(int64_t)k * n + i] * w;
+                    float w = y[i];
+#pragma unroll 32
+                    for (int l = 0; l < m; ++l) w -= V[(int64_t)l * n + i] * hs[l];
+                    y[i] = w;
+                    if (yc) ycache[i - i0] = w;
+                    ss += w * w;
                 }
-                block_sums<float, CHUNK_EXTRA>(ex, scr);
-                if (tid == 0) {
-                    pH2[(int64_t)m * G + blk] = ex[0];
-                    pH2[(int64_t)(m + 1) * G + blk] = 0.f;
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        if (k < nd) pH2[(int64_t)(m + 2 + k) * G + blk] = ex[2 + k];
-                }
+                return ss;
+            };
+            cta_dots<float, CW>(V, m, y, n, i0, i1, false, red, pH + blk, G);
+            if (!grid_sync(a.o.bar, epoch, err, a.o.spin)) { publish(); return; }
+            grid_columns<float>(pH, G, m, hs);
+            __syncthreads();
+            hj = hs[jj];
+            const float ww = bb;
+            {
+                float s1[1] = {update()};
+                block_sums<float, 1>(s1, scr, nw);
+                if (tid == 0) pB[blk] = s1[0];
             }
             if (!grid_sync(a.o.bar, epoch, err, a.o.spin)) { publish(); return; }
-            grid_columns<float>(pH2, G, m + (anc ? 2 + nd : 0), hs);
-            __syncthreads();
-            hj += hs[jj];
-            float s1[1] = {update(m)};
-            block_sums<float, 1>(s1, scr);
-            if (tid == 0) pB2[blk] = s1[0];
-            if (!grid_sync(a.o.bar, epoch, err, a.o.spin)) { publish(); return; }
             float t1[1];
-            grid_totals<float, 1>(pB2, G, bc + 9, t1);
+            grid_totals<float, 1>(pB, G, bc + 15, t1);
             bb = t1[0];
+            if (bb < 0.5f * ww) {   // second projection (same decision in every CTA)
+                cta_dots<float, CW>(V, m, y, n, i0, i1, false, red, pH2 + blk, G);
+                if (!grid_sync(a.o.bar, epoch, err, a.o.spin)) { publish(); return; }
+                grid_columns<float>(pH2, G, m, hs);
+                __syncthreads();
+                hj += hs[jj];
+                float s1[1] = {update()};
+                block_sums<float, 1>(s1, scr, nw);
+                if (tid == 0) pB2[blk] = s1[0];
+                if (!grid_sync(a.o.bar, epoch, err, a.o.spin)) { publish(); return; }
+                grid_totals<float, 1>(pB2, G, bc + 6, t1);
+                bb = t1[0];
+            }
         }
         const float alpha_j = alpha0 + hj;
         const float beta_j = sqrtf(bb);
@@ -1095,9 +1243,22 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_chunk32(ChunkArgs a) {
             rec_b[done] = beta_j;
             rec_m[done] = mj;
         }
+        if (tid == 0) {
+            pro.sa[jj] = alpha_j;
+            pro.sb[jj] = beta_j;
+        }
+        pro.advance();
+        if constexpr (ANC) {
+#pragma unroll
+            for (int q = 0; q < NA; ++q) {
+                dm[q] = dc[q];
+                dc[q] = sv[2 + q] / beta_j;
+            }
+        }
         ++done;
         if (brk) {
             brk_m = m;
+            __syncthreads();
             publish();
             return;
         }
@@ -1116,12 +1277,17 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_chunk32(ChunkArgs a) {
 // so every CTA takes the same barrier sequence: the per-solve decisions that
 // change it (second projection, breakdown, end of the chunk) are recomputed
 // by every CTA from the solves' partial sums, in the same order, so all CTAs
-// agree.  Solves stop within a launch only at their chunk end or at a
+// agree.  The omega estimates belong to a solve's own CTAs, so their verdict
+// reaches the others one step later: v_{j+1} over the threshold makes the
+// steps j+1 and j+2 project, with the threshold a quarter of the one of the
+// single-solve kernels for that step of growth.  All solves project together:
+// one solve's projection already costs everybody its two barriers, and solves
+// that start over at the same time come due at about the same time.  Solves stop within a launch only at their chunk end or at a
 // breakdown; the host checks convergence between launches.
 
 struct BatchSolve {
     ChunkArgs c;                 // per-solve arguments (c.o.bar unused)
-    float *pitem;                // [c.nitems] alpha partials of the solve's items
+    float *pitem;                // [2 c.nitems] alpha and u.w partials of the solve's items
     int cta0, ncta;              // CTAs owning the solve's rows
     int active;                  // takes part in this launch
     int pad;
@@ -1177,18 +1343,21 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_batch32(BatchArgs B) {
     float *red = hs + ps;
     float *scr = red + orth_redsz(ps, CW);
     float *bc = scr + 8 * ORTH_WARPS;
+    ProSmem pro(batch_raw + (chunk_smem(ps) - pro_floats(ps) * sizeof(float)), ps);
     const int64_t n = Mp ? Mp->c.o.n : 0;
     const int64_t chunk = (n + Gs - 1) / Gs;
     const int64_t i0 = min(n, (int64_t)lb * chunk), i1 = min(n, i0 + chunk);
+    if (Mp) pro.load(Mp->c.o.pro, ps, Mp->c.o.alpha, Mp->c.o.beta, Mp->c.j0);
+    float dc = Mp ? __ldcg(Mp->c.o.pro + 2 * ps + 1) : 0.f;            // u.v_j, u.v_{j-1} (see k_chunk32)
+    float dm = Mp ? __ldcg(Mp->c.o.pro + 2 * ps + 1 + ANC_MAX) : 0.f;
+    int owed = Mp ? __ldcg((const int *)(Mp->c.o.pro + 2 * ps)) : 0;   // projections its estimates still ask for
     float *V = Mp ? (float *)Mp->c.o.V : nullptr;
     float *pA = Mp ? (float *)Mp->c.o.part : nullptr;
-    float *pH = pA + PA_COLS * Gs, *pB = pH + (int64_t)ps * Gs, *pH2 = pB + Gs, *pB2 = pH2 + (int64_t)ps * Gs;
+    float *pH = pA + PA_COLS * Gs, *pB = pH + (int64_t)ps * Gs, *pH2 = pB + Gs, *pB2 = pH2 + (int64_t)ps * Gs,
+          *pW = pB2 + Gs;
     const float *au = Mp ? (const float *)Mp->c.o.anc_u : nullptr;
     const float *ar = Mp ? (const float *)Mp->c.o.anc_r : nullptr;
-    const float *ay = Mp ? (const float *)Mp->c.o.defl : nullptr;
-    const bool anc = au != nullptr;
-    const int nd = anc ? Mp->c.o.ndefl : 0;
-    const int nx = anc ? 3 + nd : 0;
+    const bool anc = au != nullptr;          // no deflation vectors: one state a solve
     int done = 0;
     for (int step = 0; step < B.steps; ++step) {
         // ---- H*psi of every running solve, all items over all CTAs: each
@@ -1206,15 +1375,20 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_batch32(BatchArgs B) {
                 const bool first = tj == S.c.j0 && S.c.first_from_v;
                 const float *x = first ? (const float *)S.c.o.V + (int64_t)tj * S.c.o.n : S.c.buf[tj & 1];
                 const float sc = first ? 1.f : 1.f / bprev[g.x];
-                float ap = hv32_item(S.c.items[g.y], x, S.c.slot, S.c.op, ism[grp], lt, GroupSync{1 + grp}, sc);
-                // group sum of the alpha partial (named barrier of the group)
-                ap = warp_sum<float>(ap);
-                if ((lt & 31) == 0) scr[grp * 8 + (lt >> 5)] = ap;
+                const AncCols ac{(const float *)S.c.o.anc_u, nullptr, 0, 0};
+                float ap[2] = {0.f, 0.f};
+                hv32_item<1>(S.c.items[g.y], x, S.c.slot, S.c.op, ism[grp], lt, GroupSync{1 + grp}, sc, ac, ap);
+                // group sums of the alpha and u.w partials (named barrier of the group)
+                const float a0 = warp_sum<float>(ap[0]), a1 = warp_sum<float>(ap[1]);
+                if ((lt & 31) == 0) {
+                    scr[grp * 16 + (lt >> 5)] = a0;
+                    scr[grp * 16 + 8 + (lt >> 5)] = a1;
+                }
                 GroupSync{1 + grp}();
-                if (lt == 0) {
+                if (lt < 2) {
                     float t = 0.f;
-                    for (int q = 0; q < 8; ++q) t += scr[grp * 8 + q];
-                    S.pitem[g.y] = t;
+                    for (int q = 0; q < 8; ++q) t += scr[grp * 16 + 8 * lt + q];
+                    S.pitem[(int64_t)lt * S.c.nitems + g.y] = t;
                 }
             }
             GroupSync{1 + grp}();
@@ -1229,145 +1403,129 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_batch32(BatchArgs B) {
         const float *x = run ? (first ? V + (int64_t)jj * n : Mp->c.buf[jj & 1]) : nullptr;
         const float sc = first ? 1.f : (me >= 0 ? 1.f / bprev[me] : 1.f);
         float *y = run ? Mp->c.buf[(jj + 1) & 1] : nullptr;
-        float ex[CHUNK_EXTRA];
-#pragma unroll
-        for (int q = 0; q < CHUNK_EXTRA; ++q) ex[q] = 0.f;
-        float alpha0 = 0.f;
+        const int nw = (int)min((int64_t)ORTH_WARPS, max((int64_t)1, (chunk + 31) / 32));
+        float alpha0 = 0.f, mj = 0.f, hj = 0.f, ud = 0.f;
         if (run) {
-            {   // alpha from the item partials, fixed order
-                float t = 0.f;
-                if (tid < 32) {
-                    t = strided_sum<float>(Mp->pitem, tid, Mp->c.nitems, 32);
+            float uw = 0.f;
+            {   // alpha (and u.w) from the item partials, fixed order
+                if (tid < 64) {
+                    float t = strided_sum<float>(Mp->pitem + (int64_t)(tid >> 5) * Mp->c.nitems, tid & 31, Mp->c.nitems, 32);
                     t = warp_sum<float>(t);
-                    if (tid == 0) bc[0] = t;
+                    if ((tid & 31) == 0) bc[tid >> 5] = t;
                 }
                 __syncthreads();
                 alpha0 = bc[0];
+                uw = bc[1] - alpha0 * dc - (jj > 0 ? bprev[me] * dm : 0.f);
             }
             float *vj = V + (int64_t)jj * n;
             const float *vjm = V + (int64_t)(jj > 0 ? jj - 1 : 0) * n;
             const float *s0 = Mp->c.slot[0], *s1 = Mp->c.slot[1], *s2 = Mp->c.slot[2];
+            float sv[3] = {0.f, 0.f, 0.f};
             for (int64_t i = i0 + tid; i < i1; i += ORTH_THREADS) {
                 const float v = x[i] * sc;
                 if (!first) vj[i] = v;
                 float w = (s0[i] + s1[i] + s2[i]) - alpha0 * v;
                 if (jj > 0) w -= bprev[me] * vjm[i];
-                y[i] = w;
                 if (anc) {
-                    ex[0] += au[i] * w;
-                    ex[1] += ar[i] * v;
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        if (k < nd) ex[2 + k] += ay[(int64_t)k * n + i] * w;
+                    sv[1] += ar[i] * v;
+                    w -= uw * au[i];
+                    sv[2] += au[i] * w;
                 }
+                y[i] = w;
+                sv[0] += w * w;
             }
-            __syncthreads();
-            cta_dots<float, CW>(V, m, y, n, i0, i1, true, red, pH + lb, Gs);
-            if (anc) {
-                block_sums<float, CHUNK_EXTRA>(ex, scr);
-                if (tid == 0) {
-                    pH[(int64_t)(m + 1) * Gs + lb] = ex[0];
-                    pH[(int64_t)(m + 2) * Gs + lb] = ex[1];
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        if (k < nd) pH[(int64_t)(m + 3 + k) * Gs + lb] = ex[2 + k];
+            block_sums<float, 3>(sv, scr, nw);
+            if (tid == 0) {
+                pW[lb] = sv[0];
+                pW[Gs + lb] = sv[1];
+                pW[2 * Gs + lb] = sv[2];
+                if (lb == 0) {
+                    B.st[4 * me + 0] = alpha0;
+                    B.st[4 * me + 1] = 0.f;          // h_j of a projection
                 }
             }
         }
         if (!grid_sync(B.bar, epoch, B.err, B.spin)) break;
-        float hj = 0.f, mj = 0.f;
-        auto update = [&](int xoff) -> float {
-            float ss = 0.f;
-            for (int64_t i = i0 + tid; i < i1; i += ORTH_THREADS) {
-                float w = y[i];
-#pragma unroll 32
-                for (int l = 0; l < m; ++l) w -= V[(int64_t)l * n + i] * hs[l];
-                if (anc) {
-                    w -= hs[xoff] * au[i];
-                    for (int k = 0; k < nd; ++k) w -= hs[xoff + 2 + k] * ay[(int64_t)k * n + i];
-                }
-                y[i] = w;
-                ss += w * w;
-            }
-            return ss;
-        };
-        if (run) {
-            grid_columns<float>(pH, Gs, m + 1 + nx, hs);
-            __syncthreads();
-            hj = hs[jj];
-            mj = anc ? hs[m + 2] : 0.f;
-            if (lb == 0 && tid == 0) {
-                B.st[4 * me + 0] = alpha0 + hj;
-                B.st[4 * me + 1] = hs[m];
-                B.st[4 * me + 2] = 0.f;
-            }
-            float s1[1] = {update(m + 1)};
-            block_sums<float, 1>(s1, scr);
-            if (tid == 0) pB[lb] = s1[0];
-        }
-        if (!grid_sync(B.bar, epoch, B.err, B.spin)) break;
-        // every CTA: beta^2 and the second-projection decision of every solve
+        // every CTA: w.w and whether the step projects, of every solve
         if (tid == 0) any_p2 = 0;
         __syncthreads();
         for (int s = tid; s < ns; s += ORTH_THREADS) {
             const BatchSolve &S = B.s[s];
             p2[s] = 0;
             if (!alive[s] || S.c.j0 + step >= S.c.jend) continue;
-            const float *pBs = (const float *)S.c.o.part + (PA_COLS + (int64_t)S.c.o.pstride) * S.ncta;
-            float t = 0.f;
-            t = strided_sum<float>(pBs, 0, S.ncta, 1);
-            bbb[s] = t;
+            const float *pWs = (const float *)S.c.o.part + (PA_COLS + 2 * (int64_t)S.c.o.pstride + 2) * S.ncta;
+            bbb[s] = strided_sum<float>(pWs, 0, S.ncta, 1);
             balpha[s] = __ldcg(B.st + 4 * s + 0);
-            if (t < 0.5f * __ldcg(B.st + 4 * s + 1)) {
-                p2[s] = 1;
-                any_p2 = 1;
-            }
+            const int ow = step == 0 ? __ldcg((const int *)(S.c.o.pro + 2 * S.c.o.pstride)) : __float_as_int(__ldcg(B.st + 4 * s + 3));
+            p2[s] = 1;
+            if (ow > 0 || pro_always<float>(S.c.j0 + step + 1, S.c.o.n)) any_p2 = 1;
         }
         __syncthreads();
-        if (any_p2) {
+        auto update = [&]() -> float {
+            float ss = 0.f;
+            for (int64_t i = i0 + tid; i < i1; i += ORTH_THREADS) {
+                float w = y[i];
+#pragma unroll 32
+                for (int l = 0; l < m; ++l) w -= V[(int64_t)l * n + i] * hs[l];
+                y[i] = w;
+                ss += w * w;
+            }
+            return ss;
+        };
+        if (run) {
+            float t2[2];
+            grid_totals<float, 2>(pW + Gs, Gs, bc + 2, t2);
+            mj = t2[0];
+            ud = t2[1];
+            if (tid == 0) {
+                pro.sa[jj] = alpha0;
+                pro.sb[jj] = sqrtf(bbb[me]);
+            }
+            __syncthreads();
+            const bool over = pro_step<float>(pro.so, pro.sp, pro.sa, pro.sb, pro.sn, jj, 0.25f * Pro<float>::DELTA);
+            if (any_p2) {
+                for (int k = tid; k <= jj; k += ORTH_THREADS) pro.sn[k] = Pro<float>::EPS1;
+                if (owed > 0) --owed;
+            } else if (over) {
+                owed = 2;
+            }
+        }
+        // the projections, up to two rounds (the second for the solves that
+        // lost more than half); pH / pB, then pH2 / pB2
+        for (int round = 0; round < 2 && any_p2; ++round) {
             const bool mine = run && p2[me];
+            float *ph = round == 0 ? pH : pH2, *pb = round == 0 ? pB : pB2;
+            if (mine) cta_dots<float, CW>(V, m, y, n, i0, i1, false, red, ph + lb, Gs);
+            if (!grid_sync(B.bar, epoch, B.err, B.spin)) { done = -1; break; }
             if (mine) {
-                cta_dots<float, CW>(V, m, y, n, i0, i1, false, red, pH2 + lb, Gs);
-                if (anc) {
-#pragma unroll
-                    for (int q = 0; q < CHUNK_EXTRA; ++q) ex[q] = 0.f;
-                    for (int64_t i = i0 + tid; i < i1; i += ORTH_THREADS) {
-                        const float w = y[i];
-                        ex[0] += au[i] * w;
-#pragma unroll
-                        for (int k = 0; k < 4; ++k)
-                            if (k < nd) ex[2 + k] += ay[(int64_t)k * n + i] * w;
-                    }
-                    block_sums<float, CHUNK_EXTRA>(ex, scr);
-                    if (tid == 0) {
-                        pH2[(int64_t)m * Gs + lb] = ex[0];
-                        pH2[(int64_t)(m + 1) * Gs + lb] = 0.f;
-#pragma unroll
-                        for (int k = 0; k < 4; ++k)
-                            if (k < nd) pH2[(int64_t)(m + 2 + k) * Gs + lb] = ex[2 + k];
-                    }
-                }
-            }
-            if (!grid_sync(B.bar, epoch, B.err, B.spin)) break;
-            if (mine) {
-                grid_columns<float>(pH2, Gs, m + (anc ? 2 + nd : 0), hs);
+                grid_columns<float>(ph, Gs, m, hs);
                 __syncthreads();
-                if (lb == 0 && tid == 0) B.st[4 * me + 2] = hs[jj];
-                float s1[1] = {update(m)};
-                block_sums<float, 1>(s1, scr);
-                if (tid == 0) pB2[lb] = s1[0];
+                hj += hs[jj];
+                if (lb == 0 && tid == 0) B.st[4 * me + 1] = hj;
+                float s1[1] = {update()};
+                block_sums<float, 1>(s1, scr, nw);
+                if (tid == 0) pb[lb] = s1[0];
             }
-            if (!grid_sync(B.bar, epoch, B.err, B.spin)) break;
+            if (!grid_sync(B.bar, epoch, B.err, B.spin)) { done = -1; break; }
+            if (tid == 0) any_p2 = 0;
+            __syncthreads();
             for (int s = tid; s < ns; s += ORTH_THREADS) {
                 if (!p2[s]) continue;
                 const BatchSolve &S = B.s[s];
-                const float *pB2s = (const float *)S.c.o.part + (PA_COLS + 2 * (int64_t)S.c.o.pstride + 1) * S.ncta;
-                float t = 0.f;
-                t = strided_sum<float>(pB2s, 0, S.ncta, 1);
+                const float *pBs = (const float *)S.c.o.part +
+                                   (PA_COLS + (round + 1) * (int64_t)S.c.o.pstride + round) * S.ncta;
+                const float t = strided_sum<float>(pBs, 0, S.ncta, 1);
+                const bool again = round == 0 && t < 0.5f * bbb[s];
                 bbb[s] = t;
-                balpha[s] += __ldcg(B.st + 4 * s + 2);
+                balpha[s] = __ldcg(B.st + 4 * s + 0) + __ldcg(B.st + 4 * s + 1);
+                p2[s] = again;
+                if (again) any_p2 = 1;
             }
             __syncthreads();
+        }
+        if (done < 0) {                              // a barrier ran out
+            done = 0;
+            break;
         }
         // every CTA: beta, breakdown, next scale of every solve that ran
         for (int s = tid; s < ns; s += ORTH_THREADS) {
@@ -1390,11 +1548,27 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_batch32(BatchArgs B) {
                 rec_a[done] = balpha[me];
                 rec_b[done] = bprev[me];
                 rec_m[done] = mj;
+                B.st[4 * me + 3] = __int_as_float(owed);   // read by all after the next step's barriers
             }
+            if (tid == 0) {
+                pro.sa[jj] = balpha[me];
+                pro.sb[jj] = bprev[me];
+            }
+            dm = dc;
+            dc = anc ? ud / bprev[me] : 0.f;
+            pro.advance();
             ++done;
         }
     }
     // publish the completed iterations of the own solve
+    __syncthreads();
+    if (me >= 0 && lb == 0 && done > 0) {
+        pro.store(Mp->c.o.pro, ps, Mp->c.j0 + done - 1, owed);
+        if (tid == 0) {
+            Mp->c.o.pro[2 * ps + 1] = dc;
+            Mp->c.o.pro[2 * ps + 1 + ANC_MAX] = dm;
+        }
+    }
     if (me >= 0 && lb == 0 && tid == 0) {
         const ChunkArgs &a = Mp->c;
         for (int q = 0; q < done; ++q) {
@@ -1692,22 +1866,22 @@ int ensure_lanczos(Ctx &c, int64_t n, int cap, bool mixed) {
     if (mixed) {
         // the persistent chunk kernel of the mixed method
         const size_t csm = chunk_smem(pstride);
-        // the row cache takes what one CTA per SM leaves: the CTA's rows of
-        // the work vector and of as many basis vectors as fit
+        // the row cache: the CTA's rows of the work vector and of the last two
+        // basis vectors, where they fit beside the rest
         const int64_t rows = (n + nsm - 1) / nsm;
         const int cs = (int)((rows + 3) & ~(int64_t)3);
         const size_t coff = chunk_cache_off(pstride), vbytes = (size_t)cs * sizeof(float);
         int vc = 0;
-        if (chunk_cache_enabled() && coff + 2 * vbytes <= CHUNK_SMEM_MAX)
-            vc = (int)std::min<int64_t>(cap + 1, (int64_t)((CHUNK_SMEM_MAX - coff - vbytes) / vbytes));
+        if (chunk_cache_enabled() && coff + 3 * vbytes <= CHUNK_SMEM_MAX) vc = 2;
         const size_t csm_vc = vc > 0 ? coff + (size_t)(vc + 1) * vbytes : csm;
-        NSS_CUDA_TRY(c, allow_smem((const void *)k_chunk32, std::max(csm, csm_vc)));
+        for (const void *fn : {(const void *)k_chunk32<false>, (const void *)k_chunk32<true>})
+            NSS_CUDA_TRY(c, allow_smem(fn, std::max(csm, csm_vc)));
         int occ2 = 0;
-        NSS_CUDA_TRY(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ2, (const void *)k_chunk32, ORTH_THREADS,
+        NSS_CUDA_TRY(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ2, (const void *)k_chunk32<true>, ORTH_THREADS,
                                                                       csm_vc));
         if (occ2 < 1 && vc > 0) {   // no room for the cache after all: run without it
             vc = 0;
-            NSS_CUDA_TRY(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ2, (const void *)k_chunk32, ORTH_THREADS,
+            NSS_CUDA_TRY(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ2, (const void *)k_chunk32<true>, ORTH_THREADS,
                                                                           csm));
         }
         if (occ2 >= 1) {
@@ -1727,10 +1901,11 @@ int ensure_lanczos(Ctx &c, int64_t n, int cap, bool mixed) {
         z.vcur = vc;
     }
     NSS_CUDA_TRY(c, ctx_alloc(c, &z.jdev, 1));
+    NSS_CUDA_TRY(c, ctx_alloc(c, &z.pro, (size_t)2 * pstride + PRO_TAIL));
     NSS_CUDA_TRY(c, ctx_alloc(c, &z.evecs, (size_t)4 * n));
     // scalars, projection coefficients, restart scratch alpha/beta, refinement
     NSS_CUDA_TRY(c, ctx_alloc(c, &z.scal, (size_t)S_NSCAL + 4 * (cap + 2) + 8));
-    const size_t part = std::max((size_t)(cap + 2) * NBLK, (size_t)(2 * pstride + PA_COLS + 2) * (size_t)nsm);
+    const size_t part = std::max((size_t)(cap + 2) * NBLK, (size_t)(2 * pstride + 2 * PA_COLS + 2) * (size_t)nsm);
     NSS_CUDA_TRY(c, ctx_alloc(c, &z.part, part));
     NSS_CUDA_TRY(c, ctx_alloc(c, &z.counter, 4));
     NSS_CUDA_TRY(c, ctx_alloc(c, &z.alpha, (size_t)cap + 1));
@@ -1855,6 +2030,7 @@ int run_lanczos(Ctx &c, T *V, T *w, int neigen, int mmax, double tol, uint64_t s
     oa.h_m = z.d_h_ab + 2 * (cap + 1);
     oa.spin = wait_limit();
     oa.jdev = nullptr;
+    oa.pro = z.pro;
     // the launched chunks keep vcur current too, so that a replayed chunk
     // can follow one
     oa.vcur = c.use_graphs ? z.vcur : nullptr;
@@ -1877,6 +2053,10 @@ int run_lanczos(Ctx &c, T *V, T *w, int neigen, int mmax, double tol, uint64_t s
     bool from_v = true;   // the next chunk starts from V[j0] (start, restart)
     auto enqueue_chunk = [&](int j0, int slot) -> int {
         const int jend = std::min(mmax, j0 + CHECK);
+        if (from_v) {
+            ++c.launches;
+            k_pro_reset<<<1, 512, 0, st>>>(z.pro, cap + 8, Pro<T>::EPS1);
+        }
         if (use_chunk && jend > j0) {
             ChunkArgs ca;
             ca.o = oa;
@@ -1901,7 +2081,7 @@ int run_lanczos(Ctx &c, T *V, T *w, int neigen, int mmax, double tol, uint64_t s
                 cudaEventCreate(&ct.b);
                 cudaEventRecord(ct.a, st);
             }
-            cudaError_t e = cudaLaunchCooperativeKernel((const void *)k_chunk32, dim3(z.orth_grid),
+            cudaError_t e = cudaLaunchCooperativeKernel(anc ? (const void *)k_chunk32<true> : (const void *)k_chunk32<false>, dim3(z.orth_grid),
                                                         dim3(ORTH_THREADS), args, z.chunk_smem_vc, st);
             if (c.time_chunks) {
                 cudaEventRecord(ct.b, st);
@@ -2168,7 +2348,7 @@ int run_lanczos(Ctx &c, T *V, T *w, int neigen, int mmax, double tol, uint64_t s
 void lanczos_release(Ctx &c) {
     DevLanczos &z = c.lz;
     void *ptrs[] = {z.V, z.w, z.V32, z.w32, z.anc32, z.wbuf32, z.slot32, z.evecs, z.rrw, z.scal, z.part, z.counter,
-                    z.alpha, z.beta, z.theta, z.resid, z.svec, z.flags, z.pitem, z.vcur, z.jdev};
+                    z.alpha, z.beta, z.theta, z.resid, z.svec, z.flags, z.pitem, z.vcur, z.jdev, z.pro};
     if (z.gx) cudaGraphExecDestroy(z.gx);
     for (void *p : ptrs) ctx_free(c, p);
     if (z.h_flags) cudaFreeHost(z.h_flags);
@@ -2527,6 +2707,8 @@ int engine_start_run(BatchEngine &E, BatchState &B) {
     NSS_CUDA_TRY(c0, cudaMemsetAsync(z.flags, 0, F_NFLAGS * sizeof(int), st));
     NSS_CUDA_TRY(c0, cudaMemsetAsync(z.beta, 0, (z.cap + 1) * sizeof(double), st));
     NSS_CUDA_TRY(c0, cudaMemsetAsync(z.slot32 + B.n, 0, (size_t)2 * B.n * sizeof(float), st));
+    ++c0.launches;
+    k_pro_reset<<<1, 512, 0, st>>>(z.pro, z.cap + 8, Pro<float>::EPS1);
     B.j0 = 0;
     B.from_v = true;
     B.have_upper = false;
@@ -2563,7 +2745,7 @@ int engine_add(BatchEngine &E, Ctx &c, uint64_t seed, int nitermax, double tol, 
     if (!z.pitem || z.cap_pitem < c.sb.nitems32) {
         ctx_free(c, z.pitem);
         z.pitem = nullptr;
-        NSS_CUDA_TRY(c0, ctx_alloc(c, &z.pitem, (size_t)std::max(c.sb.nitems32, 1)));
+        NSS_CUDA_TRY(c0, ctx_alloc(c, &z.pitem, (size_t)2 * std::max(c.sb.nitems32, 1)));
         z.cap_pitem = c.sb.nitems32;
     }
     if ((rc = engine_start_run(E, B))) return rc;
@@ -2655,6 +2837,7 @@ int engine_step(BatchEngine &E, int max_done, int *ndone, int *ids, double *ener
             oa.h_flags = z.d_h_flags;
             oa.h_m = z.d_h_ab + 2 * (z.cap + 1);
             oa.spin = wait_limit();
+            oa.pro = z.pro;
             const bool anc = B.phase == 2;
             oa.anc_u = anc ? (const void *)B.as.u32 : nullptr;
             oa.anc_r = anc ? (const void *)B.as.r32 : nullptr;
@@ -2771,6 +2954,8 @@ int engine_step(BatchEngine &E, int max_done, int *ndone, int *ids, double *ener
                 normalize_dev<float>(z, vn, B.n, st, c0.launches);
                 NSS_CUDA_TRY(c0, cudaMemsetAsync(z.beta + (m - 1), 0, sizeof(double), st));
                 NSS_CUDA_TRY(c0, cudaMemsetAsync(z.flags, 0, F_NFLAGS * sizeof(int), st));
+                ++c0.launches;
+                k_pro_reset<<<1, 512, 0, st>>>(z.pro, z.cap + 8, Pro<float>::EPS1);
                 z.h_ab[(z.cap + 1) + m - 1] = 0.0;
                 hf[F_STOP] = 0;
                 hf[F_BREAK] = 0;
