@@ -126,6 +126,8 @@ struct DevLanczos {
     // of CHECK iterations with the key it was captured for
     void *vcur = nullptr;        // [n] doubles' room
     int *jdev = nullptr;
+    uint64_t *xch = nullptr;     // tagged exchange words of the cooperative Lanczos kernels
+    size_t xwords = 0;
     float *pro = nullptr;        // omega estimates of the partial reorthogonalisation (see k_lanczos.cu)
     cudaGraphExec_t gx = nullptr;
     uint64_t gx_gen = 0;

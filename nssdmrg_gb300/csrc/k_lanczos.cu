@@ -352,6 +352,11 @@ struct OrthArgs {
     // (the next step projects whatever its estimates say) and, anchored, the
     // products of u and y_k with v_j and with v_{j-1}
     float *pro;
+    // tagged exchange (see xchg_totals): the last epoch of the previous
+    // launch, the words of the totals, of the columns' partials and of the
+    // columns' totals
+    unsigned *xep;
+    uint64_t *xtot, *xpart, *xcol;   // xcol: plain values
 };
 
 // The omega recurrence's constants per basis type: level after a projection,
@@ -420,6 +425,9 @@ constexpr int PA_COLS = 8;       // per-CTA values of the first phase (alpha, u.
 // critical path; grid_exit zeroes the counter when the last CTA leaves.
 // Bounded: a wait that runs out sets flags[F_ERR] and every later barrier
 // returns false at once, so the kernel always ends.
+// orders the writes that this thread has seen before its later stores (the
+// lighter fence: __threadfence is sequentially consistent)
+__device__ __forceinline__ void fence_acq_rel() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned *p) {
     unsigned v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -432,7 +440,7 @@ __device__ __forceinline__ bool grid_sync(unsigned *bar, unsigned &epoch, int *e
     if (threadIdx.x == 0) {
         int good = 1;
         epoch += gridDim.x;
-        __threadfence();
+        fence_acq_rel();
         atomicAdd(bar, 1u);
         uint32_t it = 0;
         while (ld_acquire_u32(bar) < epoch) {
@@ -455,16 +463,6 @@ __device__ __forceinline__ void grid_exit(unsigned *bar) {
             atomicExch(bar + 1, 0u);
         }
     }
-}
-
-// leaving after a barrier that failed: the host learns of it through the
-// mapped flag mirror at its next check, before it reads any result
-__device__ __forceinline__ void fail_exit(unsigned *bar, int *h_flags) {
-    if (threadIdx.x == 0) {
-        h_flags[F_ERR] = 1;
-        __threadfence_system();
-    }
-    grid_exit(bar);
 }
 
 // CTA sums of NV values at once, valid in thread 0; only the first nw warps
@@ -587,13 +585,180 @@ __device__ __forceinline__ R multi_reduce(R (&d)[CW], int lane) {
     return d[0];
 }
 
+// Tagged exchange between the CTAs of k_orth.  A grid barrier costs an atomic
+// per CTA on one address and a poll (1.6 us over 152 CTAs), and the partials
+// are read and summed by everybody only after it (0.6-1.2 us more).  In k_orth
+// the values are all that travels (every CTA works on its own rows), so no
+// fence is needed: every CTA stores its values as 64-bit words (32 bits of
+// value, 32 of epoch); the last CTA polls them, sums and stores the totals as
+// tagged words, which the others poll: barrier and sum in two hops.  A CTA
+// stores epoch e+1 only after it has read the totals of e, and the last CTA its
+// totals of e+1 only after every word of e+1, so one buffer of each is enough.
+// Epochs grow from launch to launch (*xep); a run starts with words and epoch
+// zeroed.  With the column sums shared out (xchg_columns): FP64 solves of 3 958
+// states 3.28 -> 3.12 ms, of 66 600 10.07 -> 9.85 ms.  Where the exchange has
+// to publish other writes too (k_chunk32), its fences make it slower than the
+// barrier: 2.8 us against 2.6 us for barrier and sum, 7 us with seven values;
+// and every CTA polling all words, 152 x 152 readers of the same lines, took
+// 4 us.
+constexpr int XMAX = 192;        // CTAs of a cooperative launch at most
+constexpr int XCOLS = 9;         // words per epoch (double: two a value), the last for the flag
+
+template <class R>
+struct XW { static constexpr int words = sizeof(R) / 4; };
+
+__device__ __forceinline__ void st_word(uint64_t *p, uint32_t v, unsigned ep) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"((uint64_t)v | ((uint64_t)ep << 32)) : "memory");
+}
+template <bool ACQ>
+__device__ __forceinline__ uint64_t ld_word(const uint64_t *p) {
+    uint64_t w;
+    if (ACQ) asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(p) : "memory");
+    else asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(p) : "memory");
+    return w;
+}
+// value q of a set of `n` values, words `stride` apart: word k of the value at p + (q * words + k) * stride
+__device__ __forceinline__ void st_value(uint64_t *p, int64_t, float v, unsigned ep) {
+    st_word(p, __float_as_uint(v), ep);
+}
+__device__ __forceinline__ void st_value(uint64_t *p, int64_t stride, double v, unsigned ep) {
+    st_word(p, (uint32_t)__double2loint(v), ep);
+    st_word(p + stride, (uint32_t)__double2hiint(v), ep);
+}
+// polls until the value carries the epoch; false when the limit ran out
+template <bool ACQ = false>
+__device__ __forceinline__ bool ld_value(const uint64_t *p, int64_t, unsigned ep, float &v, const int *err, uint32_t spin) {
+    uint32_t it = 0;
+    for (;;) {
+        const uint64_t w = ld_word<ACQ>(p);
+        if ((unsigned)(w >> 32) == ep) {
+            v = __uint_as_float((uint32_t)w);
+            return true;
+        }
+        if (++it > spin || ((it & 255u) == 0 && *(volatile const int *)err)) return false;
+    }
+}
+template <bool ACQ = false>
+__device__ __forceinline__ bool ld_value(const uint64_t *p, int64_t stride, unsigned ep, double &v, const int *err,
+                                         uint32_t spin) {
+    uint32_t it = 0;
+    for (;;) {
+        const uint64_t w0 = ld_word<ACQ>(p), w1 = ld_word<ACQ>(p + stride);
+        if ((unsigned)(w0 >> 32) == ep && (unsigned)(w1 >> 32) == ep) {
+            v = __hiloint2double((int)(uint32_t)w1, (int)(uint32_t)w0);
+            return true;
+        }
+        if (++it > spin || ((it & 255u) == 0 && *(volatile const int *)err)) return false;
+    }
+}
+
+// out[q] = sum over the CTAs of v[q] (valid in thread 0), in the order of
+// grid_totals; xs: [NV][G] in shared memory.  FENCE: also a barrier, after
+// which the CTAs see each other's global writes from before it; else only
+// the values travel.  flag (may be null): the last CTA's value (thread 0), on
+// return everybody's.  False when a wait ran out (sets *err).
+template <class R, int NV, bool FENCE>
+__device__ __forceinline__ bool xchg_totals(uint64_t *xtot, unsigned &ep, const R (&v)[NV], int G, R *xs, R *bc,
+                                            R (&out)[NV], int *err, uint32_t spin, int *flag = nullptr) {
+    constexpr int W = XW<R>::words;
+    static_assert(NV * W < XCOLS, "words per CTA");
+    __shared__ int xflag;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int last = G - 1;
+    uint64_t *res = xtot + (size_t)XCOLS * XMAX;     // the totals
+    ++ep;
+    bool good = true;
+    __syncthreads();                                 // xs, bc and xflag of the last exchange are read
+    if ((int)blockIdx.x != last) {
+        if (tid == 0) {
+            if (FENCE) fence_acq_rel();
+#pragma unroll
+            for (int q = 0; q < NV; ++q) st_value(xtot + (size_t)(q * W) * XMAX + blockIdx.x, XMAX, v[q], ep);
+        }
+        if (tid < NV) {
+            R x = (R)0;
+            good = ld_value<FENCE>(res + tid * W, 1, ep, x, err, spin);
+            bc[tid] = x;
+        }
+        if (flag && tid == NV) {
+            float f = 0.f;
+            good = ld_value(res + XCOLS - 1, 0, ep, f, err, spin);
+            xflag = __float_as_int(f);
+        }
+        if (!good) atomicExch(err, 1);
+    } else {
+        if (tid == 0)
+#pragma unroll
+            for (int q = 0; q < NV; ++q) xs[q * G + last] = v[q];
+        if (tid < last) {
+#pragma unroll
+            for (int q = 0; q < NV; ++q) {
+                R x = (R)0;
+                good = good && ld_value<FENCE>(xtot + (size_t)(q * W) * XMAX + tid, XMAX, ep, x, err, spin);
+                xs[q * G + tid] = x;
+            }
+            if (!good) atomicExch(err, 1);
+        }
+        if (!__syncthreads_and(good)) good = false;
+        if (warp < NV && good) {
+            R t = (R)0;
+            for (int b = lane; b < G; b += 32) t += xs[warp * G + b];
+            t = warp_sum<R>(t);
+            if (lane == 0) {
+                bc[warp] = t;
+                if (FENCE) fence_acq_rel();
+                st_value(res + warp * W, 1, t, ep);
+                if (flag && warp == 0) {
+                    st_word(res + XCOLS - 1, (uint32_t)*flag, ep);
+                    xflag = *flag;
+                }
+            }
+        }
+    }
+    if (!__syncthreads_and(good)) return false;
+    if (flag) *flag = xflag;
+#pragma unroll
+    for (int q = 0; q < NV; ++q) out[q] = bc[q];
+    return true;
+}
+
+// hs[l] = sum over the CTAs of column l's partial (l < ncol), which every CTA
+// has stored at xpart (st_value, epoch ep + 1): CTA l mod G sums column l, in
+// the order of grid_columns, and all read the totals after an exchange (summed
+// by every CTA instead, 100 FP64 columns took each SM's FP64 pipe 10 us).
+template <class R>
+__device__ __forceinline__ bool xchg_columns(const uint64_t *xpart, R *xcol, uint64_t *xtot, unsigned &ep, int G, int ncol,
+                                             R *hs, R *xs, R *bc, int *err, uint32_t spin) {
+    constexpr int W = XW<R>::words;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    ++ep;
+    bool good = true;
+    for (int l = blockIdx.x + warp * G; l < ncol; l += ORTH_WARPS * G) {
+        R t = (R)0;
+        for (int b = lane; b < G; b += 32) {
+            R x = (R)0;
+            good = good && ld_value(xpart + (size_t)l * W * XMAX + b, XMAX, ep, x, err, spin);
+            t += x;
+        }
+        t = warp_sum<R>(t);
+        if (lane == 0) xcol[l] = t;
+    }
+    if (!good) atomicExch(err, 1);
+    if (!__syncthreads_and(good)) return false;
+    float none[1] = {0.f}, sum[1];
+    if (!xchg_totals<float, 1, true>(xtot, ep, none, G, (float *)xs, (float *)bc, sum, err, spin)) return false;
+    for (int l = tid; l < ncol; l += ORTH_THREADS) hs[l] = __ldcg(xcol + l);
+    __syncthreads();
+    return true;
+}
+
 // CTA partials of h[l] = V[l] . w (l < m) over rows [i0, i1), plus w.w as
-// column m when `ww`; written to out[l*G] (out = region + blockIdx.x).  Work
+// column m when `ww`; handed to store(l, sum).  Work
 // items are (CW-column group, row quarter); a lane runs down the rows of its
 // item accumulating CW columns in registers, then one multi_reduce.
-template <class T, int CW>
+template <class T, int CW, class Store>
 __device__ __forceinline__ void cta_dots(const T *__restrict__ V, int m, const T *__restrict__ w, int64_t n,
-                                         int64_t i0, int64_t i1, bool ww, T *red, T *out, int G) {
+                                         int64_t i0, int64_t i1, bool ww, T *red, Store store) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int ncol = m + (ww ? 1 : 0);
     const int ng = (ncol + CW - 1) / CW;
@@ -631,7 +796,7 @@ __device__ __forceinline__ void cta_dots(const T *__restrict__ V, int m, const T
     for (int l = threadIdx.x; l < ncol; l += ORTH_THREADS) {
         T s = (T)0;
         for (int q = 0; q < nq; ++q) s += red[q * rs + l];
-        out[(int64_t)l * G] = s;
+        store(l, s);
     }
 }
 
@@ -661,10 +826,14 @@ __host__ __device__ inline int orth_redsz(int pstride, int cw) {
 // v_{j+1}, alpha, beta
 __host__ __device__ inline size_t pro_floats(int pstride) { return 5 * (size_t)((pstride + 3) & ~3); }
 
-// shared memory of k_orth in bytes: hs, red, scratch (T), the recurrence
+// shared memory of the orthogonalisation in bytes: hs, red, scratch (T), the
+// recurrence; k_orth has the exchanged values of a CTA after it
 __host__ __device__ inline size_t orth_smem(int pstride, int cw, size_t tsize) {
     const size_t t = (size_t)(pstride + orth_redsz(pstride, cw) + 8 * ORTH_WARPS + 16) * tsize;
     return ((t + 15) & ~(size_t)15) + pro_floats(pstride) * sizeof(float);
+}
+__host__ __device__ inline size_t orth_smem_x(int pstride, int cw, size_t tsize) {
+    return orth_smem(pstride, cw, tsize) + XCOLS * XMAX * sizeof(float);
 }
 
 // The recurrence's shared arrays
@@ -717,11 +886,7 @@ __device__ __forceinline__ bool pro_always(int m, int64_t n) {
 template <class T, int CW>
 __global__ void __launch_bounds__(ORTH_THREADS, 1) k_orth(OrthArgs a) {
     int *flags = a.flags;
-    unsigned epoch = 0;
-    if (*(volatile int *)&flags[F_STOP]) {           // set before this launch: uniform
-        grid_exit(a.bar);
-        return;
-    }
+    if (*(volatile int *)&flags[F_STOP]) return;     // set before this launch: uniform
     extern __shared__ __align__(16) unsigned char osm_raw[];
     T *osm = (T *)osm_raw;
     const int ps = a.pstride;
@@ -729,6 +894,7 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_orth(OrthArgs a) {
     T *red = hs + ps;
     T *scr = red + orth_redsz(ps, CW);               // [8 x 16] block sums, then [16] broadcasts
     T *bc = scr + 8 * ORTH_WARPS;
+    T *xs = (T *)(osm_raw + orth_smem(ps, CW, sizeof(T)));
     ProSmem pro(osm_raw + (orth_smem(ps, CW, sizeof(T)) - pro_floats(ps) * sizeof(float)), ps);
     const int G = gridDim.x, blk = blockIdx.x, tid = threadIdx.x;
     const int64_t n = a.n;
@@ -739,17 +905,30 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_orth(OrthArgs a) {
     const int j = a.jdev ? *(volatile const int *)a.jdev : a.j, m = j + 1;
     const T *vj = V + (int64_t)j * n;
     const T *vjm = V + (int64_t)(j > 0 ? j - 1 : 0) * n;
-    T *pA = (T *)a.part, *pH = pA + PA_COLS * G, *pB = pH + (int64_t)ps * G, *pH2 = pB + G,
-      *pB2 = pH2 + (int64_t)ps * G, *pW = pB2 + G;
     int *err = flags + F_ERR;
+    unsigned ep = *(volatile unsigned *)a.xep;       // advanced when the launch ends
+    constexpr int W = XW<T>::words;
+    auto column = [&](int l, T t) { st_value(a.xpart + (size_t)l * W * XMAX + blk, XMAX, t, ep + 1); };
+    // leaving: the next launch's epochs follow this one's.  A wait that ran out
+    // is reported through the mapped flag mirror, which the host reads before
+    // any result.
+    auto leave = [&](bool failed) {
+        if (tid != 0) return;
+        if (failed) {
+            a.h_flags[F_ERR] = 1;
+            __threadfence_system();
+        } else if (blk == 0) {
+            *a.xep = ep;
+        }
+    };
     const T *au = (const T *)a.anc_u, *ar = (const T *)a.anc_r, *ay = (const T *)a.defl;
-    const bool anc = au != nullptr;
+    const bool anc = sizeof(T) == 4 && au != nullptr;   // the refinement's bases are FP32
     const int nd = anc ? a.ndefl : 0;
 
     // the host's stop request (host memory: issued first, consumed just
     // before the first barrier so the read overlaps the first phase)
     int host_stop = 0;
-    if (blk == 0 && tid == 0) host_stop = *(volatile const int *)(a.h_flags + F_NFLAGS);
+    if (blk == G - 1 && tid == 0) host_stop = *(volatile const int *)(a.h_flags + F_NFLAGS);
     // alpha = v_j . w; anchored also u.w, r.v_j and y_k.w
     T av[PA_COLS];
 #pragma unroll
@@ -768,33 +947,30 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_orth(OrthArgs a) {
     const T beta_m = j > 0 ? (T)__ldcg(a.beta + j - 1) : (T)0;
     if (!pro_always<T>(m, n)) pro.load(a.pro, ps, a.alpha, a.beta, j);
     int force = __ldcg((const int *)(a.pro + 2 * ps));
-    if (anc) {
-        block_sums<T, PA_COLS>(av, scr, nw);
-        if (tid == 0)
-#pragma unroll
-            for (int q = 0; q < PA_COLS; ++q) pA[q * G + blk] = av[q];
-    } else {
-        T a1[1] = {av[0]};
-        block_sums<T, 1>(a1, scr, nw);
-        if (tid == 0) pA[blk] = a1[0];
-    }
-    if (blk == 0 && tid == 0) flags[F_HOST] = host_stop;
-    if (!grid_sync(a.bar, epoch, err, a.spin)) { fail_exit(a.bar, a.h_flags); return; }
-    if (__ldcg(&flags[F_HOST])) {
-        if (blk == 0 && tid == 0) flags[F_STOP] = 1;
-        grid_exit(a.bar);
-        return;
-    }
+    // no exchange here needs a fence: every CTA works on its own rows, and only
+    // the values and the last CTA's stop request travel
     T tot[PA_COLS];
-    if (anc) {
-        grid_totals<T, PA_COLS>(pA, G, bc, tot);
-        if (blk == 0 && tid == 0) a.h_m[j] = (double)tot[2];
-    } else {
-        T t1[1];
-        grid_totals<T, 1>(pA, G, bc, t1);
+    bool ok;
+    if constexpr (sizeof(T) == 4) {
+        if (anc) {
+            block_sums<T, PA_COLS>(av, scr, nw);
+            ok = xchg_totals<T, PA_COLS, false>(a.xtot, ep, av, G, xs, bc, tot, err, a.spin, &host_stop);
+            if (blk == 0 && tid == 0) a.h_m[j] = (double)tot[2];
+        }
+    }
+    if (!anc) {
+        T a1[1] = {av[0]}, t1[1];
+        block_sums<T, 1>(a1, scr, nw);
+        ok = xchg_totals<T, 1, false>(a.xtot, ep, a1, G, xs, bc, t1, err, a.spin, &host_stop);
 #pragma unroll
         for (int q = 0; q < PA_COLS; ++q) tot[q] = (T)0;
         tot[0] = t1[0];
+    }
+    if (!ok) { leave(true); return; }
+    if (host_stop) {
+        if (blk == 0 && tid == 0) flags[F_STOP] = 1;
+        leave(false);
+        return;
     }
     const T alpha0 = tot[0];
     const bool always = pro_always<T>(m, n);
@@ -824,23 +1000,19 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_orth(OrthArgs a) {
     T bb[1] = {(T)0};
     bool project = always;
     if (!always || anc) {
-        if (anc) {
-            block_sums<T, 1 + ANC_MAX>(ew, scr, nw);
-            if (tid == 0)
-#pragma unroll
-                for (int q = 0; q < 1 + ANC_MAX; ++q) pW[q * G + blk] = ew[q];
-        } else {
+        if constexpr (sizeof(T) == 4) {
+            if (anc) {
+                block_sums<T, 1 + ANC_MAX>(ew, scr, nw);
+                ok = xchg_totals<T, 1 + ANC_MAX, false>(a.xtot, ep, ew, G, xs, bc, ew, err, a.spin);
+                bb[0] = ew[0];
+            }
+        }
+        if (!anc) {
             T s1[1] = {ew[0]};
             block_sums<T, 1>(s1, scr, nw);
-            if (tid == 0) pW[blk] = s1[0];
+            ok = xchg_totals<T, 1, false>(a.xtot, ep, s1, G, xs, bc + 8, bb, err, a.spin);
         }
-        if (!grid_sync(a.bar, epoch, err, a.spin)) { fail_exit(a.bar, a.h_flags); return; }
-        if (anc) {
-            grid_totals<T, 1 + ANC_MAX>(pW, G, bc, ew);
-            bb[0] = ew[0];
-        } else {
-            grid_totals<T, 1>(pW, G, bc + 8, bb);
-        }
+        if (!ok) { leave(true); return; }
     }
     if (!always) {
         // does this step project?  (same decision in every CTA; beta in FP32
@@ -860,30 +1032,19 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_orth(OrthArgs a) {
     T hj = (T)0;
     if (project) {
         __syncthreads();
-        cta_dots<T, CW>(V, m, w, n, i0, i1, true, red, pH + blk, G);
-        if (!grid_sync(a.bar, epoch, err, a.spin)) { fail_exit(a.bar, a.h_flags); return; }
-        grid_columns<T>(pH, G, m + 1, hs);
-        __syncthreads();
-        const T ww = hs[m];
-        hj = hs[j];
-        {
-            T s1[1] = {cta_update<T>(V, m, w, n, i0, i1, hs)};
-            block_sums<T, 1>(s1, scr, nw);
-            if (tid == 0) pB[blk] = s1[0];
-        }
-        if (!grid_sync(a.bar, epoch, err, a.spin)) { fail_exit(a.bar, a.h_flags); return; }
-        grid_totals<T, 1>(pB, G, bc + 9, bb);
-        if (bb[0] < (T)0.5 * ww) {   // second projection (same decision in every CTA)
-            cta_dots<T, CW>(V, m, w, n, i0, i1, false, red, pH2 + blk, G);
-            if (!grid_sync(a.bar, epoch, err, a.spin)) { fail_exit(a.bar, a.h_flags); return; }
-            grid_columns<T>(pH2, G, m, hs);
-            __syncthreads();
+        T ww = (T)0;
+        for (int pass = 0; pass < 2; ++pass) {       // a second time when the first took more than half (same in every CTA)
+            cta_dots<T, CW>(V, m, w, n, i0, i1, pass == 0, red, column);
+            if (!xchg_columns<T>(a.xpart, (T *)a.xcol, a.xtot, ep, G, pass == 0 ? m + 1 : m, hs, xs, bc + 8, err, a.spin)) {
+                leave(true);
+                return;
+            }
+            if (pass == 0) ww = hs[m];
             hj += hs[j];
             T s1[1] = {cta_update<T>(V, m, w, n, i0, i1, hs)};
             block_sums<T, 1>(s1, scr, nw);
-            if (tid == 0) pB2[blk] = s1[0];
-            if (!grid_sync(a.bar, epoch, err, a.spin)) { fail_exit(a.bar, a.h_flags); return; }
-            grid_totals<T, 1>(pB2, G, bc + 10, bb);
+            if (!xchg_totals<T, 1, false>(a.xtot, ep, s1, G, xs, bc + 9 + pass, bb, err, a.spin)) { leave(true); return; }
+            if (!(bb[0] < (T)0.5 * ww)) break;
         }
     }
     const T alpha_j = alpha0 + hj;
@@ -941,7 +1102,7 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_orth(OrthArgs a) {
             __threadfence_system();
         }
     }
-    grid_exit(a.bar);
+    leave(false);
 }
 
 // ---------------------------------------------------------------------------
@@ -1202,7 +1363,7 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_chunk32(ChunkArgs a) {
                 }
                 return ss;
             };
-            cta_dots<float, CW>(V, m, y, n, i0, i1, false, red, pH + blk, G);
+            cta_dots<float, CW>(V, m, y, n, i0, i1, false, red, [&](int l, float t) { pH[(int64_t)l * G + blk] = t; });
             if (!grid_sync(a.o.bar, epoch, err, a.o.spin)) { publish(); return; }
             grid_columns<float>(pH, G, m, hs);
             __syncthreads();
@@ -1218,7 +1379,7 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_chunk32(ChunkArgs a) {
             grid_totals<float, 1>(pB, G, bc + 15, t1);
             bb = t1[0];
             if (bb < 0.5f * ww) {   // second projection (same decision in every CTA)
-                cta_dots<float, CW>(V, m, y, n, i0, i1, false, red, pH2 + blk, G);
+                cta_dots<float, CW>(V, m, y, n, i0, i1, false, red, [&](int l, float t) { pH2[(int64_t)l * G + blk] = t; });
                 if (!grid_sync(a.o.bar, epoch, err, a.o.spin)) { publish(); return; }
                 grid_columns<float>(pH2, G, m, hs);
                 __syncthreads();
@@ -1495,7 +1656,9 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_batch32(BatchArgs B) {
         for (int round = 0; round < 2 && any_p2; ++round) {
             const bool mine = run && p2[me];
             float *ph = round == 0 ? pH : pH2, *pb = round == 0 ? pB : pB2;
-            if (mine) cta_dots<float, CW>(V, m, y, n, i0, i1, false, red, ph + lb, Gs);
+            if (mine)
+                cta_dots<float, CW>(V, m, y, n, i0, i1, false, red,
+                                    [&](int l, float t) { ph[(int64_t)l * Gs + lb] = t; });
             if (!grid_sync(B.bar, epoch, B.err, B.spin)) { done = -1; break; }
             if (mine) {
                 grid_columns<float>(ph, Gs, m, hs);
@@ -1824,6 +1987,11 @@ void normalize_dev(DevLanczos &z, T *x, int64_t n, cudaStream_t st, int64_t &lau
     launches += 1;   // the caller counted one launch for the normalisation
 }
 
+// words of a workspace's exchange area (w: words per value)
+inline size_t x_words(int pstride, int w) {
+    return 1 + (size_t)XCOLS * (XMAX + 1) + (size_t)w * pstride * (1 + XMAX);
+}
+
 // per-eigenvector scratch row of svec
 inline int svec_stride(int cap) { return 4 * (cap + 1); }
 
@@ -1850,7 +2018,7 @@ int ensure_lanczos(Ctx &c, int64_t n, int cap, bool mixed) {
     NSS_CUDA_TRY(c, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     const int pstride = cap + 8;   // m+1 columns plus the anchored refinement's extras
     const int cw = mixed ? OrthCW<float>::value : OrthCW<double>::value;
-    const size_t smem = orth_smem(pstride, cw, mixed ? sizeof(float) : sizeof(double));
+    const size_t smem = orth_smem_x(pstride, cw, mixed ? sizeof(float) : sizeof(double));
     const void *fn = mixed ? (const void *)k_orth<float, OrthCW<float>::value>
                            : (const void *)k_orth<double, OrthCW<double>::value>;
     NSS_CUDA_TRY(c, allow_smem(fn, smem));
@@ -1860,7 +2028,7 @@ int ensure_lanczos(Ctx &c, int64_t n, int cap, bool mixed) {
         c.err = "nss_eigh: Krylov basis too large for the orthogonalisation kernel's shared memory";
         return NSS_ERR_INVALID;
     }
-    z.orth_grid = nsm;      // one CTA per SM, all resident (cooperative launch)
+    z.orth_grid = std::min(nsm, XMAX);      // one CTA per SM, all resident (cooperative launch)
     z.orth_smem = smem;
     z.chunk_ok = false;
     if (mixed) {
@@ -1901,6 +2069,9 @@ int ensure_lanczos(Ctx &c, int64_t n, int cap, bool mixed) {
         z.vcur = vc;
     }
     NSS_CUDA_TRY(c, ctx_alloc(c, &z.jdev, 1));
+    // exchange words: epoch (one word), totals, column partials, column totals
+    z.xwords = x_words(pstride, mixed ? 1 : 2);
+    NSS_CUDA_TRY(c, ctx_alloc(c, &z.xch, z.xwords));
     NSS_CUDA_TRY(c, ctx_alloc(c, &z.pro, (size_t)2 * pstride + PRO_TAIL));
     NSS_CUDA_TRY(c, ctx_alloc(c, &z.evecs, (size_t)4 * n));
     // scalars, projection coefficients, restart scratch alpha/beta, refinement
@@ -1990,6 +2161,8 @@ int run_lanczos(Ctx &c, T *V, T *w, int neigen, int mmax, double tol, uint64_t s
     NSS_CUDA_TRY(c, cudaMemsetAsync(z.flags, 0, F_NFLAGS * sizeof(int), st));
     NSS_CUDA_TRY(c, cudaMemsetAsync(z.beta, 0, (cap + 1) * sizeof(double), st));
     NSS_CUDA_TRY(c, cudaMemsetAsync(z.counter, 0, 4 * sizeof(unsigned), st));
+    // epochs start over: no word of an earlier run may carry one of this run's
+    NSS_CUDA_TRY(c, cudaMemsetAsync(z.xch, 0, z.xwords * sizeof(uint64_t), st));
     const int vb = 608;   // 4 CTAs per SM for elementwise kernels
     uint64_t restarts = 0;
     if (anc) {
@@ -2031,6 +2204,10 @@ int run_lanczos(Ctx &c, T *V, T *w, int neigen, int mmax, double tol, uint64_t s
     oa.spin = wait_limit();
     oa.jdev = nullptr;
     oa.pro = z.pro;
+    oa.xep = (unsigned *)z.xch;
+    oa.xtot = z.xch + 1;
+    oa.xcol = oa.xtot + (size_t)XCOLS * (XMAX + 1);
+    oa.xpart = oa.xcol + (size_t)XW<T>::words * (cap + 8);
     // the launched chunks keep vcur current too, so that a replayed chunk
     // can follow one
     oa.vcur = c.use_graphs ? z.vcur : nullptr;
@@ -2348,7 +2525,7 @@ int run_lanczos(Ctx &c, T *V, T *w, int neigen, int mmax, double tol, uint64_t s
 void lanczos_release(Ctx &c) {
     DevLanczos &z = c.lz;
     void *ptrs[] = {z.V, z.w, z.V32, z.w32, z.anc32, z.wbuf32, z.slot32, z.evecs, z.rrw, z.scal, z.part, z.counter,
-                    z.alpha, z.beta, z.theta, z.resid, z.svec, z.flags, z.pitem, z.vcur, z.jdev, z.pro};
+                    z.alpha, z.beta, z.theta, z.resid, z.svec, z.flags, z.pitem, z.vcur, z.jdev, z.pro, z.xch};
     if (z.gx) cudaGraphExecDestroy(z.gx);
     for (void *p : ptrs) ctx_free(c, p);
     if (z.h_flags) cudaFreeHost(z.h_flags);
