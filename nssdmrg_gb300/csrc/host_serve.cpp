@@ -93,8 +93,15 @@ struct Server {
 
 namespace {
 
+// A worker's context comes and goes under the device lock as well: library
+// handles, streams and allocations then never change beside a launch or a
+// graph capture of another thread.
 void run_request(Server *S, std::shared_ptr<Request> r) {
-    nss_ctx *ctx = nss_create(S->device, 0);
+    nss_ctx *ctx = nullptr;
+    {
+        std::lock_guard<std::mutex> g(S->gpu);
+        ctx = nss_create(S->device, 0);
+    }
     int rc = ctx ? NSS_OK : NSS_ERR_CUDA;
     if (ctx) {
         Ctx &c = ctx_of(ctx);
@@ -115,6 +122,7 @@ void run_request(Server *S, std::shared_ptr<Request> r) {
             nss_dmrg_destroy(d);
         }
         r->peak_bytes = c.peak_used;
+        std::lock_guard<std::mutex> g(S->gpu);
         nss_destroy(ctx);
     }
     std::lock_guard<std::mutex> lk(S->mu);
