@@ -81,6 +81,24 @@ struct DevSb {
     int mma_nplanes = 0, mma_grid = 0;
     bool mma_split = true;
     alignas(64) unsigned char mma_map_a[128] = {}, mma_map_b[128] = {};
+    // FP64 product on the tensor cores (k_sector_split.cu), sections of the
+    // arena: digit pool [rows][64] bf16, scale exponents, FP32 copy of the
+    // vector, the two output planes, work items with their per-CTA ranges,
+    // packing jobs, A x B terms and output tiles (sp_nitems = 0: not used)
+    uint32_t *d_sp_pool = nullptr;
+    int *d_sp_exp = nullptr, *d_sp_tcol = nullptr, *d_sp_dptr = nullptr, *d_sp_dcol = nullptr;
+    float *d_sp_x32 = nullptr, *d_sp_dval = nullptr;
+    int64_t *d_sp_out = nullptr;
+    int *d_sp_out0 = nullptr;
+    double *d_sp_tval = nullptr;
+    struct SplitItem *d_sp_items = nullptr;
+    int2 *d_sp_rng = nullptr;
+    struct SplitJob *d_sp_jobs_w = nullptr, *d_sp_jobs_hl = nullptr, *d_sp_jobs_hr = nullptr;
+    struct SplitTerm *d_sp_terms = nullptr;
+    struct SplitTile *d_sp_tiles = nullptr;
+    size_t sp_pack_smem = 0;
+    int sp_nitems = 0, sp_njobs = 0, sp_ntiles = 0, sp_bn = 64, sp_grid = 0;
+    alignas(64) unsigned char sp_map_a[128] = {}, sp_map_b[128] = {};
 };
 
 // Device-side Lanczos state, kept resident between nss_eigh and nss_rdm.

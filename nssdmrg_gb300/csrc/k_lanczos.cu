@@ -2556,7 +2556,7 @@ int lanczos_eigh(Ctx &c, int neigen, int nitermax, double tol, uint64_t seed, in
     c.chunk_cols = 0.0;
     cudaStream_t st = c.stream;
     // the tensor-core pipeline's error word belongs to this solve
-    if (mixed && s.d_tc_err) NSS_CUDA_TRY(c, cudaMemsetAsync(s.d_tc_err, 0, sizeof(int), st));
+    if (s.d_tc_err) NSS_CUDA_TRY(c, cudaMemsetAsync(s.d_tc_err, 0, sizeof(int), st));
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
@@ -2785,7 +2785,7 @@ int lanczos_eigh(Ctx &c, int neigen, int nitermax, double tol, uint64_t seed, in
     cudaEventDestroy(e1);
     if (rc) return rc;
     if (ce != cudaSuccess) { c.err = cudaGetErrorString(ce); return NSS_ERR_CUDA; }
-    if (mixed && c.sb.d_tc_err) {
+    if ((mixed || c.sb.sp_nitems) && c.sb.d_tc_err) {
         int tc_err = 0;
         NSS_CUDA_TRY(c, cudaMemcpy(&tc_err, c.sb.d_tc_err, sizeof(int), cudaMemcpyDeviceToHost));
         if (tc_err) {

@@ -10,6 +10,7 @@
 #include "hv_tile.cuh"
 #include "host_sparse.hpp"
 #include "sector_mma.cuh"
+#include "sector_split.cuh"
 
 #include <algorithm>
 #include <atomic>
@@ -81,27 +82,29 @@ constexpr int TILE = 16;
 constexpr int TILE32 = 32;
 
 // Sections of the pool's arena: each array at a 256-byte boundary (at least
-// 16 bytes, so that every pointer is distinct and valid).
+// 16 bytes, so that every pointer is distinct and valid), those with a host
+// source first, so that one copy of `host` bytes fills them; the sections that
+// the device fills follow (they are many times larger and not copied).
 struct Stager {
     struct Item {
         void **dst;
         const void *src;
         size_t bytes, off;
     };
-    std::vector<Item> items;
-    size_t total = 0;
+    std::vector<Item> items, dev;
+    size_t host = 0, device = 0;
     template <class T>
     void add(T **dst, const std::vector<T> &v) {
         const size_t bytes = v.size() * sizeof(T);
-        items.push_back({(void **)dst, (const void *)v.data(), bytes, total});
-        total += (std::max<size_t>(bytes, 16) + 255) / 256 * 256;
+        items.push_back({(void **)dst, (const void *)v.data(), bytes, host});
+        host += (std::max<size_t>(bytes, 16) + 255) / 256 * 256;
     }
     // a section the device fills (no host source, not copied)
     template <class T>
     void add_dev(T **dst, size_t count) {
         const size_t bytes = count * sizeof(T);
-        items.push_back({(void **)dst, nullptr, bytes, total});
-        total += (std::max<size_t>(bytes, 16) + 255) / 256 * 256;
+        dev.push_back({(void **)dst, nullptr, bytes, device});
+        device += (std::max<size_t>(bytes, 16) + 255) / 256 * 256;
     }
 };
 
@@ -141,19 +144,20 @@ int stage_commit(Ctx &c, Stager &sg) {
     // the previous upload's copy out of the staging buffer may still be in
     // flight on the stream (two uploads with no solve between them)
     NSS_CUDA_TRY(c, cudaStreamSynchronize(c.stream));
-    if (c.sb_arena_cap < sg.total) {
+    const size_t total = sg.host + sg.device;
+    if (c.sb_arena_cap < total) {
         ctx_free(c, c.sb_arena);
         c.sb_arena = nullptr;
         c.sb_arena_cap = 0;
-        const size_t cap = sg.total + sg.total / 4;   // headroom: the pool size varies from step to step
+        const size_t cap = total + total / 4;   // headroom: the pool size varies from step to step
         NSS_CUDA_TRY(c, ctx_alloc(c, &c.sb_arena, cap));
         c.sb_arena_cap = cap;
     }
-    if (c.sb_stage_cap < sg.total) {
+    if (c.sb_stage_cap < sg.host) {
         if (c.sb_stage) cudaFreeHost(c.sb_stage);
         c.sb_stage = nullptr;
         c.sb_stage_cap = 0;
-        const size_t cap = sg.total + sg.total / 4;
+        const size_t cap = sg.host + sg.host / 4;
         NSS_CUDA_TRY(c, cudaHostAlloc((void **)&c.sb_stage, cap, cudaHostAllocDefault));
         c.sb_stage_cap = cap;
     }
@@ -166,16 +170,17 @@ int stage_commit(Ctx &c, Stager &sg) {
     std::vector<Piece> pieces;
     constexpr size_t PIECE = (size_t)1 << 20;
     for (const auto &it : sg.items)
-        if (it.bytes && it.src)
+        if (it.bytes)
             for (size_t o = 0; o < it.bytes; o += PIECE)
                 pieces.push_back({c.sb_stage + it.off + o, (const char *)it.src + o, std::min(PIECE, it.bytes - o)});
     parallel_for((int)pieces.size(), [&](int i) { std::memcpy(pieces[i].dst, pieces[i].src, pieces[i].bytes); },
-                 sg.total > ((size_t)4 << 20));
-    NSS_CUDA_TRY(c, cudaMemcpyAsync(c.sb_arena, c.sb_stage, sg.total, cudaMemcpyHostToDevice, c.stream));
+                 sg.host > ((size_t)4 << 20));
+    NSS_CUDA_TRY(c, cudaMemcpyAsync(c.sb_arena, c.sb_stage, sg.host, cudaMemcpyHostToDevice, c.stream));
     for (const auto &it : sg.items) {
         *it.dst = (void *)(c.sb_arena + it.off);
-        if (it.src) c.sb.h2d_bytes += (int64_t)it.bytes;
+        c.sb.h2d_bytes += (int64_t)it.bytes;
     }
+    for (const auto &it : sg.dev) *it.dst = (void *)(c.sb_arena + sg.host + it.off);
     return NSS_OK;
 }
 
@@ -534,6 +539,8 @@ int sb_upload(Ctx &c, const nss_sb_desc *d, bool trusted) {
     }
     s.ntiles32 = (int)tiles32.size();
     std::vector<int> tc_err(1, 0);
+    SplitPlan sp;
+    if (split_wanted(s)) split_layout(s, rowptr, col, val, nsm, sp);
 
     Stager sg;
     sg.add_dev(&s.d_hl32, (size_t)hl_tot);
@@ -575,6 +582,24 @@ int sb_upload(Ctx &c, const nss_sb_desc *d, bool trusted) {
     sg.add(&s.d_ab_col, col);
     sg.add(&s.d_ab_val, val);
     sg.add(&s.d_tiles, tiles);
+    sg.add(&s.d_sp_items, sp.items);
+    sg.add(&s.d_sp_rng, sp.rng);
+    sg.add(&s.d_sp_jobs_w, sp.jobs_w);
+    sg.add(&s.d_sp_jobs_hl, sp.jobs_hl);
+    sg.add(&s.d_sp_jobs_hr, sp.jobs_hr);
+    sg.add(&s.d_sp_terms, sp.terms);
+    sg.add(&s.d_sp_tcol, sp.tcol);
+    sg.add(&s.d_sp_tval, sp.tval);
+    sg.add(&s.d_sp_dptr, sp.dptr);
+    sg.add(&s.d_sp_dcol, sp.dcol);
+    sg.add(&s.d_sp_dval, sp.dval);
+    sg.add(&s.d_sp_tiles, sp.tiles);
+    const bool split = !sp.items.empty();
+    sg.add_dev(&s.d_sp_exp, (size_t)sp.nexp);
+    sg.add_dev(&s.d_sp_x32, split ? (size_t)s.n : 0);
+    sg.add_dev(&s.d_sp_out, split ? 2 * (size_t)s.n : 0);
+    sg.add_dev(&s.d_sp_out0, split ? 2 * (size_t)s.n : 0);
+    sg.add_dev(&s.d_sp_pool, (size_t)sp.pool_rows * (SP_KC / 2));
     int rc;
     if ((rc = stage_commit(c, sg))) return rc;
     NSS_CUDA_TRY(c, cudaMemsetAsync(s.d_hl, 0, (size_t)hl_tot * sizeof(double), c.stream));
@@ -590,6 +615,7 @@ int sb_upload(Ctx &c, const nss_sb_desc *d, bool trusted) {
         NSS_CUDA_TRY(c, cudaGetLastError());
     }
     if ((rc = mma_finish(c, plan))) return rc;
+    if ((rc = split_finish(c, sp))) return rc;
     NSS_CUDA_TRY(c, cudaStreamSynchronize(c.stream));
     static std::atomic<uint64_t> g_gen{0};
     s.gen = ++g_gen;
@@ -773,6 +799,7 @@ int hv_device(Ctx &c, const double *d_v, double *d_hv, const int *stop) {
         c.err = "nss_hv: no superblock uploaded";
         return NSS_ERR_STATE;
     }
+    if (s.sp_nitems) return hv_device_split(c, d_v, d_hv, stop);
     k_hv_fp64<<<s.ntiles, 256, 0, c.stream>>>(d_v, d_hv, s.d_tiles, s.d_dls, s.d_drs, s.d_off, s.d_hl,
                                               s.d_hl_off, s.d_hr, s.d_hr_off, s.d_term_ptr, s.d_terms,
                                               s.d_ab_rowptr, s.d_ab_col, s.d_ab_val, stop);

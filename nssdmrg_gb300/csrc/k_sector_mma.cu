@@ -54,8 +54,8 @@
 // the copies it issued, the MMA lane for its MMAs, and the CTA frees its
 // TMEM and returns.
 #include "sector_mma.cuh"
+#include "tc_common.cuh"
 
-#include <cuda.h>
 #include <cudaTypedefs.h>
 
 #include <algorithm>
@@ -77,66 +77,11 @@ __host__ __device__ constexpr uint32_t idesc_tf32(int bn) {
     return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(MM_M >> 4) << 24);
 }
 
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-// shared-memory matrix descriptor: K-major, 128-byte swizzle, 8-row groups
-// 1024 bytes apart (SBO), start address in 16-byte units
-__device__ __forceinline__ uint64_t desc_sw128(uint32_t saddr) {
-    uint64_t d = (uint64_t)((saddr & 0x3FFFF) >> 4);
-    d |= (uint64_t)1 << 16;                 // LBO (unused for swizzled K-major)
-    d |= (uint64_t)(1024 >> 4) << 32;       // SBO
-    d |= (uint64_t)1 << 46;                 // descriptor version
-    d |= (uint64_t)2 << 61;                 // SWIZZLE_128B
-    return d;
-}
-
 __device__ __forceinline__ void mma_tf32(uint32_t tmem, uint64_t ad, uint64_t bd, uint32_t idesc, uint32_t acc) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem),
         "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
-}
-
-__device__ __forceinline__ void mma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-                 : "memory");
-}
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-
-// bounded wait for the phase of the given parity; false when it ran out or
-// when another role has already given up (*abort)
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t spin, volatile int *abort) {
-    for (uint32_t it = 0; it <= spin; ++it) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}\n"
-            : "=r"(ok)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (ok) return true;
-        if ((it & 63u) == 63u && *abort) return false;
-    }
-    return false;
-}
-
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-            dst),
-        "l"((uint64_t)map), "r"(x), "r"(y), "r"(bar)
-        : "memory");
 }
 
 // x rounded to TF32 (10 explicit mantissa bits), to nearest with ties away
@@ -476,6 +421,34 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
     return fn;
 }
 
+}  // namespace
+
+int tc_tensor_map(Ctx &c, unsigned char *out, CUtensorMapDataType type, int esize, void *pool, int cols, int64_t rows,
+                  int box_rows) {
+    auto enc = encode_fn();
+    if (!enc) {
+        c.err = "nss_sb_upload: cuTensorMapEncodeTiled is not available from the driver";
+        return NSS_ERR_CUDA;
+    }
+    const cuuint64_t gdim[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+    const cuuint64_t gstride[1] = {(cuuint64_t)cols * esize};
+    const cuuint32_t estr[2] = {1, 1};
+    const cuuint32_t box[2] = {(cuuint32_t)cols, (cuuint32_t)box_rows};
+    alignas(64) CUtensorMap map;
+    const CUresult cr = enc(&map, type, 2, pool, gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (cr != CUDA_SUCCESS) {
+        c.err = "nss_sb_upload: cuTensorMapEncodeTiled failed (" + std::to_string((int)cr) + ")";
+        return NSS_ERR_CUDA;
+    }
+    static_assert(sizeof(CUtensorMap) == 128, "tensor map storage");
+    std::memcpy(out, &map, sizeof(map));
+    return NSS_OK;
+}
+
+namespace {
+
 template <int BN, int KPS>
 int launch_mma(Ctx &c, const CUtensorMap &ma, const CUtensorMap &mb, uint32_t spin, const int *stop) {
     static std::atomic<bool> done{false};
@@ -600,29 +573,12 @@ int mma_finish(Ctx &c, const MmaPlan &p) {
     s.mma_split = p.split;
     s.mma_nplanes = p.nplanes;
     s.mma_grid = p.grid;
-    // two tensor maps over the pool, [plane rows] x 32 FP32 with 128-byte
-    // rows and the 128-byte swizzle: boxes of 128 rows (A) and of BN rows (B)
-    auto enc = encode_fn();
-    if (!enc) {
-        c.err = "nss_sb_upload: cuTensorMapEncodeTiled is not available from the driver";
-        return NSS_ERR_CUDA;
-    }
-    const cuuint64_t gdim[2] = {(cuuint64_t)MM_KC, (cuuint64_t)p.plane_rows};
-    const cuuint64_t gstride[1] = {(cuuint64_t)MM_KC * sizeof(float)};
-    const cuuint32_t estr[2] = {1, 1};
-    for (int which = 0; which < 2; ++which) {
-        alignas(64) CUtensorMap map;
-        const cuuint32_t box[2] = {(cuuint32_t)MM_KC, (cuuint32_t)(which == 0 ? MM_M : p.bn)};
-        const CUresult cr = enc(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, (void *)s.d_mma_pool, gdim, gstride, box,
-                                estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (cr != CUDA_SUCCESS) {
-            c.err = "nss_sb_upload: cuTensorMapEncodeTiled failed (" + std::to_string((int)cr) + ")";
-            return NSS_ERR_CUDA;
-        }
-        static_assert(sizeof(CUtensorMap) == sizeof(s.mma_map_a), "tensor map storage");
-        std::memcpy(which == 0 ? s.mma_map_a : s.mma_map_b, &map, sizeof(map));
-    }
+    // two tensor maps over the pool, [plane rows] x 32 FP32: boxes of 128 rows
+    // (A) and of BN rows (B)
+    for (int which = 0; which < 2; ++which)
+        if (int rc = tc_tensor_map(c, which == 0 ? s.mma_map_a : s.mma_map_b, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4,
+                                   s.d_mma_pool, MM_KC, p.plane_rows, which == 0 ? MM_M : p.bn))
+            return rc;
     return NSS_OK;
 }
 

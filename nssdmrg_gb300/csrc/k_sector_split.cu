@@ -1,0 +1,788 @@
+// FP64 superblock product on the tensor cores.
+//
+// GB300's FP64 pipe does 1.0-1.2 TFLOP/s, its bf16 tensor cores 1 900.  The
+// dense part of the direct product (src/DMRG_SUPERBLOCK_SETUP.f90:767-796),
+//     D_k = H_L(k) W_k + W_k H_R(k)^T ,   W_k = psi_k as row-major [Dl x Dr],
+// is formed here from exact integer products (the error-free splitting of
+// Ozaki, Ogita, Oishi and Rump, "Error-free transformations of matrix
+// multiplication by using fast routines of matrix multiplication", Numer.
+// Algorithms 59 (2012)):
+//   * Every row of an operand gets a power of two 2^e above its largest element,
+//     and each element becomes the integer nearest x 2^(61-e), written as seven
+//     digits of nine bits, -256 .. 255 (the first below 128), each exact in bf16.
+//   * The products of digits i and j (0 .. 6) with i + j = d <= 6 (28 pairs) are
+//     accumulated in FP32 tensor memory, one accumulator per d.  They are
+//     integers, exact below 2^24: over K = 64 columns (one slab) that holds for
+//     d = 3 and 4, over two slabs for d = 2, over four for d = 0 and 1, whatever
+//     the digits are; d = 5 and 6 (unit 2^-59 of the largest product) are read
+//     every four slabs as one FP32 sum.
+//   * The epilogue warps collect the weighted sums in 96 bits per output; the
+//     last kernel rounds them once to FP64.
+// So a product's error is one rounding plus about 2^-57 of (largest H in the
+// row) (largest W in the column), below that of a chain of FP64 FMAs: measured
+// against products in 64 bits 1.3-4.9e-16 where the chains had 1.7-8.7e-16.
+// The left and right products go to two planes; the last kernel adds them and
+// the A x B terms (:808-857).
+//
+// What bounds it: a slab of a 128 x 64 tile is 40 MMAs (digit i of A against
+// digits 0 .. 6-i of B, which lie one after the other in shared memory and land
+// in the accumulators i .. 6, N <= 256), measured at ~130 cycles each for N
+// from 64 to 256.  Draining the accumulators of every slab took 7 700 cycles
+// (conversions), longer than the MMAs: hence the periods above.  In digit order
+// the accumulator d is complete after digit d, so it is drained while the next
+// digits run.
+//
+// Kernel: persistent, one CTA per SM, 10 warps: one lane issues the TMA copies
+// (seven A digit boxes, released one by one as their MMAs finish; the seven B
+// boxes double buffered), one lane the MMAs, eight warps drain.  Every wait is
+// bounded as in k_sector_mma.cu.
+#include "sector_split.cuh"
+#include "tc_common.cuh"
+
+#include <algorithm>
+#include <atomic>
+#include <cmath>
+#include <cstring>
+
+namespace nss {
+
+namespace {
+
+constexpr int SP_THREADS = 320;            // producer, MMA, 8 epilogue warps
+constexpr int SP_EPI0 = 2, SP_NEPI = 8;
+constexpr int SP_BADEXP = 1 << 20;         // scale exponent of a row with an Inf or NaN
+
+// instruction descriptor, kind::f16: D FP32, A and B bf16, both K-major
+__device__ __forceinline__ constexpr uint32_t idesc_bf16(int n) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(SP_M >> 4) << 24);
+}
+
+__device__ __forceinline__ void mma_bf16(uint32_t tmem, uint64_t ad, uint64_t bd, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem),
+        "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
+}
+
+// x as an integer multiple of 2^(e - 61), rounded to nearest (|x| < 2^e), plus
+// the offset that makes all seven base-512 digits non-negative
+__device__ __forceinline__ uint64_t to_fixed(double x, int e) {
+    const uint64_t b = (uint64_t)__double_as_longlong(x);
+    const int ex = (int)(b >> 52) & 0x7ff;
+    const uint64_t man = (b & 0xfffffffffffffull) | ((uint64_t)(ex ? 1 : 0) << 52);
+    // x = man 2^(max(ex,1) - 1075); shift by max(ex,1) - 1075 + 61 - e <= 8
+    const int sh = (ex ? ex : 1) - 1014 - e;
+    uint64_t m;
+    if (sh >= 0) {
+        m = man << sh;
+    } else {
+        const int r = -sh;
+        m = r > 54 ? 0 : ((man + ((uint64_t)1 << (r - 1))) >> r);
+    }
+    const int64_t v = (b >> 63) ? -(int64_t)m : (int64_t)m;
+    constexpr uint64_t OFFSET = 256ull * (1ull + (1ull << 9) + (1ull << 18) + (1ull << 27) + (1ull << 36) +
+                                          (1ull << 45) + (1ull << 54));
+    return (uint64_t)(v + (int64_t)OFFSET);
+}
+
+// digit q (0: the most significant) as bf16 bits
+__device__ __forceinline__ uint32_t digit_bf16(uint64_t u, int q) {
+    const uint32_t f = q == 0 ? (uint32_t)(u >> 54) : ((uint32_t)(u >> (9 * (SP_D - 1 - q))) & 511u);
+    return __float_as_uint(__uint_as_float(0x4B000000u | f) - 8388864.0f) >> 16;
+}
+
+// (s0 2^42 + r) 2^e rounded to nearest even, in integer arithmetic
+__device__ __forceinline__ double fixed_to_double(int s0, int64_t r, int e) {
+    uint64_t l = ((uint64_t)(int64_t)s0 << 42) + (uint64_t)r;
+    int64_t h = (int64_t)(s0 >> 22) + (r >> 63) + (l < (uint64_t)r ? 1 : 0);
+    const uint64_t sign = (uint64_t)h & 0x8000000000000000ull;
+    if (sign) {
+        l = 0 - l;
+        h = ~h + (l == 0 ? 1 : 0);
+    }
+    if (((uint64_t)h | l) == 0) return 0.0;
+    // normalised: the leading bit at bit 63 of u, the rest below it in l
+    uint64_t u = (uint64_t)h;
+    int lz;
+    if (u) {
+        lz = __clzll((long long)u);                  // at least 36: h has 28 bits
+        u = (u << lz) | (l >> (64 - lz));
+        l <<= lz;
+    } else {
+        const int z = __clzll((long long)l);
+        u = l << z;
+        l = 0;
+        lz = 64 + z;
+    }
+    uint64_t m = u >> 11;
+    const uint32_t low = (uint32_t)u & 0x7ffu;
+    if (low > 0x400u || (low == 0x400u && (l || (m & 1)))) ++m;
+    const int ex = 127 - lz + e + 1023;
+    if (ex <= 0) return __longlong_as_double((long long)sign);          // below the normal range
+    if (ex >= 2047) return __longlong_as_double((long long)(sign | 0x7ff0000000000000ull));
+    return __longlong_as_double((long long)(sign | (((uint64_t)(ex - 1) << 52) + m)));
+}
+
+// high word of |x| -> scale exponent e with |x| < 2^e for the largest such word of a row
+__device__ __forceinline__ int scale_exp(uint32_t hiabs) {
+    const int ex = (int)(hiabs >> 20);
+    if (ex >= 0x7ff) return SP_BADEXP;
+    return (ex ? ex : 1) - 1022;
+}
+
+// FP32 value of x 2^-e by its bits (conversions run at the FP64 pipe's rate),
+// truncated; for products that are far below FP64 rounding
+__device__ __forceinline__ float trunc32(double x, int e) {
+    const uint64_t b = (uint64_t)__double_as_longlong(x);
+    const int ex = ((int)(b >> 52) & 0x7ff) - 896 - e;
+    if (ex <= 0) return 0.f;
+    const uint32_t s = (uint32_t)(b >> 32) & 0x80000000u;
+    return __uint_as_float(s | ((uint32_t)min(ex, 254) << 23) | ((uint32_t)(b >> 29) & 0x7fffffu));
+}
+
+}  // namespace
+
+// Digits of SP_ROWS rows of one operand per CTA, one warp a row.  The strip
+// (rows of a row-major matrix, or its columns: kind 1) is read once into shared
+// memory with all loads in flight; the row's largest high word gives the scale;
+// then chunk by chunk a lane turns two elements into 2 x 7 digits, whole
+// 128-byte rows per store.  Integer arithmetic only: 45 operations an element,
+// and 14 bytes written.  A strip beyond SP_STRIP columns is read twice, chunk by
+// chunk.
+constexpr int SP_STRIP = 768;
+__global__ void __launch_bounds__(32 * SP_ROWS) k_split_pack(const double *__restrict__ x, const SplitJob *__restrict__ jobs,
+                                                             uint32_t *__restrict__ pool, int *__restrict__ exps,
+                                                             float *__restrict__ x32, const int *stop) {
+    if (stop && *stop) return;
+    extern __shared__ double strip[];
+    const SplitJob J = jobs[blockIdx.x];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const double *X = x + J.src;
+    const int r = J.r0 + warp;                       // the warp's row
+    const bool on = r < J.rows;
+    const int nch = (J.k + SP_KC - 1) / SP_KC;
+    const int part = J.k <= SP_STRIP ? J.k : SP_KC;  // columns staged at once
+    const int ld = part | 1;
+    const double *mine = strip + warp * ld;
+    auto load = [&](int k0, int kn) {
+        if (J.kind == 0) {
+            if (on)
+#pragma unroll 8
+                for (int k = lane; k < kn; k += 32) strip[warp * ld + k] = X[(int64_t)r * J.ld + k0 + k];
+        } else {
+            const int c = threadIdx.x % SP_ROWS;
+            const bool in = J.r0 + c < J.rows;
+#pragma unroll 8
+            for (int k = threadIdx.x / SP_ROWS; k < kn; k += 32)
+                strip[c * ld + k] = in ? X[(int64_t)(k0 + k) * J.ld + J.r0 + c] : 0.0;
+        }
+    };
+    uint32_t m = 0;
+    for (int k0 = 0; k0 < J.k; k0 += part) {
+        const int kn = min(part, J.k - k0);
+        if (k0) __syncthreads();
+        load(k0, kn);
+        __syncthreads();
+        if (on)
+            for (int k = lane; k < kn; k += 32) m = max(m, (uint32_t)__double2hiint(mine[k]) & 0x7fffffffu);
+    }
+    m = __reduce_max_sync(0xffffffffu, m);
+    const int e = scale_exp(m);
+    if (on && lane == 0) exps[J.exp + r] = e;
+    for (int c = 0; c < nch; ++c) {
+        int k0 = c * SP_KC, kn = min(SP_KC, J.k - k0), at = k0;
+        if (J.k > SP_STRIP) {
+            __syncthreads();
+            load(k0, kn);
+            __syncthreads();
+            at = 0;
+        }
+        if (!on) continue;
+        const double a = 2 * lane < kn ? mine[at + 2 * lane] : 0.0, b = 2 * lane + 1 < kn ? mine[at + 2 * lane + 1] : 0.0;
+        uint64_t ua = 0, ub = 0;
+        if (e < SP_BADEXP) {
+            ua = to_fixed(a, e);
+            ub = to_fixed(b, e);
+        }
+        if (x32 && J.kind == 0) {
+            float *o = x32 + J.src + (int64_t)r * J.ld + k0 + 2 * lane;
+            if (2 * lane < kn) o[0] = e < SP_BADEXP ? trunc32(a, e) : 0.f;
+            if (2 * lane + 1 < kn) o[1] = e < SP_BADEXP ? trunc32(b, e) : 0.f;
+        }
+#pragma unroll
+        for (int q = 0; q < SP_D; ++q)
+            pool[((int64_t)J.row + (int64_t)(c * SP_D + q) * J.rows + r) * (SP_KC / 2) + lane] =
+                e < SP_BADEXP ? (digit_bf16(ua, q) | (digit_bf16(ub, q) << 16)) : 0u;
+    }
+}
+
+namespace {
+
+template <int BN>
+struct SplitCfg {
+    static constexpr int A_BYTES = SP_M * 128, B_BYTES = BN * 128;      // one digit box
+    static constexpr int SMEM = SP_D * A_BYTES + 2 * SP_D * B_BYTES + 1024;
+    static constexpr int HALF = BN / 2;
+    static constexpr uint32_t TCOLS = BN == 64 ? 512 : 256;
+    static_assert(SMEM <= 232448 - 256, "shared memory plan");
+};
+
+__device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(addr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+}  // namespace
+
+template <int BN>
+__global__ void __launch_bounds__(SP_THREADS, 1) k_sector_split(const __grid_constant__ CUtensorMap map_a,
+                                                                 const __grid_constant__ CUtensorMap map_b,
+                                                                 const SplitItem *__restrict__ items,
+                                                                 const int2 *__restrict__ ranges,
+                                                                 int64_t *__restrict__ out, int *__restrict__ out0,
+                                                                 int64_t plane, uint32_t spin, int *err, const int *stop) {
+    using C = SplitCfg<BN>;
+    if (stop && *stop) return;   // before any TMEM allocation: uniform exit
+    extern __shared__ uint8_t sp_raw[];
+    uint8_t *smem = (uint8_t *)(((uintptr_t)sp_raw + 1023) & ~(uintptr_t)1023);
+    uint8_t *sa = smem, *sbuf = smem + SP_D * C::A_BYTES;
+    __shared__ __align__(8) uint64_t fulla[SP_D], emptya[SP_D], fullb[2], emptyb[2], tfull[SP_D], tempty, drain;
+    __shared__ uint32_t tmem_base;
+    __shared__ int abort_s;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int2 rg = ranges[blockIdx.x];
+    if (threadIdx.x == 0) {
+        for (int q = 0; q < SP_D; ++q) {
+            mbar_init(smem_u32(&fulla[q]), 1);
+            mbar_init(smem_u32(&emptya[q]), 1);
+            mbar_init(smem_u32(&tfull[q]), 1);
+        }
+        for (int q = 0; q < 2; ++q) {
+            mbar_init(smem_u32(&fullb[q]), 1);
+            mbar_init(smem_u32(&emptyb[q]), 1);
+        }
+        mbar_init(smem_u32(&tempty), SP_NEPI);
+        mbar_init(smem_u32(&drain), 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)&map_a) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)&map_b) : "memory");
+        abort_s = 0;
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
+                     "r"(C::TCOLS));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tmem_base;
+    volatile int *abort = &abort_s;
+    const uint32_t drain_spin = spin > (1u << 22) ? spin : (1u << 22);
+    auto give_up = [&]() {
+        *abort = 1;
+        atomicExch(err, 1);
+    };
+    auto slabs = [](int k) { return (k + SP_KC - 1) / SP_KC; };
+    // slab c of nk: is accumulator d read after it? (see the periods above)
+    auto due = [](int d, int c, int nk) {
+        return c == nk - 1 || d == 3 || d == 4 || (d == 2 ? (c & 1) == 1 : (c & 3) == 3);
+    };
+
+    if (warp == 0 && lane == 0) {
+        // ---- TMA producer
+        int it = 0;                   // slabs issued
+        int na = 0, nb = 0;           // A boxes and B buffers issued
+        bool ok = true;
+        for (int i = rg.x; i < rg.y && ok && !*abort; ++i) {
+            const SplitItem m = items[i];
+            const int nk = slabs(m.k);
+            for (int c = 0; c < nk && ok; ++c, ++it) {
+                const int bs = it & 1;
+                if (!mbar_wait(smem_u32(&emptyb[bs]), ((uint32_t)(it >> 1) & 1u) ^ 1u, spin, abort)) { give_up(); ok = false; break; }
+                const uint32_t fb = smem_u32(&fullb[bs]);
+                mbar_expect_tx(fb, (uint32_t)(SP_D * C::B_BYTES));
+                for (int q = 0; q < SP_D; ++q)
+                    tma_load_2d(smem_u32(sbuf + (size_t)(bs * SP_D + q) * C::B_BYTES), &map_b, 0,
+                                m.b_row + (c * SP_D + q) * m.b_rows + m.n0, fb);
+                ++nb;
+                for (int q = 0; q < SP_D; ++q) {
+                    if (!mbar_wait(smem_u32(&emptya[q]), ((uint32_t)it & 1u) ^ 1u, spin, abort)) { give_up(); ok = false; break; }
+                    const uint32_t fa = smem_u32(&fulla[q]);
+                    mbar_expect_tx(fa, (uint32_t)C::A_BYTES);
+                    tma_load_2d(smem_u32(sa + (size_t)q * C::A_BYTES), &map_a, 0, m.a_row + (c * SP_D + q) * m.a_rows + m.m0, fa);
+                    ++na;
+                }
+            }
+        }
+        // no copy of this CTA may still be landing when it leaves (bounded, by a
+        // limit of its own, and not cut short by the abort flag)
+        volatile int never = 0;
+        for (int q = 0; q < SP_D; ++q) {
+            const int fills = na / SP_D + (q < na % SP_D ? 1 : 0);
+            if (fills && !mbar_wait(smem_u32(&fulla[q]), (uint32_t)(fills - 1) & 1u, drain_spin, &never)) atomicExch(err, 1);
+        }
+        for (int q = 0; q < 2; ++q) {
+            const int fills = (nb + 1 - q) / 2;
+            if (fills && !mbar_wait(smem_u32(&fullb[q]), (uint32_t)(fills - 1) & 1u, drain_spin, &never)) atomicExch(err, 1);
+        }
+    } else if (warp == 1 && lane == 0) {
+        // ---- MMA issuer
+        int it = 0;
+        bool issued = false, ok = true;
+        for (int i = rg.x; i < rg.y && ok && !*abort; ++i) {
+            const int k = items[i].k, nk = slabs(k);
+            for (int c = 0; c < nk && ok; ++c, ++it) {
+                const int bs = it & 1;
+                const int ks = min(SP_KC / 16, (k - c * SP_KC + 15) / 16);   // K steps with anything in them
+                if (!mbar_wait(smem_u32(&tempty), ((uint32_t)it & 1u) ^ 1u, spin, abort) ||
+                    !mbar_wait(smem_u32(&fullb[bs]), (uint32_t)(it >> 1) & 1u, spin, abort)) {
+                    give_up();
+                    ok = false;
+                    break;
+                }
+                const uint32_t b0 = smem_u32(sbuf + (size_t)bs * SP_D * C::B_BYTES);
+#pragma unroll
+                for (int q = 0; q < SP_D; ++q) {
+                    if (!mbar_wait(smem_u32(&fulla[q]), (uint32_t)it & 1u, spin, abort)) {
+                        give_up();
+                        ok = false;
+                        break;
+                    }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t a0 = smem_u32(sa + (size_t)q * C::A_BYTES);
+                    // digit q of A against digits 0 .. 6-q of B: accumulators
+                    // q .. 6, n0 columns on from there
+                    auto mma = [&](int kk, int n0, int n, uint32_t acc) {
+                        mma_bf16(tmem + (uint32_t)(q * BN + n0), desc_sw128(a0 + kk * 32),
+                                 desc_sw128(b0 + (uint32_t)n0 * 128 + kk * 32), idesc_bf16(n), acc);
+                    };
+                    const int n = (SP_D - q) * BN;
+                    for (int kk = 0; kk < ks; ++kk) {
+                        if (q == 0 && kk == 0 && (c & 3) != 0) {
+                            // accumulators that go on (d = 0, 1, 5, 6, and 2 in odd
+                            // slabs) beside those that start over
+                            const int d0 = (c & 1) ? 3 : 2;
+                            mma(0, 0, d0 * BN, 1u);
+                            mma(0, d0 * BN, (5 - d0) * BN, 0u);
+                            mma(0, 5 * BN, 2 * BN, 1u);
+                            continue;
+                        }
+                        const uint32_t acc = (q > 0 || kk > 0) ? 1u : 0u;
+#pragma unroll
+                        for (int n0 = 0; n0 < n; n0 += 256) mma(kk, n0, min(256, n - n0), acc);
+                    }
+                    issued = true;
+                    mma_commit(smem_u32(&emptya[q]));   // this A box may be refilled
+                    if (due(q, c, nk)) mma_commit(smem_u32(&tfull[q]));   // ... and accumulator q is complete
+                }
+                if (ok) mma_commit(smem_u32(&emptyb[bs]));
+            }
+        }
+        if (issued) {   // every MMA of this lane done before the CTA frees its TMEM
+            mma_commit(smem_u32(&drain));
+            volatile int never = 0;
+            if (!mbar_wait(smem_u32(&drain), 0u, drain_spin, &never)) atomicExch(err, 1);
+        }
+    } else if (warp >= SP_EPI0) {
+        // ---- epilogue: warp w owns TMEM lanes 32 (w % 4) .. +31 (its rows) and
+        // half of the columns
+        const int qr = warp & 3, h = (warp - SP_EPI0) >> 2;
+        const uint32_t tq = tmem + ((uint32_t)(32 * qr) << 16) + (uint32_t)(h * C::HALF);
+        uint32_t par[SP_D];           // parities of the next completion of each accumulator
+#pragma unroll
+        for (int d = 0; d < SP_D; ++d) par[d] = 0u;
+        for (int i = rg.x; i < rg.y && !*abort; ++i) {
+            const SplitItem m = items[i];
+            const int nk = slabs(m.k);
+            // the output is (s0 2^42 + sum) 2^-6 units of d = 4
+            int s0[C::HALF];
+            int64_t sum[C::HALF];
+#pragma unroll
+            for (int j = 0; j < C::HALF; ++j) sum[j] = s0[j] = 0;
+            bool ok = true;
+            for (int c = 0; c < nk && ok; ++c) {
+                auto ready = [&](int d) -> bool {
+                    bool got = true;
+                    if (lane == 0) got = mbar_wait(smem_u32(&tfull[d]), par[d], spin, abort);
+                    par[d] ^= 1u;
+                    if (__shfl_sync(0xffffffffu, got ? 1 : 0, 0) == 0) {
+                        if (lane == 0) give_up();
+                        return false;
+                    }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    return true;
+                };
+#pragma unroll
+                for (int d = 0; d < 5; ++d) {
+                    if (!ok || !due(d, c, nk)) continue;
+                    if (!(ok = ready(d))) continue;
+#pragma unroll
+                    for (int c0 = 0; c0 < C::HALF; c0 += 16) {
+                        uint32_t r[16];
+                        tmem_ld16(tq + (uint32_t)(d * BN + c0), r);
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) {
+                            const int x = __float2int_rn(__uint_as_float(r[j]));
+                            if (d == 0) s0[c0 + j] += x;
+                            else sum[c0 + j] += (int64_t)x * (int64_t)(1ll << (42 - 9 * d));
+                        }
+                    }
+                }
+                if (ok && due(5, c, nk)) {
+                    ok = ready(5) && ready(6);
+                    if (ok)
+#pragma unroll
+                        for (int c0 = 0; c0 < C::HALF; c0 += 16) {
+                            uint32_t r5[16], r6[16];
+                            tmem_ld16(tq + (uint32_t)(5 * BN + c0), r5);
+                            tmem_ld16(tq + (uint32_t)(6 * BN + c0), r6);
+#pragma unroll
+                            for (int j = 0; j < 16; ++j)
+                                sum[c0 + j] += __float2int_rn(fmaf(__uint_as_float(r6[j]), 0x1p-12f, __uint_as_float(r5[j]) * 0x1p-3f));
+                        }
+                }
+                if (!ok) break;
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&tempty));
+            }
+            if (!ok) break;
+            const int il = m.m0 + 32 * qr + lane, ir0 = m.n0 + h * C::HALF;
+            if (il < m.dl) {
+                // the planes are column-major: a warp's 32 rows of a column are
+                // one run (row-major, a lane writing its own row, took 16 000
+                // cycles an item)
+                const int64_t o = (int64_t)m.plane * plane + m.off + (int64_t)ir0 * m.dl + il;
+#pragma unroll
+                for (int j = 0; j < C::HALF; ++j)
+                    if (ir0 + j < m.dr) {
+                        out[o + (int64_t)j * m.dl] = sum[j];
+                        out0[o + (int64_t)j * m.dl] = s0[j];
+                    }
+            }
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(C::TCOLS));
+}
+
+// hv = plane 0 + plane 1 (rounded to FP64) + sum_t A W_q B^T, one CTA per 8 x
+// 32 outputs of a sector, a warp a row.  Per term A's row and B's columns give
+// their dominant (column, value).  The entries of A's row beside it (below 2^-40
+// of A's largest: rounding left by the renormalisation, up to a block sector's
+// width of them) are summed in FP32 against the FP32 copy of W, which is scaled
+// by its rows' powers of two: an error of 2^-61 of the term.  A lane holds one
+// such entry, its gather is broadcast, eight gathers in flight.  Two FP64
+// operations a term and output, spread over all SMs (in the GEMM's epilogue
+// they would hold one SM's FP64 pipe for 8 us a tile); the chain of dependent
+// loads bounds it, hence the tile and term records.
+struct SplitTerms {
+    const SplitTerm *terms;
+    const int *tcol, *dptr, *dcol, *exps;
+    const double *tval;
+    const float *dval;
+    const DevTerm *csr;
+    const int *ab_rp, *ab_col;
+    const double *ab_val;
+};
+
+__global__ void __launch_bounds__(256, 4) k_split_terms(const double *__restrict__ v, const float *__restrict__ v32,
+                                                     const int64_t *__restrict__ planes,
+                                                     const int *__restrict__ planes0, int64_t n, double *__restrict__ hv,
+                                                     const SplitTile *__restrict__ tiles, SplitTerms T, const int *stop) {
+    if (stop && *stop) return;
+    __shared__ double dense[8][33];
+    const SplitTile t = tiles[blockIdx.x];
+    {   // the two planes (column-major), eight rows of four columns a warp
+        const int r = threadIdx.x & 7, c = threadIdx.x >> 3, il = t.row0 + r, ir = t.col0 + c;
+        double x = 0.0;
+        if (il < t.dl && ir < t.dr) {
+            const int64_t e = t.off + (int64_t)ir * t.dl + il;
+            const int64_t p0 = planes[e], p1 = planes[n + e];
+            const int q0 = planes0[e], q1 = planes0[n + e];
+            // scale exponents: H_L row, W column; W row, H_R row
+            const int x0 = T.exps[t.exp + il], x1 = T.exps[t.exp + 2 * t.dl + t.dr + ir];
+            const int y0 = T.exps[t.exp + t.dl + t.dr + il], y1 = T.exps[t.exp + t.dl + ir];
+            x = (x0 >= SP_BADEXP || x1 >= SP_BADEXP || y0 >= SP_BADEXP || y1 >= SP_BADEXP)
+                    ? __longlong_as_double(0x7ff8000000000000ll)
+                    : fixed_to_double(q0, p0, x0 + x1 - 56) + fixed_to_double(q1, p1, y0 + y1 - 56);
+        }
+        dense[r][c] = x;
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const int il = t.row0 + (threadIdx.x >> 5), ir = t.col0 + lane;
+    if (il >= t.dl) return;                          // whole warps
+    const bool in = ir < t.dr;
+    const int64_t e0 = t.off + (int64_t)il * t.dr + ir;
+    double acc = 0.0;
+    bool dusty = false;
+    // the dominant entries, four terms' loads in flight
+    for (int tb = t.t0; tb < t.t1; tb += 4) {
+        SplitTerm tm[4];
+        int aj[4], bj[4];
+        double c[4], w[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) tm[q] = T.terms[min(tb + q, t.t1 - 1)];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const bool on = tb + q < t.t1 && !tm[q].general;
+            dusty = dusty || tm[q].general || tm[q].dust >= 0;
+            aj[q] = on ? T.tcol[tm[q].a + il] : -1;
+            bj[q] = on && in ? T.tcol[tm[q].b + ir] : -1;
+            c[q] = (on ? T.tval[tm[q].a + il] : 0.0) * (on && in ? T.tval[tm[q].b + ir] : 0.0);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            w[q] = aj[q] >= 0 && bj[q] >= 0 ? v[tm[q].off + (int64_t)aj[q] * tm[q].drq + bj[q]] : 0.0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (aj[q] >= 0 && bj[q] >= 0) acc = fma(c[q], w[q], acc);
+    }
+    if (dusty)
+        for (int ti = t.t0; ti < t.t1; ++ti) {
+            const SplitTerm tm = T.terms[ti];
+            if (tm.general) {                        // several sizeable entries in a row: the CSR loop
+                if (!in) continue;
+                const DevTerm c = T.csr[tm.term];
+                const double *W = v + tm.off;
+                for (int ja = T.ab_rp[c.a_rp + il]; ja < T.ab_rp[c.a_rp + il + 1]; ++ja) {
+                    const int64_t row = (int64_t)T.ab_col[ja] * tm.drq;
+                    double cb = 0.0;
+                    for (int jb = T.ab_rp[c.b_rp + ir]; jb < T.ab_rp[c.b_rp + ir + 1]; ++jb)
+                        cb = fma(T.ab_val[jb], W[row + T.ab_col[jb]], cb);
+                    acc = fma(T.ab_val[ja], cb, acc);
+                }
+                continue;
+            }
+            if (tm.dust < 0) continue;
+            const int p0 = T.dptr[tm.dust + il], p1 = T.dptr[tm.dust + il + 1];   // uniform over the warp
+            const int bj = in ? T.tcol[tm.b + ir] : -1;
+            const float *W32 = v32 + tm.off + max(bj, 0);
+            for (int p = p0; p < p1; p += 32) {
+                const int cnt = min(32, p1 - p);
+                const int dc = lane < cnt ? T.dcol[p + lane] : 0;
+                const int ex = lane < cnt ? T.exps[tm.ew + dc] : -(1 << 20);
+                // powers of two of the input rows relative to the largest of them
+                const int top = __reduce_max_sync(0xffffffffu, ex);
+                float dv = 0.f;
+                if (lane < cnt && ex - top > -120) dv = T.dval[p + lane] * __int_as_float((127 + ex - top) << 23);
+                const int at = dc * tm.drq;
+                float s = 0.f;
+                for (int u = 0; u < cnt; u += 8) {
+                    float g[8];
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) g[q] = W32[__shfl_sync(0xffffffffu, at, u + q)];
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) s = fmaf(__shfl_sync(0xffffffffu, dv, u + q), g[q], s);
+                }
+                if (bj >= 0 && s != 0.f) {
+                    // s 2^top as a double by its bits (s is normal or negligible)
+                    const uint32_t b = __float_as_uint(s);
+                    const int e = (int)((b >> 23) & 0xff) - 127 + top + 1023;
+                    if (e > 0 && e < 2047 && ((b >> 23) & 0xff))
+                        acc = fma(__hiloint2double((int)((b & 0x80000000u) | ((uint32_t)e << 20) | ((b & 0x7fffffu) >> 3)),
+                                                   (int)(b << 29)),
+                                  T.tval[tm.b + ir], acc);
+                }
+            }
+        }
+    if (in) hv[e0] = dense[threadIdx.x >> 5][lane] + acc;
+}
+
+// ---------------------------------------------------------------------------
+// Host side
+
+bool split_wanted(const DevSb &s) {
+    const char *e = std::getenv("NSS_SPLIT64");
+    if (e && std::atoi(e) == 0) return false;
+    if (e) return true;
+    for (int k = 0; k < s.nsb; ++k)
+        if (s.dls[k] > SP_KMAX || s.drs[k] > SP_KMAX) return false;
+    return s.flops_dense >= 4e7;
+}
+
+void split_layout(const DevSb &s, const std::vector<int> &rowptr, const std::vector<int> &col,
+                  const std::vector<double> &val, int nsm, SplitPlan &p) {
+    p = SplitPlan{};
+    auto slabs = [](int d) { return (d + SP_KC - 1) / SP_KC; };
+    // pool rows and scale exponents of the four operands of every sector
+    int64_t row = 0;
+    struct Rows {
+        int hl, hr, w, wt, ehl, ehr, ew, ewt;
+    };
+    std::vector<Rows> rs(s.nsb);
+    auto jobs = [](std::vector<SplitJob> &v, int64_t src, int ld, int rows, int k, int kind, int row0, int exp0) {
+        for (int r = 0; r < rows; r += SP_ROWS) v.push_back(SplitJob{src, ld, rows, k, r, kind, row0, exp0, 0});
+    };
+    int64_t tiles32 = 0;
+    for (int k = 0; k < s.nsb; ++k) {
+        const int dl = s.dls[k], dr = s.drs[k];
+        Rows &R = rs[k];
+        auto take = [&](int rows, int kk) {
+            const int r0 = (int)row;
+            row += (int64_t)SP_D * slabs(kk) * rows;
+            return r0;
+        };
+        R.hl = take(dl, dl);
+        R.hr = take(dr, dr);
+        R.w = take(dl, dr);
+        R.wt = take(dr, dl);
+        R.ehl = p.nexp;
+        R.ehr = R.ehl + dl;
+        R.ew = R.ehr + dr;
+        R.ewt = R.ew + dl;
+        p.nexp = R.ewt + dr;
+        jobs(p.jobs_hl, s.hl_off[k], dl, dl, dl, 0, R.hl, R.ehl);
+        jobs(p.jobs_hr, s.hr_off[k], dr, dr, dr, 0, R.hr, R.ehr);
+        jobs(p.jobs_w, s.off[k], dr, dl, dr, 0, R.w, R.ew);
+        jobs(p.jobs_w, s.off[k], dr, dr, dl, 1, R.wt, R.ewt);
+        tiles32 += 2 * (int64_t)((dl + SP_M - 1) / SP_M) * ((dr + 31) / 32);
+        for (int a = 0; a < dl; a += 8)
+            for (int b = 0; b < dr; b += 32)
+                p.tiles.push_back(SplitTile{a, b, dl, dr, s.term_ptr[k], s.term_ptr[k + 1], R.ehl, 0, s.off[k]});
+        p.kmax = std::max({p.kmax, dl, dr});
+    }
+    row += SP_M;   // a box that starts near the end of the pool stays inside it
+    p.pool_rows = row;
+    // the longest packing jobs first
+    std::stable_sort(p.jobs_w.begin(), p.jobs_w.end(), [](const SplitJob &a, const SplitJob &b) { return a.k > b.k; });
+    // a slab of 32 columns takes nearly as long as one of 64 (7 MMAs a K step
+    // against 10, 4 500 against 5 200 cycles): the narrow tile only where the
+    // narrow items still go one to a CTA and its shorter epilogue shows
+    p.bn = tiles32 <= nsm ? 32 : 64;
+    for (int k = 0; k < s.nsb; ++k) {
+        const int dl = s.dls[k], dr = s.drs[k];
+        const Rows &R = rs[k];
+        for (int m0 = 0; m0 < dl; m0 += SP_M)
+            for (int n0 = 0; n0 < dr; n0 += p.bn) {
+                p.items.push_back(SplitItem{R.hl, R.wt, dl, dr, dl, dl, dr, m0, n0, 0, s.off[k]});
+                p.items.push_back(SplitItem{R.w, R.hr, dl, dr, dr, dl, dr, m0, n0, 1, s.off[k]});
+            }
+    }
+    // longest first onto the least loaded CTA (an item costs its slabs plus
+    // about one of epilogue)
+    std::stable_sort(p.items.begin(), p.items.end(),
+                     [&](const SplitItem &a, const SplitItem &b) { return slabs(a.k) > slabs(b.k); });
+    const int G = (int)std::min<size_t>(p.items.size(), (size_t)std::max(1, nsm));
+    std::vector<int64_t> load(G, 0);
+    std::vector<std::vector<int>> own(G);
+    for (size_t e = 0; e < p.items.size(); ++e) {
+        const int b = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+        load[b] += slabs(p.items[e].k) + 1;
+        own[b].push_back((int)e);
+    }
+    p.grid = G;
+    std::vector<SplitItem> ordered;
+    ordered.reserve(p.items.size());
+    for (int g = 0; g < G; ++g) {
+        const int start = (int)ordered.size();
+        for (int e : own[g]) ordered.push_back(p.items[e]);
+        p.rng.push_back(make_int2(start, (int)ordered.size()));
+    }
+    p.items.swap(ordered);
+    // A x B terms: the dominant entry of every row, and the small rest of A's
+    constexpr double SMALL = 0x1p-40;
+    for (size_t ti = 0; ti < s.terms.size(); ++ti) {
+        const DevTerm &tm = s.terms[ti];
+        SplitTerm t{0, 0, 0, -1, (int)ti, s.drs[tm.in_sec], rs[tm.in_sec].ew, 0, s.off[tm.in_sec]};
+        for (int side = 0; side < 2; ++side) {
+            const int64_t rp = side == 0 ? tm.a_rp : tm.b_rp;
+            const int nrow = side == 0 ? tm.a_nrow : tm.b_nrow;
+            double mx = 0.0;
+            bool multi = false;
+            for (int i = 0; i < nrow; ++i) multi = multi || rowptr[rp + i + 1] - rowptr[rp + i] > 1;
+            if (multi)
+                for (int j = rowptr[rp]; j < rowptr[rp + nrow]; ++j) mx = std::max(mx, std::fabs(val[j]));
+            (side == 0 ? t.a : t.b) = (int)p.tcol.size();
+            const bool dusty = multi && side == 0;
+            if (multi && side == 1) t.general = 1;
+            if (dusty) {
+                t.dust = (int)p.dptr.size();
+                p.dptr.push_back((int)p.dcol.size());
+            }
+            for (int i = 0; i < nrow; ++i) {
+                const int p0 = rowptr[rp + i], p1 = rowptr[rp + i + 1];
+                int top = -1;
+                for (int j = p0; j < p1; ++j)
+                    if (top < 0 || std::fabs(val[j]) > std::fabs(val[top])) top = j;
+                p.tcol.push_back(top < 0 ? -1 : col[top]);
+                p.tval.push_back(top < 0 ? 0.0 : val[top]);
+                if (!dusty) continue;
+                for (int j = p0; j < p1; ++j) {
+                    if (j == top || val[j] == 0.0) continue;
+                    if (std::fabs(val[j]) > SMALL * mx || mx > 0x1p60 || mx < 0x1p-60) t.general = 1;
+                    p.dcol.push_back(col[j]);
+                    p.dval.push_back((float)val[j]);
+                }
+                p.dptr.push_back((int)p.dcol.size());
+            }
+        }
+        p.terms.push_back(t);
+    }
+}
+
+int split_finish(Ctx &c, const SplitPlan &p) {
+    DevSb &s = c.sb;
+    if (p.items.empty()) return NSS_OK;
+    const int part = p.kmax <= SP_STRIP ? p.kmax : SP_STRIP;   // widest strip of a job
+    const size_t smem = (size_t)SP_ROWS * (part | 1) * sizeof(double);
+    s.sp_pack_smem = smem;
+    NSS_CUDA_TRY(c, cudaFuncSetAttribute(k_split_pack, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)(SP_ROWS * (SP_STRIP | 1) * sizeof(double))));
+    c.launches += 2;
+    k_split_pack<<<(unsigned)p.jobs_hl.size(), 32 * SP_ROWS, smem, c.stream>>>(s.d_hl, s.d_sp_jobs_hl, s.d_sp_pool, s.d_sp_exp,
+                                                                            nullptr, nullptr);
+    k_split_pack<<<(unsigned)p.jobs_hr.size(), 32 * SP_ROWS, smem, c.stream>>>(s.d_hr, s.d_sp_jobs_hr, s.d_sp_pool, s.d_sp_exp,
+                                                                            nullptr, nullptr);
+    NSS_CUDA_TRY(c, cudaGetLastError());
+    s.sp_nitems = (int)p.items.size();
+    s.sp_njobs = (int)p.jobs_w.size();
+    s.sp_ntiles = (int)p.tiles.size();
+    s.sp_bn = p.bn;
+    s.sp_grid = p.grid;
+    for (int which = 0; which < 2; ++which)
+        if (int rc = tc_tensor_map(c, which == 0 ? s.sp_map_a : s.sp_map_b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, s.d_sp_pool,
+                                   SP_KC, p.pool_rows, which == 0 ? SP_M : p.bn))
+            return rc;
+    return NSS_OK;
+}
+
+namespace {
+
+template <int BN>
+int launch_split(Ctx &c, const int *stop) {
+    static std::atomic<bool> done{false};
+    if (!done.load()) {
+        NSS_CUDA_TRY(c, cudaFuncSetAttribute(k_sector_split<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitCfg<BN>::SMEM));
+        done.store(true);
+    }
+    DevSb &s = c.sb;
+    alignas(64) CUtensorMap ma, mb;
+    std::memcpy(&ma, s.sp_map_a, sizeof(ma));
+    std::memcpy(&mb, s.sp_map_b, sizeof(mb));
+    k_sector_split<BN><<<s.sp_grid, SP_THREADS, SplitCfg<BN>::SMEM, c.stream>>>(ma, mb, s.d_sp_items, s.d_sp_rng, s.d_sp_out, s.d_sp_out0, s.n,
+                                                                               wait_limit(), s.d_tc_err, stop);
+    return NSS_OK;
+}
+
+}  // namespace
+
+int hv_device_split(Ctx &c, const double *d_v, double *d_hv, const int *stop) {
+    DevSb &s = c.sb;
+    c.launches += 3;
+    k_split_pack<<<(unsigned)s.sp_njobs, 32 * SP_ROWS, s.sp_pack_smem, c.stream>>>(d_v, s.d_sp_jobs_w, s.d_sp_pool, s.d_sp_exp, s.d_sp_x32, stop);
+    if (int rc = s.sp_bn == 64 ? launch_split<64>(c, stop) : launch_split<32>(c, stop)) return rc;
+    SplitTerms T{s.d_sp_terms, s.d_sp_tcol, s.d_sp_dptr, s.d_sp_dcol, s.d_sp_exp, s.d_sp_tval, s.d_sp_dval, s.d_terms,
+                 s.d_ab_rowptr, s.d_ab_col, s.d_ab_val};
+    k_split_terms<<<(unsigned)s.sp_ntiles, 256, 0, c.stream>>>(d_v, s.d_sp_x32, s.d_sp_out, s.d_sp_out0, s.n, d_hv, s.d_sp_tiles, T, stop);
+    NSS_CUDA_TRY(c, cudaGetLastError());
+    return NSS_OK;
+}
+
+}  // namespace nss
