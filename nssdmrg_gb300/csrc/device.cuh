@@ -31,6 +31,19 @@ struct DevTerm {          // one A x B term, grouped by output sector
     int64_t a_rp, b_rp;   // offsets of the rowptr arrays in the pools
 };
 
+// Tiles and terms of k_hv_fp64 (k_matvec.cu)
+struct HvRec {
+    int dl, dr, row0, col0;
+    int t0, t1, csr, pad;        // the sector's terms; csr: some term's rows hold several entries
+    int64_t off, hlo, hro;
+};
+struct HvTerm {
+    int64_t off;                 // the input sector's offset in psi
+    int drq, a, b;               // its Dr; first entries of A's rows at ell[a + il], of B's at ell[b + ir]
+    int64_t a_rp, b_rp;          // CSR rows
+    int kind, unit_b;            // 0 one entry a row, 1 A has more, 2 B has; B's entries all +-1
+};
+
 struct DevSb {
     bool valid = false;
     uint64_t gen = 0;                  // upload generation (process-wide count)
@@ -55,6 +68,11 @@ struct DevSb {
     double *d_ab_val = nullptr;
     int4 *d_tiles = nullptr;
     int ntiles = 0;
+    HvRec *d_hv_recs = nullptr;        // k_hv_fp64 (unless the split path has the superblock)
+    HvTerm *d_hv_terms = nullptr;
+    int *d_ell_col = nullptr;
+    double *d_ell_val = nullptr;
+    int nhv = 0;
     // FP32 copies for the mixed-precision path
     float *d_hl32 = nullptr, *d_hr32 = nullptr, *d_ab_val32 = nullptr;
     int *d_ab_rowptr32 = nullptr, *d_ab_col32 = nullptr;   // pruned FP32 A/B pool

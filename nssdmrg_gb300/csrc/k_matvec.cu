@@ -80,6 +80,7 @@ namespace {
 
 constexpr int TILE = 16;
 constexpr int TILE32 = 32;
+constexpr int HV_TR = 8, HV_TC = 16;   // output tile of k_hv_fp64
 
 // Sections of the pool's arena: each array at a 256-byte boundary (at least
 // 16 bytes, so that every pointer is distinct and valid), those with a host
@@ -394,12 +395,48 @@ int sb_upload(Ctx &c, const nss_sb_desc *d, bool trusted) {
         for (auto &t : by_out[k]) s.terms.push_back(t);
         s.term_ptr.push_back((int)s.terms.size());
     }
-    // tiles
+    // tiles (k_noalloc.cu)
     std::vector<int4> tiles;
     for (int k = 0; k < s.nsb; ++k)
         for (int r = 0; r < s.dls[k]; r += TILE)
             for (int cc = 0; cc < s.drs[k]; cc += TILE) tiles.push_back(make_int4(k, r, cc, 0));
     s.ntiles = (int)tiles.size();
+    // k_hv_fp64's terms, with the first entry of every row, and its tiles,
+    // longest first
+    const bool split = split_wanted(s);
+    std::vector<HvTerm> hv_terms;
+    std::vector<HvRec> hv_recs;
+    std::vector<int> ell_col;
+    std::vector<double> ell_val;
+    if (!split) {
+        for (const DevTerm &t : s.terms) {
+            HvTerm h{s.off[t.in_sec], s.drs[t.in_sec], 0, 0, t.a_rp, t.b_rp, 0, 1};
+            for (int side = 0; side < 2; ++side) {
+                const int64_t rp = side == 0 ? t.a_rp : t.b_rp;
+                const int nrow = side == 0 ? t.a_nrow : t.b_nrow;
+                (side == 0 ? h.a : h.b) = (int)ell_col.size();
+                for (int i = 0; i < nrow; ++i) {
+                    const int p0 = rowptr[rp + i], p1 = rowptr[rp + i + 1];
+                    ell_col.push_back(p1 > p0 ? col[p0] : -1);
+                    ell_val.push_back(p1 > p0 ? val[p0] : 0.0);
+                    if (p1 - p0 > 1) h.kind = std::max(h.kind, side == 0 ? 1 : 2);
+                    if (side == 1 && p1 > p0 && std::fabs(val[p0]) != 1.0) h.unit_b = 0;
+                }
+            }
+            hv_terms.push_back(h);
+        }
+        for (int k = 0; k < s.nsb; ++k) {
+            int csr = 0;
+            for (int t = s.term_ptr[k]; t < s.term_ptr[k + 1]; ++t) csr |= hv_terms[t].kind > 0;
+            for (int r = 0; r < s.dls[k]; r += HV_TR)
+                for (int cc = 0; cc < s.drs[k]; cc += HV_TC)
+                    hv_recs.push_back(HvRec{s.dls[k], s.drs[k], r, cc, s.term_ptr[k], s.term_ptr[k + 1], csr, 0, s.off[k],
+                                            s.hl_off[k], s.hr_off[k]});
+        }
+        std::stable_sort(hv_recs.begin(), hv_recs.end(),
+                         [](const HvRec &x, const HvRec &y) { return x.dl + x.dr > y.dl + y.dr; });
+    }
+    s.nhv = (int)hv_recs.size();
 
     // FP32 copies for the mixed path, and its 32x32 tiles.  The FP32 A/B
     // pool drops entries below 1e-12 of the largest entry of their matrix:
@@ -540,7 +577,7 @@ int sb_upload(Ctx &c, const nss_sb_desc *d, bool trusted) {
     s.ntiles32 = (int)tiles32.size();
     std::vector<int> tc_err(1, 0);
     SplitPlan sp;
-    if (split_wanted(s)) split_layout(s, rowptr, col, val, nsm, sp);
+    if (split) split_layout(s, rowptr, col, val, nsm, sp);
 
     Stager sg;
     sg.add_dev(&s.d_hl32, (size_t)hl_tot);
@@ -594,7 +631,10 @@ int sb_upload(Ctx &c, const nss_sb_desc *d, bool trusted) {
     sg.add(&s.d_sp_dcol, sp.dcol);
     sg.add(&s.d_sp_dval, sp.dval);
     sg.add(&s.d_sp_tiles, sp.tiles);
-    const bool split = !sp.items.empty();
+    sg.add(&s.d_hv_recs, hv_recs);
+    sg.add(&s.d_hv_terms, hv_terms);
+    sg.add(&s.d_ell_col, ell_col);
+    sg.add(&s.d_ell_val, ell_val);
     sg.add_dev(&s.d_sp_exp, (size_t)sp.nexp);
     sg.add_dev(&s.d_sp_x32, split ? (size_t)s.n : 0);
     sg.add_dev(&s.d_sp_out, split ? 2 * (size_t)s.n : 0);
@@ -623,87 +663,157 @@ int sb_upload(Ctx &c, const nss_sb_desc *d, bool trusted) {
     return NSS_OK;
 }
 
-// One CTA per 16x16 output tile; thread (ty,tx) owns W_k[row0+ty][col0+tx].
-// GB300 issues FP64 at about 1/64 of its FP32 rate, so this kernel is bound
-// by the FP64 pipe; the operand tiles are staged in shared memory only to
-// keep the loads coalesced.
-__global__ void __launch_bounds__(256) k_hv_fp64(
-    const double *__restrict__ v, double *__restrict__ hv, const int4 *__restrict__ tiles,
-    const int *__restrict__ dls, const int *__restrict__ drs, const int64_t *__restrict__ off,
-    const double *__restrict__ hlp, const int64_t *__restrict__ hl_off,
-    const double *__restrict__ hrp, const int64_t *__restrict__ hr_off,
-    const int *__restrict__ term_ptr, const DevTerm *__restrict__ terms,
-    const int *__restrict__ ab_rp, const int *__restrict__ ab_col, const double *__restrict__ ab_val,
-    const int *stop) {
-    if (stop && *stop) return;   // the Lanczos loop has already finished
-    __shared__ double sa[TILE][33];
-    __shared__ double sb[32][TILE + 1];
-    const int4 t = tiles[blockIdx.x];
-    const int k = t.x, row0 = t.y, col0 = t.z;
-    const int dl = dls[k], dr = drs[k];
-    const int64_t o = off[k];
-    const double *W = v + o;
-    const double *HL = hlp + hl_off[k];
-    const double *HR = hrp + hr_off[k];
-    const int tid = threadIdx.x, ty = tid / TILE, tx = tid % TILE;
-    const int il = row0 + ty, ir = col0 + tx;
-    double acc = 0.0;
+// One CTA of four warps per 8 x 16 output tile, a thread an output.
+// The FP64 pipe takes a warp's FMA every 64 cycles (1.0-1.2 TFLOP/s over the
+// GPU) and bounds the kernel: so the K loops stop at the sector's edge, four
+// warps (one per quarter of an SM) are a tile, which spreads a small superblock
+// over four times as many SMs as 16 x 16 outputs on eight warps did, and the
+// next 32 columns of K are loaded into registers while the current ones are
+// multiplied.  Sums run in the same order as there.  A x B terms: Out[ai][bi]
+// += A[ai][aj] B[bi][bj] W_q[aj][bj] (:808-857).  Where all rows hold one entry,
+// four terms' loads are in flight; where rows of A hold more (the
+// renormalised sign operator leaves rounding-level entries in its whole block,
+// 40 a row), half a warp takes a row, a lane an entry, eight gathers in flight,
+// instead of every thread walking the row by itself; a factor of +-1 is a sign
+// flip and no FP64 multiplication.  Against the 16 x 16 form, results bit for
+// bit the same: Hubbard m = 256 (66 600 states) 88 -> 60 us a product, 582
+// states 4.1 -> 3.4 us, FP64 solves of 3 958 states 3.12 -> 2.32 ms, of 66 600
+// 9.85 -> 7.60 ms.
+__device__ __forceinline__ double hv_times(double b, double x, bool unit) {
+    if (!unit) return b * x;
+    return __hiloint2double(__double2hiint(x) ^ (__double2hiint(b) & 0x80000000), __double2loint(x));
+}
 
-    // H_L W : sum_j HL[il][j] W[j][ir]   (the H^L x 1^R loop, :784-796)
-    for (int j0 = 0; j0 < dl; j0 += 32) {
-        for (int e = tid; e < TILE * 32; e += 256) {
-            int r = e / 32, cc = e % 32;
-            int gi = row0 + r, gj = j0 + cc;
-            sa[r][cc] = (gi < dl && gj < dl) ? HL[(int64_t)gi * dl + gj] : 0.0;
+struct HvOps {
+    const double *hl, *hr;
+    const HvTerm *terms;
+    const int *ell_col;
+    const double *ell_val;
+    const int *ab_rp, *ab_col;
+    const double *ab_val;
+};
+
+__global__ void __launch_bounds__(HV_TR *HV_TC) k_hv_fp64(const double *__restrict__ v, double *__restrict__ hv,
+                                                           const HvRec *__restrict__ recs, HvOps op, const int *stop) {
+    if (stop && *stop) return;   // the Lanczos loop has already finished
+    constexpr int NT = HV_TR * HV_TC, KC = 32;
+    __shared__ double sa[HV_TR][KC + 1];
+    __shared__ double sb[KC][HV_TC + 1];
+    const HvRec t = recs[blockIdx.x];
+    const int dl = t.dl, dr = t.dr;
+    const double *W = v + t.off, *HL = op.hl + t.hlo, *HR = op.hr + t.hro;
+    const int tid = threadIdx.x, ty = tid / HV_TC, tx = tid % HV_TC;
+    const int il = t.row0 + ty, ir = t.col0 + tx;
+    const int c0 = (dl + KC - 1) / KC, c1 = (dr + KC - 1) / KC;
+    double ra[HV_TR * KC / NT], rb[KC * HV_TC / NT];
+    // chunk c of the K loops: H_L W (sum_j HL[il][j] W[j][ir], :784-796), then
+    // W H_R^T (sum_j W[il][j] HR[ir][j], :767-779)
+    auto load = [&](int c) {
+        const bool left = c < c0;
+        const int j0 = (left ? c : c - c0) * KC, K = left ? dl : dr;
+#pragma unroll
+        for (int q = 0; q < HV_TR * KC / NT; ++q) {
+            const int e = tid + q * NT, gi = t.row0 + e / KC, gj = j0 + e % KC;
+            ra[q] = (gi < dl && gj < K) ? (left ? HL[(int64_t)gi * dl + gj] : W[(int64_t)gi * dr + gj]) : 0.0;
         }
-        for (int e = tid; e < 32 * TILE; e += 256) {
-            int r = e / TILE, cc = e % TILE;
-            int gj = j0 + r, gc = col0 + cc;
-            sb[r][cc] = (gj < dl && gc < dr) ? W[(int64_t)gj * dr + gc] : 0.0;
-        }
-        __syncthreads();
-#pragma unroll 8
-        for (int j = 0; j < 32; ++j) acc = fma(sa[ty][j], sb[j][tx], acc);
-        __syncthreads();
-    }
-    // W H_R^T : sum_j W[il][j] HR[ir][j]   (the 1^L x H^R loop, :767-779)
-    for (int j0 = 0; j0 < dr; j0 += 32) {
-        for (int e = tid; e < TILE * 32; e += 256) {
-            int r = e / 32, cc = e % 32;
-            int gi = row0 + r, gj = j0 + cc;
-            sa[r][cc] = (gi < dl && gj < dr) ? W[(int64_t)gi * dr + gj] : 0.0;
-        }
-        for (int e = tid; e < 32 * TILE; e += 256) {
-            int r = e / TILE, cc = e % TILE;   // sb[j][x] = HR[col0+x][j0+j]
-            int gr = col0 + cc, gj = j0 + r;
-            sb[r][cc] = (gr < dr && gj < dr) ? HR[(int64_t)gr * dr + gj] : 0.0;
-        }
-        __syncthreads();
-#pragma unroll 8
-        for (int j = 0; j < 32; ++j) acc = fma(sa[ty][j], sb[j][tx], acc);
-        __syncthreads();
-    }
-    // sum_t A W_q B^T : Out[ai][bi] += A[ai][aj] B[bi][bj] W_q[aj][bj] (:808-857)
-    __shared__ AbStage<double, TILE, TILE> S;
-    const bool in = il < dl && ir < dr;
-    for (int tb = term_ptr[k]; tb < term_ptr[k + 1]; tb += AB_MAXT) {
-        const int nt = min(AB_MAXT, term_ptr[k + 1] - tb);
-        ab_stage<double, TILE, TILE>(S, v, tb, nt, row0, col0, dl, dr, drs, off, terms, ab_rp, ab_col, ab_val,
-                                     threadIdx.x, blockDim.x, CtaSync{});
-        if (in) {
-            if (!S.multi) {
-                for (int tt = 0; tt < nt; ++tt) {
-                    const int aj = S.ac[tt][ty], bj = S.bc[tt][tx];
-                    if (aj >= 0 && bj >= 0)
-                        acc = fma(S.av[tt][ty] * S.bv[tt][tx], S.wq[tt][(int64_t)aj * S.drq[tt] + bj], acc);
-                }
+#pragma unroll
+        for (int q = 0; q < KC * HV_TC / NT; ++q) {
+            const int e = tid + q * NT;
+            if (left) {
+                const int gj = j0 + e / HV_TC, gc = t.col0 + e % HV_TC;
+                rb[q] = (gj < dl && gc < dr) ? W[(int64_t)gj * dr + gc] : 0.0;
             } else {
-                acc = ab_csr<double>(acc, v, tb, nt, il, ir, drs, off, terms, ab_rp, ab_col, ab_val);
+                const int gr = t.col0 + e / KC, gj = j0 + e % KC;
+                rb[q] = (gr < dr && gj < dr) ? HR[(int64_t)gr * dr + gj] : 0.0;
             }
         }
+    };
+    double acc = 0.0;
+    load(0);
+    for (int c = 0; c < c0 + c1; ++c) {
+        const bool left = c < c0;
+        const int kn = min(KC, left ? dl - c * KC : dr - (c - c0) * KC);
+#pragma unroll
+        for (int q = 0; q < HV_TR * KC / NT; ++q) {
+            const int e = tid + q * NT;
+            sa[e / KC][e % KC] = ra[q];
+        }
+#pragma unroll
+        for (int q = 0; q < KC * HV_TC / NT; ++q) {
+            const int e = tid + q * NT;
+            if (left) sb[e / HV_TC][e % HV_TC] = rb[q];
+            else sb[e % KC][e / KC] = rb[q];
+        }
+        __syncthreads();
+        if (c + 1 < c0 + c1) load(c + 1);
+#pragma unroll 8
+        for (int j = 0; j < kn; ++j) acc = fma(sa[ty][j], sb[j][tx], acc);
         __syncthreads();
     }
-    if (in) hv[o + (int64_t)il * dr + ir] = acc;
+    const bool in = il < dl && ir < dr;
+    if (!t.csr) {
+        for (int tb = t.t0; tb < t.t1; tb += 4) {
+            int aj[4], bj[4];
+            double f[4], w[4];
+            HvTerm tm[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) tm[q] = op.terms[min(tb + q, t.t1 - 1)];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const bool on = in && tb + q < t.t1;
+                aj[q] = on ? op.ell_col[tm[q].a + il] : -1;
+                bj[q] = on ? op.ell_col[tm[q].b + ir] : -1;
+                f[q] = on ? hv_times(op.ell_val[tm[q].b + ir], op.ell_val[tm[q].a + il], tm[q].unit_b) : 0.0;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                w[q] = aj[q] >= 0 && bj[q] >= 0 ? v[tm[q].off + (int64_t)aj[q] * tm[q].drq + bj[q]] : 0.0;
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (aj[q] >= 0 && bj[q] >= 0) acc = fma(f[q], w[q], acc);
+        }
+    } else {
+        const int hl16 = tid & 15;                   // lane of the half warp that holds the row
+        for (int ti = t.t0; ti < t.t1; ++ti) {
+            const HvTerm tm = op.terms[ti];
+            const double *Wq = v + tm.off;
+            if (tm.kind == 2) {                      // rows of B with several entries
+                if (in)
+                    for (int ja = op.ab_rp[tm.a_rp + il]; ja < op.ab_rp[tm.a_rp + il + 1]; ++ja) {
+                        const int64_t row = (int64_t)op.ab_col[ja] * tm.drq;
+                        double cb = 0.0;
+                        for (int jb = op.ab_rp[tm.b_rp + ir]; jb < op.ab_rp[tm.b_rp + ir + 1]; ++jb)
+                            cb = fma(op.ab_val[jb], Wq[row + op.ab_col[jb]], cb);
+                        acc = fma(op.ab_val[ja], cb, acc);
+                    }
+                continue;
+            }
+            const int bj = in ? op.ell_col[tm.b + ir] : -1;
+            const double bv = in ? op.ell_val[tm.b + ir] : 0.0;
+            const int p0 = il < dl ? op.ab_rp[tm.a_rp + il] : 0;
+            const int cnt = il < dl ? op.ab_rp[tm.a_rp + il + 1] - p0 : 0;
+            const int most = max(cnt, __shfl_xor_sync(0xffffffffu, cnt, 16));
+            for (int base = 0; base < most; base += 16) {
+                const bool mine = base + hl16 < cnt;
+                const int ec = mine ? op.ab_col[p0 + base + hl16] : 0;
+                const double ev = mine ? op.ab_val[p0 + base + hl16] : 0.0;
+                for (int u = 0; u < 16 && base + u < most; u += 8) {
+                    double g[8];
+#pragma unroll
+                    for (int x = 0; x < 8; ++x) {
+                        const int c = __shfl_sync(0xffffffffu, ec, u + x, 16);
+                        g[x] = bj >= 0 && base + u + x < cnt ? Wq[(int64_t)c * tm.drq + bj] : 0.0;
+                    }
+#pragma unroll
+                    for (int x = 0; x < 8; ++x) {
+                        const double a = __shfl_sync(0xffffffffu, ev, u + x, 16);
+                        if (bj >= 0 && base + u + x < cnt) acc = fma(a, hv_times(bv, g[x], tm.unit_b), acc);
+                    }
+                }
+            }
+        }
+    }
+    if (in) hv[t.off + (int64_t)il * dr + ir] = acc;
 }
 
 // FP32 variant for the mixed-precision Lanczos phase: 32x32 output tiles,
@@ -800,9 +910,9 @@ int hv_device(Ctx &c, const double *d_v, double *d_hv, const int *stop) {
         return NSS_ERR_STATE;
     }
     if (s.sp_nitems) return hv_device_split(c, d_v, d_hv, stop);
-    k_hv_fp64<<<s.ntiles, 256, 0, c.stream>>>(d_v, d_hv, s.d_tiles, s.d_dls, s.d_drs, s.d_off, s.d_hl,
-                                              s.d_hl_off, s.d_hr, s.d_hr_off, s.d_term_ptr, s.d_terms,
-                                              s.d_ab_rowptr, s.d_ab_col, s.d_ab_val, stop);
+    k_hv_fp64<<<s.nhv, HV_TR * HV_TC, 0, c.stream>>>(
+        d_v, d_hv, s.d_hv_recs,
+        HvOps{s.d_hl, s.d_hr, s.d_hv_terms, s.d_ell_col, s.d_ell_val, s.d_ab_rowptr, s.d_ab_col, s.d_ab_val}, stop);
     c.launches += 1;
     NSS_CUDA_TRY(c, cudaGetLastError());
     return NSS_OK;
