@@ -109,10 +109,12 @@ struct Stager {
     }
 };
 
-// Dense sector operators from their CSR rows: one thread per row of one
-// sector's H_L or H_R (rows of both sides in one launch), duplicates summed
-// as the host build did; the blocks are zeroed beforehand.  FP32 copies
-// follow in k_dense32.
+// Dense sector operators from their CSR rows: one warp per row of one
+// sector's H_L or H_R (rows of both sides in one launch), 32 entries at a time,
+// duplicates summed in their order as the host build did (one lane takes a
+// batch that holds a column twice); the blocks are zeroed beforehand.  FP32
+// copies follow in k_dense32.  (A thread per row wrote 300 entries one after
+// the other: 62 us at Hubbard m = 250, 187 us at spin-1 m = 400.)
 struct DenseRows {
     const int *rowptr;      // per side: all sectors' rows, global entry offsets
     const int *col;
@@ -124,8 +126,9 @@ __global__ void __launch_bounds__(256) k_densify(DenseRows L, DenseRows R, int n
                                                   const int *__restrict__ dls, const int *__restrict__ drs,
                                                   const int64_t *__restrict__ hl_off, const int64_t *__restrict__ hr_off,
                                                   double *__restrict__ hl, double *__restrict__ hr) {
-    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (t >= (int64_t)nrow_l + nrow_r) return;
+    const int64_t t = blockIdx.x * (int64_t)(blockDim.x / 32) + threadIdx.x / 32;
+    if (t >= (int64_t)nrow_l + nrow_r) return;       // whole warps
+    const int lane = threadIdx.x & 31;
     const bool right = t >= nrow_l;
     const DenseRows &D = right ? R : L;
     const int g = (int)(right ? t - nrow_l : t);
@@ -133,7 +136,19 @@ __global__ void __launch_bounds__(256) k_densify(DenseRows L, DenseRows R, int n
     const int d = right ? drs[k] : dls[k];
     const int i = (int)(g - D.row_first[k]);
     double *row = (right ? hr + hr_off[k] : hl + hl_off[k]) + (int64_t)i * d;
-    for (int p = D.rowptr[g]; p < D.rowptr[g + 1]; ++p) row[D.col[p]] += D.val[p];
+    const int p1 = D.rowptr[g + 1];
+    for (int p0 = D.rowptr[g]; p0 < p1; p0 += 32) {
+        const int p = p0 + lane;
+        const int c = p < p1 ? D.col[p] : -1 - lane;
+        const double x = p < p1 ? D.val[p] : 0.0;
+        const bool twice = __popc(__match_any_sync(0xffffffffu, c)) > 1;
+        if (!__any_sync(0xffffffffu, twice)) {
+            if (p < p1) row[c] += x;
+        } else if (lane == 0) {
+            for (int q = p0; q < min(p1, p0 + 32); ++q) row[D.col[q]] += D.val[q];
+        }
+        __syncwarp();
+    }
 }
 
 __global__ void __launch_bounds__(256) k_dense32(const double *__restrict__ x, float *__restrict__ y, int64_t n) {
@@ -647,7 +662,7 @@ int sb_upload(Ctx &c, const nss_sb_desc *d, bool trusted) {
     {
         const int64_t nr = nrow_l + nrow_r;
         c.launches += 3;
-        k_densify<<<(unsigned)((nr + 255) / 256), 256, 0, c.stream>>>(dr_dev[0], dr_dev[1], (int)nrow_l, (int)nrow_r,
+        k_densify<<<(unsigned)((nr + 7) / 8), 256, 0, c.stream>>>(dr_dev[0], dr_dev[1], (int)nrow_l, (int)nrow_r,
                                                                       s.d_dls, s.d_drs, s.d_hl_off, s.d_hr_off,
                                                                       s.d_hl, s.d_hr);
         k_dense32<<<608, 256, 0, c.stream>>>(s.d_hl, s.d_hl32, hl_tot);
