@@ -56,9 +56,15 @@ int tune_choose(Ctx &c, const DevSb &s, int *tc_min_dl, int *bn) {
     {
         std::lock_guard<std::mutex> lk(g_mu);
         Entry &e = g_table[{c.device, cls}];
+        // the likely winner first, since every superblock uploaded before the
+        // first solve of its class gets it: from 100 MFLOP of dense work the
+        // tensor cores (mixed solves, plans 0 / 1 / 2: 60 MFLOP 3.3 / 3.9 / 4.0 ms,
+        // 148 MFLOP 4.8 / 4.4 / 4.5, 474 MFLOP 9.5 / 6.8 / 6.2)
+        static const int small_first[NCAND] = {0, 1, 2}, large_first[NCAND] = {2, 1, 0};
+        const int *order = s.flops_dense >= 1e8 ? large_first : small_first;
         int untried = -1;
-        for (int k = 0; k < ncand && untried < 0; ++k)
-            if (e.solves[k] == 0) untried = k;
+        for (int q = 0; q < NCAND && untried < 0; ++q)
+            if (order[q] < ncand && e.solves[order[q]] == 0) untried = order[q];
         if (untried >= 0) {
             cand = untried;
         } else {
