@@ -94,6 +94,24 @@ struct Stager {
     };
     std::vector<Item> items, dev;
     size_t host = 0, device = 0;
+    // a section gathered from several host arrays (straight from the caller's
+    // matrices: collecting them in a vector first cost a second copy and the
+    // page faults of fresh memory, most of an upload's host time)
+    struct Part {
+        const void *src;
+        size_t bytes, off;      // offset in the arena
+    };
+    std::vector<Part> parts;
+    template <class T>
+    void add_gather(T **dst, size_t count) {
+        items.push_back({(void **)dst, nullptr, count * sizeof(T), host});
+        host += (std::max<size_t>(count * sizeof(T), 16) + 255) / 256 * 256;
+    }
+    // the next `count` elements of the section `dst` was added for, at element `at`
+    template <class T>
+    void part(size_t item, const T *src, size_t count, size_t at) {
+        if (count) parts.push_back({(const void *)src, count * sizeof(T), items[item].off + at * sizeof(T)});
+    }
     template <class T>
     void add(T **dst, const std::vector<T> &v) {
         const size_t bytes = v.size() * sizeof(T);
@@ -185,10 +203,13 @@ int stage_commit(Ctx &c, Stager &sg) {
     };
     std::vector<Piece> pieces;
     constexpr size_t PIECE = (size_t)1 << 20;
+    auto cut = [&](const void *src, size_t off, size_t bytes) {
+        for (size_t o = 0; o < bytes; o += PIECE)
+            pieces.push_back({c.sb_stage + off + o, (const char *)src + o, std::min(PIECE, bytes - o)});
+    };
     for (const auto &it : sg.items)
-        if (it.bytes)
-            for (size_t o = 0; o < it.bytes; o += PIECE)
-                pieces.push_back({c.sb_stage + it.off + o, (const char *)it.src + o, std::min(PIECE, it.bytes - o)});
+        if (it.src) cut(it.src, it.off, it.bytes);
+    for (const auto &p : sg.parts) cut(p.src, p.off, p.bytes);
     parallel_for((int)pieces.size(), [&](int i) { std::memcpy(pieces[i].dst, pieces[i].src, pieces[i].bytes); },
                  sg.host > ((size_t)4 << 20));
     NSS_CUDA_TRY(c, cudaMemcpyAsync(c.sb_arena, c.sb_stage, sg.host, cudaMemcpyHostToDevice, c.stream));
@@ -307,59 +328,27 @@ int sb_upload(Ctx &c, const nss_sb_desc *d, bool trusted) {
         return NSS_ERR_INVALID;
     }
     struct PackedRows {
-        std::vector<int> rowptr, col, row_sec;
-        std::vector<double> val;
+        std::vector<int> rowptr, row_sec;
         std::vector<int64_t> row_first;
     } pk[2];
-    const bool big_pool = nnz_l + nnz_r > 100000;
-    run_pair(
-        [&] {
-            for (int side = 0; side < 2; ++side) {
-                PackedRows &P = pk[side];
-                P.rowptr.reserve((size_t)(side ? nrow_r : nrow_l) + 1);
-                P.rowptr.push_back(0);
-                P.row_first.reserve(s.nsb);
-                P.row_sec.reserve((size_t)(side ? nrow_r : nrow_l));
-                int64_t rows = 0;
-                for (int k = 0; k < s.nsb; ++k) {
-                    const nss_csr &M = side ? d->hright[k] : d->hleft[k];
-                    const int base = P.rowptr.back();
-                    P.row_first.push_back(rows);
-                    for (int i = 0; i < M.nrow; ++i) {
-                        P.rowptr.push_back(base + M.rowptr[i + 1]);
-                        P.row_sec.push_back(k);
-                    }
-                    rows += M.nrow;
-                }
+    for (int side = 0; side < 2; ++side) {
+        PackedRows &P = pk[side];
+        P.rowptr.reserve((size_t)(side ? nrow_r : nrow_l) + 1);
+        P.rowptr.push_back(0);
+        P.row_first.reserve(s.nsb);
+        P.row_sec.reserve((size_t)(side ? nrow_r : nrow_l));
+        int64_t rows = 0;
+        for (int k = 0; k < s.nsb; ++k) {
+            const nss_csr &M = side ? d->hright[k] : d->hleft[k];
+            const int base = P.rowptr.back();
+            P.row_first.push_back(rows);
+            for (int i = 0; i < M.nrow; ++i) {
+                P.rowptr.push_back(base + M.rowptr[i + 1]);
+                P.row_sec.push_back(k);
             }
-        },
-        [&] {
-            std::vector<int64_t> at(2 * (size_t)s.nsb);
-            for (int side = 0; side < 2; ++side) {
-                PackedRows &P = pk[side];
-                P.col.resize((size_t)(side ? nnz_r : nnz_l));
-                P.val.resize((size_t)(side ? nnz_r : nnz_l));
-                int64_t a = 0;
-                for (int k = 0; k < s.nsb; ++k) {
-                    at[(size_t)side * s.nsb + k] = a;
-                    const nss_csr &M = side ? d->hright[k] : d->hleft[k];
-                    a += M.rowptr[M.nrow];
-                }
-            }
-            // the sectors' entries copied in parallel
-            parallel_for(2 * s.nsb, [&](int t) {
-                const int side = t / s.nsb, k = t % s.nsb;
-                PackedRows &P = pk[side];
-                const nss_csr &M = side ? d->hright[k] : d->hleft[k];
-                const int nz = M.rowptr[M.nrow];
-                const int64_t o = at[(size_t)t];
-                if (nz) {
-                    std::memcpy(P.col.data() + o, M.colidx, sizeof(int) * (size_t)nz);
-                    std::memcpy(P.val.data() + o, M.vals, sizeof(double) * (size_t)nz);
-                }
-            }, big_pool, 6);
-        },
-        big_pool);
+            rows += M.nrow;
+        }
+    }
 
     // A x B terms, regrouped by output sector
     std::vector<std::vector<DevTerm>> by_out(s.nsb);
@@ -623,8 +612,17 @@ int sb_upload(Ctx &c, const nss_sb_desc *d, bool trusted) {
     DenseRows dr_dev[2];
     for (int side = 0; side < 2; ++side) {
         sg.add((int **)&dr_dev[side].rowptr, pk[side].rowptr);
-        sg.add((int **)&dr_dev[side].col, pk[side].col);
-        sg.add((double **)&dr_dev[side].val, pk[side].val);
+        const size_t it = sg.items.size();
+        sg.add_gather((int **)&dr_dev[side].col, (size_t)(side ? nnz_r : nnz_l));
+        sg.add_gather((double **)&dr_dev[side].val, (size_t)(side ? nnz_r : nnz_l));
+        size_t at = 0;
+        for (int k = 0; k < s.nsb; ++k) {
+            const nss_csr &M = side ? d->hright[k] : d->hleft[k];
+            const size_t nz = (size_t)M.rowptr[M.nrow];
+            sg.part(it, M.colidx, nz, at);
+            sg.part(it + 1, M.vals, nz, at);
+            at += nz;
+        }
         sg.add((int **)&dr_dev[side].row_sec, pk[side].row_sec);
         sg.add((int64_t **)&dr_dev[side].row_first, pk[side].row_first);
     }
