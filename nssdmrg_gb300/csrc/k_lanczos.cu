@@ -356,7 +356,7 @@ struct OrthArgs {
     // launch, the words of the totals, of the columns' partials and of the
     // columns' totals
     unsigned *xep;
-    uint64_t *xtot, *xpart, *xcol;   // xcol: plain values
+    uint64_t *xtot, *xpart, *xcol;
 };
 
 // The omega recurrence's constants per basis type: level after a projection,
@@ -561,25 +561,27 @@ __device__ __forceinline__ void grid_columns(const R *p, int G, int ncol, R *hs)
     }
 }
 
-// Reduce CW per-lane values over the 32 lanes of a warp at once (butterfly
-// with exchange: 31 shuffles for all CW columns); lane L ends with the sum of
-// column L % CW in d[0].
-template <class R, int CW>
-__device__ __forceinline__ R multi_reduce(R (&d)[CW], int lane) {
-    if (CW < 32) {
+// Sums of d[0..N) over groups of P lanes (butterfly with exchange while a lane
+// holds more than one value, N <= P): d[0] ends as the group's sum of value
+// (lane % P) * N / P.  The order of the additions, lanes P/2 apart first, does
+// not depend on N.
+template <class R, int N, int P>
+__device__ __forceinline__ R multi_reduce(R (&d)[N], int lane) {
+    static_assert(N <= P, "every value needs a lane");
 #pragma unroll
-        for (int s = 16; s >= CW; s >>= 1)
+    for (int s = P / 2, cnt = N; s >= 1; s >>= 1) {
+        if (cnt > 1) {
+            const bool upper = (lane & s) != 0;
+            cnt >>= 1;
 #pragma unroll
-            for (int c = 0; c < CW; ++c) d[c] += __shfl_xor_sync(0xffffffffu, d[c], s);
-    }
-#pragma unroll
-    for (int s = CW / 2; s >= 1; s >>= 1) {
-        const bool upper = (lane & s) != 0;
-#pragma unroll
-        for (int c = 0; c < s; ++c) {
-            const R send = upper ? d[c] : d[c + s];
-            const R keep = upper ? d[c + s] : d[c];
-            d[c] = keep + __shfl_xor_sync(0xffffffffu, send, s);
+            for (int c = 0; c < N / 2; ++c)
+                if (c < cnt) {
+                    const R send = upper ? d[c] : d[c + cnt];
+                    const R keep = upper ? d[c + cnt] : d[c];
+                    d[c] = keep + __shfl_xor_sync(0xffffffffu, send, s);
+                }
+        } else {
+            d[0] += __shfl_xor_sync(0xffffffffu, d[0], s);
         }
     }
     return d[0];
@@ -610,11 +612,9 @@ struct XW { static constexpr int words = sizeof(R) / 4; };
 __device__ __forceinline__ void st_word(uint64_t *p, uint32_t v, unsigned ep) {
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"((uint64_t)v | ((uint64_t)ep << 32)) : "memory");
 }
-template <bool ACQ>
 __device__ __forceinline__ uint64_t ld_word(const uint64_t *p) {
     uint64_t w;
-    if (ACQ) asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(p) : "memory");
-    else asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(p) : "memory");
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(p) : "memory");
     return w;
 }
 // value q of a set of `n` values, words `stride` apart: word k of the value at p + (q * words + k) * stride
@@ -626,11 +626,10 @@ __device__ __forceinline__ void st_value(uint64_t *p, int64_t stride, double v, 
     st_word(p + stride, (uint32_t)__double2hiint(v), ep);
 }
 // polls until the value carries the epoch; false when the limit ran out
-template <bool ACQ = false>
 __device__ __forceinline__ bool ld_value(const uint64_t *p, int64_t, unsigned ep, float &v, const int *err, uint32_t spin) {
     uint32_t it = 0;
     for (;;) {
-        const uint64_t w = ld_word<ACQ>(p);
+        const uint64_t w = ld_word(p);
         if ((unsigned)(w >> 32) == ep) {
             v = __uint_as_float((uint32_t)w);
             return true;
@@ -638,12 +637,11 @@ __device__ __forceinline__ bool ld_value(const uint64_t *p, int64_t, unsigned ep
         if (++it > spin || ((it & 255u) == 0 && *(volatile const int *)err)) return false;
     }
 }
-template <bool ACQ = false>
 __device__ __forceinline__ bool ld_value(const uint64_t *p, int64_t stride, unsigned ep, double &v, const int *err,
                                          uint32_t spin) {
     uint32_t it = 0;
     for (;;) {
-        const uint64_t w0 = ld_word<ACQ>(p), w1 = ld_word<ACQ>(p + stride);
+        const uint64_t w0 = ld_word(p), w1 = ld_word(p + stride);
         if ((unsigned)(w0 >> 32) == ep && (unsigned)(w1 >> 32) == ep) {
             v = __hiloint2double((int)(uint32_t)w1, (int)(uint32_t)w0);
             return true;
@@ -652,12 +650,38 @@ __device__ __forceinline__ bool ld_value(const uint64_t *p, int64_t stride, unsi
     }
 }
 
+// x[q] = the value at p + lane + 32 q (for those below G): all words in flight
+// at once, where one ld_value after the other takes an L2 round trip each
+template <class R, int Q>
+__device__ __forceinline__ bool ld_values(const uint64_t *p, int64_t stride, int lane, int G, unsigned ep, R (&x)[Q],
+                                          const int *err, uint32_t spin) {
+    constexpr int W = XW<R>::words;
+    uint32_t it = 0;
+    for (;;) {
+        uint64_t w[Q][W];
+        bool all = true;
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+#pragma unroll
+            for (int k = 0; k < W; ++k)
+                w[q][k] = lane + 32 * q < G ? ld_word(p + k * stride + lane + 32 * q) : (uint64_t)ep << 32;
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+#pragma unroll
+            for (int k = 0; k < W; ++k) all = all && (unsigned)(w[q][k] >> 32) == ep;
+            if constexpr (W == 1) x[q] = __uint_as_float((uint32_t)w[q][0]);
+            else x[q] = __hiloint2double((int)(uint32_t)w[q][1], (int)(uint32_t)w[q][0]);
+        }
+        if (all) return true;
+        if (++it > spin || ((it & 255u) == 0 && *(volatile const int *)err)) return false;
+    }
+}
+
 // out[q] = sum over the CTAs of v[q] (valid in thread 0), in the order of
-// grid_totals; xs: [NV][G] in shared memory.  FENCE: also a barrier, after
-// which the CTAs see each other's global writes from before it; else only
-// the values travel.  flag (may be null): the last CTA's value (thread 0), on
+// grid_totals; xs: [NV][G] in shared memory.  Only the values travel: no
+// barrier, no fence.  flag (may be null): the last CTA's value (thread 0), on
 // return everybody's.  False when a wait ran out (sets *err).
-template <class R, int NV, bool FENCE>
+template <class R, int NV>
 __device__ __forceinline__ bool xchg_totals(uint64_t *xtot, unsigned &ep, const R (&v)[NV], int G, R *xs, R *bc,
                                             R (&out)[NV], int *err, uint32_t spin, int *flag = nullptr) {
     constexpr int W = XW<R>::words;
@@ -671,13 +695,12 @@ __device__ __forceinline__ bool xchg_totals(uint64_t *xtot, unsigned &ep, const 
     __syncthreads();                                 // xs, bc and xflag of the last exchange are read
     if ((int)blockIdx.x != last) {
         if (tid == 0) {
-            if (FENCE) fence_acq_rel();
 #pragma unroll
             for (int q = 0; q < NV; ++q) st_value(xtot + (size_t)(q * W) * XMAX + blockIdx.x, XMAX, v[q], ep);
         }
         if (tid < NV) {
             R x = (R)0;
-            good = ld_value<FENCE>(res + tid * W, 1, ep, x, err, spin);
+            good = ld_value(res + tid * W, 1, ep, x, err, spin);
             bc[tid] = x;
         }
         if (flag && tid == NV) {
@@ -690,15 +713,13 @@ __device__ __forceinline__ bool xchg_totals(uint64_t *xtot, unsigned &ep, const 
         if (tid == 0)
 #pragma unroll
             for (int q = 0; q < NV; ++q) xs[q * G + last] = v[q];
-        if (tid < last) {
-#pragma unroll
-            for (int q = 0; q < NV; ++q) {
-                R x = (R)0;
-                good = good && ld_value<FENCE>(xtot + (size_t)(q * W) * XMAX + tid, XMAX, ep, x, err, spin);
-                xs[q * G + tid] = x;
-            }
-            if (!good) atomicExch(err, 1);
+        for (int k = tid; k < NV * last; k += ORTH_THREADS) {
+            const int q = k / last, b = k - q * last;
+            R x = (R)0;
+            good = good && ld_value(xtot + (size_t)(q * W) * XMAX + b, XMAX, ep, x, err, spin);
+            xs[q * G + b] = x;
         }
+        if (!good) atomicExch(err, 1);
         if (!__syncthreads_and(good)) good = false;
         if (warp < NV && good) {
             R t = (R)0;
@@ -706,7 +727,6 @@ __device__ __forceinline__ bool xchg_totals(uint64_t *xtot, unsigned &ep, const 
             t = warp_sum<R>(t);
             if (lane == 0) {
                 bc[warp] = t;
-                if (FENCE) fence_acq_rel();
                 st_value(res + warp * W, 1, t, ep);
                 if (flag && warp == 0) {
                     st_word(res + XCOLS - 1, (uint32_t)*flag, ep);
@@ -724,78 +744,103 @@ __device__ __forceinline__ bool xchg_totals(uint64_t *xtot, unsigned &ep, const 
 
 // hs[l] = sum over the CTAs of column l's partial (l < ncol), which every CTA
 // has stored at xpart (st_value, epoch ep + 1): CTA l mod G sums column l, in
-// the order of grid_columns, and all read the totals after an exchange (summed
-// by every CTA instead, 100 FP64 columns took each SM's FP64 pipe 10 us).
+// the order of grid_columns, and stores the total as tagged words at xcol,
+// which all poll (summed by every CTA instead, 100 FP64 columns took each SM's
+// FP64 pipe 10 us).  A CTA writes its partials and totals of a later epoch only
+// after it has read all totals of this one, so one buffer of each is enough.
 template <class R>
-__device__ __forceinline__ bool xchg_columns(const uint64_t *xpart, R *xcol, uint64_t *xtot, unsigned &ep, int G, int ncol,
-                                             R *hs, R *xs, R *bc, int *err, uint32_t spin) {
+__device__ __forceinline__ bool xchg_columns(const uint64_t *xpart, uint64_t *xcol, unsigned &ep, int G, int ncol, R *hs,
+                                             int *err, uint32_t spin) {
     constexpr int W = XW<R>::words;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     ++ep;
     bool good = true;
     for (int l = blockIdx.x + warp * G; l < ncol; l += ORTH_WARPS * G) {
+        const uint64_t *p = xpart + (size_t)l * W * XMAX;
+        R x[XMAX / 32];
+        good = good && ld_values<R, XMAX / 32>(p, XMAX, lane, G, ep, x, err, spin);
         R t = (R)0;
-        for (int b = lane; b < G; b += 32) {
-            R x = (R)0;
-            good = good && ld_value(xpart + (size_t)l * W * XMAX + b, XMAX, ep, x, err, spin);
-            t += x;
-        }
+#pragma unroll
+        for (int q = 0; q < XMAX / 32; ++q)
+            if (lane + 32 * q < G) t += x[q];
+        good = __all_sync(0xffffffffu, good);
         t = warp_sum<R>(t);
-        if (lane == 0) xcol[l] = t;
+        if (lane == 0 && good) st_value(xcol + (size_t)l * W, 1, t, ep);
+    }
+    for (int l = tid; l < ncol; l += ORTH_THREADS) {
+        R x = (R)0;
+        good = good && ld_value(xcol + (size_t)l * W, 1, ep, x, err, spin);
+        hs[l] = x;
     }
     if (!good) atomicExch(err, 1);
-    if (!__syncthreads_and(good)) return false;
-    float none[1] = {0.f}, sum[1];
-    if (!xchg_totals<float, 1, true>(xtot, ep, none, G, (float *)xs, (float *)bc, sum, err, spin)) return false;
-    for (int l = tid; l < ncol; l += ORTH_THREADS) hs[l] = __ldcg(xcol + l);
-    __syncthreads();
-    return true;
+    return __syncthreads_and(good);
+}
+
+// One item of cta_dots: CW columns from l0 over the rows [r0, r1).  P lanes go
+// along the rows and 32 / P side by side along the columns, so a lane holds
+// CW P / 32 sums; rows beyond a lane's would only add zeros, so the result is
+// bit for bit that of P = 32.
+template <class T, int CW, int P>
+__device__ __forceinline__ void dots_item(const T *__restrict__ V, int m, const T *__restrict__ w, int64_t n, int l0,
+                                          int64_t r0, int64_t r1, int ncol, T *red) {
+    constexpr int N = CW * P / 32;
+    const int lane = threadIdx.x & 31, rl = lane % P, lb = l0 + (lane / P) * N;
+    T acc[N];
+#pragma unroll
+    for (int c = 0; c < N; ++c) acc[c] = (T)0;
+    if (lb + N <= m) {
+        for (int64_t r = r0 + rl; r < r1; r += P) {
+            const T wv = w[r];
+            const T *vr = V + (int64_t)lb * n + r;
+#pragma unroll
+            for (int c = 0; c < N; ++c) acc[c] += vr[(int64_t)c * n] * wv;
+        }
+    } else {
+        for (int64_t r = r0 + rl; r < r1; r += P) {
+            const T wv = w[r];
+#pragma unroll
+            for (int c = 0; c < N; ++c) {
+                const int l = lb + c;
+                if (l < m) acc[c] += V[(int64_t)l * n + r] * wv;
+                else if (l < ncol) acc[c] += wv * wv;
+            }
+        }
+    }
+    const T s = multi_reduce<T, N, P>(acc, lane);
+    const int l = lb + rl * N / P;
+    if (rl % (P / N) == 0 && l < ncol) red[l] = s;
 }
 
 // CTA partials of h[l] = V[l] . w (l < m) over rows [i0, i1), plus w.w as
-// column m when `ww`; handed to store(l, sum).  Work
-// items are (CW-column group, row quarter); a lane runs down the rows of its
-// item accumulating CW columns in registers, then one multi_reduce.
+// column m when `ww`; handed to store(l, sum).  Work items are (CW-column
+// group, row quarter), a warp each.  A DADD on the whole warp holds an SM
+// quarter's FP64 pipe for 64 cycles whatever its lanes hold, so with a few
+// rows per quarter (12 per CTA at 1 800 states) the lanes go along the columns
+// instead, and the totals are exchanged in two hops (xchg_columns): a step that
+// projects at every iteration, 1 500 states, 30 columns: 31 -> 16 us, a chain of
+// 20 spins with 40 states kept 21.8 -> 17.6 ms.
 template <class T, int CW, class Store>
 __device__ __forceinline__ void cta_dots(const T *__restrict__ V, int m, const T *__restrict__ w, int64_t n,
                                          int64_t i0, int64_t i1, bool ww, T *red, Store store) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int warp = threadIdx.x >> 5;
     const int ncol = m + (ww ? 1 : 0);
     const int ng = (ncol + CW - 1) / CW;
     const int nq = ng >= ORTH_WARPS ? 1 : ORTH_WARPS / ng;
     const int rs = ng * CW;
-    const int64_t len = i1 - i0, qlen = (len + nq - 1) / nq;
-    for (int item = warp; item < ng * nq; item += ORTH_WARPS) {
-        const int g = item % ng, q = item / ng, l0 = g * CW;
+    const unsigned len = (unsigned)(i1 - i0), qlen = (len + nq - 1) / nq;   // a CTA's rows: 32-bit divisions
+    const int nqe = qlen > 0 ? (int)((len + qlen - 1) / qlen) : 1;          // quarters with rows
+    for (int item = warp; item < ng * nqe; item += ORTH_WARPS) {
+        const int g = item % ng, q = item / ng;
         const int64_t r0 = i0 + (int64_t)q * qlen, r1 = min(i1, r0 + qlen);
-        T acc[CW];
-#pragma unroll
-        for (int c = 0; c < CW; ++c) acc[c] = (T)0;
-        if (l0 + CW <= m) {
-            for (int64_t r = r0 + lane; r < r1; r += 32) {
-                const T wv = w[r];
-                const T *vr = V + (int64_t)l0 * n + r;
-#pragma unroll
-                for (int c = 0; c < CW; ++c) acc[c] += vr[(int64_t)c * n] * wv;
-            }
-        } else {
-            for (int64_t r = r0 + lane; r < r1; r += 32) {
-                const T wv = w[r];
-#pragma unroll
-                for (int c = 0; c < CW; ++c) {
-                    const int l = l0 + c;
-                    if (l < m) acc[c] += V[(int64_t)l * n + r] * wv;
-                    else if (ww && l == m) acc[c] += wv * wv;
-                }
-            }
-        }
-        const T s = multi_reduce<T, CW>(acc, lane);
-        if (lane < CW && l0 + lane < ncol) red[q * rs + l0 + lane] = s;
+        T *rq = red + q * rs;
+        if (qlen > 16) dots_item<T, CW, 32>(V, m, w, n, g * CW, r0, r1, ncol, rq);
+        else if (qlen > 4) dots_item<T, CW, 16>(V, m, w, n, g * CW, r0, r1, ncol, rq);
+        else dots_item<T, CW, 4>(V, m, w, n, g * CW, r0, r1, ncol, rq);
     }
     __syncthreads();
     for (int l = threadIdx.x; l < ncol; l += ORTH_THREADS) {
         T s = (T)0;
-        for (int q = 0; q < nq; ++q) s += red[q * rs + l];
+        for (int q = 0; q < nqe; ++q) s += red[q * rs + l];
         store(l, s);
     }
 }
@@ -886,7 +931,12 @@ __device__ __forceinline__ bool pro_always(int m, int64_t n) {
 template <class T, int CW>
 __global__ void __launch_bounds__(ORTH_THREADS, 1) k_orth(OrthArgs a) {
     int *flags = a.flags;
-    if (*(volatile int *)&flags[F_STOP]) return;     // set before this launch: uniform
+    // the launch's state, loads issued together
+    const int stop = *(volatile int *)&flags[F_STOP];
+    const int j = a.jdev ? *(volatile const int *)a.jdev : a.j, m = j + 1;
+    unsigned ep = *(volatile unsigned *)a.xep;       // advanced when the launch ends
+    int force = __ldcg((const int *)(a.pro + 2 * a.pstride));
+    if (stop) return;                                // set before this launch: uniform
     extern __shared__ __align__(16) unsigned char osm_raw[];
     T *osm = (T *)osm_raw;
     const int ps = a.pstride;
@@ -902,11 +952,9 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_orth(OrthArgs a) {
     const int64_t i0 = min(n, (int64_t)blk * chunk), i1 = min(n, i0 + chunk);
     const int nw = (int)min((int64_t)ORTH_WARPS, max((int64_t)1, (chunk + 31) / 32));   // warps with rows
     T *V = (T *)a.V, *w = (T *)a.w;
-    const int j = a.jdev ? *(volatile const int *)a.jdev : a.j, m = j + 1;
     const T *vj = V + (int64_t)j * n;
     const T *vjm = V + (int64_t)(j > 0 ? j - 1 : 0) * n;
     int *err = flags + F_ERR;
-    unsigned ep = *(volatile unsigned *)a.xep;       // advanced when the launch ends
     constexpr int W = XW<T>::words;
     auto column = [&](int l, T t) { st_value(a.xpart + (size_t)l * W * XMAX + blk, XMAX, t, ep + 1); };
     // leaving: the next launch's epochs follow this one's.  A wait that ran out
@@ -946,7 +994,6 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_orth(OrthArgs a) {
     }
     const T beta_m = j > 0 ? (T)__ldcg(a.beta + j - 1) : (T)0;
     if (!pro_always<T>(m, n)) pro.load(a.pro, ps, a.alpha, a.beta, j);
-    int force = __ldcg((const int *)(a.pro + 2 * ps));
     // no exchange here needs a fence: every CTA works on its own rows, and only
     // the values and the last CTA's stop request travel
     T tot[PA_COLS];
@@ -954,14 +1001,14 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_orth(OrthArgs a) {
     if constexpr (sizeof(T) == 4) {
         if (anc) {
             block_sums<T, PA_COLS>(av, scr, nw);
-            ok = xchg_totals<T, PA_COLS, false>(a.xtot, ep, av, G, xs, bc, tot, err, a.spin, &host_stop);
+            ok = xchg_totals<T, PA_COLS>(a.xtot, ep, av, G, xs, bc, tot, err, a.spin, &host_stop);
             if (blk == 0 && tid == 0) a.h_m[j] = (double)tot[2];
         }
     }
     if (!anc) {
         T a1[1] = {av[0]}, t1[1];
         block_sums<T, 1>(a1, scr, nw);
-        ok = xchg_totals<T, 1, false>(a.xtot, ep, a1, G, xs, bc, t1, err, a.spin, &host_stop);
+        ok = xchg_totals<T, 1>(a.xtot, ep, a1, G, xs, bc, t1, err, a.spin, &host_stop);
 #pragma unroll
         for (int q = 0; q < PA_COLS; ++q) tot[q] = (T)0;
         tot[0] = t1[0];
@@ -1003,14 +1050,14 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_orth(OrthArgs a) {
         if constexpr (sizeof(T) == 4) {
             if (anc) {
                 block_sums<T, 1 + ANC_MAX>(ew, scr, nw);
-                ok = xchg_totals<T, 1 + ANC_MAX, false>(a.xtot, ep, ew, G, xs, bc, ew, err, a.spin);
+                ok = xchg_totals<T, 1 + ANC_MAX>(a.xtot, ep, ew, G, xs, bc, ew, err, a.spin);
                 bb[0] = ew[0];
             }
         }
         if (!anc) {
             T s1[1] = {ew[0]};
             block_sums<T, 1>(s1, scr, nw);
-            ok = xchg_totals<T, 1, false>(a.xtot, ep, s1, G, xs, bc + 8, bb, err, a.spin);
+            ok = xchg_totals<T, 1>(a.xtot, ep, s1, G, xs, bc + 8, bb, err, a.spin);
         }
         if (!ok) { leave(true); return; }
     }
@@ -1035,7 +1082,7 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_orth(OrthArgs a) {
         T ww = (T)0;
         for (int pass = 0; pass < 2; ++pass) {       // a second time when the first took more than half (same in every CTA)
             cta_dots<T, CW>(V, m, w, n, i0, i1, pass == 0, red, column);
-            if (!xchg_columns<T>(a.xpart, (T *)a.xcol, a.xtot, ep, G, pass == 0 ? m + 1 : m, hs, xs, bc + 8, err, a.spin)) {
+            if (!xchg_columns<T>(a.xpart, a.xcol, ep, G, pass == 0 ? m + 1 : m, hs, err, a.spin)) {
                 leave(true);
                 return;
             }
@@ -1043,7 +1090,7 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_orth(OrthArgs a) {
             hj += hs[j];
             T s1[1] = {cta_update<T>(V, m, w, n, i0, i1, hs)};
             block_sums<T, 1>(s1, scr, nw);
-            if (!xchg_totals<T, 1, false>(a.xtot, ep, s1, G, xs, bc + 9 + pass, bb, err, a.spin)) { leave(true); return; }
+            if (!xchg_totals<T, 1>(a.xtot, ep, s1, G, xs, bc + 9 + pass, bb, err, a.spin)) { leave(true); return; }
             if (!(bb[0] < (T)0.5 * ww)) break;
         }
     }
@@ -1098,8 +1145,8 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_orth(OrthArgs a) {
                 flags[F_STOP] = 2;
                 a.h_flags[F_BREAK] = m;
                 a.h_flags[F_STOP] = 2;
+                __threadfence_system();
             }
-            __threadfence_system();
         }
     }
     leave(false);
