@@ -260,10 +260,17 @@ namespace nss {
 //   HV_LEFT   H_L W                               -> slot 1
 //   HV_RIGHT  W H_R^T                             -> slot 2
 //   HV_TERMS  A x B terms                         -> slot 0
-// Sectors whose tiles have long K loops (Dl or Dr > 64) are split into the
+// Sectors whose tiles have long K loops (Dl or Dr > HV_SPLIT) are split into the
 // last three so the parts run on different SMs; the result is slot 0 +
 // slot 1 + slot 2 (regions of slots 1 and 2 that no item writes stay zero).
+// An iteration lasts as long as its longest item, and a superblock has fewer
+// items than the 304 groups of the grid; but a part costs a load round of its
+// own, which a batch of solves, with more items than groups, pays: solves of
+// 16 900 states (54 x 54 sectors) 1.99 -> 1.92 ms and of 66 600 2.30 -> 2.28 ms
+// from 64 to 48; 32 is no better there and costs a batch of 16 3 %, a solve of
+// 66 600 20 % (more items than groups).
 enum { HV_FULL = 0, HV_LEFT = 1, HV_RIGHT = 2, HV_TERMS = 3 };
+constexpr int HV_SPLIT = 48;
 constexpr int HV_KMAX = 128;            // K extent staged at once
 constexpr int SA_LD = HV_KMAX + 4;      // A rows: float4 reads along K
 constexpr int SB_LD = 34;               // B rows: float2 reads along the columns

@@ -1305,7 +1305,10 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_chunk32(ChunkArgs a) {
         float ap[1 + NA];
 #pragma unroll
         for (int q = 0; q < 1 + NA; ++q) ap[q] = 0.f;
-        for (int ti = 2 * blk + grp; ti < a.nitems; ti += 2 * G)
+        // longest items first, one to every CTA before a second joins it (two
+        // neighbours of the order per CTA: 1.90 against 1.67 ms at 15 200
+        // states, 22 CTAs busy with 44 items)
+        for (int ti = blk + grp * G; ti < a.nitems; ti += 2 * G)
             hv32_item<NA>(a.items[ti], x, a.slot, a.op, ism[grp], lt, GroupSync{1 + grp}, sc, ac, ap);
         block_sums<float, 1 + NA>(ap, scr);
         if (tid == 0)

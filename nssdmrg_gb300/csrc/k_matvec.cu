@@ -496,7 +496,7 @@ int sb_upload(Ctx &c, const nss_sb_desc *d, bool trusted) {
     // split into H_L, H_R and A x B parts when a K loop is long
     std::vector<int4> items32;
     for (int k = 0; k < s.nsb; ++k) {
-        const bool split = std::max(s.dls[k], s.drs[k]) > 64;
+        const bool split = std::max(s.dls[k], s.drs[k]) > HV_SPLIT;
         for (int r = 0; r < s.dls[k]; r += TILE32)
             for (int cc = 0; cc < s.drs[k]; cc += TILE32) {
                 if (split) {
