@@ -863,28 +863,34 @@ __device__ __forceinline__ T cta_update(const T *__restrict__ V, int m, T *__res
 template <class T>
 struct OrthCW { static constexpr int value = sizeof(T) == 4 ? 32 : 16; };
 
+// also the exchanged values of a CTA (xchg_totals), up to PA_COLS + 1 of XMAX CTAs
 __host__ __device__ inline int orth_redsz(int pstride, int cw) {
-    return ORTH_WARPS * cw > pstride + cw ? ORTH_WARPS * cw : pstride + cw;
+    const int dots = ORTH_WARPS * cw > pstride + cw ? ORTH_WARPS * cw : pstride + cw;
+    return dots > (PA_COLS + 1) * XMAX ? dots : (PA_COLS + 1) * XMAX;
 }
+
+// A Krylov basis of more columns than this leaves no room for the recurrence:
+// its solve projects at every step
+constexpr int PRO_MAX_PS = 4096;
 
 // floats of the omega recurrence in shared memory: estimates of v_j, v_{j-1},
 // v_{j+1}, alpha, beta
-__host__ __device__ inline size_t pro_floats(int pstride) { return 5 * (size_t)((pstride + 3) & ~3); }
+__host__ __device__ inline size_t pro_floats(int pstride) {
+    return pstride <= PRO_MAX_PS ? 5 * (size_t)((pstride + 3) & ~3) : 0;
+}
 
 // shared memory of the orthogonalisation in bytes: hs, red, scratch (T), the
-// recurrence; k_orth has the exchanged values of a CTA after it
+// recurrence
 __host__ __device__ inline size_t orth_smem(int pstride, int cw, size_t tsize) {
     const size_t t = (size_t)(pstride + orth_redsz(pstride, cw) + 8 * ORTH_WARPS + 16) * tsize;
     return ((t + 15) & ~(size_t)15) + pro_floats(pstride) * sizeof(float);
-}
-__host__ __device__ inline size_t orth_smem_x(int pstride, int cw, size_t tsize) {
-    return orth_smem(pstride, cw, tsize) + XCOLS * XMAX * sizeof(float);
 }
 
 // The recurrence's shared arrays
 struct ProSmem {
     float *so, *sp, *sn, *sa, *sb;
-    __device__ ProSmem(void *base, int ps) {
+    const bool on;
+    __device__ ProSmem(void *base, int ps) : on(ps <= PRO_MAX_PS) {
         const int st = (ps + 3) & ~3;
         so = (float *)base;
         sp = so + st;
@@ -894,12 +900,28 @@ struct ProSmem {
     }
     // state of step j from global memory (estimates, alpha_k, beta_k, k < j)
     __device__ __forceinline__ void load(const float *pro, int ps, const double *alpha, const double *beta, int j) {
-        for (int k = threadIdx.x; k < j; k += blockDim.x) {
+        for (int k = threadIdx.x; on && k < j; k += blockDim.x) {
             so[k] = __ldcg(pro + k);
             sp[k] = __ldcg(pro + ps + k);
             sa[k] = (float)__ldcg(alpha + k);
             sb[k] = (float)__ldcg(beta + k);
         }
+    }
+    // (one thread) alpha_j, beta_j
+    __device__ __forceinline__ void set(int j, float alpha, float beta) {
+        if (!on) return;
+        sa[j] = alpha;
+        sb[j] = beta;
+    }
+    // does v_{j+1} lose more than `limit`?
+    template <class T>
+    __device__ __forceinline__ bool over(int j, float limit = (float)Pro<T>::DELTA) {
+        return on ? pro_step<T>(so, sp, sa, sb, sn, j, limit) : true;
+    }
+    // step j projects
+    template <class T>
+    __device__ __forceinline__ void projected(int j) {
+        for (int k = threadIdx.x; on && k <= j; k += blockDim.x) sn[k] = (float)Pro<T>::EPS1;
     }
     // after step j: the new estimates become v_{j+1}'s
     __device__ __forceinline__ void advance() {
@@ -909,7 +931,7 @@ struct ProSmem {
         sn = t;
     }
     __device__ __forceinline__ void store(float *pro, int ps, int j, int force) const {
-        for (int k = threadIdx.x; k <= j; k += blockDim.x) {
+        for (int k = threadIdx.x; on && k <= j; k += blockDim.x) {
             pro[k] = so[k];
             pro[ps + k] = sp[k];
         }
@@ -924,8 +946,8 @@ struct ProSmem {
 // exhausting it the estimates' model no longer holds.
 constexpr int64_t PRO_MIN_N = 3072;
 template <class T>
-__device__ __forceinline__ bool pro_always(int m, int64_t n) {
-    return sizeof(T) == 8 ? n < PRO_MIN_N : 8 * (int64_t)m > n;
+__device__ __forceinline__ bool pro_always(int m, int64_t n, int ps) {
+    return ps > PRO_MAX_PS || (sizeof(T) == 8 ? n < PRO_MIN_N : 8 * (int64_t)m > n);
 }
 
 template <class T, int CW>
@@ -944,7 +966,7 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_orth(OrthArgs a) {
     T *red = hs + ps;
     T *scr = red + orth_redsz(ps, CW);               // [8 x 16] block sums, then [16] broadcasts
     T *bc = scr + 8 * ORTH_WARPS;
-    T *xs = (T *)(osm_raw + orth_smem(ps, CW, sizeof(T)));
+    T *xs = red;                                     // between two uses of red
     ProSmem pro(osm_raw + (orth_smem(ps, CW, sizeof(T)) - pro_floats(ps) * sizeof(float)), ps);
     const int G = gridDim.x, blk = blockIdx.x, tid = threadIdx.x;
     const int64_t n = a.n;
@@ -993,7 +1015,7 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_orth(OrthArgs a) {
         }
     }
     const T beta_m = j > 0 ? (T)__ldcg(a.beta + j - 1) : (T)0;
-    if (!pro_always<T>(m, n)) pro.load(a.pro, ps, a.alpha, a.beta, j);
+    if (!pro_always<T>(m, n, ps)) pro.load(a.pro, ps, a.alpha, a.beta, j);
     // no exchange here needs a fence: every CTA works on its own rows, and only
     // the values and the last CTA's stop request travel
     T tot[PA_COLS];
@@ -1020,7 +1042,7 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_orth(OrthArgs a) {
         return;
     }
     const T alpha0 = tot[0];
-    const bool always = pro_always<T>(m, n);
+    const bool always = pro_always<T>(m, n, ps);
     // three-term step (and the anchor projections); ww = w.w, and what is left
     // of w along u and y_k, taken off when w is normalised: alpha v_j and
     // beta v_{j-1} bring back alpha and beta times the rounding-level products
@@ -1064,16 +1086,13 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_orth(OrthArgs a) {
     if (!always) {
         // does this step project?  (same decision in every CTA; beta in FP32
         // is enough for the estimates)
-        if (tid == 0) {
-            pro.sa[j] = (float)alpha0;
-            pro.sb[j] = sqrtf((float)bb[0]);
-        }
+        if (tid == 0) pro.set(j, (float)alpha0, sqrtf((float)bb[0]));
         __syncthreads();
-        const bool over = pro_step<T>(pro.so, pro.sp, pro.sa, pro.sb, pro.sn, j);
+        const bool over = pro.template over<T>(j);
         project = over || force;
         if (project) {
             force = over && !force;
-            for (int k = tid; k <= j; k += ORTH_THREADS) pro.sn[k] = Pro<T>::EPS1;
+            pro.template projected<T>(j);
         }
     }
     T hj = (T)0;
@@ -1389,17 +1408,14 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_chunk32(ChunkArgs a) {
         }
         float bb = sv[0];
         const float mj = sv[1];
-        if (tid == 0) {
-            pro.sa[jj] = alpha0;
-            pro.sb[jj] = sqrtf(bb);
-        }
+        if (tid == 0) pro.set(jj, alpha0, sqrtf(bb));
         __syncthreads();
         // does this step project?  (same decision in every CTA)
-        const bool over = pro_step<float>(pro.so, pro.sp, pro.sa, pro.sb, pro.sn, jj);
+        const bool over = pro.over<float>(jj);
         float hj = 0.f;
-        if (over || force || pro_always<float>(m, n)) {
+        if (over || force || pro_always<float>(m, n, ps)) {
             force = over && !force;
-            for (int k = tid; k <= jj; k += ORTH_THREADS) pro.sn[k] = Pro<float>::EPS1;
+            pro.projected<float>(jj);
             // w -= V h
             auto update = [&]() -> float {
                 float ss = 0.f;
@@ -1454,10 +1470,7 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_chunk32(ChunkArgs a) {
             rec_b[done] = beta_j;
             rec_m[done] = mj;
         }
-        if (tid == 0) {
-            pro.sa[jj] = alpha_j;
-            pro.sb[jj] = beta_j;
-        }
+        if (tid == 0) pro.set(jj, alpha_j, beta_j);
         pro.advance();
         if constexpr (ANC) {
 #pragma unroll
@@ -1669,7 +1682,7 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_batch32(BatchArgs B) {
             balpha[s] = __ldcg(B.st + 4 * s + 0);
             const int ow = step == 0 ? __ldcg((const int *)(S.c.o.pro + 2 * S.c.o.pstride)) : __float_as_int(__ldcg(B.st + 4 * s + 3));
             p2[s] = 1;
-            if (ow > 0 || pro_always<float>(S.c.j0 + step + 1, S.c.o.n)) any_p2 = 1;
+            if (ow > 0 || pro_always<float>(S.c.j0 + step + 1, S.c.o.n, S.c.o.pstride)) any_p2 = 1;
         }
         __syncthreads();
         auto update = [&]() -> float {
@@ -1688,14 +1701,11 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_batch32(BatchArgs B) {
             grid_totals<float, 2>(pW + Gs, Gs, bc + 2, t2);
             mj = t2[0];
             ud = t2[1];
-            if (tid == 0) {
-                pro.sa[jj] = alpha0;
-                pro.sb[jj] = sqrtf(bbb[me]);
-            }
+            if (tid == 0) pro.set(jj, alpha0, sqrtf(bbb[me]));
             __syncthreads();
-            const bool over = pro_step<float>(pro.so, pro.sp, pro.sa, pro.sb, pro.sn, jj, 0.25f * Pro<float>::DELTA);
+            const bool over = pro.over<float>(jj, 0.25f * Pro<float>::DELTA);
             if (any_p2) {
-                for (int k = tid; k <= jj; k += ORTH_THREADS) pro.sn[k] = Pro<float>::EPS1;
+                pro.projected<float>(jj);
                 if (owed > 0) --owed;
             } else if (over) {
                 owed = 2;
@@ -1763,10 +1773,7 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_batch32(BatchArgs B) {
                 rec_m[done] = mj;
                 B.st[4 * me + 3] = __int_as_float(owed);   // read by all after the next step's barriers
             }
-            if (tid == 0) {
-                pro.sa[jj] = balpha[me];
-                pro.sb[jj] = bprev[me];
-            }
+            if (tid == 0) pro.set(jj, balpha[me], bprev[me]);
             dm = dc;
             dc = anc ? ud / bprev[me] : 0.f;
             pro.advance();
@@ -2068,7 +2075,7 @@ int ensure_lanczos(Ctx &c, int64_t n, int cap, bool mixed) {
     NSS_CUDA_TRY(c, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     const int pstride = cap + 8;   // m+1 columns plus the anchored refinement's extras
     const int cw = mixed ? OrthCW<float>::value : OrthCW<double>::value;
-    const size_t smem = orth_smem_x(pstride, cw, mixed ? sizeof(float) : sizeof(double));
+    const size_t smem = orth_smem(pstride, cw, mixed ? sizeof(float) : sizeof(double));
     const void *fn = mixed ? (const void *)k_orth<float, OrthCW<float>::value>
                            : (const void *)k_orth<double, OrthCW<double>::value>;
     NSS_CUDA_TRY(c, allow_smem(fn, smem));
