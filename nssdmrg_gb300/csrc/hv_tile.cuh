@@ -272,8 +272,9 @@ namespace nss {
 enum { HV_FULL = 0, HV_LEFT = 1, HV_RIGHT = 2, HV_TERMS = 3 };
 constexpr int HV_SPLIT = 48;
 constexpr int HV_KMAX = 128;            // K extent staged at once
-constexpr int SA_LD = HV_KMAX + 4;      // A rows: float4 reads along K
-constexpr int SB_LD = 34;               // B rows: float2 reads along the columns
+constexpr int SA_LD = HV_KMAX + 4;      // rows along K: float4 reads, eight rows apart in different banks
+constexpr int SB_FULL = 64 * 32;        // a FULL item's second B operand in sb, rows SB_LD apart
+constexpr int SB_LD = 64 + 4;
 
 // A work item with everything it needs to start its operand loads, so that
 // these depend on one load only: (sector, row0, col0, part), (Dl, Dr, first
@@ -286,75 +287,81 @@ struct ItemRec {
 __device__ __forceinline__ int64_t lohi(int lo, int hi) { return (int64_t)(unsigned)lo | ((int64_t)hi << 32); }
 
 struct __align__(16) Item32Smem {
-    float sa[32][SA_LD];                // A rows x K
-    float sb[HV_KMAX][SB_LD];           // K x B columns
-    AbStage<float, 32, 32> S;
+    float sa[32 * SA_LD];               // A: rows x K
+    float sb[32 * SA_LD];               // B: K x columns (H_L W) or columns x K (W H_R^T)
+                                        // (W's part of both: then the tile's four K shares)
+    union {
+        struct {
+            int2 ta[AB_MAXT][32], tb[AB_MAXT][32];   // (column, value) of A's rows, B's columns (col_pos)
+            int4 hd[AB_MAXT];
+        };
+        AbStage<float, 32, 32> S;       // rows of several elements
+    };
 };
 
-// K loop over staged operands: sa[r][k0..k0+kn4) x sb[k0..k0+kn4)[cols]
-__device__ __forceinline__ void item_mma(const Item32Smem &sm, int k0, int kn4, int ty, int tx, float (&acc)[2][2]) {
-#pragma unroll 2
-    for (int j = k0; j < k0 + kn4; j += 4) {
-        const float4 a0 = *reinterpret_cast<const float4 *>(&sm.sa[ty][j]);
-        const float4 a1 = *reinterpret_cast<const float4 *>(&sm.sa[ty + 16][j]);
-        const float av0[4] = {a0.x, a0.y, a0.z, a0.w}, av1[4] = {a1.x, a1.y, a1.z, a1.w};
+// A thread's columns are eight apart; stored side by side it reads them as one vector
+__device__ __forceinline__ int col_pos(int x) { return 4 * (x & 7) + (x >> 3); }
+
+// Asynchronous copies into shared memory (zero when !in; the address is then not read)
+template <int BYTES>
+__device__ __forceinline__ void cp_async(void *dst, const void *src, bool in) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
+                 "n"(BYTES), "r"(in ? BYTES : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// dst[r * LD + c] = src[r * ld + c], r < 32, c < kn4: zero from `rows` and `kn` on
+__device__ __forceinline__ void stage_rows(float *dst, int LD, const float *src, int64_t ld, int rows, int kn, int kn4,
+                                           int lt) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int r = (lt >> 5) + 8 * q;
+        const float *p = r < rows ? src + r * ld : src;
+        for (int c = lt & 31; c < kn4; c += 32) {
+            const bool in = r < rows && c < kn;
+            cp_async<4>(dst + r * LD + c, in ? p + c : src, in);
+        }
+    }
+}
+// dst[k * 32 + col_pos(x)] = src[k * ld + x], x < 32, k < kn4: zero from `cols` and `kn` on
+__device__ __forceinline__ void stage_cols(float *dst, const float *src, int64_t ld, int cols, int kn, int kn4, int lt) {
+    const int x = lt & 31;
+    for (int k = lt >> 5; k < kn4; k += 8) {
+        const bool in = k < kn && x < cols;
+        cp_async<4>(dst + k * 32 + col_pos(x), in ? src + k * ld + x : src, in);
+    }
+}
+
+// acc[i][j] += A[4 ty + i][k] B[k][tx + 8 j] over the K steps of four s, s + 4,
+// ... < n4; ROWS: B is stored as columns x K
+template <bool ROWS>
+__device__ __forceinline__ void item_mma(const float *sa, const float *sb, int ldb, int s, int n4, int ty, int tx,
+                                         float (&acc)[4][4]) {
+    for (; s < n4; s += 4) {
+        const int k = 4 * s;
+        float a[4][4], b[4][4];                      // [row][k], [k][column]
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float4 t = *reinterpret_cast<const float4 *>(sa + (4 * ty + i) * SA_LD + k);
+            a[i][0] = t.x; a[i][1] = t.y; a[i][2] = t.z; a[i][3] = t.w;
+        }
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            const float2 b = *reinterpret_cast<const float2 *>(&sm.sb[j + q][2 * tx]);
-            acc[0][0] = fmaf(av0[q], b.x, acc[0][0]);
-            acc[0][1] = fmaf(av0[q], b.y, acc[0][1]);
-            acc[1][0] = fmaf(av1[q], b.x, acc[1][0]);
-            acc[1][1] = fmaf(av1[q], b.y, acc[1][1]);
-        }
-    }
-}
-
-// Staged operands of one phase into columns [k0, k0 + ext) of sa / rows of
-// sb: A[r][c] and B[c][x] of H_L W (ph 0) or W H_R^T (ph 1), K range
-// [kb, kb + kn), zero beyond kn; EXT (64 or 128) is the staged extent, so a
-// thread loads EXT/8 elements per operand, all in flight before the stores.
-template <int EXT>
-__device__ __forceinline__ void item_load(int ph, const float *__restrict__ H, const float *__restrict__ W, int dl,
-                                          int dr, int row0, int col0, int kb, int kn, int lt, float *ra, float *rb) {
-    constexpr int PER = 32 * EXT / 256;
-    constexpr int SH = EXT == 64 ? 6 : 7;
+            const float4 t = *reinterpret_cast<const float4 *>(ROWS ? sb + (tx + 8 * q) * ldb + k : sb + (k + q) * 32 + 4 * tx);
+            const float u[4] = {t.x, t.y, t.z, t.w};
 #pragma unroll
-    for (int q = 0; q < PER; ++q) {
-        const int e = lt + q * 256;
-        const int r = e >> SH, c = e & (EXT - 1);
-        const int gi = row0 + r;
-        float x = 0.f;
-        if (gi < dl && c < kn) x = ph == 0 ? H[(int64_t)gi * dl + kb + c] : W[(int64_t)gi * dr + kb + c];
-        ra[q] = x;
-        float y = 0.f;
-        if (ph == 0) {
-            const int c2 = e >> 5, xx = e & 31, gc = col0 + xx;
-            if (gc < dr && c2 < kn) y = W[(int64_t)(kb + c2) * dr + gc];
-        } else {
-            const int xx = e >> SH, gr = col0 + xx;
-            if (gr < dr && c < kn) y = H[(int64_t)gr * dr + kb + c];
+            for (int j = 0; j < 4; ++j) {
+                if (ROWS) b[j][q] = u[j];
+                else b[q][j] = u[j];
+            }
         }
-        rb[q] = y;
-    }
-}
-
-template <int EXT>
-__device__ __forceinline__ void item_store(Item32Smem &sm, int ph, int k0, int kn4, int lt, const float *ra,
-                                           const float *rb) {
-    constexpr int PER = 32 * EXT / 256;
-    constexpr int SH = EXT == 64 ? 6 : 7;
 #pragma unroll
-    for (int q = 0; q < PER; ++q) {
-        const int e = lt + q * 256;
-        const int r = e >> SH, c = e & (EXT - 1);
-        if (c < kn4) sm.sa[r][k0 + c] = ra[q];
-        if (ph == 0) {
-            const int c2 = e >> 5, xx = e & 31;
-            if (c2 < kn4) sm.sb[k0 + c2][xx] = rb[q];
-        } else {
-            const int xx = e >> SH;
-            if (c < kn4) sm.sb[k0 + c][xx] = rb[q];
-        }
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i][q], b[q][j], acc[i][j]);
     }
 }
 
@@ -367,161 +374,213 @@ struct AncCols {
 };
 constexpr int ANC_MAX = 5;              // u and up to four y
 
-// One item by 256 threads (lt = thread index in the group): each thread owns
-// rows {ty, ty+16} x columns {2tx, 2tx+1}, so a K step of four costs two
-// float4 and four float2 shared-memory reads for sixteen FMAs.  The staged
-// operands are loaded with every load of a thread in flight before its
-// stores: a FULL item (both K <= 64) stages both products in one round (H_L
-// part in columns 0..63, H_R part in 64..127), a LEFT / RIGHT item its K
-// range (<= HV_KMAX) in one round per 128.  The A x B tables (and the
-// per-term offsets) are read in the same round.  The outputs times `scale`
-// go to the item's slot; this thread's share of sum_i (v[i] scale)
-// (out[i] scale) over its outputs is added to p[0], those of u.out and
-// y_k.out to p[1..NA].
+// One item by 256 threads (lt = thread index in the group).  An iteration of
+// the persistent kernel waits for its slowest item, and a group has one item
+// as a rule, so what counts is an item's latency: operands, A x B tables and
+// the outputs' own W go out in one round of asynchronous copies; the gathers
+// of the first four terms are in flight during the products.  In the products
+// a thread holds 4 x 4 outputs for every fourth K step of four (eight floats
+// read from shared memory for sixteen FMAs; at 2 x 2 outputs shared memory's
+// 128 B a clock took 130 clk a step); the four shares are added in shared
+// memory, after which a thread owns row r, columns {cx, cx + 8, cx + 16,
+// cx + 24}.  keep: this group's last item was the same one, so the tiles of
+// H_L and H_R and the tables are still in shared memory.  An item of 39 x 40 states and
+// three terms 9.7k -> 6.2k clk, a part of K = 106 13.4k -> 6.5k; an iteration of
+// 66 600 states 14.2 -> 9.3 us, solves of it 2.36 -> 1.87 ms, of 16 900 states
+// 1.92 -> 1.56 ms.  The staging (2.2k to 2.8k) is the L2's latency: plain loads
+// through registers took as long.
+// The outputs times `scale` go to the item's slot; this thread's share of
+// sum_i (v[i] scale) (out[i] scale) over its outputs is added to p[0], those
+// of u.out and y_k.out to p[1..NA].
 template <int NA, class Sync>
 __device__ __forceinline__ void hv32_item(const ItemRec &it, const float *__restrict__ v, float *const *slots,
                                           const Hv32Ops &op, Item32Smem &sm, int lt, Sync sync, float scale,
-                                          const AncCols &ac, float (&p)[1 + NA]) {
+                                          const AncCols &ac, float (&p)[1 + NA], bool keep) {
     const int row0 = it.a.y, col0 = it.a.z, part = it.a.w;
     const int dl = it.b.x, dr = it.b.y, t0 = it.b.z, t1 = it.b.w;
     const int64_t o = lohi(it.c.x, it.c.y);
     const float *W = v + o;
-    const float *HLk = op.hl + lohi(it.d.x, it.d.y), *HRk = op.hr + lohi(it.d.z, it.d.w);
-    const int ty = lt / 16, tx = lt % 16;
-    float acc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+    const float *HL = op.hl + lohi(it.d.x, it.d.y) + (int64_t)row0 * dl;
+    const float *HR = op.hr + lohi(it.d.z, it.d.w) + (int64_t)col0 * dr;
+    const float *Wr = W + (int64_t)row0 * dr;
+    const int rows = dl - row0, cols = dr - col0;
+    const int r = lt >> 3, cx = lt & 7;
     const bool terms = part == HV_FULL || part == HV_TERMS;
     const int eo = terms ? it.c.z : -1;
-    constexpr int NE = AB_MAXT * 64 / 256;
-    int2 ee[NE];
-    int4 hd = make_int4(0, 0, 0, 0);
     const int nt0 = min(AB_MAXT, t1 - t0);
-    // first batch of the A x B table, issued with the operand loads
-    auto ell_load = [&](int tb, int nt) {
+    auto stage_terms = [&](int tb, int nt) {
         const int2 *src = op.ell + eo + (int64_t)(tb - t0) * 64;
-#pragma unroll
-        for (int q = 0; q < NE; ++q) {
-            const int e = lt + q * 256;
-            ee[q] = e < nt * 64 ? src[e] : make_int2(-1, 0);
+        for (int e = lt; e < nt * 64; e += 256) {
+            const int tt = e >> 6, x = e & 63;
+            cp_async<8>(x < 32 ? &sm.ta[tt][x] : &sm.tb[tt][col_pos(x - 32)], src + e, true);
         }
-        if (lt < nt) hd = op.term_hdr[tb + lt];
+        if (lt < nt) cp_async<16>(&sm.hd[lt], op.term_hdr + tb + lt, true);
     };
-    if (eo >= 0 && nt0 > 0) ell_load(t0, nt0);
+    // K range [kb, kb + kn) of a LEFT or RIGHT item; kh: H is there already
+    auto stage_part = [&](int kb, int kn, bool kh) {
+        const int kn4 = (kn + 3) & ~3;
+        if (part == HV_LEFT) {
+            if (!kh) stage_rows(sm.sa, SA_LD, HL + kb, dl, rows, kn, kn4, lt);
+            stage_cols(sm.sb, W + (int64_t)kb * dr + col0, dr, cols, kn, kn4, lt);
+        } else {
+            stage_rows(sm.sa, SA_LD, Wr + kb, dr, rows, kn, kn4, lt);
+            if (!kh) stage_rows(sm.sb, SA_LD, HR + kb, dr, cols, kn, kn4, lt);
+        }
+    };
+    const int K = part == HV_LEFT ? dl : dr;
+    if (!keep) sync();                               // the last item's reads are done
     if (part == HV_FULL) {
-        float ra[8], rb[8];
-        item_load<64>(0, HLk, W, dl, dr, row0, col0, 0, dl, lt, ra, rb);
-        float rc[8], rd[8];
-        item_load<64>(1, HRk, W, dl, dr, row0, col0, 0, dr, lt, rc, rd);
         const int kl4 = (dl + 3) & ~3, kr4 = (dr + 3) & ~3;
-        item_store<64>(sm, 0, 0, kl4, lt, ra, rb);
-        item_store<64>(sm, 1, 64, kr4, lt, rc, rd);
+        if (!keep) {
+            stage_rows(sm.sa, SA_LD, HL, dl, rows, dl, kl4, lt);
+            stage_rows(sm.sb + SB_FULL, SB_LD, HR, dr, cols, dr, kr4, lt);
+        }
+        stage_cols(sm.sb, W + col0, dr, cols, dl, kl4, lt);
+        stage_rows(sm.sa + 64, SA_LD, Wr, dr, rows, dr, kr4, lt);
+    } else if (part != HV_TERMS) {
+        stage_part(0, min(HV_KMAX, K), keep && K <= HV_KMAX);
+    }
+    if (eo >= 0 && nt0 > 0 && !(keep && t1 - t0 <= AB_MAXT)) stage_terms(t0, nt0);
+    float wv[4], uv[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const bool in = r < rows && cx + 8 * j < cols;
+        const int64_t at = (int64_t)r * dr + col0 + cx + 8 * j;
+        wv[j] = in ? Wr[at] : 0.f;
+        uv[j] = NA > 0 && ac.u && in ? ac.u[o + (int64_t)row0 * dr + at] : 0.f;
+    }
+    cp_async_wait();
+    sync();
+    // W_q[aj][bj] of term tt of the staged batch for the thread's outputs
+    auto gather = [&](int tt, float (&g)[4]) {
+        const int aj = sm.ta[tt][r].x;
+        const int4 b0 = *reinterpret_cast<const int4 *>(&sm.tb[tt][4 * cx]);
+        const int4 b1 = *reinterpret_cast<const int4 *>(&sm.tb[tt][4 * cx + 2]);
+        const int4 hd = sm.hd[tt];
+        const float *q = v + lohi(hd.x, hd.y) + (int64_t)aj * hd.z;
+        g[0] = (aj | b0.x) >= 0 ? q[b0.x] : 0.f;
+        g[1] = (aj | b0.z) >= 0 ? q[b0.z] : 0.f;
+        g[2] = (aj | b1.x) >= 0 ? q[b1.x] : 0.f;
+        g[3] = (aj | b1.z) >= 0 ? q[b1.z] : 0.f;
+    };
+    float g[4][4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+        if (eo >= 0 && u < nt0) gather(u, g[u]);
+    float y[4] = {0.f, 0.f, 0.f, 0.f};
+    if (part != HV_TERMS) {
+        const int tx = lt & 7, ty = ((lt >> 3) & 3) + 4 * ((lt >> 5) & 1), kq = lt >> 6;
+        float acc[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+        if (part == HV_FULL) {
+            const int nl = (dl + 3) >> 2, nr = (dr + 3) >> 2;
+            item_mma<false>(sm.sa, sm.sb, 0, kq, nl, ty, tx, acc);
+            item_mma<true>(sm.sa + 64, sm.sb + SB_FULL, SB_LD, (kq - nl) & 3, nr, ty, tx, acc);
+        } else {
+            for (int kb = 0; kb < K; kb += HV_KMAX) {
+                const int kn = min(HV_KMAX, K - kb);
+                if (kb > 0) {
+                    sync();
+                    stage_part(kb, kn, false);
+                    cp_async_wait();
+                    sync();
+                }
+                if (part == HV_LEFT) item_mma<false>(sm.sa, sm.sb, 0, kq, (kn + 3) >> 2, ty, tx, acc);
+                else item_mma<true>(sm.sa, sm.sb, SA_LD, kq, (kn + 3) >> 2, ty, tx, acc);
+            }
+        }
+        // the shares go where W was: H stays for the next iteration
+        auto share = [&](int q, int row) -> float4 * {
+            float *d = part == HV_RIGHT ? sm.sa + (q * 32 + row) * 32
+                       : part == HV_LEFT || q < 2 ? sm.sb + (q * 32 + row) * 32 : sm.sa + row * SA_LD + 64 + (q - 2) * 32;
+            return reinterpret_cast<float4 *>(d);
+        };
         sync();
-        item_mma(sm, 0, kl4, ty, tx, acc);
-        item_mma(sm, 64, kr4, ty, tx, acc);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) share(kq, 4 * ty + i)[tx] = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
         sync();
-    } else if (part == HV_LEFT || part == HV_RIGHT) {
-        const int ph = part == HV_LEFT ? 0 : 1;
-        const int K = ph == 0 ? dl : dr;
-        const float *H = ph == 0 ? HLk : HRk;
-        for (int kb = 0; kb < K; kb += HV_KMAX) {
-            const int kn = min(HV_KMAX, K - kb), kn4 = (kn + 3) & ~3;
-            float ra[16], rb[16];
-            item_load<HV_KMAX>(ph, H, W, dl, dr, row0, col0, kb, kn, lt, ra, rb);
-            item_store<HV_KMAX>(sm, ph, 0, kn4, lt, ra, rb);
-            sync();
-            item_mma(sm, 0, kn4, ty, tx, acc);
-            sync();
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const float4 t = share(q, r)[cx];
+            y[0] += t.x;
+            y[1] += t.y;
+            y[2] += t.z;
+            y[3] += t.w;
         }
     }
-    if (terms) {
-        AbStage<float, 32, 32> &S = sm.S;
-        for (int tb = t0; tb < t1; tb += AB_MAXT) {
-            const int nt = min(AB_MAXT, t1 - tb);
-            bool multi = false;
-            if (eo >= 0) {
-                if (tb != t0) ell_load(tb, nt);
-                if (lt < nt) {
-                    S.wq[lt] = v + ((int64_t)(unsigned)hd.x | ((int64_t)hd.y << 32));
-                    S.drq[lt] = hd.z;
-                }
-#pragma unroll
-                for (int q = 0; q < NE; ++q) {
-                    const int e = lt + q * 256;
-                    if (e < nt * 64) {
-                        const int tt = e >> 6, r = e & 63;
-                        if (r < 32) {
-                            S.ac[tt][r] = ee[q].x;
-                            S.av[tt][r] = __int_as_float(ee[q].y);
-                        } else {
-                            S.bc[tt][r - 32] = ee[q].x;
-                            S.bv[tt][r - 32] = __int_as_float(ee[q].y);
-                        }
-                    }
-                }
+    for (int tb = t0; terms && tb < t1; tb += AB_MAXT) {
+        const int nt = min(AB_MAXT, t1 - tb);
+        if (eo >= 0) {
+            if (tb != t0) {
                 sync();
-            } else {
-                ab_stage<float, 32, 32>(S, v, tb, nt, row0, col0, dl, dr, op.drs, op.off, op.terms, op.ab_rp,
-                                        op.ab_col, op.ab_val, lt, 256, sync);
-                multi = S.multi != 0;
+                stage_terms(tb, nt);
+                cp_async_wait();
+                sync();
             }
-            if (!multi) {
-                // the gathers of eight terms issued before their FMAs
-                for (int t8 = 0; t8 < nt; t8 += 8) {
-                    float g[8][2][2], f[8][2][2];
+            for (int t4 = 0; t4 < nt; t4 += 4) {
+                if (tb != t0 || t4 != 0)
 #pragma unroll
-                    for (int u = 0; u < 8; ++u) {
-                        const int tt = t8 + u;
-                        const bool on = tt < nt;
-                        const float *Wq = on ? S.wq[tt] : nullptr;
-                        const int drq = on ? S.drq[tt] : 0;
+                    for (int u = 0; u < 4; ++u)
+                        if (t4 + u < nt) gather(t4 + u, g[u]);
 #pragma unroll
-                        for (int rr = 0; rr < 2; ++rr)
-#pragma unroll
-                            for (int cc = 0; cc < 2; ++cc) {
-                                const int aj = on ? S.ac[tt][ty + 16 * rr] : -1;
-                                const int bj = on ? S.bc[tt][2 * tx + cc] : -1;
-                                const bool hit = aj >= 0 && bj >= 0;
-                                f[u][rr][cc] = hit ? S.av[tt][ty + 16 * rr] * S.bv[tt][2 * tx + cc] : 0.f;
-                                g[u][rr][cc] = hit ? Wq[(int64_t)aj * drq + bj] : 0.f;
-                            }
+                for (int u = 0; u < 4; ++u)
+                    if (t4 + u < nt) {
+                        const float av = __int_as_float(sm.ta[t4 + u][r].y);
+                        const int4 b0 = *reinterpret_cast<const int4 *>(&sm.tb[t4 + u][4 * cx]);
+                        const int4 b1 = *reinterpret_cast<const int4 *>(&sm.tb[t4 + u][4 * cx + 2]);
+                        y[0] = fmaf(av * __int_as_float(b0.y), g[u][0], y[0]);
+                        y[1] = fmaf(av * __int_as_float(b0.w), g[u][1], y[1]);
+                        y[2] = fmaf(av * __int_as_float(b1.y), g[u][2], y[2]);
+                        y[3] = fmaf(av * __int_as_float(b1.w), g[u][3], y[3]);
                     }
+            }
+        } else {
+            AbStage<float, 32, 32> &S = sm.S;
+            ab_stage<float, 32, 32>(S, v, tb, nt, row0, col0, dl, dr, op.drs, op.off, op.terms, op.ab_rp, op.ab_col,
+                                    op.ab_val, lt, 256, sync);
+            if (!S.multi) {
+                for (int tt = 0; tt < nt; ++tt) {
+                    const int aj = S.ac[tt][r];
+                    const float *q = S.wq[tt] + (int64_t)aj * S.drq[tt];
 #pragma unroll
-                    for (int u = 0; u < 8; ++u)
-#pragma unroll
-                        for (int rr = 0; rr < 2; ++rr)
-#pragma unroll
-                            for (int cc = 0; cc < 2; ++cc) acc[rr][cc] = fmaf(f[u][rr][cc], g[u][rr][cc], acc[rr][cc]);
+                    for (int j = 0; j < 4; ++j) {
+                        const int bj = S.bc[tt][cx + 8 * j];
+                        if ((aj | bj) >= 0) y[j] = fmaf(S.av[tt][r] * S.bv[tt][cx + 8 * j], q[bj], y[j]);
+                    }
                 }
             } else {
-                for (int rr = 0; rr < 2; ++rr)
-                    for (int cc = 0; cc < 2; ++cc) {
-                        const int il = row0 + ty + 16 * rr, ir = col0 + 2 * tx + cc;
-                        if (il < dl && ir < dr)
-                            acc[rr][cc] = ab_csr<float>(acc[rr][cc], v, tb, nt, il, ir, op.drs, op.off, op.terms,
-                                                        op.ab_rp, op.ab_col, op.ab_val);
-                    }
+                for (int j = 0; j < 4; ++j)
+                    if (r < rows && cx + 8 * j < cols)
+                        y[j] = ab_csr<float>(y[j], v, tb, nt, row0 + r, col0 + cx + 8 * j, op.drs, op.off, op.terms,
+                                             op.ab_rp, op.ab_col, op.ab_val);
             }
             sync();
         }
     }
-    float *out = slots[part == HV_LEFT ? 1 : (part == HV_RIGHT ? 2 : 0)] + o;
+    float *out = slots[part == HV_LEFT ? 1 : (part == HV_RIGHT ? 2 : 0)] + o + (int64_t)row0 * dr;
 #pragma unroll
-    for (int rr = 0; rr < 2; ++rr)
+    for (int j = 0; j < 4; ++j) {
+        y[j] *= scale;
+        if (r < rows && cx + 8 * j < cols) out[(int64_t)r * dr + col0 + cx + 8 * j] = y[j];
+        else y[j] = 0.f;
+        p[0] = fmaf(wv[j] * scale, y[j], p[0]);
+        if constexpr (NA > 0) p[1] = fmaf(uv[j], y[j], p[1]);
+    }
+    if constexpr (NA > 1) {
 #pragma unroll
-        for (int cc = 0; cc < 2; ++cc) {
-            const int il = row0 + ty + 16 * rr, ir = col0 + 2 * tx + cc;
-            if (il < dl && ir < dr) {
-                const int64_t idx2 = (int64_t)il * dr + ir;
-                const float y = acc[rr][cc] * scale;
-                out[idx2] = y;
-                p[0] = fmaf(W[idx2] * scale, y, p[0]);
-                if constexpr (NA > 0) {
-                    if (ac.u) p[1] = fmaf(ac.u[o + idx2], y, p[1]);
+        for (int k = 0; k < NA - 1; ++k)
+            if (k < ac.nd) {
+                const float *yk = ac.y + (int64_t)k * ac.n + o + (int64_t)row0 * dr + (int64_t)r * dr + col0 + cx;
+                float z[4];
 #pragma unroll
-                    for (int k = 0; k < NA - 1; ++k)
-                        if (k < ac.nd) p[2 + k] = fmaf(ac.y[(int64_t)k * ac.n + o + idx2], y, p[2 + k]);
-                }
+                for (int j = 0; j < 4; ++j) z[j] = r < rows && cx + 8 * j < cols ? yk[8 * j] : 0.f;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) p[2 + k] = fmaf(z[j], y[j], p[2 + k]);
             }
-        }
+    }
 }
 
 }  // namespace nss

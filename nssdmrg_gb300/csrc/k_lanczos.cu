@@ -1270,12 +1270,17 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_chunk32(ChunkArgs a) {
     // u.v_j, y_k.v_j and u.v_{j-1}, y_k.v_{j-1}: rounding level, but alpha v_j
     // and beta v_{j-1} in the three-term step would let them grow
     constexpr int NA = ANC ? ANC_MAX : 0;            // anchor columns
-    float dc[NA + 1], dm[NA + 1];
-#pragma unroll
-    for (int q = 0; q < NA; ++q) {
-        dc[q] = __ldcg(a.o.pro + 2 * ps + 1 + q);
-        dm[q] = __ldcg(a.o.pro + 2 * ps + 1 + ANC_MAX + q);
+    __shared__ float dc[ANC_MAX], dm[ANC_MAX];
+    if (tid < NA) {
+        dc[tid] = __ldcg(a.o.pro + 2 * ps + 1 + tid);
+        dm[tid] = __ldcg(a.o.pro + 2 * ps + 1 + ANC_MAX + tid);
     }
+    // the group's first work item, as a rule its only one
+    __shared__ ItemRec irec[2];
+    const int ti0 = blk + grp * G;
+    const bool one = ti0 + 2 * G >= a.nitems;
+    if (ti0 < a.nitems && lt == 0) irec[grp] = a.items[ti0];
+    __syncthreads();
     int force = __ldcg((const int *)(a.o.pro + 2 * ps));
     int done = 0, brk_m = 0;
     // CTA 0 publishes the completed iterations (device arrays, host mirrors)
@@ -1286,12 +1291,10 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_chunk32(ChunkArgs a) {
         }
         if (blk == 0 && done > 0) {
             pro.store(a.o.pro, ps, a.j0 + done - 1, force);
-            if (tid == 0)
-#pragma unroll
-                for (int q = 0; q < NA; ++q) {
-                    a.o.pro[2 * ps + 1 + q] = dc[q];
-                    a.o.pro[2 * ps + 1 + ANC_MAX + q] = dm[q];
-                }
+            if (tid < NA) {
+                a.o.pro[2 * ps + 1 + tid] = dc[tid];
+                a.o.pro[2 * ps + 1 + ANC_MAX + tid] = dm[tid];
+            }
         }
         if (blk == 0 && tid == 0) {
             for (int q = 0; q < done; ++q) {
@@ -1327,19 +1330,17 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_chunk32(ChunkArgs a) {
         // longest items first, one to every CTA before a second joins it (two
         // neighbours of the order per CTA: 1.90 against 1.67 ms at 15 200
         // states, 22 CTAs busy with 44 items)
-        for (int ti = blk + grp * G; ti < a.nitems; ti += 2 * G)
-            hv32_item<NA>(a.items[ti], x, a.slot, a.op, ism[grp], lt, GroupSync{1 + grp}, sc, ac, ap);
+        for (int ti = ti0; ti < a.nitems; ti += 2 * G) {
+            const ItemRec it = ti == ti0 ? irec[grp] : a.items[ti];
+            hv32_item<NA>(it, x, a.slot, a.op, ism[grp], lt, GroupSync{1 + grp}, sc, ac, ap, one && jj > a.j0);
+        }
         block_sums<float, 1 + NA>(ap, scr);
         if (tid == 0)
 #pragma unroll
             for (int q = 0; q < 1 + NA; ++q) pA[q * G + blk] = ap[q];
         if (blk == 0 && tid == 0) flags[F_HOST] = host_stop;
         if (!grid_sync(a.o.bar, epoch, err, a.o.spin)) { publish(); return; }
-        if (__ldcg(&flags[F_HOST])) {
-            if (blk == 0 && tid == 0) flags[F_STOP] = 1;
-            publish();
-            return;
-        }
+        const int stop = __ldcg(&flags[F_HOST]);     // looked at below, with the totals
         const float *s0 = a.slot[0], *s1 = a.slot[1], *s2 = a.slot[2];
         // the three-term step's H v_j of the thread's first row, loaded before
         // the alpha total so that the two L2 round trips overlap
@@ -1348,6 +1349,11 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_chunk32(ChunkArgs a) {
         if (if0 < i1) hv0 = s0[if0] + s1[if0] + s2[if0];
         float tot[1 + NA];
         grid_totals<float, 1 + NA>(pA, G, bc, tot);
+        if (stop) {
+            if (blk == 0 && tid == 0) flags[F_STOP] = 1;
+            publish();
+            return;
+        }
 #pragma unroll
         for (int q = 0; q < NA; ++q) tot[1 + q] -= tot[0] * dc[q] + beta_prev * dm[q];
         const float alpha0 = tot[0];
@@ -1472,12 +1478,9 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_chunk32(ChunkArgs a) {
         }
         if (tid == 0) pro.set(jj, alpha_j, beta_j);
         pro.advance();
-        if constexpr (ANC) {
-#pragma unroll
-            for (int q = 0; q < NA; ++q) {
-                dm[q] = dc[q];
-                dc[q] = sv[2 + q] / beta_j;
-            }
+        if (tid < NA) {
+            dm[tid] = dc[tid];
+            dc[tid] = bc[8 + 2 + tid] / beta_j;      // the totals of sv
         }
         ++done;
         if (brk) {
@@ -1601,7 +1604,8 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_batch32(BatchArgs B) {
                 const float sc = first ? 1.f : 1.f / bprev[g.x];
                 const AncCols ac{(const float *)S.c.o.anc_u, nullptr, 0, 0};
                 float ap[2] = {0.f, 0.f};
-                hv32_item<1>(S.c.items[g.y], x, S.c.slot, S.c.op, ism[grp], lt, GroupSync{1 + grp}, sc, ac, ap);
+                hv32_item<1>(S.c.items[g.y], x, S.c.slot, S.c.op, ism[grp], lt, GroupSync{1 + grp}, sc, ac, ap,
+                             false);
                 // group sums of the alpha and u.w partials (named barrier of the group)
                 const float a0 = warp_sum<float>(ap[0]), a1 = warp_sum<float>(ap[1]);
                 if ((lt & 31) == 0) {
