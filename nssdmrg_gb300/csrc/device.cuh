@@ -34,7 +34,7 @@ struct DevTerm {          // one A x B term, grouped by output sector
 // Tiles and terms of k_hv_fp64 (k_matvec.cu)
 struct HvRec {
     int dl, dr, row0, col0;
-    int t0, t1, csr, pad;        // the sector's terms; csr: some term's rows hold several entries
+    int t0, t1, csr, cost;       // the sector's terms; csr: some term's rows hold several entries; cost: FMAs an output
     int64_t off, hlo, hro;
 };
 struct HvTerm {
@@ -72,7 +72,8 @@ struct DevSb {
     HvTerm *d_hv_terms = nullptr;
     int *d_ell_col = nullptr;
     double *d_ell_val = nullptr;
-    int nhv = 0;
+    int nhv = 0, hv_grid = 0, hv_nsm = 0;   // its tiles, CTAs, the GPU's SMs
+    int *d_hv_queue = nullptr;         // tiles handed out, CTAs that left (both 0 between launches)
     // FP32 copies for the mixed-precision path
     float *d_hl32 = nullptr, *d_hr32 = nullptr, *d_ab_val32 = nullptr;
     int *d_ab_rowptr32 = nullptr, *d_ab_col32 = nullptr;   // pruned FP32 A/B pool

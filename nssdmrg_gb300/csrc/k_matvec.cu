@@ -80,7 +80,9 @@ namespace {
 
 constexpr int TILE = 16;
 constexpr int TILE32 = 32;
-constexpr int HV_TR = 8, HV_TC = 16;   // output tile of k_hv_fp64
+constexpr int HV_TR = 4, HV_TC = 8;    // output tile of a warp of k_hv_fp64
+constexpr int HV_WARPS = 4;            // warps of its CTAs, one per quarter of an SM
+constexpr int HV_CTAS = 5;             // CTAs per SM at most: more tiles are handed out by a queue
 
 // Sections of the pool's arena: each array at a 256-byte boundary (at least
 // 16 bytes, so that every pointer is distinct and valid), those with a host
@@ -430,15 +432,20 @@ int sb_upload(Ctx &c, const nss_sb_desc *d, bool trusted) {
             hv_terms.push_back(h);
         }
         for (int k = 0; k < s.nsb; ++k) {
-            int csr = 0;
-            for (int t = s.term_ptr[k]; t < s.term_ptr[k + 1]; ++t) csr |= hv_terms[t].kind > 0;
+            // FMAs per output: the two K loops and, per term, a row of A
+            int csr = 0, cost = s.dls[k] + s.drs[k];
+            for (int t = s.term_ptr[k]; t < s.term_ptr[k + 1]; ++t) {
+                const DevTerm &tm = s.terms[t];
+                csr |= hv_terms[t].kind > 0;
+                cost += (rowptr[tm.a_rp + tm.a_nrow] - rowptr[tm.a_rp]) / std::max(tm.a_nrow, 1);
+            }
             for (int r = 0; r < s.dls[k]; r += HV_TR)
                 for (int cc = 0; cc < s.drs[k]; cc += HV_TC)
-                    hv_recs.push_back(HvRec{s.dls[k], s.drs[k], r, cc, s.term_ptr[k], s.term_ptr[k + 1], csr, 0, s.off[k],
+                    hv_recs.push_back(HvRec{s.dls[k], s.drs[k], r, cc, s.term_ptr[k], s.term_ptr[k + 1], csr, cost, s.off[k],
                                             s.hl_off[k], s.hr_off[k]});
         }
         std::stable_sort(hv_recs.begin(), hv_recs.end(),
-                         [](const HvRec &x, const HvRec &y) { return x.dl + x.dr > y.dl + y.dr; });
+                         [](const HvRec &x, const HvRec &y) { return x.cost > y.cost; });
     }
     s.nhv = (int)hv_recs.size();
 
@@ -481,6 +488,9 @@ int sb_upload(Ctx &c, const nss_sb_desc *d, bool trusted) {
     int nsm = 0;
     NSS_CUDA_TRY(c, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c.device));
     mma_layout(s, tc_thr, tc_bn, c.mma_split, nsm, plan);
+    s.hv_nsm = nsm;
+    s.hv_grid = s.nhv <= 2 * HV_WARPS * nsm ? (s.nhv + HV_WARPS - 1) / HV_WARPS
+                                            : nsm * std::min(HV_CTAS, (s.nhv + HV_WARPS * nsm - 1) / (HV_WARPS * nsm));
     std::vector<char> on_tc(s.nsb, 0);
     for (int k : plan.sectors) on_tc[k] = 1;
     std::vector<int4> tiles32;
@@ -645,6 +655,8 @@ int sb_upload(Ctx &c, const nss_sb_desc *d, bool trusted) {
     sg.add(&s.d_sp_dval, sp.dval);
     sg.add(&s.d_sp_tiles, sp.tiles);
     sg.add(&s.d_hv_recs, hv_recs);
+    const std::vector<int> hv_queue(2, 0);
+    sg.add(&s.d_hv_queue, hv_queue);
     sg.add(&s.d_hv_terms, hv_terms);
     sg.add(&s.d_ell_col, ell_col);
     sg.add(&s.d_ell_val, ell_val);
@@ -676,22 +688,28 @@ int sb_upload(Ctx &c, const nss_sb_desc *d, bool trusted) {
     return NSS_OK;
 }
 
-// One CTA of four warps per 8 x 16 output tile, a thread an output.
+// A warp per 4 x 8 output tile, a thread an output.
 // The FP64 pipe takes a warp's FMA every 64 cycles (1.0-1.2 TFLOP/s over the
-// GPU) and bounds the kernel: so the K loops stop at the sector's edge, four
-// warps (one per quarter of an SM) are a tile, which spreads a small superblock
-// over four times as many SMs as 16 x 16 outputs on eight warps did, and the
+// GPU) and bounds the kernel: the K loops stop at the sector's edge, and the
 // next 32 columns of K are loaded into registers while the current ones are
-// multiplied.  Sums run in the same order as there.  A x B terms: Out[ai][bi]
-// += A[ai][aj] B[bi][bj] W_q[aj][bj] (:808-857).  Where all rows hold one entry,
-// four terms' loads are in flight; where rows of A hold more (the
-// renormalised sign operator leaves rounding-level entries in its whole block,
-// 40 a row), half a warp takes a row, a lane an entry, eight gathers in flight,
-// instead of every thread walking the row by itself; a factor of +-1 is a sign
-// flip and no FP64 multiplication.  Against the 16 x 16 form, results bit for
-// bit the same: Hubbard m = 256 (66 600 states) 88 -> 60 us a product, 582
-// states 4.1 -> 3.4 us, FP64 solves of 3 958 states 3.12 -> 2.32 ms, of 66 600
-// 9.85 -> 7.60 ms.
+// multiplied.  What is left is balance: every quarter of an SM has a pipe of its
+// own.  Up to two tiles for each (2 * 4 * 152) the CTAs get four each; above,
+// every SM the same number of CTAs (at most five), and a warp that is done takes
+// its next tile from a queue, longest first.  Tiles of 8 x 16 on four warps,
+// one CTA each, left SMs with five CTAs beside others with four, and waited for
+// each other at barriers.  Up to five CTAs against three and four: 51.5 against 58.8
+// and 53.0 us at 66 600 states, 76 against 90 and 85 at 93 000.
+// A x B terms: Out[ai][bi] += A[ai][aj] B[bi][bj] W_q[aj][bj] (:808-857).  Where
+// all rows hold one entry, four terms' loads are in flight; where rows of A hold
+// more (the renormalised sign operator leaves rounding-level entries in its
+// whole block, 40 a row), a row's eight lanes hold two entries each, eight
+// gathers in flight, instead of every thread walking the row by itself; a
+// factor of +-1 is a sign flip and no FP64 multiplication.  (Gathers a round
+// ahead of the FMAs need 126 registers and were slower: 57.7 us.)
+// Bit for bit the results of 16 x 16 tiles on eight warps, in us: Hubbard
+// 66 600 states 88 -> 60 (8 x 16) -> 51.5, spin-1/2 39 200 states 28.0 (8 x 16)
+// -> 22.9, spin-1 60 900 states 37.3 -> 34.8, 582 states 4.1 -> 3.4; FP64 solves
+// of 3 958 states 3.12 -> 2.32 -> 2.13 ms, of 66 600 9.85 -> 7.11 -> 6.14 ms.
 __device__ __forceinline__ double hv_times(double b, double x, bool unit) {
     if (!unit) return b * x;
     return __hiloint2double(__double2hiint(x) ^ (__double2hiint(b) & 0x80000000), __double2loint(x));
@@ -706,127 +724,149 @@ struct HvOps {
     const double *ab_val;
 };
 
-__global__ void __launch_bounds__(HV_TR *HV_TC) k_hv_fp64(const double *__restrict__ v, double *__restrict__ hv,
-                                                           const HvRec *__restrict__ recs, HvOps op, const int *stop) {
-    if (stop && *stop) return;   // the Lanczos loop has already finished
-    constexpr int NT = HV_TR * HV_TC, KC = 32;
-    __shared__ double sa[HV_TR][KC + 1];
-    __shared__ double sb[KC][HV_TC + 1];
-    const HvRec t = recs[blockIdx.x];
-    const int dl = t.dl, dr = t.dr;
-    const double *W = v + t.off, *HL = op.hl + t.hlo, *HR = op.hr + t.hro;
-    const int tid = threadIdx.x, ty = tid / HV_TC, tx = tid % HV_TC;
-    const int il = t.row0 + ty, ir = t.col0 + tx;
-    const int c0 = (dl + KC - 1) / KC, c1 = (dr + KC - 1) / KC;
-    double ra[HV_TR * KC / NT], rb[KC * HV_TC / NT];
-    // chunk c of the K loops: H_L W (sum_j HL[il][j] W[j][ir], :784-796), then
-    // W H_R^T (sum_j W[il][j] HR[ir][j], :767-779)
-    auto load = [&](int c) {
-        const bool left = c < c0;
-        const int j0 = (left ? c : c - c0) * KC, K = left ? dl : dr;
+__global__ void __launch_bounds__(32 * HV_WARPS) k_hv_fp64(const double *__restrict__ v, double *__restrict__ hv,
+                                                           const HvRec *__restrict__ recs, HvOps op, int ntiles,
+                                                           int nsm, int *queue, const int *stop) {
+    if (stop && *stop) return;   // the Lanczos loop has already finished (the same for every CTA)
+    constexpr int KC = 32;
+    __shared__ double sa_[HV_WARPS][HV_TR][KC + 1];
+    __shared__ double sb_[HV_WARPS][KC][HV_TC + 1];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, grid = gridDim.x;
+    double(*sa)[KC + 1] = sa_[warp];
+    double(*sb)[HV_TC + 1] = sb_[warp];
+    const int ty = lane / HV_TC, tx = lane % HV_TC;
+    const bool queued = ntiles > HV_WARPS * grid;
+    // longest tiles first, a CTA's four a grid apart in the order; the warp that
+    // may be left without one is another in each CTA of an SM
+    int tile = (int)((warp + blockIdx.x / nsm) % HV_WARPS) * grid + blockIdx.x, next = ntiles;
+    for (; tile < ntiles; tile = next) {
+        const HvRec t = recs[tile];
+        const int dl = t.dl, dr = t.dr;
+        const double *W = v + t.off, *HL = op.hl + t.hlo, *HR = op.hr + t.hro;
+        const int il = t.row0 + ty, ir = t.col0 + tx;
+        const int c0 = (dl + KC - 1) / KC, c1 = (dr + KC - 1) / KC;
+        double ra[HV_TR], rb[HV_TC];
+        // chunk c of the K loops: H_L W (sum_j HL[il][j] W[j][ir], :784-796), then
+        // W H_R^T (sum_j W[il][j] HR[ir][j], :767-779)
+        auto load = [&](int c) {
+            const bool left = c < c0;
+            const int j0 = (left ? c : c - c0) * KC, K = left ? dl : dr, gk = j0 + lane;
+            const double *A = (left ? HL : W) + (int64_t)t.row0 * K + gk;
 #pragma unroll
-        for (int q = 0; q < HV_TR * KC / NT; ++q) {
-            const int e = tid + q * NT, gi = t.row0 + e / KC, gj = j0 + e % KC;
-            ra[q] = (gi < dl && gj < K) ? (left ? HL[(int64_t)gi * dl + gj] : W[(int64_t)gi * dr + gj]) : 0.0;
-        }
-#pragma unroll
-        for (int q = 0; q < KC * HV_TC / NT; ++q) {
-            const int e = tid + q * NT;
+            for (int q = 0; q < HV_TR; ++q) ra[q] = t.row0 + q < dl && gk < K ? A[(int64_t)q * K] : 0.0;
             if (left) {
-                const int gj = j0 + e / HV_TC, gc = t.col0 + e % HV_TC;
-                rb[q] = (gj < dl && gc < dr) ? W[(int64_t)gj * dr + gc] : 0.0;
+                const int gj = j0 + ty;
+                const double *B = W + (int64_t)gj * dr + ir;
+#pragma unroll
+                for (int q = 0; q < HV_TC; ++q)
+                    rb[q] = gj + HV_TR * q < dl && ir < dr ? B[(int64_t)(HV_TR * q) * dr] : 0.0;
             } else {
-                const int gr = t.col0 + e / KC, gj = j0 + e % KC;
-                rb[q] = (gr < dr && gj < dr) ? HR[(int64_t)gr * dr + gj] : 0.0;
+                const double *B = HR + (int64_t)t.col0 * dr + gk;
+#pragma unroll
+                for (int q = 0; q < HV_TC; ++q) rb[q] = t.col0 + q < dr && gk < dr ? B[(int64_t)q * dr] : 0.0;
             }
-        }
-    };
-    double acc = 0.0;
-    load(0);
-    for (int c = 0; c < c0 + c1; ++c) {
-        const bool left = c < c0;
-        const int kn = min(KC, left ? dl - c * KC : dr - (c - c0) * KC);
+        };
+        double acc = 0.0;
+        load(0);
+        for (int c = 0; c < c0 + c1; ++c) {
+            const bool left = c < c0;
+            const int kn = min(KC, left ? dl - c * KC : dr - (c - c0) * KC);
 #pragma unroll
-        for (int q = 0; q < HV_TR * KC / NT; ++q) {
-            const int e = tid + q * NT;
-            sa[e / KC][e % KC] = ra[q];
-        }
+            for (int q = 0; q < HV_TR; ++q) sa[q][lane] = ra[q];
 #pragma unroll
-        for (int q = 0; q < KC * HV_TC / NT; ++q) {
-            const int e = tid + q * NT;
-            if (left) sb[e / HV_TC][e % HV_TC] = rb[q];
-            else sb[e % KC][e / KC] = rb[q];
-        }
-        __syncthreads();
-        if (c + 1 < c0 + c1) load(c + 1);
+            for (int q = 0; q < HV_TC; ++q) {
+                if (left) sb[ty + HV_TR * q][tx] = rb[q];
+                else sb[lane][q] = rb[q];
+            }
+            __syncwarp();
+            if (c + 1 < c0 + c1) load(c + 1);
 #pragma unroll 8
-        for (int j = 0; j < kn; ++j) acc = fma(sa[ty][j], sb[j][tx], acc);
-        __syncthreads();
-    }
-    const bool in = il < dl && ir < dr;
-    if (!t.csr) {
-        for (int tb = t.t0; tb < t.t1; tb += 4) {
-            int aj[4], bj[4];
-            double f[4], w[4];
-            HvTerm tm[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) tm[q] = op.terms[min(tb + q, t.t1 - 1)];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const bool on = in && tb + q < t.t1;
-                aj[q] = on ? op.ell_col[tm[q].a + il] : -1;
-                bj[q] = on ? op.ell_col[tm[q].b + ir] : -1;
-                f[q] = on ? hv_times(op.ell_val[tm[q].b + ir], op.ell_val[tm[q].a + il], tm[q].unit_b) : 0.0;
-            }
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-                w[q] = aj[q] >= 0 && bj[q] >= 0 ? v[tm[q].off + (int64_t)aj[q] * tm[q].drq + bj[q]] : 0.0;
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-                if (aj[q] >= 0 && bj[q] >= 0) acc = fma(f[q], w[q], acc);
+            for (int j = 0; j < kn; ++j) acc = fma(sa[ty][j], sb[j][tx], acc);
+            __syncwarp();
         }
-    } else {
-        const int hl16 = tid & 15;                   // lane of the half warp that holds the row
-        for (int ti = t.t0; ti < t.t1; ++ti) {
-            const HvTerm tm = op.terms[ti];
-            const double *Wq = v + tm.off;
-            if (tm.kind == 2) {                      // rows of B with several entries
-                if (in)
-                    for (int ja = op.ab_rp[tm.a_rp + il]; ja < op.ab_rp[tm.a_rp + il + 1]; ++ja) {
-                        const int64_t row = (int64_t)op.ab_col[ja] * tm.drq;
-                        double cb = 0.0;
-                        for (int jb = op.ab_rp[tm.b_rp + ir]; jb < op.ab_rp[tm.b_rp + ir + 1]; ++jb)
-                            cb = fma(op.ab_val[jb], Wq[row + op.ab_col[jb]], cb);
-                        acc = fma(op.ab_val[ja], cb, acc);
-                    }
-                continue;
+        if (queued) {
+            if (lane == 0) next = HV_WARPS * grid + atomicAdd(queue, 1);
+            next = __shfl_sync(0xffffffffu, next, 0);
+        }
+        const bool in = il < dl && ir < dr;
+        if (!t.csr) {
+            for (int tb = t.t0; tb < t.t1; tb += 4) {
+                int aj[4], bj[4];
+                double f[4], w[4];
+                HvTerm tm[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) tm[q] = op.terms[min(tb + q, t.t1 - 1)];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const bool on = in && tb + q < t.t1;
+                    aj[q] = on ? op.ell_col[tm[q].a + il] : -1;
+                    bj[q] = on ? op.ell_col[tm[q].b + ir] : -1;
+                    f[q] = on ? hv_times(op.ell_val[tm[q].b + ir], op.ell_val[tm[q].a + il], tm[q].unit_b) : 0.0;
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    w[q] = aj[q] >= 0 && bj[q] >= 0 ? v[tm[q].off + (int64_t)aj[q] * tm[q].drq + bj[q]] : 0.0;
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    if (aj[q] >= 0 && bj[q] >= 0) acc = fma(f[q], w[q], acc);
             }
-            const int bj = in ? op.ell_col[tm.b + ir] : -1;
-            const double bv = in ? op.ell_val[tm.b + ir] : 0.0;
-            const int p0 = il < dl ? op.ab_rp[tm.a_rp + il] : 0;
-            const int cnt = il < dl ? op.ab_rp[tm.a_rp + il + 1] - p0 : 0;
-            const int most = max(cnt, __shfl_xor_sync(0xffffffffu, cnt, 16));
-            for (int base = 0; base < most; base += 16) {
-                const bool mine = base + hl16 < cnt;
-                const int ec = mine ? op.ab_col[p0 + base + hl16] : 0;
-                const double ev = mine ? op.ab_val[p0 + base + hl16] : 0.0;
-                for (int u = 0; u < 16 && base + u < most; u += 8) {
-                    double g[8];
+        } else {
+            for (int ti = t.t0; ti < t.t1; ++ti) {
+                const HvTerm tm = op.terms[ti];
+                const double *Wq = v + tm.off;
+                if (tm.kind == 2) {                  // rows of B with several entries
+                    if (in)
+                        for (int ja = op.ab_rp[tm.a_rp + il]; ja < op.ab_rp[tm.a_rp + il + 1]; ++ja) {
+                            const int64_t row = (int64_t)op.ab_col[ja] * tm.drq;
+                            double cb = 0.0;
+                            for (int jb = op.ab_rp[tm.b_rp + ir]; jb < op.ab_rp[tm.b_rp + ir + 1]; ++jb)
+                                cb = fma(op.ab_val[jb], Wq[row + op.ab_col[jb]], cb);
+                            acc = fma(op.ab_val[ja], cb, acc);
+                        }
+                    continue;
+                }
+                const int bj = in ? op.ell_col[tm.b + ir] : -1;
+                const double bv = in ? op.ell_val[tm.b + ir] : 0.0;
+                const int p0 = il < dl ? op.ab_rp[tm.a_rp + il] : 0;
+                const int cnt = il < dl ? op.ab_rp[tm.a_rp + il + 1] - p0 : 0;
+                int most = cnt;                      // of the tile's rows, HV_TC lanes each
 #pragma unroll
-                    for (int x = 0; x < 8; ++x) {
-                        const int c = __shfl_sync(0xffffffffu, ec, u + x, 16);
-                        g[x] = bj >= 0 && base + u + x < cnt ? Wq[(int64_t)c * tm.drq + bj] : 0.0;
+                for (int o = HV_TC; o < 32; o <<= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
+                for (int base = 0; base < most; base += 2 * HV_TC) {
+                    int ec[2];                       // entries base + tx, base + HV_TC + tx of the lane's row
+                    double ev[2];
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const bool mine = base + h * HV_TC + tx < cnt;
+                        ec[h] = mine ? op.ab_col[p0 + base + h * HV_TC + tx] : 0;
+                        ev[h] = mine ? op.ab_val[p0 + base + h * HV_TC + tx] : 0.0;
                     }
 #pragma unroll
-                    for (int x = 0; x < 8; ++x) {
-                        const double a = __shfl_sync(0xffffffffu, ev, u + x, 16);
-                        if (bj >= 0 && base + u + x < cnt) acc = fma(a, hv_times(bv, g[x], tm.unit_b), acc);
+                    for (int h = 0; h < 2; ++h) {
+                        const int b0 = base + h * HV_TC;
+                        if (b0 >= most) break;
+                        double g[HV_TC];
+#pragma unroll
+                        for (int x = 0; x < HV_TC; ++x) {
+                            const int c = __shfl_sync(0xffffffffu, ec[h], x, HV_TC);
+                            g[x] = bj >= 0 && b0 + x < cnt ? Wq[(int64_t)c * tm.drq + bj] : 0.0;
+                        }
+#pragma unroll
+                        for (int x = 0; x < HV_TC; ++x) {
+                            const double a = __shfl_sync(0xffffffffu, ev[h], x, HV_TC);
+                            if (bj >= 0 && b0 + x < cnt) acc = fma(a, hv_times(bv, g[x], tm.unit_b), acc);
+                        }
                     }
                 }
             }
         }
+        if (in) hv[t.off + (int64_t)il * dr + ir] = acc;
     }
-    if (in) hv[t.off + (int64_t)il * dr + ir] = acc;
+    // every tile is taken: the last warp to leave clears the queue
+    if (queued && lane == 0 && atomicAdd(queue + 1, 1) == HV_WARPS * grid - 1) {
+        queue[0] = 0;
+        queue[1] = 0;
+    }
 }
 
 // FP32 variant for the mixed-precision Lanczos phase: 32x32 output tiles,
@@ -923,9 +963,10 @@ int hv_device(Ctx &c, const double *d_v, double *d_hv, const int *stop) {
         return NSS_ERR_STATE;
     }
     if (s.sp_nitems) return hv_device_split(c, d_v, d_hv, stop);
-    k_hv_fp64<<<s.nhv, HV_TR * HV_TC, 0, c.stream>>>(
+    k_hv_fp64<<<s.hv_grid, 32 * HV_WARPS, 0, c.stream>>>(
         d_v, d_hv, s.d_hv_recs,
-        HvOps{s.d_hl, s.d_hr, s.d_hv_terms, s.d_ell_col, s.d_ell_val, s.d_ab_rowptr, s.d_ab_col, s.d_ab_val}, stop);
+        HvOps{s.d_hl, s.d_hr, s.d_hv_terms, s.d_ell_col, s.d_ell_val, s.d_ab_rowptr, s.d_ab_col, s.d_ab_val}, s.nhv,
+        s.hv_nsm, s.d_hv_queue, stop);
     c.launches += 1;
     NSS_CUDA_TRY(c, cudaGetLastError());
     return NSS_OK;
