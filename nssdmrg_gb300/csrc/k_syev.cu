@@ -136,30 +136,39 @@ __global__ void __launch_bounds__(TRD_THREADS, 1)
         if (j <= i) A[i * ld + j] = R[(int64_t)pm[i] * n + pm[j]];
     }
     __syncthreads();
+    // reflector of column k by warp 0 (dlarfg: H x = beta e_1); ss: the lane's
+    // share of its squares below the subdiagonal.  The two quotients are one
+    // division in two lanes
+    auto reflect = [&](int k, double ss) {
+        ss = wsum(ss);
+        const double alpha = A[(k + 1) * ld + k];
+        double t = 0.0, beta = alpha, scal = 0.0;
+        if (ss > 0.0) {
+            beta = -copysign(sqrt(fma(alpha, alpha, ss)), alpha);
+            const double quo = (lane == 0 ? beta - alpha : 1.0) / (lane == 0 ? beta : alpha - beta);
+            t = __shfl_sync(0xffffffffu, quo, 0);
+            scal = __shfl_sync(0xffffffffu, quo, 1);
+        }
+        if (lane == 0) {
+            sh[0] = t;
+            sh[2] = scal;
+            td[eo + k] = A[k * ld + k];
+            te[eo + k] = beta;
+            tau[eo + k] = t;
+        }
+    };
+    auto squares = [&](int k) {                     // of a column that no update touches
+        double ss = 0.0;
+        for (int i = k + 2 + lane; i < n; i += 32) {
+            const double x = A[i * ld + k];
+            ss = fma(x, x, ss);
+        }
+        return ss;
+    };
+    if (warp == 0 && n > 2) reflect(0, squares(0));
     for (int k = 0; k + 2 < n; ++k) {
         const int m = n - k - 1;                    // trailing rows k+1 .. n-1
-        if (warp == 0) {
-            double ss = 0.0;
-            for (int i = k + 2 + lane; i < n; i += 32) {
-                const double x = A[i * ld + k];
-                ss = fma(x, x, ss);
-            }
-            ss = wsum(ss);
-            if (lane == 0) {
-                const double alpha = A[(k + 1) * ld + k];
-                double t = 0.0, beta = alpha, scal = 0.0;
-                if (ss > 0.0) {                      // dlarfg: H x = beta e_1
-                    beta = -copysign(sqrt(fma(alpha, alpha, ss)), alpha);
-                    t = (beta - alpha) / beta;
-                    scal = 1.0 / (alpha - beta);
-                }
-                sh[0] = t;
-                sh[2] = scal;
-                td[eo + k] = A[k * ld + k];
-                te[eo + k] = beta;
-                tau[eo + k] = t;
-            }
-        }
+        const bool ahead = k + 3 < n;               // there is a next column
         __syncthreads();
         const double t = sh[0];
         for (int i = tid; i < m; i += TRD_THREADS) {
@@ -168,7 +177,10 @@ __global__ void __launch_bounds__(TRD_THREADS, 1)
             Vq[(int64_t)k * n + k + 1 + i] = x;
         }
         __syncthreads();
-        if (t == 0.0) continue;                      // uniform: t is shared
+        if (t == 0.0) {                              // uniform: t is shared
+            if (warp == 0 && ahead) reflect(k + 1, squares(k + 1));
+            continue;
+        }
         // p = t A v over the trailing block (symmetric reads of the lower
         // triangle): four threads per row, each with two accumulators, so the
         // whole CTA streams FMAs instead of one warp reduction per row
@@ -204,16 +216,29 @@ __global__ void __launch_bounds__(TRD_THREADS, 1)
         const double K = sh[3];
         for (int i = tid; i < m; i += TRD_THREADS) w[i] = fma(K, v[i], w[i]);   // w = p - (t/2)(p.v) v
         __syncthreads();
-        for (int i = warp; i < m; i += NW) {         // A -= v w^T + w v^T (lower triangle)
-            const int r = k + 1 + i;
-            const double vi = v[i], wi = w[i];
-            for (int j = lane; j <= i; j += 32) {
-                const int c = k + 1 + j;
-                A[r * ld + c] = fma(-vi, w[j], fma(-wi, v[j], A[r * ld + c]));   // two FMAs
+        // A -= v w^T + w v^T (lower triangle): warp 0 the first column, from
+        // which it forms the next reflector while the others update the rest
+        auto updated = [&](int i, int j) {           // two FMAs
+            double &x = A[(k + 1 + i) * ld + k + 1 + j];
+            x = fma(-v[i], w[j], fma(-w[i], v[j], x));
+            return x;
+        };
+        if (ahead && warp == 0) {
+            if (lane < 2) updated(lane, 0);
+            double ss = 0.0;
+            for (int i = 2 + lane; i < m; i += 32) {
+                const double x = updated(i, 0);
+                ss = fma(x, x, ss);
             }
+            __syncwarp();
+            reflect(k + 1, ss);
+        } else {
+            for (int i = ahead ? warp - 1 : warp; i < m; i += ahead ? NW - 1 : NW)
+                for (int j = lane; j <= i; j += 32)
+                    if (j > 0 || !ahead) updated(i, j);
         }
-        __syncthreads();
     }
+    __syncthreads();
     if (tid == 0) {
         if (n >= 2) {
             td[eo + n - 2] = A[(n - 2) * ld + n - 2];
@@ -283,16 +308,15 @@ __global__ void __launch_bounds__(TRD_THREADS, 1)
                 double ss = 0.0;
                 for (int i = k + 2 + lane; i < n; i += 32) ss = fma(colk[i], colk[i], ss);
                 ss = wsum(ss);
+                const double alpha = colk[k + 1];
+                double beta = alpha, quo = 0.0;      // lane 0: tau, lane 1: the scale (one division for both)
+                if (ss > 0.0) {
+                    beta = -copysign(sqrt(fma(alpha, alpha, ss)), alpha);
+                    quo = (lane == 0 ? beta - alpha : 1.0) / (lane == 0 ? beta : alpha - beta);
+                }
+                if (lane < 2) sb[lane] = quo;
                 if (lane == 0) {
-                    const double alpha = colk[k + 1];
-                    double t = 0.0, beta = alpha, scal = 0.0;
-                    if (ss > 0.0) {
-                        beta = -copysign(sqrt(fma(alpha, alpha, ss)), alpha);
-                        t = (beta - alpha) / beta;
-                        scal = 1.0 / (alpha - beta);
-                    }
-                    sb[0] = t;
-                    sb[1] = scal;
+                    const double t = quo;
                     td[eo + k] = colk[k];
                     te[eo + k] = beta;
                     tau[eo + k] = t;
@@ -342,10 +366,12 @@ __global__ void __launch_bounds__(TRD_THREADS, 1)
         __syncthreads();
         if (tid == 0) {
             double x = 0.0;
-            for (int u = 0; u < NW; ++u) x += red[u];
+            for (int u = 0; u < min(NW, ncol - jj0); ++u) x += red[u];   // the warps that had columns
             sb[2] = x;
         }
         cl.sync();                                   // p and the p.v shares published
+        auto pval = [&](int i) { return cl.map_shared_rank(pb, (k + 1 + i) % C)[(k + 1 + i) / C]; };
+        const double p0 = tid < m ? pval(tid) : 0.0; // in flight beside the shares
         if (warp == 0) {
             double x = lane < C ? cl.map_shared_rank(sb, lane)[2] : 0.0;
             x = wsum(x);
@@ -354,10 +380,7 @@ __global__ void __launch_bounds__(TRD_THREADS, 1)
         __syncthreads();
         const double K = kk;
         if (t != 0.0)
-            for (int i = tid; i < m; i += TRD_THREADS) {
-                const int g = k + 1 + i;
-                w[i] = fma(K, v[i], cl.map_shared_rank(pb, g % C)[g / C]);
-            }
+            for (int i = tid; i < m; i += TRD_THREADS) w[i] = fma(K, v[i], i == tid ? p0 : pval(i));
         __syncthreads();
         if (t != 0.0)
             for (int jj = jj0 + warp; jj < ncol; jj += NW) {
