@@ -326,7 +326,8 @@ int sb_upload(Ctx &c, const nss_sb_desc *d, bool trusted = false);
 void sb_release(Ctx &c, bool free_arena);
 // `stop` (may be null): a device flag; the kernels return at once when set
 int hv_device(Ctx &c, const double *d_v, double *d_hv, const int *stop = nullptr);
-int hv_device_fp32(Ctx &c, const float *d_v, float *d_hv, const int *stop = nullptr);
+// add_planes false: the tensor-core sectors' part stays in sb.d_mma_out (mma_nplanes planes)
+int hv_device_fp32(Ctx &c, const float *d_v, float *d_hv, const int *stop = nullptr, bool add_planes = true);
 // k_sector_mma.cu: the dense sector products of the routed sectors into the
 // two output planes (the "terms only" tiles of k_hv_fp32 add them)
 int hv_device_mma(Ctx &c, const float *d_v, const int *stop = nullptr);

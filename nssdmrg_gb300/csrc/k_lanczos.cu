@@ -357,6 +357,10 @@ struct OrthArgs {
     // columns' totals
     unsigned *xep;
     uint64_t *xtot, *xpart, *xcol;
+    // H v_j's tensor-core part, still to be added to w: tcn planes of n (FP32
+    // only; null: w is complete)
+    const float *tc = nullptr;
+    int tcn = 0;
 };
 
 // The omega recurrence's constants per basis type: level after a projection,
@@ -950,6 +954,10 @@ __device__ __forceinline__ bool pro_always(int m, int64_t n, int ps) {
     return ps > PRO_MAX_PS || (sizeof(T) == 8 ? n < PRO_MIN_N : 8 * (int64_t)m > n);
 }
 
+// Rows of a thread whose loads go out together (a store to w would order the
+// next row's loads behind it; a CTA has five rows a thread at 398 000 states)
+constexpr int ROWS = 4;
+
 template <class T, int CW>
 __global__ void __launch_bounds__(ORTH_THREADS, 1) k_orth(OrthArgs a) {
     int *flags = a.flags;
@@ -1003,15 +1011,45 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_orth(OrthArgs a) {
     T av[PA_COLS];
 #pragma unroll
     for (int q = 0; q < PA_COLS; ++q) av[q] = (T)0;
-    for (int64_t i = i0 + tid; i < i1; i += ORTH_THREADS) {
-        const T wi = w[i], vi = vj[i];
-        av[0] += vi * wi;
-        if (anc) {
-            av[1] += au[i] * wi;
-            av[2] += ar[i] * vi;
+    for (int64_t b0 = i0 + tid; b0 < i1; b0 += ROWS * ORTH_THREADS) {
+        T wv[ROWS], vv[ROWS], uv[ROWS], rv[ROWS];
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
-                if (k < nd) av[3 + k] += ay[(int64_t)k * n + i] * wi;
+        for (int u = 0; u < ROWS; ++u) {
+            const int64_t i = b0 + u * ORTH_THREADS;
+            const bool ok = i < i1;
+            wv[u] = ok ? w[i] : (T)0;
+            vv[u] = ok ? vj[i] : (T)0;
+            uv[u] = anc && ok ? au[i] : (T)0;
+            rv[u] = anc && ok ? ar[i] : (T)0;
+        }
+        if constexpr (sizeof(T) == 4) {
+            if (a.tc) {                              // H v_j's tensor-core part, plane 0 first
+                float d[ROWS];
+#pragma unroll
+                for (int u = 0; u < ROWS; ++u) d[u] = b0 + u * ORTH_THREADS < i1 ? a.tc[b0 + u * ORTH_THREADS] : 0.f;
+                for (int p = 1; p < a.tcn; ++p)
+#pragma unroll
+                    for (int u = 0; u < ROWS; ++u)
+                        if (b0 + u * ORTH_THREADS < i1) d[u] += a.tc[(int64_t)p * n + b0 + u * ORTH_THREADS];
+#pragma unroll
+                for (int u = 0; u < ROWS; ++u) {
+                    wv[u] += d[u];
+                    if (b0 + u * ORTH_THREADS < i1) w[b0 + u * ORTH_THREADS] = wv[u];
+                }
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < ROWS; ++u) {
+            const int64_t i = b0 + u * ORTH_THREADS;
+            if (i >= i1) break;
+            av[0] += vv[u] * wv[u];
+            if (anc) {
+                av[1] += uv[u] * wv[u];
+                av[2] += rv[u] * vv[u];
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (k < nd) av[3 + k] += ay[(int64_t)k * n + i] * wv[u];
+            }
         }
     }
     const T beta_m = j > 0 ? (T)__ldcg(a.beta + j - 1) : (T)0;
@@ -1050,21 +1088,36 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_orth(OrthArgs a) {
     T ew[1 + ANC_MAX];
 #pragma unroll
     for (int q = 0; q < 1 + ANC_MAX; ++q) ew[q] = (T)0;
-    for (int64_t i = i0 + tid; i < i1; i += ORTH_THREADS) {
-        T x = w[i] - alpha0 * vj[i];
-        if (j > 0) x -= beta_m * vjm[i];
-        if (anc) {
-            x -= tot[1] * au[i];
+    for (int64_t b0 = i0 + tid; b0 < i1; b0 += ROWS * ORTH_THREADS) {
+        T wv[ROWS], vv[ROWS], pv[ROWS], uv[ROWS];
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
-                if (k < nd) x -= tot[3 + k] * ay[(int64_t)k * n + i];
-            ew[1] += au[i] * x;
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-                if (k < nd) ew[2 + k] += ay[(int64_t)k * n + i] * x;
+        for (int u = 0; u < ROWS; ++u) {
+            const int64_t i = b0 + u * ORTH_THREADS;
+            const bool ok = i < i1;
+            wv[u] = ok ? w[i] : (T)0;
+            vv[u] = ok ? vj[i] : (T)0;
+            pv[u] = ok && j > 0 ? vjm[i] : (T)0;
+            uv[u] = anc && ok ? au[i] : (T)0;
         }
-        w[i] = x;
-        if (!always) ew[0] += x * x;
+#pragma unroll
+        for (int u = 0; u < ROWS; ++u) {
+            const int64_t i = b0 + u * ORTH_THREADS;
+            if (i >= i1) break;
+            T x = wv[u] - alpha0 * vv[u];
+            if (j > 0) x -= beta_m * pv[u];
+            if (anc) {
+                x -= tot[1] * uv[u];
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (k < nd) x -= tot[3 + k] * ay[(int64_t)k * n + i];
+                ew[1] += uv[u] * x;
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (k < nd) ew[2 + k] += ay[(int64_t)k * n + i] * x;
+            }
+            w[i] = x;
+            if (!always) ew[0] += x * x;
+        }
     }
     T bb[1] = {(T)0};
     bool project = always;
@@ -1134,17 +1187,29 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_orth(OrthArgs a) {
             const T inv = bc[12];
             T *vn = V + (int64_t)m * n;
             T *vc = (T *)a.vcur;
-            for (int64_t i = i0 + tid; i < i1; i += ORTH_THREADS) {
-                T x = w[i];
-                if (anc) {
-                    x -= ew[1] * au[i];
+            for (int64_t b0 = i0 + tid; b0 < i1; b0 += ROWS * ORTH_THREADS) {
+                T wv[ROWS], uv[ROWS];
 #pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        if (k < nd) x -= ew[2 + k] * ay[(int64_t)k * n + i];
+                for (int u = 0; u < ROWS; ++u) {
+                    const int64_t i = b0 + u * ORTH_THREADS;
+                    wv[u] = i < i1 ? w[i] : (T)0;
+                    uv[u] = anc && i < i1 ? au[i] : (T)0;
                 }
-                x *= inv;
-                vn[i] = x;
-                if (vc) vc[i] = x;
+#pragma unroll
+                for (int u = 0; u < ROWS; ++u) {
+                    const int64_t i = b0 + u * ORTH_THREADS;
+                    if (i >= i1) break;
+                    T x = wv[u];
+                    if (anc) {
+                        x -= ew[1] * uv[u];
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            if (k < nd) x -= ew[2 + k] * ay[(int64_t)k * n + i];
+                    }
+                    x *= inv;
+                    vn[i] = x;
+                    if (vc) vc[i] = x;
+                }
             }
         }
     }
@@ -2168,7 +2233,9 @@ int hv_t(Ctx &c, const T *v, T *hv, const int *stop);
 template <>
 int hv_t<double>(Ctx &c, const double *v, double *hv, const int *stop) { return hv_device(c, v, hv, stop); }
 template <>
-int hv_t<float>(Ctx &c, const float *v, float *hv, const int *stop) { return hv_device_fp32(c, v, hv, stop); }
+int hv_t<float>(Ctx &c, const float *v, float *hv, const int *stop) {
+    return hv_device_fp32(c, v, hv, stop, false);    // k_orth adds the tensor-core planes
+}
 
 // Anchored refinement of one eigenvector (mixed precision, second phase):
 // the FP64 anchor u with theta0 = u.H.u and r = H u - theta0 u; the caller
@@ -2269,6 +2336,10 @@ int run_lanczos(Ctx &c, T *V, T *w, int neigen, int mmax, double tol, uint64_t s
     oa.xtot = z.xch + 1;
     oa.xcol = oa.xtot + (size_t)XCOLS * (XMAX + 1);
     oa.xpart = oa.xcol + (size_t)XW<T>::words * (cap + 8);
+    if (sizeof(T) == sizeof(float) && c.sb.mma_nitems) {
+        oa.tc = c.sb.d_mma_out;
+        oa.tcn = c.sb.mma_nplanes;
+    }
     // the launched chunks keep vcur current too, so that a replayed chunk
     // can follow one
     oa.vcur = c.use_graphs ? z.vcur : nullptr;

@@ -914,7 +914,7 @@ __global__ void __launch_bounds__(256) k_add_planes(float *__restrict__ hv, cons
     }
 }
 
-int hv_device_fp32(Ctx &c, const float *d_v, float *d_hv, const int *stop) {
+int hv_device_fp32(Ctx &c, const float *d_v, float *d_hv, const int *stop, bool add_planes) {
     DevSb &s = c.sb;
     if (!s.valid) {
         c.err = "nss_hv: no superblock uploaded";
@@ -947,6 +947,7 @@ int hv_device_fp32(Ctx &c, const float *d_v, float *d_hv, const int *stop) {
     NSS_CUDA_TRY(c, cudaEventRecord(c.hv_join, c.hv_side));
     if (int rc = hv_device_mma(c, d_v, stop)) return rc;
     NSS_CUDA_TRY(c, cudaStreamWaitEvent(c.stream, c.hv_join, 0));
+    if (!add_planes) return NSS_OK;
     int nsm = 0;
     NSS_CUDA_TRY(c, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c.device));
     k_add_planes<<<(unsigned)std::min<int64_t>(4 * nsm, (s.n + 255) / 256), 256, 0, c.stream>>>(
