@@ -2105,6 +2105,29 @@ __global__ void k_to32(float *__restrict__ out, const double *__restrict__ x, do
         out[i] = (float)(x[i] * s);
 }
 
+// The FP32 vectors of an anchored run: v = (float)(r s), the start vector,
+// u32 = (float)u, r32 = (float)r
+__global__ void k_anchor32(float *__restrict__ v, float *__restrict__ u32, float *__restrict__ r32,
+                           const double *__restrict__ u, const double *__restrict__ r, double s, int64_t n) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        v[i] = (float)(r[i] * s);
+        u32[i] = (float)u[i];
+        r32[i] = (float)r[i];
+    }
+}
+
+// The start of a batched solve's run: k_pro_reset, and zeros in the flags, beta
+// and the product slots that no item may write (one launch instead of four
+// calls a solve)
+__global__ void k_run_reset(float *pro, int ps, float eps1, int *flags, double *beta, int nbeta, float *slots, int64_t nslots) {
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t k = t; k < 2 * ps; k += nt) pro[k] = eps1;
+    if (t < PRO_TAIL) pro[2 * ps + t] = 0.f;
+    if (t < F_NFLAGS) flags[t] = 0;
+    for (int64_t k = t; k < nbeta; k += nt) beta[k] = 0.0;
+    for (int64_t k = t; k < nslots; k += nt) slots[k] = 0.f;
+}
+
 // x <- x / ||x|| on stream st (two launches)
 template <class T>
 void normalize_dev(DevLanczos &z, T *x, int64_t n, cudaStream_t st, int64_t &launches) {
@@ -2791,10 +2814,8 @@ int lanczos_eigh(Ctx &c, int neigen, int nitermax, double tol, uint64_t seed, in
         auto refine = [&](int e, double beta0) -> int {
             double *u = z.evecs + (int64_t)e * n;
             float *u32 = z.anc32, *r32 = z.anc32 + n, *y32 = z.anc32 + 2 * n;
-            c.launches += 3 + e;
-            k_to32<<<608, 256, 0, st>>>(z.V32, z.w, 1.0 / beta0, n);
-            k_to32<<<608, 256, 0, st>>>(u32, u, 1.0, n);
-            k_to32<<<608, 256, 0, st>>>(r32, z.w, 1.0, n);
+            c.launches += 1 + e;
+            k_anchor32<<<608, 256, 0, st>>>(z.V32, u32, r32, u, z.w, 1.0 / beta0, n);
             for (int f = 0; f < e; ++f)
                 k_to32<<<608, 256, 0, st>>>(y32 + (int64_t)f * n, z.evecs + (int64_t)f * n, 1.0, n);
             AnchorSpec as{u, u32, r32, y32, e, th[e], u};
@@ -2973,10 +2994,14 @@ struct BatchEngine {
     float *d_st = nullptr;
     unsigned *d_q = nullptr;     // item queue heads of a launch
     double *h_res = nullptr;     // [BATCH_MAX][8] pinned refinement results
+    cudaEvent_t forked = nullptr, joined[BATCH_MAX] = {};   // the solves' own streams leave and rejoin c0's
     size_t smem_set = 0;         // dynamic shared memory of its launches (the most any round needed)
     ~BatchEngine() {
         if (!c0) return;
         cudaStreamSynchronize(c0->stream);
+        if (forked) cudaEventDestroy(forked);
+        for (cudaEvent_t e : joined)
+            if (e) cudaEventDestroy(e);
         ctx_free(*c0, d_solves);
         ctx_free(*c0, d_gitems);
         ctx_free(*c0, d_st);
@@ -3001,6 +3026,7 @@ int engine_init(BatchEngine &E, Ctx &c0) {
     NSS_CUDA_TRY(c0, ctx_alloc(c0, &E.d_q, (size_t)CHUNK_MAXIT));
     NSS_CUDA_TRY(c0, cudaMallocHost((void **)&E.h_solves, sizeof(BatchSolve) * BATCH_MAX));
     NSS_CUDA_TRY(c0, cudaMallocHost((void **)&E.h_res, sizeof(double) * 8 * BATCH_MAX));
+    NSS_CUDA_TRY(c0, cudaEventCreateWithFlags(&E.forked, cudaEventDisableTiming));
     NSS_CUDA_TRY(c0, cudaMemsetAsync(c0.lz.counter, 0, 4 * sizeof(unsigned), c0.stream));
     NSS_CUDA_TRY(c0, cudaMemsetAsync(c0.lz.flags, 0, F_NFLAGS * sizeof(int), c0.stream));
     return NSS_OK;
@@ -3013,11 +3039,9 @@ int engine_start_run(BatchEngine &E, BatchState &B) {
     for (int i = 0; i < F_NFLAGS + 8; ++i) hf[i] = 0;
     for (int i = 0; i < 3 * (z.cap + 1); ++i) z.h_ab[i] = 0.0;
     cudaStream_t st = c0.stream;
-    NSS_CUDA_TRY(c0, cudaMemsetAsync(z.flags, 0, F_NFLAGS * sizeof(int), st));
-    NSS_CUDA_TRY(c0, cudaMemsetAsync(z.beta, 0, (z.cap + 1) * sizeof(double), st));
-    NSS_CUDA_TRY(c0, cudaMemsetAsync(z.slot32 + B.n, 0, (size_t)2 * B.n * sizeof(float), st));
     ++c0.launches;
-    k_pro_reset<<<1, 512, 0, st>>>(z.pro, z.cap + 8, Pro<float>::EPS1);
+    k_run_reset<<<(unsigned)std::min<int64_t>(152, (2 * B.n + 255) / 256), 256, 0, st>>>(
+        z.pro, z.cap + 8, Pro<float>::EPS1, z.flags, z.beta, z.cap + 1, z.slot32 + B.n, 2 * B.n);
     B.j0 = 0;
     B.from_v = true;
     B.have_upper = false;
@@ -3283,48 +3307,64 @@ int engine_step(BatchEngine &E, int max_done, int *ndone, int *ids, double *ener
     }
     for (int b = 0; b < (int)E.solves.size(); ++b)
         if (E.solves[b].phase == 3) p3.push_back(b);
-    // follow-up work, queued back to back: refinement results land in h_res
-    double *r = c0.lz.scal + S_NSCAL + 4 * (c0.lz.cap + 2);
+    // follow-up work, every solve on its own context's stream and scratch:
+    // refinement results land in h_res.  Its kernels are latency (60 us a solve
+    // of a few thousand states); one after the other on the engine's stream
+    // they took a third of a batch's device time
+    auto fork = [&](BatchState &B) -> int {
+        if (B.c->stream != st) NSS_CUDA_TRY(c0, cudaStreamWaitEvent(B.c->stream, E.forked, 0));
+        return NSS_OK;
+    };
+    auto join = [&](BatchState &B, int slot) -> int {
+        if (B.c->stream == st) return NSS_OK;
+        if (!E.joined[slot]) NSS_CUDA_TRY(c0, cudaEventCreateWithFlags(&E.joined[slot], cudaEventDisableTiming));
+        NSS_CUDA_TRY(c0, cudaEventRecord(E.joined[slot], B.c->stream));
+        NSS_CUDA_TRY(c0, cudaStreamWaitEvent(st, E.joined[slot], 0));
+        return NSS_OK;
+    };
     auto fp64_energy = [&](BatchState &B, int slot, bool anchor) -> int {
         Ctx &c = *B.c;
         DevLanczos &z = c.lz;
-        const cudaStream_t keep = c.stream;
-        c.stream = st;
-        int r2 = hv_device(c, z.evecs, z.w);
-        c.stream = keep;
-        if (r2) { c0.err = c.err; return r2; }
+        const cudaStream_t s = c.stream;
+        double *r = z.scal + S_NSCAL + 4 * (z.cap + 2);
+        if (int r2 = hv_device(c, z.evecs, z.w)) { c0.err = c.err; return r2; }
         ++B.numop;
         c0.launches += 2;
-        k_rq<<<NBLK, 256, 0, st>>>(z.evecs, z.w, B.n, z.part, r, c0.lz.counter);
-        if (anchor) k_anchor_r<<<NBLK, 256, 0, st>>>(z.evecs, z.w, B.n, z.part, r, c0.lz.counter);
-        else k_resid<<<NBLK, 256, 0, st>>>(z.evecs, z.w, B.n, z.part, r, c0.lz.counter);
-        NSS_CUDA_TRY(c0, cudaMemcpyAsync(E.h_res + 8 * slot, r, 8 * sizeof(double), cudaMemcpyDeviceToHost, st));
+        k_rq<<<NBLK, 256, 0, s>>>(z.evecs, z.w, B.n, z.part, r, z.counter);
+        if (anchor) k_anchor_r<<<NBLK, 256, 0, s>>>(z.evecs, z.w, B.n, z.part, r, z.counter);
+        else k_resid<<<NBLK, 256, 0, s>>>(z.evecs, z.w, B.n, z.part, r, z.counter);
+        NSS_CUDA_TRY(c0, cudaMemcpyAsync(E.h_res + 8 * slot, r, 8 * sizeof(double), cudaMemcpyDeviceToHost, s));
         return NSS_OK;
     };
+    if (!p1.empty() || !p2.empty() || !p3.empty()) NSS_CUDA_TRY(c0, cudaEventRecord(E.forked, st));
     int rc = NSS_OK;
     for (int b : p1) {
         BatchState &B = E.solves[b];
         DevLanczos &z = B.c->lz;
         const int m = B.m_done;
-        NSS_CUDA_TRY(c0, cudaMemcpyAsync(z.svec, B.svec.data(), (size_t)m * sizeof(double), cudaMemcpyHostToDevice, st));
+        const cudaStream_t s = B.c->stream;
+        if ((rc = fork(B))) return rc;
+        NSS_CUDA_TRY(c0, cudaMemcpyAsync(z.svec, B.svec.data(), (size_t)m * sizeof(double), cudaMemcpyHostToDevice, s));
         c0.launches += 2;
-        k_ritz<float><<<NBLK, 256, (size_t)m * sizeof(double), st>>>(z.V32, m, B.n, z.svec, m, 1, z.evecs);
-        normalize_dev<double>(z, z.evecs, B.n, st, c0.launches);
-        if ((rc = fp64_energy(B, b, true))) return rc;
+        k_ritz<float><<<NBLK, 256, (size_t)m * sizeof(double), s>>>(z.V32, m, B.n, z.svec, m, 1, z.evecs);
+        normalize_dev<double>(z, z.evecs, B.n, s, c0.launches);
+        if ((rc = fp64_energy(B, b, true)) || (rc = join(B, b))) return rc;
     }
     for (int b : p2) {
         BatchState &B = E.solves[b];
         DevLanczos &z = B.c->lz;
+        const cudaStream_t s = B.c->stream;
+        if ((rc = fork(B))) return rc;
         NSS_CUDA_TRY(c0, cudaMemcpyAsync(z.svec, B.cvec.data(), B.cvec.size() * sizeof(double), cudaMemcpyHostToDevice,
-                                         st));
+                                         s));
         c0.launches += 2;
-        k_ritz_anchor<float><<<NBLK, 256, B.cvec.size() * sizeof(double), st>>>(z.V32, B.m_done, B.n, z.svec, z.evecs,
-                                                                                z.evecs);
-        normalize_dev<double>(z, z.evecs, B.n, st, c0.launches);
-        if ((rc = fp64_energy(B, b, false))) return rc;
+        k_ritz_anchor<float><<<NBLK, 256, B.cvec.size() * sizeof(double), s>>>(z.V32, B.m_done, B.n, z.svec, z.evecs,
+                                                                               z.evecs);
+        normalize_dev<double>(z, z.evecs, B.n, s, c0.launches);
+        if ((rc = fp64_energy(B, b, false)) || (rc = join(B, b))) return rc;
     }
     for (int b : p3)
-        if ((rc = fp64_energy(E.solves[b], b, false))) return rc;
+        if ((rc = fork(E.solves[b])) || (rc = fp64_energy(E.solves[b], b, false)) || (rc = join(E.solves[b], b))) return rc;
     NSS_CUDA_TRY(c0, cudaStreamSynchronize(st));
     auto finish = [&](BatchState &B, int slot) -> int {
         const double *hr = E.h_res + 8 * slot;
@@ -3349,10 +3389,8 @@ int engine_step(BatchEngine &E, int max_done, int *ndone, int *ids, double *ener
             continue;
         }
         float *u32 = z.anc32, *r32 = z.anc32 + B.n;
-        c0.launches += 3;
-        k_to32<<<608, 256, 0, st>>>(z.V32, z.w, 1.0 / beta0, B.n);
-        k_to32<<<608, 256, 0, st>>>(u32, z.evecs, 1.0, B.n);
-        k_to32<<<608, 256, 0, st>>>(r32, z.w, 1.0, B.n);
+        ++c0.launches;
+        k_anchor32<<<608, 256, 0, st>>>(z.V32, u32, r32, z.evecs, z.w, 1.0 / beta0, B.n);
         B.as = AnchorSpec{z.evecs, u32, r32, z.anc32 + 2 * B.n, 0, B.theta0, z.evecs};
         if ((rc = engine_start_run(E, B))) return rc;
         B.phase = 2;
