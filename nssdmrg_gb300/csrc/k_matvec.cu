@@ -512,7 +512,7 @@ int sb_upload(Ctx &c, const nss_sb_desc *d, bool trusted) {
                 if (split) {
                     items32.push_back(make_int4(k, r, cc, HV_LEFT));
                     items32.push_back(make_int4(k, r, cc, HV_RIGHT));
-                    if (s.term_ptr[k + 1] > s.term_ptr[k]) items32.push_back(make_int4(k, r, cc, HV_TERMS));
+                    items32.push_back(make_int4(k, r, cc, HV_TERMS));   // without terms: zeros, the slot is read
                 } else {
                     items32.push_back(make_int4(k, r, cc, HV_FULL));
                 }
