@@ -680,15 +680,16 @@ def run_gpu(args):
         desc0 = d.export_superblock()
         op_bytes = 4 * sum(desc0.dls[k] ** 2 + desc0.drs[k] ** 2 for k in range(desc0.nsb))
         mbar = tcols / max(tit, 1)
-        # per iteration: the basis read by the projections and by the update
-        # (2 m N floats), ~10 N floats of vector traffic (slots, three-term
-        # step, next vector), the FP32 sector blocks read by the H*psi items
-        bytes_it = 2 * 4 * n * mbar + 40 * n + op_bytes
+        # per iteration: ~10 N floats of vector traffic (slots, three-term
+        # step, next vector) and the FP32 sector blocks read by the H*psi
+        # items; the few steps that project against the basis (2 m N floats
+        # each) are not counted
+        bytes_it = 40 * n + op_bytes
         t_it = tms / 1e3 / max(tit, 1)
         chunk = {"launches": tl, "iterations": int(tit), "ms_per_launch": tms / max(tl, 1),
                  "us_per_iteration": t_it * 1e6, "mean_basis_m": mbar, "bytes_per_iteration": bytes_it,
                  "achieved_gbs": bytes_it / t_it / 1e9,
-                 "flops_per_iteration": f_hv + 4 * n * mbar, "achieved_tflops": (f_hv + 4 * n * mbar) / t_it / 1e12}
+                 "flops_per_iteration": f_hv, "achieved_tflops": f_hv / t_it / 1e12}
     if args.profile:
         if rank == 0:
             print(json.dumps({"profile_run": True, "ms_per_step": head["ms_per_step"],

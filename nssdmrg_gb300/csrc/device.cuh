@@ -250,6 +250,8 @@ struct Ctx {
     void *solver = nullptr;      // cusolverDnHandle_t
     DevSb sb;
     DevLanczos lz;
+    char *lz_arena = nullptr, *lz_host = nullptr;   // its arrays, its host mirrors (kept from solve to solve)
+    size_t lz_arena_bytes = 0, lz_host_bytes = 0;
     DevRdm rdm;
     DevRenorm ren;
     int64_t launches = 0;        // kernels of this library launched
@@ -397,7 +399,7 @@ void batch_destroy(BatchEngine *e);
 int batch_add(BatchEngine *e, Ctx &c, uint64_t seed, int nitermax, double tol, int *id);
 int batch_step(BatchEngine *e, int max_done, int *ndone, int *ids, double *energies, int *numops);
 int batch_inflight(const BatchEngine *e);
-void lanczos_release(Ctx &c);
+void lanczos_release(Ctx &c, bool keep = false);
 
 // k_syev.cu: FP64 eigensolver of the rho blocks.  Blocks up to SYEV_MAX
 // are reduced to tridiagonal form in one CTA (k_trd); larger ones, up to

@@ -2144,22 +2144,65 @@ inline size_t x_words(int pstride, int w) {
 // per-eigenvector scratch row of svec
 inline int svec_stride(int cap) { return 4 * (cap + 1); }
 
+// Memory for a Lanczos workspace.  A DMRG run solves another size at every
+// step; allocating and freeing two dozen arrays took 100 to 260 us a step
+// (of 2 ms in a chain of 20 spins), so they are sections of one block that the
+// context keeps while it fits: with a quarter to spare (64 MB at most), given
+// back when less than a quarter of it would be used (above 64 MB) and with the
+// context.  A context with a budget allocates each array for itself, so that
+// what it holds is what the solve needs.
+int workspace(Ctx &c, const std::vector<std::pair<void **, size_t>> &want) {
+    if (c.budget) {
+        for (auto &w : want) {
+            char *p = nullptr;
+            NSS_CUDA_TRY(c, ctx_alloc(c, &p, w.second));
+            *w.first = p;
+        }
+        return NSS_OK;
+    }
+    auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    size_t need = 0;
+    for (auto &w : want) need += up(w.second);
+    constexpr size_t SMALL = (size_t)64 << 20;
+    if (need > c.lz_arena_bytes || (c.lz_arena_bytes > SMALL && need < c.lz_arena_bytes / 4)) {
+        ctx_free(c, c.lz_arena);
+        c.lz_arena = nullptr;
+        c.lz_arena_bytes = 0;
+        const size_t roomy = std::max(need + std::min(need / 4, SMALL), (size_t)8 << 20);
+        if (ctx_alloc(c, &c.lz_arena, roomy) == cudaSuccess) {
+            c.lz_arena_bytes = roomy;
+        } else {
+            cudaGetLastError();                      // no room for the spare part
+            NSS_CUDA_TRY(c, ctx_alloc(c, &c.lz_arena, need));
+            c.lz_arena_bytes = need;
+        }
+    }
+    size_t at = 0;
+    for (auto &w : want) {
+        *w.first = c.lz_arena + at;
+        at += up(w.second);
+    }
+    return NSS_OK;
+}
+
 int ensure_lanczos(Ctx &c, int64_t n, int cap, bool mixed) {
     DevLanczos &z = c.lz;
     // reuse only buffers shaped for this mode: the FP64 method needs a whole
     // FP64 basis in V, the mixed one an FP32 basis in V32
     if (z.V && z.n == n && z.cap >= cap && (mixed ? (z.V32 != nullptr) : z.full64)) return NSS_OK;
-    lanczos_release(c);
+    lanczos_release(c, true);
     z.n = n;
     z.cap = cap;
+    std::vector<std::pair<void **, size_t>> want;    // the workspace's arrays and their bytes
+    auto add = [&](auto *p, size_t count) { want.push_back({(void **)p, std::max<size_t>(count * sizeof(**p), 16)}); };
     if (mixed) {
-        NSS_CUDA_TRY(c, ctx_alloc(c, &z.V32, (size_t)(cap + 1) * n));
-        NSS_CUDA_TRY(c, ctx_alloc(c, &z.w32, (size_t)n));
-        NSS_CUDA_TRY(c, ctx_alloc(c, &z.anc32, (size_t)6 * n));   // FP32 anchor, residual, deflation set
-        NSS_CUDA_TRY(c, ctx_alloc(c, &z.V, (size_t)n));   // FP64 refinement scratch
+        add(&z.V32, (size_t)(cap + 1) * n);
+        add(&z.w32, (size_t)n);
+        add(&z.anc32, (size_t)6 * n);   // FP32 anchor, residual, deflation set
+        add(&z.V, (size_t)n);   // FP64 refinement scratch
         z.full64 = false;
     } else {
-        NSS_CUDA_TRY(c, ctx_alloc(c, &z.V, (size_t)(cap + 1) * n));
+        add(&z.V, (size_t)(cap + 1) * n);
         z.full64 = true;
     }
     int dev = 0, nsm = 0;
@@ -2202,8 +2245,8 @@ int ensure_lanczos(Ctx &c, int64_t n, int cap, bool mixed) {
                                                                           csm));
         }
         if (occ2 >= 1) {
-            NSS_CUDA_TRY(c, ctx_alloc(c, &z.wbuf32, (size_t)2 * n));
-            NSS_CUDA_TRY(c, ctx_alloc(c, &z.slot32, (size_t)3 * n));
+            add(&z.wbuf32, (size_t)2 * n);
+            add(&z.slot32, (size_t)3 * n);
             z.chunk_smem = csm;
             z.chunk_vc = vc;
             z.chunk_cs = vc > 0 ? cs : 0;
@@ -2211,34 +2254,48 @@ int ensure_lanczos(Ctx &c, int64_t n, int cap, bool mixed) {
             z.chunk_ok = true;
         }
     }
-    NSS_CUDA_TRY(c, ctx_alloc(c, &z.w, (size_t)n));
-    {
-        double *vc = nullptr;
-        NSS_CUDA_TRY(c, ctx_alloc(c, &vc, (size_t)n));
-        z.vcur = vc;
-    }
-    NSS_CUDA_TRY(c, ctx_alloc(c, &z.jdev, 1));
+    add(&z.w, (size_t)n);
+    double *vcur = nullptr;
+    add(&vcur, (size_t)n);
+    add(&z.jdev, 1);
     // exchange words: epoch (one word), totals, column partials, column totals
     z.xwords = x_words(pstride, mixed ? 1 : 2);
-    NSS_CUDA_TRY(c, ctx_alloc(c, &z.xch, z.xwords));
-    NSS_CUDA_TRY(c, ctx_alloc(c, &z.pro, (size_t)2 * pstride + PRO_TAIL));
-    NSS_CUDA_TRY(c, ctx_alloc(c, &z.evecs, (size_t)4 * n));
+    add(&z.xch, z.xwords);
+    add(&z.pro, (size_t)2 * pstride + PRO_TAIL);
+    add(&z.evecs, (size_t)4 * n);
     // scalars, projection coefficients, restart scratch alpha/beta, refinement
-    NSS_CUDA_TRY(c, ctx_alloc(c, &z.scal, (size_t)S_NSCAL + 4 * (cap + 2) + 8));
+    add(&z.scal, (size_t)S_NSCAL + 4 * (cap + 2) + 8);
     const size_t part = std::max((size_t)(cap + 2) * NBLK, (size_t)(2 * pstride + 2 * PA_COLS + 2) * (size_t)nsm);
-    NSS_CUDA_TRY(c, ctx_alloc(c, &z.part, part));
-    NSS_CUDA_TRY(c, ctx_alloc(c, &z.counter, 4));
-    NSS_CUDA_TRY(c, ctx_alloc(c, &z.alpha, (size_t)cap + 1));
-    NSS_CUDA_TRY(c, ctx_alloc(c, &z.beta, (size_t)cap + 1));
-    NSS_CUDA_TRY(c, ctx_alloc(c, &z.theta, 8));
-    NSS_CUDA_TRY(c, ctx_alloc(c, &z.resid, 8));
-    NSS_CUDA_TRY(c, ctx_alloc(c, &z.svec, (size_t)4 * svec_stride(cap)));
-    NSS_CUDA_TRY(c, ctx_alloc(c, &z.flags, F_NFLAGS));
-    // host-mapped mirrors: alpha, beta, anchor couplings m; flags + the host's stop request
-    NSS_CUDA_TRY(c, cudaHostAlloc((void **)&z.h_ab, 3 * (size_t)(cap + 1) * sizeof(double), cudaHostAllocMapped));
-    NSS_CUDA_TRY(c, cudaHostAlloc((void **)&z.h_flags, (F_NFLAGS + 8) * sizeof(int), cudaHostAllocMapped));
-    NSS_CUDA_TRY(c, cudaHostGetDevicePointer((void **)&z.d_h_ab, z.h_ab, 0));
-    NSS_CUDA_TRY(c, cudaHostGetDevicePointer((void **)&z.d_h_flags, z.h_flags, 0));
+    add(&z.part, part);
+    add(&z.counter, 4);
+    add(&z.alpha, (size_t)cap + 1);
+    add(&z.beta, (size_t)cap + 1);
+    add(&z.theta, 8);
+    add(&z.resid, 8);
+    add(&z.svec, (size_t)4 * svec_stride(cap));
+    add(&z.flags, F_NFLAGS);
+    // host-mapped mirrors: flags + the host's stop request; alpha, beta, anchor couplings m
+    const size_t hflags = 256, hbytes = hflags + 3 * (size_t)(cap + 1) * sizeof(double);
+    static_assert((F_NFLAGS + 8) * sizeof(int) <= 256, "flag mirror");
+    if (hbytes > c.lz_host_bytes) {
+        if (c.lz_host) cudaFreeHost(c.lz_host);
+        c.lz_host = nullptr;
+        c.lz_host_bytes = 0;
+        NSS_CUDA_TRY(c, cudaHostAlloc((void **)&c.lz_host, hbytes, cudaHostAllocMapped));
+        c.lz_host_bytes = hbytes;
+    }
+    char *dh = nullptr;
+    NSS_CUDA_TRY(c, cudaHostGetDevicePointer((void **)&dh, c.lz_host, 0));
+    if (int rc = workspace(c, want)) {
+        z.vcur = vcur;
+        lanczos_release(c, true);
+        return rc;
+    }
+    z.vcur = vcur;
+    z.h_flags = (int *)c.lz_host;
+    z.h_ab = (double *)(c.lz_host + hflags);
+    z.d_h_flags = (int *)dh;
+    z.d_h_ab = (double *)(dh + hflags);
     NSS_CUDA_TRY(c, cudaMemsetAsync(z.counter, 0, 4 * sizeof(unsigned), c.stream));
     return NSS_OK;
 }
@@ -2677,14 +2734,25 @@ int run_lanczos(Ctx &c, T *V, T *w, int neigen, int mmax, double tol, uint64_t s
 
 }  // namespace
 
-void lanczos_release(Ctx &c) {
+// keep: the block of the workspace's arrays and the host mirrors stay for the next
+void lanczos_release(Ctx &c, bool keep) {
     DevLanczos &z = c.lz;
-    void *ptrs[] = {z.V, z.w, z.V32, z.w32, z.anc32, z.wbuf32, z.slot32, z.evecs, z.rrw, z.scal, z.part, z.counter,
-                    z.alpha, z.beta, z.theta, z.resid, z.svec, z.flags, z.pitem, z.vcur, z.jdev, z.pro, z.xch};
     if (z.gx) cudaGraphExecDestroy(z.gx);
-    for (void *p : ptrs) ctx_free(c, p);
-    if (z.h_flags) cudaFreeHost(z.h_flags);
-    if (z.h_ab) cudaFreeHost(z.h_ab);
+    ctx_free(c, z.rrw);
+    ctx_free(c, z.pitem);
+    if (c.budget) {
+        void *ptrs[] = {z.V, z.w, z.V32, z.w32, z.anc32, z.wbuf32, z.slot32, z.evecs, z.scal, z.part, z.counter,
+                        z.alpha, z.beta, z.theta, z.resid, z.svec, z.flags, z.vcur, z.jdev, z.pro, z.xch};
+        for (void *p : ptrs) ctx_free(c, p);
+    }
+    if (!keep) {
+        ctx_free(c, c.lz_arena);
+        c.lz_arena = nullptr;
+        c.lz_arena_bytes = 0;
+        if (c.lz_host) cudaFreeHost(c.lz_host);
+        c.lz_host = nullptr;
+        c.lz_host_bytes = 0;
+    }
     z = DevLanczos{};
 }
 
@@ -3073,6 +3141,7 @@ int engine_add(BatchEngine &E, Ctx &c, uint64_t seed, int nitermax, double tol, 
     B.upper.assign(4, 0.0);
     int rc = ensure_lanczos(c, B.n, B.mmax + 1, true);
     if (rc) { c0.err = c.err; return rc; }
+    NSS_CUDA_TRY(c0, cudaStreamSynchronize(c.stream));   // the engine works on its own stream
     DevLanczos &z = c.lz;
     if (!z.chunk_ok) { c0.err = "nss_batch_add: the persistent kernel does not fit this Krylov basis"; return NSS_ERR_INVALID; }
     if (!z.pitem || z.cap_pitem < c.sb.nitems32) {
