@@ -22,8 +22,8 @@
 // H on its span, so Ritz values are as accurate as with a projection at every
 // step; the threshold lies lower (struct Pro) so that the vectors are too.  On
 // the measured superblocks 4 to 12 of 50 to 100 steps project.  A projection
-// reads the basis twice (2 N m sizeof(T) bytes) and costs two more grid
-// barriers.  Against projecting at every step, solves went from 5.6 to 3.3 ms
+// reads the basis twice (2 N m sizeof(T) bytes) and costs two more grid-wide
+// exchanges.  Against projecting at every step, solves went from 5.6 to 3.3 ms
 // (FP64, N = 3 958), 13.1 to 10.1 ms (FP64, 66 600), 2.72 to 2.52 ms (mixed,
 // 66 600), 13.9 to 10.8 ms (mixed, 398 000), and 16 batched solves of up to
 // 9 500 states from 10.9 to 10.1 ms.
@@ -31,14 +31,15 @@
 // Per iteration j (m = j+1 basis vectors) two kinds of launch:
 //   sector H*psi   w = H v_j                      (k_hv_* kernels)
 //   k_orth         one cooperative launch, one CTA per SM, each CTA owning a
-//                  contiguous slice of the rows; grid barriers separate
+//                  contiguous slice of the rows; exchanges of sums separate
 //                    alpha = v_j . w
 //                    w -= alpha v_j + beta_{j-1} v_{j-1};  beta^2 = w.w
 //                    (at a projecting step: h = V_m^T w; w -= V_m h, beta^2 =
 //                    w.w, again if it fell by more than half)
 //                    v_{j+1} = w / beta, or the breakdown flag
-// Every grid-level sum is reduced by every CTA in the same fixed order, so
-// all CTAs hold bitwise identical scalars and take the same branches.
+// Every grid-level sum is formed in one fixed order, by one CTA in k_orth
+// (xchg_totals) and by every CTA alike in the persistent kernels, so all CTAs
+// hold bitwise identical scalars and take the same branches.
 //
 // The tridiagonal problem (m <= a few hundred) is a chain of dependent FP64
 // operations, which GB300's narrow FP64 pipe runs slowly on one SM; it is
