@@ -2441,6 +2441,7 @@ int run_lanczos(Ctx &c, T *V, T *w, int neigen, int mmax, double tol, uint64_t s
     if (use_chunk)   // slot 1 and 2 regions that no item writes must read as zero
         NSS_CUDA_TRY(c, cudaMemsetAsync(z.slot32 + n, 0, (size_t)2 * n * sizeof(float), st));
     bool from_v = true;   // the next chunk starts from V[j0] (start, restart)
+    int jdev_next = -1;   // the step that queued replays leave in *jdev (-1: not known)
     auto enqueue_chunk = [&](int j0, int slot) -> int {
         const int jend = std::min(mmax, j0 + CHECK);
         if (from_v) {
@@ -2498,9 +2499,13 @@ int run_lanczos(Ctx &c, T *V, T *w, int neigen, int mmax, double tol, uint64_t s
             if (from_v)
                 NSS_CUDA_TRY_R(c, cudaMemcpyAsync(z.vcur, V + (int64_t)j0 * n, (size_t)n * sizeof(T),
                                                   cudaMemcpyDeviceToDevice, st), -1);
-            k_seti<<<1, 1, 0, st>>>(z.jdev, j0);
+            if (jdev_next != j0) {                   // else the replay before left it there
+                k_seti<<<1, 1, 0, st>>>(z.jdev, j0);
+                ++c.launches;
+            }
             NSS_CUDA_TRY_R(c, cudaGraphLaunch(z.gx, st), -1);
-            c.launches += 1 + z.gx_launches;
+            jdev_next = jend;
+            c.launches += z.gx_launches;
             ++c.graph_replays;
             from_v = false;
             cudaEventRecord(evs[slot], st);
@@ -2639,6 +2644,7 @@ int run_lanczos(Ctx &c, T *V, T *w, int neigen, int mmax, double tol, uint64_t s
             hf[F_STOP] = 0;
             hf[F_BREAK] = 0;
             from_v = true;
+            jdev_next = -1;       // the chunk ended early
             slot = 0;
             pend_end = enqueue_chunk(m_done, slot);
             if (pend_end < 0) { rc = NSS_ERR_CUDA; break; }
