@@ -63,6 +63,7 @@
 // 1e-7), whose FP64 residual ||H psi - E psi|| is reported.  On GB300 the
 // FP64 pipe runs at about 1/70 of the FP32 one (1.06 against 78 TFLOP/s
 // measured), which is what the mixed method buys.
+#include "batch_words.hpp"
 #include "device.cuh"
 #include "host_tridiag.hpp"
 #include "hv_tile.cuh"
@@ -1591,7 +1592,7 @@ struct BatchArgs {
     int ns;
     int nitems;                  // items of all active solves
     const int2 *gitems;          // (solve, item) in processing order
-    float *st;                   // [4 ns] per-solve scalars published inside an iteration
+    float *st;                   // [ST_WORDS ns] per-solve scalars published inside an iteration (batch_words.hpp)
     unsigned *bar;               // global barrier
     int *err;
     int steps;                   // iterations of this launch
@@ -1734,8 +1735,8 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_batch32(BatchArgs B) {
                 pW[Gs + lb] = sv[1];
                 pW[2 * Gs + lb] = sv[2];
                 if (lb == 0) {
-                    B.st[4 * me + 0] = alpha0;
-                    B.st[4 * me + 1] = 0.f;          // h_j of a projection
+                    B.st[ST_WORDS * me + ST_ALPHA] = alpha0;
+                    B.st[ST_WORDS * me + ST_HJ] = 0.f;          // h_j of a projection
                 }
             }
         }
@@ -1749,8 +1750,9 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_batch32(BatchArgs B) {
             if (!alive[s] || S.c.j0 + step >= S.c.jend) continue;
             const float *pWs = (const float *)S.c.o.part + (PA_COLS + 2 * (int64_t)S.c.o.pstride + 2) * S.ncta;
             bbb[s] = strided_sum<float>(pWs, 0, S.ncta, 1);
-            balpha[s] = __ldcg(B.st + 4 * s + 0);
-            const int ow = step == 0 ? __ldcg((const int *)(S.c.o.pro + 2 * S.c.o.pstride)) : __float_as_int(__ldcg(B.st + 4 * s + 3));
+            balpha[s] = __ldcg(B.st + ST_WORDS * s + ST_ALPHA);
+            const int ow = step == 0 ? __ldcg((const int *)(S.c.o.pro + 2 * S.c.o.pstride))
+                                     : __float_as_int(__ldcg(B.st + ST_WORDS * s + owed_word(step - 1)));
             p2[s] = 1;
             if (ow > 0 || pro_always<float>(S.c.j0 + step + 1, S.c.o.n, S.c.o.pstride)) any_p2 = 1;
         }
@@ -1794,7 +1796,7 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_batch32(BatchArgs B) {
                 grid_columns<float>(ph, Gs, m, hs);
                 __syncthreads();
                 hj += hs[jj];
-                if (lb == 0 && tid == 0) B.st[4 * me + 1] = hj;
+                if (lb == 0 && tid == 0) B.st[ST_WORDS * me + ST_HJ] = hj;
                 float s1[1] = {update()};
                 block_sums<float, 1>(s1, scr, nw);
                 if (tid == 0) pb[lb] = s1[0];
@@ -1810,7 +1812,7 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_batch32(BatchArgs B) {
                 const float t = strided_sum<float>(pBs, 0, S.ncta, 1);
                 const bool again = round == 0 && t < 0.5f * bbb[s];
                 bbb[s] = t;
-                balpha[s] = __ldcg(B.st + 4 * s + 0) + __ldcg(B.st + 4 * s + 1);
+                balpha[s] = __ldcg(B.st + ST_WORDS * s + ST_ALPHA) + __ldcg(B.st + ST_WORDS * s + ST_HJ);
                 p2[s] = again;
                 if (again) any_p2 = 1;
             }
@@ -1841,7 +1843,7 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_batch32(BatchArgs B) {
                 rec_a[done] = balpha[me];
                 rec_b[done] = bprev[me];
                 rec_m[done] = mj;
-                B.st[4 * me + 3] = __int_as_float(owed);   // read by all after the next step's barriers
+                B.st[ST_WORDS * me + owed_word(step)] = __int_as_float(owed);   // read by all in the next step
             }
             if (tid == 0) pro.set(jj, balpha[me], bprev[me]);
             dm = dc;
@@ -3097,7 +3099,7 @@ int engine_init(BatchEngine &E, Ctx &c0) {
         if (rc) return rc;
     }
     NSS_CUDA_TRY(c0, ctx_alloc(c0, &E.d_solves, (size_t)BATCH_MAX));
-    NSS_CUDA_TRY(c0, ctx_alloc(c0, &E.d_st, (size_t)4 * BATCH_MAX));
+    NSS_CUDA_TRY(c0, ctx_alloc(c0, &E.d_st, (size_t)ST_WORDS * BATCH_MAX));
     NSS_CUDA_TRY(c0, ctx_alloc(c0, &E.d_q, (size_t)CHUNK_MAXIT));
     NSS_CUDA_TRY(c0, cudaMallocHost((void **)&E.h_solves, sizeof(BatchSolve) * BATCH_MAX));
     NSS_CUDA_TRY(c0, cudaMallocHost((void **)&E.h_res, sizeof(double) * 8 * BATCH_MAX));
