@@ -65,6 +65,7 @@
 // measured), which is what the mixed method buys.
 #include "batch_words.hpp"
 #include "device.cuh"
+#include "func_limits.hpp"
 #include "host_tridiag.hpp"
 #include "hv_tile.cuh"
 
@@ -98,24 +99,6 @@ double mixed_tol() {
     }();
     return v;
 }
-// Raise a kernel's dynamic shared-memory limit on the current device to at
-// least `bytes`.  The attribute belongs to the kernel, shared by every
-// context of the process, so it only ever grows: a context sized for a
-// smaller basis must not take the room a larger one was set up with.
-inline cudaError_t allow_smem(const void *fn, size_t bytes) {
-    if (bytes <= 48 * 1024) return cudaSuccess;
-    static std::mutex mu;
-    static std::map<std::pair<int, const void *>, size_t> done;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    std::lock_guard<std::mutex> lk(mu);
-    size_t &cur = done[{dev, fn}];
-    if (bytes <= cur) return cudaSuccess;
-    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e == cudaSuccess) cur = bytes;
-    return e;
-}
-
 constexpr int ORTH_THREADS = 512;
 constexpr int ORTH_WARPS = ORTH_THREADS / 32;
 

@@ -53,13 +53,13 @@
 // runs out sets the error word, every role stops, the producer waits for
 // the copies it issued, the MMA lane for its MMAs, and the CTA frees its
 // TMEM and returns.
+#include "func_limits.hpp"
 #include "sector_mma.cuh"
 #include "tc_common.cuh"
 
 #include <cudaTypedefs.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cstring>
 #include <vector>
 
@@ -451,12 +451,7 @@ namespace {
 
 template <int BN, int KPS>
 int launch_mma(Ctx &c, const CUtensorMap &ma, const CUtensorMap &mb, uint32_t spin, const int *stop) {
-    static std::atomic<bool> done{false};
-    if (!done.load()) {
-        NSS_CUDA_TRY(c, cudaFuncSetAttribute(k_sector_mma<BN, KPS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             MmaCfg<BN>::SMEM));
-        done.store(true);
-    }
+    NSS_CUDA_TRY(c, allow_smem((const void *)k_sector_mma<BN, KPS>, MmaCfg<BN>::SMEM));
     DevSb &s = c.sb;
     k_sector_mma<BN, KPS><<<s.mma_grid, MM_THREADS, MmaCfg<BN>::SMEM, c.stream>>>(
         ma, mb, s.d_mma_items, s.d_mma_rng, s.d_mma_out, s.n, c.mma_lolo ? 1 : 0, spin, s.d_tc_err, stop);

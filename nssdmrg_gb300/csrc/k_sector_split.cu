@@ -36,11 +36,11 @@
 // (seven A digit boxes, released one by one as their MMAs finish; the seven B
 // boxes double buffered), one lane the MMAs, eight warps drain.  Every wait is
 // bounded as in k_sector_mma.cu.
+#include "func_limits.hpp"
 #include "sector_split.cuh"
 #include "tc_common.cuh"
 
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <cstring>
 
@@ -733,8 +733,7 @@ int split_finish(Ctx &c, const SplitPlan &p) {
     const int part = p.kmax <= SP_STRIP ? p.kmax : SP_STRIP;   // widest strip of a job
     const size_t smem = (size_t)SP_ROWS * (part | 1) * sizeof(double);
     s.sp_pack_smem = smem;
-    NSS_CUDA_TRY(c, cudaFuncSetAttribute(k_split_pack, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(SP_ROWS * (SP_STRIP | 1) * sizeof(double))));
+    NSS_CUDA_TRY(c, allow_smem((const void *)k_split_pack, smem));
     c.launches += 2;
     k_split_pack<<<(unsigned)p.jobs_hl.size(), 32 * SP_ROWS, smem, c.stream>>>(s.d_hl, s.d_sp_jobs_hl, s.d_sp_pool, s.d_sp_exp,
                                                                             nullptr, nullptr);
@@ -757,11 +756,7 @@ namespace {
 
 template <int BN>
 int launch_split(Ctx &c, const int *stop) {
-    static std::atomic<bool> done{false};
-    if (!done.load()) {
-        NSS_CUDA_TRY(c, cudaFuncSetAttribute(k_sector_split<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitCfg<BN>::SMEM));
-        done.store(true);
-    }
+    NSS_CUDA_TRY(c, allow_smem((const void *)k_sector_split<BN>, SplitCfg<BN>::SMEM));
     DevSb &s = c.sb;
     alignas(64) CUtensorMap ma, mb;
     std::memcpy(&ma, s.sp_map_a, sizeof(ma));

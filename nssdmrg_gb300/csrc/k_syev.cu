@@ -45,6 +45,7 @@
 //             block, and the host recomputes that block's vectors with the
 //             library eigensolver.
 #include "device.cuh"
+#include "func_limits.hpp"
 
 #include <cooperative_groups.h>
 
@@ -1560,8 +1561,7 @@ int syev_trd_cl_size(int *nmax_out) {
     // found once per process (thread-safe initialisation)
     static const Limits lim = [] {
         int csize = 0, nmax = 0;
-        cudaFuncSetAttribute(k_trd_cl<false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        cudaFuncSetAttribute(k_trd_cl<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        raise_attribute((const void *)k_trd_cl<false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         const int smem = 200 * 1024;
         cudaFuncSetAttribute(k_trd_cl<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         cudaLaunchConfig_t cfg = {};
@@ -1603,6 +1603,7 @@ int syev_trd_cl(const double *rho, const int64_t *rho_off, const int *dims, cons
     const size_t smem = ((size_t)(glob ? 4 : ncmax + 4) * maxn + 2 * ncmax + 8) * sizeof(double);
     auto kern = glob ? k_trd_cl<true> : k_trd_cl<false>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) e = raise_attribute((const void *)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return (int)e;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at[1];
