@@ -73,7 +73,6 @@ struct DevSb {
     int *d_ell_col = nullptr;
     double *d_ell_val = nullptr;
     int nhv = 0, hv_grid = 0, hv_nsm = 0;   // its tiles, CTAs, the GPU's SMs
-    int *d_hv_queue = nullptr;         // tiles handed out, CTAs that left (both 0 between launches)
     // FP32 copies for the mixed-precision path
     float *d_hl32 = nullptr, *d_hr32 = nullptr, *d_ab_val32 = nullptr;
     int *d_ab_rowptr32 = nullptr, *d_ab_col32 = nullptr;   // pruned FP32 A/B pool

@@ -82,7 +82,7 @@ constexpr int TILE = 16;
 constexpr int TILE32 = 32;
 constexpr int HV_TR = 4, HV_TC = 8;    // output tile of a warp of k_hv_fp64
 constexpr int HV_WARPS = 4;            // warps of its CTAs, one per quarter of an SM
-constexpr int HV_CTAS = 5;             // CTAs per SM at most: more tiles are handed out by a queue
+constexpr int HV_CTAS = 5;             // CTAs per SM at most
 
 // Sections of the pool's arena: each array at a 256-byte boundary (at least
 // 16 bytes, so that every pointer is distinct and valid), those with a host
@@ -655,8 +655,6 @@ int sb_upload(Ctx &c, const nss_sb_desc *d, bool trusted) {
     sg.add(&s.d_sp_dval, sp.dval);
     sg.add(&s.d_sp_tiles, sp.tiles);
     sg.add(&s.d_hv_recs, hv_recs);
-    const std::vector<int> hv_queue(2, 0);
-    sg.add(&s.d_hv_queue, hv_queue);
     sg.add(&s.d_hv_terms, hv_terms);
     sg.add(&s.d_ell_col, ell_col);
     sg.add(&s.d_ell_val, ell_val);
@@ -694,22 +692,25 @@ int sb_upload(Ctx &c, const nss_sb_desc *d, bool trusted) {
 // next 32 columns of K are loaded into registers while the current ones are
 // multiplied.  What is left is balance: every quarter of an SM has a pipe of its
 // own.  Up to two tiles for each (2 * 4 * 152) the CTAs get four each; above,
-// every SM the same number of CTAs (at most five), and a warp that is done takes
-// its next tile from a queue, longest first.  Tiles of 8 x 16 on four warps,
-// one CTA each, left SMs with five CTAs beside others with four, and waited for
-// each other at barriers.  Up to five CTAs against three and four: 51.5 against 58.8
-// and 53.0 us at 66 600 states, 76 against 90 and 85 at 93 000.
+// every SM the same number of CTAs (at most five), and what is above one tile a
+// warp is dealt backwards through the order, longest first.  The launch leaves
+// nothing behind, so products replayed from graphs do not meet; a queue of
+// tiles in memory took as long (one launch after another on one stream: 73.6
+// us against 72.5 dealt at 90 554 states, Hubbard m = 297; 80.1 against 78.3 at
+// 99 902).  At most 3 / 4 / 5 / 6 CTAs an SM: 85.2 / 76.0 / 72.9 / 101.4 us at
+// 90 554 states (the sixth is not resident), no difference at 57 902.
+// Tiles of 8 x 16 on four warps, one CTA each, left SMs with five CTAs beside
+// others with four, and waited for each other at barriers.
 // A x B terms: Out[ai][bi] += A[ai][aj] B[bi][bj] W_q[aj][bj] (:808-857).  Where
 // all rows hold one entry, four terms' loads are in flight; where rows of A hold
 // more (the renormalised sign operator leaves rounding-level entries in its
 // whole block, 40 a row), a row's eight lanes hold two entries each, eight
 // gathers in flight, instead of every thread walking the row by itself; a
 // factor of +-1 is a sign flip and no FP64 multiplication.  (Gathers a round
-// ahead of the FMAs need 126 registers and were slower: 57.7 us.)
-// Bit for bit the results of 16 x 16 tiles on eight warps, in us: Hubbard
-// 66 600 states 88 -> 60 (8 x 16) -> 51.5, spin-1/2 39 200 states 28.0 (8 x 16)
-// -> 22.9, spin-1 60 900 states 37.3 -> 34.8, 582 states 4.1 -> 3.4; FP64 solves
-// of 3 958 states 3.12 -> 2.32 -> 2.13 ms, of 66 600 9.85 -> 7.11 -> 6.14 ms.
+// ahead of the FMAs need 126 registers and were slower: 57.7 against 51.5 us.)
+// Bit for bit the results of 16 x 16 tiles on eight warps, in us, one launch
+// after another on one stream: Hubbard 66 600 states 88 -> 60 (8 x 16) -> 51.3,
+// spin-1/2 39 200 states 28.0 (8 x 16) -> 22.6, spin-1 61 200 states 37.3 -> 34.6.
 __device__ __forceinline__ double hv_times(double b, double x, bool unit) {
     if (!unit) return b * x;
     return __hiloint2double(__double2hiint(x) ^ (__double2hiint(b) & 0x80000000), __double2loint(x));
@@ -726,7 +727,7 @@ struct HvOps {
 
 __global__ void __launch_bounds__(32 * HV_WARPS) k_hv_fp64(const double *__restrict__ v, double *__restrict__ hv,
                                                            const HvRec *__restrict__ recs, HvOps op, int ntiles,
-                                                           int nsm, int *queue, const int *stop) {
+                                                           int nsm, const int *stop) {
     if (stop && *stop) return;   // the Lanczos loop has already finished (the same for every CTA)
     constexpr int KC = 32;
     __shared__ double sa_[HV_WARPS][HV_TR][KC + 1];
@@ -735,11 +736,14 @@ __global__ void __launch_bounds__(32 * HV_WARPS) k_hv_fp64(const double *__restr
     double(*sa)[KC + 1] = sa_[warp];
     double(*sb)[HV_TC + 1] = sb_[warp];
     const int ty = lane / HV_TC, tx = lane % HV_TC;
-    const bool queued = ntiles > HV_WARPS * grid;
     // longest tiles first, a CTA's four a grid apart in the order; the warp that
-    // may be left without one is another in each CTA of an SM
-    int tile = (int)((warp + blockIdx.x / nsm) % HV_WARPS) * grid + blockIdx.x, next = ntiles;
-    for (; tile < ntiles; tile = next) {
+    // may be left without one is another in each CTA of an SM.  What is above
+    // one tile a warp is dealt backwards, so that the warps with the longest
+    // first tile get the shortest second one.
+    const int all = HV_WARPS * grid, mine = (int)((warp + blockIdx.x / nsm) % HV_WARPS) * grid + blockIdx.x;
+    for (int r = 0; r * all < ntiles; ++r) {
+        const int tile = r * all + (r & 1 ? all - 1 - mine : mine);
+        if (tile >= ntiles) continue;
         const HvRec t = recs[tile];
         const int dl = t.dl, dr = t.dr;
         const double *W = v + t.off, *HL = op.hl + t.hlo, *HR = op.hr + t.hro;
@@ -783,10 +787,6 @@ __global__ void __launch_bounds__(32 * HV_WARPS) k_hv_fp64(const double *__restr
 #pragma unroll 8
             for (int j = 0; j < kn; ++j) acc = fma(sa[ty][j], sb[j][tx], acc);
             __syncwarp();
-        }
-        if (queued) {
-            if (lane == 0) next = HV_WARPS * grid + atomicAdd(queue, 1);
-            next = __shfl_sync(0xffffffffu, next, 0);
         }
         const bool in = il < dl && ir < dr;
         if (!t.csr) {
@@ -861,11 +861,6 @@ __global__ void __launch_bounds__(32 * HV_WARPS) k_hv_fp64(const double *__restr
             }
         }
         if (in) hv[t.off + (int64_t)il * dr + ir] = acc;
-    }
-    // every tile is taken: the last warp to leave clears the queue
-    if (queued && lane == 0 && atomicAdd(queue + 1, 1) == HV_WARPS * grid - 1) {
-        queue[0] = 0;
-        queue[1] = 0;
     }
 }
 
@@ -967,7 +962,7 @@ int hv_device(Ctx &c, const double *d_v, double *d_hv, const int *stop) {
     k_hv_fp64<<<s.hv_grid, 32 * HV_WARPS, 0, c.stream>>>(
         d_v, d_hv, s.d_hv_recs,
         HvOps{s.d_hl, s.d_hr, s.d_hv_terms, s.d_ell_col, s.d_ell_val, s.d_ab_rowptr, s.d_ab_col, s.d_ab_val}, s.nhv,
-        s.hv_nsm, s.d_hv_queue, stop);
+        s.hv_nsm, stop);
     c.launches += 1;
     NSS_CUDA_TRY(c, cudaGetLastError());
     return NSS_OK;
