@@ -114,7 +114,9 @@ int64_t nss_sb_upload_bytes(const nss_ctx *ctx);
 void *nss_stream(const nss_ctx *ctx);
 
 /* sparse_HxV: hv = H_sb v for host vectors of length n (must equal
- * nss_sb_dim).  spMatVec_direct_main semantics: hv is overwritten. */
+ * nss_sb_dim).  spMatVec_direct_main semantics: hv is overwritten.  A product
+ * on the tensor cores whose bounded waits run out is computed on the CUDA cores
+ * instead; it reports no error of its own. */
 int nss_hv(nss_ctx *ctx, int64_t n, const double *v, double *hv);
 /* Same on device pointers, ordered on the context's stream. */
 int nss_hv_device(nss_ctx *ctx, int64_t n, const double *d_v, double *d_hv);

@@ -209,7 +209,7 @@ int nss_hv_device(nss_ctx *ctx, int64_t n, const double *d_v, double *d_hv) {
     if (n != ctx->c.sb.n) return fail(ctx, NSS_ERR_INVALID, "nss_hv: Nloc != superblock dimension");
     if (!d_v || !d_hv) return fail(ctx, NSS_ERR_INVALID, "nss_hv: null vector");
     DeviceScope dscope(ctx->c.device);
-    return nss::hv_device(ctx->c, d_v, d_hv);
+    return nss::hv_device(ctx->c, d_v, d_hv, nullptr, true);
 }
 
 int nss_hv_device_f32(nss_ctx *ctx, int64_t n, const float *d_v, float *d_hv) {
@@ -399,7 +399,7 @@ int nss_hv(nss_ctx *ctx, int64_t n, const double *v, double *hv) {
         if (rc) return rc;
         nss::Ctx &c = ctx->c;
         NSS_CUDA_TRY(c, cudaMemcpyAsync(ctx->d_v, v, n * sizeof(double), cudaMemcpyHostToDevice, c.stream));
-        rc = nss::hv_device(c, ctx->d_v, ctx->d_hv);
+        rc = nss::hv_device(c, ctx->d_v, ctx->d_hv, nullptr, true);
         if (rc) return rc;
         NSS_CUDA_TRY(c, cudaMemcpyAsync(hv, ctx->d_hv, n * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
         NSS_CUDA_TRY(c, cudaStreamSynchronize(c.stream));

@@ -68,11 +68,11 @@ struct DevSb {
     double *d_ab_val = nullptr;
     int4 *d_tiles = nullptr;
     int ntiles = 0;
-    HvRec *d_hv_recs = nullptr;        // k_hv_fp64 (unless the split path has the superblock)
+    HvRec *d_hv_recs = nullptr;        // k_hv_fp64's tiles (none on the split path: its own tiles serve)
     HvTerm *d_hv_terms = nullptr;
     int *d_ell_col = nullptr;
     double *d_ell_val = nullptr;
-    int nhv = 0, hv_grid = 0, hv_nsm = 0;   // its tiles, CTAs, the GPU's SMs
+    int nhv = 0, hv_grid = 0, hv_nsm = 0;   // its tiles, CTAs (split path: of a redo), the GPU's SMs
     // FP32 copies for the mixed-precision path
     float *d_hl32 = nullptr, *d_hr32 = nullptr, *d_ab_val32 = nullptr;
     int *d_ab_rowptr32 = nullptr, *d_ab_col32 = nullptr;   // pruned FP32 A/B pool
@@ -114,6 +114,7 @@ struct DevSb {
     struct SplitJob *d_sp_jobs_w = nullptr, *d_sp_jobs_hl = nullptr, *d_sp_jobs_hr = nullptr;
     struct SplitTerm *d_sp_terms = nullptr;
     struct SplitTile *d_sp_tiles = nullptr;
+    int *d_sp_redo = nullptr;          // a standalone product's error word
     size_t sp_pack_smem = 0;
     int sp_nitems = 0, sp_njobs = 0, sp_ntiles = 0, sp_bn = 64, sp_grid = 0;
     alignas(64) unsigned char sp_map_a[128] = {}, sp_map_b[128] = {};
@@ -325,8 +326,11 @@ int sb_upload(Ctx &c, const nss_sb_desc *d, bool trusted = false);
 // Drop the pool; free_arena also returns its device arena and pinned
 // staging buffer (otherwise kept for the next upload).
 void sb_release(Ctx &c, bool free_arena);
-// `stop` (may be null): a device flag; the kernels return at once when set
-int hv_device(Ctx &c, const double *d_v, double *d_hv, const int *stop = nullptr);
+// `stop` (may be null): a device flag; the kernels return at once when set.
+// standalone: a product for a caller that only gets its result.  What the
+// tensor cores do not deliver (a wait that ran out) k_hv_fp64 then computes.
+// Solvers pass false and look at sb.d_tc_err with their other results.
+int hv_device(Ctx &c, const double *d_v, double *d_hv, const int *stop = nullptr, bool standalone = false);
 // add_planes false: the tensor-core sectors' part stays in sb.d_mma_out (mma_nplanes planes)
 int hv_device_fp32(Ctx &c, const float *d_v, float *d_hv, const int *stop = nullptr, bool add_planes = true);
 // k_sector_mma.cu: the dense sector products of the routed sectors into the

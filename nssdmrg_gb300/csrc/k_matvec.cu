@@ -414,34 +414,36 @@ int sb_upload(Ctx &c, const nss_sb_desc *d, bool trusted) {
     std::vector<HvRec> hv_recs;
     std::vector<int> ell_col;
     std::vector<double> ell_val;
-    if (!split) {
-        for (const DevTerm &t : s.terms) {
-            HvTerm h{s.off[t.in_sec], s.drs[t.in_sec], 0, 0, t.a_rp, t.b_rp, 0, 1};
-            for (int side = 0; side < 2; ++side) {
-                const int64_t rp = side == 0 ? t.a_rp : t.b_rp;
-                const int nrow = side == 0 ? t.a_nrow : t.b_nrow;
-                (side == 0 ? h.a : h.b) = (int)ell_col.size();
-                for (int i = 0; i < nrow; ++i) {
-                    const int p0 = rowptr[rp + i], p1 = rowptr[rp + i + 1];
-                    ell_col.push_back(p1 > p0 ? col[p0] : -1);
-                    ell_val.push_back(p1 > p0 ? val[p0] : 0.0);
-                    if (p1 - p0 > 1) h.kind = std::max(h.kind, side == 0 ? 1 : 2);
-                    if (side == 1 && p1 > p0 && std::fabs(val[p0]) != 1.0) h.unit_b = 0;
-                }
+    for (const DevTerm &t : s.terms) {
+        HvTerm h{s.off[t.in_sec], s.drs[t.in_sec], 0, 0, t.a_rp, t.b_rp, 0, 1};
+        for (int side = 0; side < 2; ++side) {
+            const int64_t rp = side == 0 ? t.a_rp : t.b_rp;
+            const int nrow = side == 0 ? t.a_nrow : t.b_nrow;
+            (side == 0 ? h.a : h.b) = (int)ell_col.size();
+            for (int i = 0; i < nrow; ++i) {
+                const int p0 = rowptr[rp + i], p1 = rowptr[rp + i + 1];
+                ell_col.push_back(p1 > p0 ? col[p0] : -1);
+                ell_val.push_back(p1 > p0 ? val[p0] : 0.0);
+                if (p1 - p0 > 1) h.kind = std::max(h.kind, side == 0 ? 1 : 2);
+                if (side == 1 && p1 > p0 && std::fabs(val[p0]) != 1.0) h.unit_b = 0;
             }
-            hv_terms.push_back(h);
         }
+        hv_terms.push_back(h);
+    }
+    std::vector<int> hv_csr(s.nsb, 0);
+    for (int k = 0; k < s.nsb; ++k)
+        for (int t = s.term_ptr[k]; t < s.term_ptr[k + 1]; ++t) hv_csr[k] |= hv_terms[t].kind > 0;
+    if (!split) {
         for (int k = 0; k < s.nsb; ++k) {
             // FMAs per output: the two K loops and, per term, a row of A
-            int csr = 0, cost = s.dls[k] + s.drs[k];
+            int cost = s.dls[k] + s.drs[k];
             for (int t = s.term_ptr[k]; t < s.term_ptr[k + 1]; ++t) {
                 const DevTerm &tm = s.terms[t];
-                csr |= hv_terms[t].kind > 0;
                 cost += (rowptr[tm.a_rp + tm.a_nrow] - rowptr[tm.a_rp]) / std::max(tm.a_nrow, 1);
             }
             for (int r = 0; r < s.dls[k]; r += HV_TR)
                 for (int cc = 0; cc < s.drs[k]; cc += HV_TC)
-                    hv_recs.push_back(HvRec{s.dls[k], s.drs[k], r, cc, s.term_ptr[k], s.term_ptr[k + 1], csr, cost, s.off[k],
+                    hv_recs.push_back(HvRec{s.dls[k], s.drs[k], r, cc, s.term_ptr[k], s.term_ptr[k + 1], hv_csr[k], cost, s.off[k],
                                             s.hl_off[k], s.hr_off[k]});
         }
         std::stable_sort(hv_recs.begin(), hv_recs.end(),
@@ -491,6 +493,7 @@ int sb_upload(Ctx &c, const nss_sb_desc *d, bool trusted) {
     s.hv_nsm = nsm;
     s.hv_grid = s.nhv <= 2 * HV_WARPS * nsm ? (s.nhv + HV_WARPS - 1) / HV_WARPS
                                             : nsm * std::min(HV_CTAS, (s.nhv + HV_WARPS * nsm - 1) / (HV_WARPS * nsm));
+    if (split) s.hv_grid = nsm * HV_CTAS;
     std::vector<char> on_tc(s.nsb, 0);
     for (int k : plan.sectors) on_tc[k] = 1;
     std::vector<int4> tiles32;
@@ -591,7 +594,7 @@ int sb_upload(Ctx &c, const nss_sb_desc *d, bool trusted) {
     s.ntiles32 = (int)tiles32.size();
     std::vector<int> tc_err(1, 0);
     SplitPlan sp;
-    if (split) split_layout(s, rowptr, col, val, nsm, sp);
+    if (split) split_layout(s, rowptr, col, val, hv_csr, nsm, sp);
 
     Stager sg;
     sg.add_dev(&s.d_hl32, (size_t)hl_tot);
@@ -658,6 +661,7 @@ int sb_upload(Ctx &c, const nss_sb_desc *d, bool trusted) {
     sg.add(&s.d_hv_terms, hv_terms);
     sg.add(&s.d_ell_col, ell_col);
     sg.add(&s.d_ell_val, ell_val);
+    sg.add_dev(&s.d_sp_redo, 1);
     sg.add_dev(&s.d_sp_exp, (size_t)sp.nexp);
     sg.add_dev(&s.d_sp_x32, split ? (size_t)s.n : 0);
     sg.add_dev(&s.d_sp_out, split ? 2 * (size_t)s.n : 0);
@@ -725,10 +729,22 @@ struct HvOps {
     const double *ab_val;
 };
 
+// What k_hv_fp64 computes of a product on the tensor cores: every tile when
+// that gave up (*err), else nothing.  A tile is an eighth of a SplitTile.
+struct HvRedo {
+    const SplitTile *tiles;
+    const int *err;
+};
+constexpr int HV_SUB = (8 / HV_TR) * (32 / HV_TC);
+
+template <bool REDO>
 __global__ void __launch_bounds__(32 * HV_WARPS) k_hv_fp64(const double *__restrict__ v, double *__restrict__ hv,
-                                                           const HvRec *__restrict__ recs, HvOps op, int ntiles,
-                                                           int nsm, const int *stop) {
+                                                           const HvRec *__restrict__ recs, HvRedo redo, HvOps op,
+                                                           int ntiles, int nsm, const int *stop) {
     if (stop && *stop) return;   // the Lanczos loop has already finished (the same for every CTA)
+    if constexpr (REDO) {
+        if (!*redo.err) return;
+    }
     constexpr int KC = 32;
     __shared__ double sa_[HV_WARPS][HV_TR][KC + 1];
     __shared__ double sb_[HV_WARPS][KC][HV_TC + 1];
@@ -744,7 +760,16 @@ __global__ void __launch_bounds__(32 * HV_WARPS) k_hv_fp64(const double *__restr
     for (int r = 0; r * all < ntiles; ++r) {
         const int tile = r * all + (r & 1 ? all - 1 - mine : mine);
         if (tile >= ntiles) continue;
-        const HvRec t = recs[tile];
+        HvRec t;
+        if constexpr (REDO) {
+            const SplitTile s = redo.tiles[tile / HV_SUB];
+            const int sub = tile % HV_SUB;
+            t = HvRec{s.dl, s.dr, s.row0 + HV_TR * (sub / (32 / HV_TC)), s.col0 + HV_TC * (sub % (32 / HV_TC)), s.t0, s.t1, s.csr,
+                      0, s.off, s.hlo, s.hro};
+            if (t.row0 >= t.dl || t.col0 >= t.dr) continue;
+        } else {
+            t = recs[tile];
+        }
         const int dl = t.dl, dr = t.dr;
         const double *W = v + t.off, *HL = op.hl + t.hlo, *HR = op.hr + t.hro;
         const int il = t.row0 + ty, ir = t.col0 + tx;
@@ -952,17 +977,22 @@ int hv_device_fp32(Ctx &c, const float *d_v, float *d_hv, const int *stop, bool 
     return NSS_OK;
 }
 
-int hv_device(Ctx &c, const double *d_v, double *d_hv, const int *stop) {
+int hv_device(Ctx &c, const double *d_v, double *d_hv, const int *stop, bool standalone) {
     DevSb &s = c.sb;
     if (!s.valid) {
         c.err = "nss_hv: no superblock uploaded";
         return NSS_ERR_STATE;
     }
-    if (s.sp_nitems) return hv_device_split(c, d_v, d_hv, stop);
-    k_hv_fp64<<<s.hv_grid, 32 * HV_WARPS, 0, c.stream>>>(
-        d_v, d_hv, s.d_hv_recs,
-        HvOps{s.d_hl, s.d_hr, s.d_hv_terms, s.d_ell_col, s.d_ell_val, s.d_ab_rowptr, s.d_ab_col, s.d_ab_val}, s.nhv,
-        s.hv_nsm, stop);
+    const HvOps op{s.d_hl, s.d_hr, s.d_hv_terms, s.d_ell_col, s.d_ell_val, s.d_ab_rowptr, s.d_ab_col, s.d_ab_val};
+    if (s.sp_nitems) {
+        if (int rc = hv_device_split(c, d_v, d_hv, stop, standalone ? s.d_sp_redo : s.d_tc_err, standalone)) return rc;
+        if (!standalone) return NSS_OK;
+        k_hv_fp64<true><<<s.hv_grid, 32 * HV_WARPS, 0, c.stream>>>(d_v, d_hv, nullptr, HvRedo{s.d_sp_tiles, s.d_sp_redo}, op,
+                                                                   s.sp_ntiles * HV_SUB, s.hv_nsm, stop);
+    } else {
+        k_hv_fp64<false><<<s.hv_grid, 32 * HV_WARPS, 0, c.stream>>>(d_v, d_hv, s.d_hv_recs, HvRedo{}, op, s.nhv, s.hv_nsm,
+                                                                    stop);
+    }
     c.launches += 1;
     NSS_CUDA_TRY(c, cudaGetLastError());
     return NSS_OK;

@@ -152,8 +152,9 @@ __device__ __forceinline__ float trunc32(double x, int e) {
 constexpr int SP_STRIP = 768;
 __global__ void __launch_bounds__(32 * SP_ROWS) k_split_pack(const double *__restrict__ x, const SplitJob *__restrict__ jobs,
                                                              uint32_t *__restrict__ pool, int *__restrict__ exps,
-                                                             float *__restrict__ x32, const int *stop) {
+                                                             float *__restrict__ x32, int *clear, const int *stop) {
     if (stop && *stop) return;
+    if (clear && blockIdx.x == 0 && threadIdx.x == 0) *clear = 0;
     extern __shared__ double strip[];
     const SplitJob J = jobs[blockIdx.x];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -608,7 +609,7 @@ bool split_wanted(const DevSb &s) {
 }
 
 void split_layout(const DevSb &s, const std::vector<int> &rowptr, const std::vector<int> &col,
-                  const std::vector<double> &val, int nsm, SplitPlan &p) {
+                  const std::vector<double> &val, const std::vector<int> &csr, int nsm, SplitPlan &p) {
     p = SplitPlan{};
     auto slabs = [](int d) { return (d + SP_KC - 1) / SP_KC; };
     // pool rows and scale exponents of the four operands of every sector
@@ -645,7 +646,8 @@ void split_layout(const DevSb &s, const std::vector<int> &rowptr, const std::vec
         tiles32 += 2 * (int64_t)((dl + SP_M - 1) / SP_M) * ((dr + 31) / 32);
         for (int a = 0; a < dl; a += 8)
             for (int b = 0; b < dr; b += 32)
-                p.tiles.push_back(SplitTile{a, b, dl, dr, s.term_ptr[k], s.term_ptr[k + 1], R.ehl, 0, s.off[k]});
+                p.tiles.push_back(SplitTile{a, b, dl, dr, s.term_ptr[k], s.term_ptr[k + 1], R.ehl, csr[k], s.off[k],
+                                            s.hl_off[k], s.hr_off[k]});
         p.kmax = std::max({p.kmax, dl, dr});
     }
     row += SP_M;   // a box that starts near the end of the pool stays inside it
@@ -736,9 +738,9 @@ int split_finish(Ctx &c, const SplitPlan &p) {
     NSS_CUDA_TRY(c, allow_smem((const void *)k_split_pack, smem));
     c.launches += 2;
     k_split_pack<<<(unsigned)p.jobs_hl.size(), 32 * SP_ROWS, smem, c.stream>>>(s.d_hl, s.d_sp_jobs_hl, s.d_sp_pool, s.d_sp_exp,
-                                                                            nullptr, nullptr);
+                                                                            nullptr, nullptr, nullptr);
     k_split_pack<<<(unsigned)p.jobs_hr.size(), 32 * SP_ROWS, smem, c.stream>>>(s.d_hr, s.d_sp_jobs_hr, s.d_sp_pool, s.d_sp_exp,
-                                                                            nullptr, nullptr);
+                                                                            nullptr, nullptr, nullptr);
     NSS_CUDA_TRY(c, cudaGetLastError());
     s.sp_nitems = (int)p.items.size();
     s.sp_njobs = (int)p.jobs_w.size();
@@ -755,24 +757,25 @@ int split_finish(Ctx &c, const SplitPlan &p) {
 namespace {
 
 template <int BN>
-int launch_split(Ctx &c, const int *stop) {
+int launch_split(Ctx &c, int *err, const int *stop) {
     NSS_CUDA_TRY(c, allow_smem((const void *)k_sector_split<BN>, SplitCfg<BN>::SMEM));
     DevSb &s = c.sb;
     alignas(64) CUtensorMap ma, mb;
     std::memcpy(&ma, s.sp_map_a, sizeof(ma));
     std::memcpy(&mb, s.sp_map_b, sizeof(mb));
     k_sector_split<BN><<<s.sp_grid, SP_THREADS, SplitCfg<BN>::SMEM, c.stream>>>(ma, mb, s.d_sp_items, s.d_sp_rng, s.d_sp_out, s.d_sp_out0, s.n,
-                                                                               wait_limit(), s.d_tc_err, stop);
+                                                                               wait_limit(), err, stop);
     return NSS_OK;
 }
 
 }  // namespace
 
-int hv_device_split(Ctx &c, const double *d_v, double *d_hv, const int *stop) {
+int hv_device_split(Ctx &c, const double *d_v, double *d_hv, const int *stop, int *err, bool clear) {
     DevSb &s = c.sb;
     c.launches += 3;
-    k_split_pack<<<(unsigned)s.sp_njobs, 32 * SP_ROWS, s.sp_pack_smem, c.stream>>>(d_v, s.d_sp_jobs_w, s.d_sp_pool, s.d_sp_exp, s.d_sp_x32, stop);
-    if (int rc = s.sp_bn == 64 ? launch_split<64>(c, stop) : launch_split<32>(c, stop)) return rc;
+    k_split_pack<<<(unsigned)s.sp_njobs, 32 * SP_ROWS, s.sp_pack_smem, c.stream>>>(d_v, s.d_sp_jobs_w, s.d_sp_pool, s.d_sp_exp,
+                                                                              s.d_sp_x32, clear ? err : nullptr, stop);
+    if (int rc = s.sp_bn == 64 ? launch_split<64>(c, err, stop) : launch_split<32>(c, err, stop)) return rc;
     SplitTerms T{s.d_sp_terms, s.d_sp_tcol, s.d_sp_dptr, s.d_sp_dcol, s.d_sp_exp, s.d_sp_tval, s.d_sp_dval, s.d_terms,
                  s.d_ab_rowptr, s.d_ab_col, s.d_ab_val};
     k_split_terms<<<(unsigned)s.sp_ntiles, 256, 0, c.stream>>>(d_v, s.d_sp_x32, s.d_sp_out, s.d_sp_out0, s.n, d_hv, s.d_sp_tiles, T, stop);

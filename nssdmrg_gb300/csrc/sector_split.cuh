@@ -48,11 +48,12 @@ struct SplitTerm {
     int64_t off;                 // offset in psi
 };
 
-// One 8 x 32 output tile of the last kernel
+// One 8 x 32 output tile of the last kernel, eight tiles of k_hv_fp64
 struct SplitTile {
     int row0, col0, dl, dr, t0, t1;
-    int exp, pad;                // the sector's scale exponents: H_L rows, H_R rows, W rows, W columns
-    int64_t off;
+    int exp;                     // the sector's scale exponents: H_L rows, H_R rows, W rows, W columns
+    int csr;                     // HvRec::csr of the sector
+    int64_t off, hlo, hro;
 };
 
 struct SplitPlan {
@@ -78,11 +79,13 @@ struct SplitPlan {
 // forces a path (comparisons, tests).
 bool split_wanted(const DevSb &s);
 // the plan from the superblock's tables and its CSR pool (rowptr, col, val)
+// (csr: HvRec::csr per sector)
 void split_layout(const DevSb &s, const std::vector<int> &rowptr, const std::vector<int> &col,
-                  const std::vector<double> &val, int nsm, SplitPlan &p);
+                  const std::vector<double> &val, const std::vector<int> &csr, int nsm, SplitPlan &p);
 // digits of H_L and H_R and the tensor maps, after the dense blocks are built
 int split_finish(Ctx &c, const SplitPlan &p);
-// hv = H v on c.stream
-int hv_device_split(Ctx &c, const double *d_v, double *d_hv, const int *stop);
+// hv = H v on c.stream.  A wait that ran out is reported in *err; clear: the
+// first kernel sets it to zero.
+int hv_device_split(Ctx &c, const double *d_v, double *d_hv, const int *stop, int *err, bool clear);
 
 }  // namespace nss
