@@ -3054,6 +3054,7 @@ struct BatchEngine {
     float *d_st = nullptr;
     unsigned *d_q = nullptr;     // item queue heads of a launch
     double *h_res = nullptr;     // [BATCH_MAX][8] pinned refinement results
+    int *h_tc = nullptr;         // [BATCH_MAX] pinned: the FP64 product gave up a wait
     cudaEvent_t forked = nullptr, joined[BATCH_MAX] = {};   // the solves' own streams leave and rejoin c0's
     size_t smem_set = 0;         // dynamic shared memory of its launches (the most any round needed)
     ~BatchEngine() {
@@ -3069,6 +3070,7 @@ struct BatchEngine {
         if (h_solves) cudaFreeHost(h_solves);
         if (h_gitems) cudaFreeHost(h_gitems);
         if (h_res) cudaFreeHost(h_res);
+        if (h_tc) cudaFreeHost(h_tc);
     }
 };
 
@@ -3086,6 +3088,7 @@ int engine_init(BatchEngine &E, Ctx &c0) {
     NSS_CUDA_TRY(c0, ctx_alloc(c0, &E.d_q, (size_t)CHUNK_MAXIT));
     NSS_CUDA_TRY(c0, cudaMallocHost((void **)&E.h_solves, sizeof(BatchSolve) * BATCH_MAX));
     NSS_CUDA_TRY(c0, cudaMallocHost((void **)&E.h_res, sizeof(double) * 8 * BATCH_MAX));
+    NSS_CUDA_TRY(c0, cudaMallocHost((void **)&E.h_tc, sizeof(int) * BATCH_MAX));
     NSS_CUDA_TRY(c0, cudaEventCreateWithFlags(&E.forked, cudaEventDisableTiming));
     NSS_CUDA_TRY(c0, cudaMemsetAsync(c0.lz.counter, 0, 4 * sizeof(unsigned), c0.stream));
     NSS_CUDA_TRY(c0, cudaMemsetAsync(c0.lz.flags, 0, F_NFLAGS * sizeof(int), c0.stream));
@@ -3388,7 +3391,12 @@ int engine_step(BatchEngine &E, int max_done, int *ndone, int *ids, double *ener
         DevLanczos &z = c.lz;
         const cudaStream_t s = c.stream;
         double *r = z.scal + S_NSCAL + 4 * (z.cap + 2);
+        // the error word of a product on the tensor cores travels with the results
+        const bool tc = c.sb.sp_nitems > 0;
+        E.h_tc[slot] = 0;
+        if (tc) NSS_CUDA_TRY(c0, cudaMemsetAsync(c.sb.d_tc_err, 0, sizeof(int), s));
         if (int r2 = hv_device(c, z.evecs, z.w)) { c0.err = c.err; return r2; }
+        if (tc) NSS_CUDA_TRY(c0, cudaMemcpyAsync(E.h_tc + slot, c.sb.d_tc_err, sizeof(int), cudaMemcpyDeviceToHost, s));
         ++B.numop;
         c0.launches += 2;
         k_rq<<<NBLK, 256, 0, s>>>(z.evecs, z.w, B.n, z.part, r, z.counter);
@@ -3427,6 +3435,12 @@ int engine_step(BatchEngine &E, int max_done, int *ndone, int *ids, double *ener
     for (int b : p3)
         if ((rc = fork(E.solves[b])) || (rc = fp64_energy(E.solves[b], b, false)) || (rc = join(E.solves[b], b))) return rc;
     NSS_CUDA_TRY(c0, cudaStreamSynchronize(st));
+    for (const std::vector<int> *p : {&p1, &p2, &p3})
+        for (int b : *p)
+            if (E.h_tc[b]) {
+                c0.err = "nss_batch: a tensor-core pipeline wait timed out (results discarded)";
+                return NSS_ERR_CUDA;
+            }
     auto finish = [&](BatchState &B, int slot) -> int {
         const double *hr = E.h_res + 8 * slot;
         B.result = hr[0] / hr[2];
@@ -3478,6 +3492,13 @@ int engine_step(BatchEngine &E, int max_done, int *ndone, int *ids, double *ener
     return NSS_OK;
 }
 
+// After a failed round: nothing of it still runs, and no solve is held
+void engine_drop(BatchEngine &E) {
+    cudaStreamSynchronize(E.c0->stream);
+    for (BatchState &B : E.solves) cudaStreamSynchronize(B.c->stream);
+    E.solves.clear();
+}
+
 }  // namespace
 
 BatchEngine *batch_create(Ctx &c0) {
@@ -3501,7 +3522,7 @@ int batch_step(BatchEngine *E, int max_done, int *ndone, int *ids, double *energ
         // a failed round drops every solve in flight, so that the engine
         // holds no context its caller may now solve alone or release; the
         // shared barrier and error word start the next round cleared
-        E->solves.clear();
+        engine_drop(*E);
         if (ndone) *ndone = 0;
         Ctx &c0 = *E->c0;
         cudaMemsetAsync(c0.lz.counter, 0, 4 * sizeof(unsigned), c0.stream);
@@ -3529,7 +3550,10 @@ int lanczos_eigh_batch(Ctx *const *cs, int nb, int nitermax, double tol, const u
     int first_rc = NSS_OK;
     for (int round = 0; round < 1000000 && !E.solves.empty(); ++round) {
         int nd = 0;
-        if ((rc = engine_step(E, nb, &nd, did.data(), en.data(), nop.data()))) return rc;
+        if ((rc = engine_step(E, nb, &nd, did.data(), en.data(), nop.data()))) {
+            engine_drop(E);
+            return rc;
+        }
         for (int q = 0; q < nd; ++q) {
             const int id = did[q] < 0 ? -did[q] : did[q];
             const int b = (int)(std::find(ids.begin(), ids.end(), id) - ids.begin());
