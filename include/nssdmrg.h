@@ -114,9 +114,13 @@ int64_t nss_sb_upload_bytes(const nss_ctx *ctx);
 void *nss_stream(const nss_ctx *ctx);
 
 /* sparse_HxV: hv = H_sb v for host vectors of length n (must equal
- * nss_sb_dim).  spMatVec_direct_main semantics: hv is overwritten.  A product
- * on the tensor cores whose bounded waits run out is computed on the CUDA cores
- * instead; it reports no error of its own. */
+ * nss_sb_dim).  spMatVec_direct_main semantics: hv is overwritten.  Every
+ * element is as accurate as a chain of FP64 sums: its error is below
+ * (operations) 2^-53 times the sum of the absolute values of its products.
+ * Large superblocks are computed on the tensor cores, relative to the largest
+ * elements of rows and columns; elements for which that is less exact (operands
+ * graded over many decades), and whole products whose bounded waits run out,
+ * are computed on the CUDA cores instead. */
 int nss_hv(nss_ctx *ctx, int64_t n, const double *v, double *hv);
 /* Same on device pointers, ordered on the context's stream. */
 int nss_hv_device(nss_ctx *ctx, int64_t n, const double *d_v, double *d_hv);

@@ -114,10 +114,16 @@ struct DevSb {
     struct SplitJob *d_sp_jobs_w = nullptr, *d_sp_jobs_hl = nullptr, *d_sp_jobs_hr = nullptr;
     struct SplitTerm *d_sp_terms = nullptr;
     struct SplitTile *d_sp_tiles = nullptr;
-    int *d_sp_redo = nullptr;          // a standalone product's error word
+    float *d_sp_size = nullptr;        // standalone products: sums of |H||W|, two planes
+    struct SplitItem *d_sp_sitems = nullptr;   // ... and their work items
+    int2 *d_sp_srng = nullptr;
+    int sp_sgrid = 0;
+    // a standalone product's words: gave up, tiles of k_hv_fp64 to compute, their list
+    int *d_sp_redo = nullptr;
+    int sp_nexp = 0;                   // scale exponents; the rows' nonzero counts follow them
     size_t sp_pack_smem = 0;
     int sp_nitems = 0, sp_njobs = 0, sp_ntiles = 0, sp_bn = 64, sp_grid = 0;
-    alignas(64) unsigned char sp_map_a[128] = {}, sp_map_b[128] = {};
+    alignas(64) unsigned char sp_map_a[128] = {}, sp_map_b[128] = {}, sp_map_s[128] = {};
 };
 
 // Device-side Lanczos state, kept resident between nss_eigh and nss_rdm.
@@ -328,7 +334,8 @@ int sb_upload(Ctx &c, const nss_sb_desc *d, bool trusted = false);
 void sb_release(Ctx &c, bool free_arena);
 // `stop` (may be null): a device flag; the kernels return at once when set.
 // standalone: a product for a caller that only gets its result.  What the
-// tensor cores do not deliver (a wait that ran out) k_hv_fp64 then computes.
+// tensor cores do not deliver (a wait that ran out, elements that their digits
+// hold less exactly than a chain of FP64 sums) k_hv_fp64 then computes.
 // Solvers pass false and look at sb.d_tc_err with their other results.
 int hv_device(Ctx &c, const double *d_v, double *d_hv, const int *stop = nullptr, bool standalone = false);
 // add_planes false: the tensor-core sectors' part stays in sb.d_mma_out (mma_nplanes planes)

@@ -82,6 +82,7 @@ constexpr int TILE = 16;
 constexpr int TILE32 = 32;
 constexpr int HV_TR = 4, HV_TC = 8;    // output tile of a warp of k_hv_fp64
 constexpr int HV_WARPS = 4;            // warps of its CTAs, one per quarter of an SM
+constexpr int HV_SUB = (8 / HV_TR) * (32 / HV_TC);   // its tiles in a SplitTile
 constexpr int HV_CTAS = 5;             // CTAs per SM at most
 
 // Sections of the pool's arena: each array at a 256-byte boundary (at least
@@ -647,6 +648,8 @@ int sb_upload(Ctx &c, const nss_sb_desc *d, bool trusted) {
     sg.add(&s.d_tiles, tiles);
     sg.add(&s.d_sp_items, sp.items);
     sg.add(&s.d_sp_rng, sp.rng);
+    sg.add(&s.d_sp_sitems, sp.sitems);
+    sg.add(&s.d_sp_srng, sp.srng);
     sg.add(&s.d_sp_jobs_w, sp.jobs_w);
     sg.add(&s.d_sp_jobs_hl, sp.jobs_hl);
     sg.add(&s.d_sp_jobs_hr, sp.jobs_hr);
@@ -661,8 +664,9 @@ int sb_upload(Ctx &c, const nss_sb_desc *d, bool trusted) {
     sg.add(&s.d_hv_terms, hv_terms);
     sg.add(&s.d_ell_col, ell_col);
     sg.add(&s.d_ell_val, ell_val);
-    sg.add_dev(&s.d_sp_redo, 1);
-    sg.add_dev(&s.d_sp_exp, (size_t)sp.nexp);
+    sg.add_dev(&s.d_sp_redo, SP_REDO_LIST + HV_SUB * sp.tiles.size());
+    sg.add_dev(&s.d_sp_exp, 2 * (size_t)sp.nexp);
+    sg.add_dev(&s.d_sp_size, split ? 2 * (size_t)s.n : 0);
     sg.add_dev(&s.d_sp_x32, split ? (size_t)s.n : 0);
     sg.add_dev(&s.d_sp_out, split ? 2 * (size_t)s.n : 0);
     sg.add_dev(&s.d_sp_out0, split ? 2 * (size_t)s.n : 0);
@@ -730,20 +734,25 @@ struct HvOps {
 };
 
 // What k_hv_fp64 computes of a product on the tensor cores: every tile when
-// that gave up (*err), else nothing.  A tile is an eighth of a SplitTile.
+// that gave up, else those on its list, of which the sides that are good come
+// from the planes of digit sums.  A tile is an eighth of a SplitTile.
 struct HvRedo {
     const SplitTile *tiles;
-    const int *err;
+    const int *words;            // sb.d_sp_redo
+    const int64_t *planes;
+    const int *planes0, *exps;
+    int64_t n;
 };
-constexpr int HV_SUB = (8 / HV_TR) * (32 / HV_TC);
 
 template <bool REDO>
 __global__ void __launch_bounds__(32 * HV_WARPS) k_hv_fp64(const double *__restrict__ v, double *__restrict__ hv,
                                                            const HvRec *__restrict__ recs, HvRedo redo, HvOps op,
                                                            int ntiles, int nsm, const int *stop) {
     if (stop && *stop) return;   // the Lanczos loop has already finished (the same for every CTA)
+    bool listed = false;
     if constexpr (REDO) {
-        if (!*redo.err) return;
+        listed = !redo.words[SP_REDO_ERR];
+        if (listed) ntiles = redo.words[SP_REDO_COUNT];
     }
     constexpr int KC = 32;
     __shared__ double sa_[HV_WARPS][HV_TR][KC + 1];
@@ -761,9 +770,12 @@ __global__ void __launch_bounds__(32 * HV_WARPS) k_hv_fp64(const double *__restr
         const int tile = r * all + (r & 1 ? all - 1 - mine : mine);
         if (tile >= ntiles) continue;
         HvRec t;
+        SplitTile s;
+        int sides = 3;
         if constexpr (REDO) {
-            const SplitTile s = redo.tiles[tile / HV_SUB];
-            const int sub = tile % HV_SUB;
+            const int word = listed ? redo.words[SP_REDO_LIST + tile] : 4 * tile + 3, id = word >> 2, sub = id % HV_SUB;
+            sides = word & 3;
+            s = redo.tiles[id / HV_SUB];
             t = HvRec{s.dl, s.dr, s.row0 + HV_TR * (sub / (32 / HV_TC)), s.col0 + HV_TC * (sub % (32 / HV_TC)), s.t0, s.t1, s.csr,
                       0, s.off, s.hlo, s.hro};
             if (t.row0 >= t.dl || t.col0 >= t.dr) continue;
@@ -795,10 +807,15 @@ __global__ void __launch_bounds__(32 * HV_WARPS) k_hv_fp64(const double *__restr
                 for (int q = 0; q < HV_TC; ++q) rb[q] = t.col0 + q < dr && gk < dr ? B[(int64_t)q * dr] : 0.0;
             }
         };
-        double acc = 0.0;
-        load(0);
-        for (int c = 0; c < c0 + c1; ++c) {
+        double acc = 0.0, part = 0.0;                // part (redo): a side's sum, the sides are added
+        const int first = REDO && !(sides & 1) ? c0 : 0, last = REDO && !(sides & 2) ? c0 : c0 + c1;
+        if (first < last) load(first);
+        for (int c = first; c < last; ++c) {
             const bool left = c < c0;
+            if (REDO && c == c0) {
+                part = acc;
+                acc = 0.0;
+            }
             const int kn = min(KC, left ? dl - c * KC : dr - (c - c0) * KC);
 #pragma unroll
             for (int q = 0; q < HV_TR; ++q) sa[q][lane] = ra[q];
@@ -808,12 +825,21 @@ __global__ void __launch_bounds__(32 * HV_WARPS) k_hv_fp64(const double *__restr
                 else sb[lane][q] = rb[q];
             }
             __syncwarp();
-            if (c + 1 < c0 + c1) load(c + 1);
+            if (c + 1 < last) load(c + 1);
 #pragma unroll 8
             for (int j = 0; j < kn; ++j) acc = fma(sa[ty][j], sb[j][tx], acc);
             __syncwarp();
         }
         const bool in = il < dl && ir < dr;
+        if constexpr (REDO) {
+            part += acc;
+            acc = 0.0;
+            if (in && sides != 3) {
+                const int64_t e = t.off + (int64_t)ir * dl + il + (sides & 1 ? redo.n : 0);
+                const int x0 = s.exp + (sides & 1 ? dl + dr + il : il), x1 = s.exp + (sides & 1 ? dl + ir : 2 * dl + dr + ir);
+                part += fixed_to_double(redo.planes0[e], redo.planes[e], redo.exps[x0] + redo.exps[x1] - 56);
+            }
+        }
         if (!t.csr) {
             for (int tb = t.t0; tb < t.t1; tb += 4) {
                 int aj[4], bj[4];
@@ -885,7 +911,7 @@ __global__ void __launch_bounds__(32 * HV_WARPS) k_hv_fp64(const double *__restr
                 }
             }
         }
-        if (in) hv[t.off + (int64_t)il * dr + ir] = acc;
+        if (in) hv[t.off + (int64_t)il * dr + ir] = REDO ? part + acc : acc;
     }
 }
 
@@ -985,9 +1011,10 @@ int hv_device(Ctx &c, const double *d_v, double *d_hv, const int *stop, bool sta
     }
     const HvOps op{s.d_hl, s.d_hr, s.d_hv_terms, s.d_ell_col, s.d_ell_val, s.d_ab_rowptr, s.d_ab_col, s.d_ab_val};
     if (s.sp_nitems) {
-        if (int rc = hv_device_split(c, d_v, d_hv, stop, standalone ? s.d_sp_redo : s.d_tc_err, standalone)) return rc;
+        if (int rc = hv_device_split(c, d_v, d_hv, stop, standalone)) return rc;
         if (!standalone) return NSS_OK;
-        k_hv_fp64<true><<<s.hv_grid, 32 * HV_WARPS, 0, c.stream>>>(d_v, d_hv, nullptr, HvRedo{s.d_sp_tiles, s.d_sp_redo}, op,
+        k_hv_fp64<true><<<s.hv_grid, 32 * HV_WARPS, 0, c.stream>>>(d_v, d_hv, nullptr, 
+            HvRedo{s.d_sp_tiles, s.d_sp_redo, s.d_sp_out, s.d_sp_out0, s.d_sp_exp, s.n}, op,
                                                                    s.sp_ntiles * HV_SUB, s.hv_nsm, stop);
     } else {
         k_hv_fp64<false><<<s.hv_grid, 32 * HV_WARPS, 0, c.stream>>>(d_v, d_hv, s.d_hv_recs, HvRedo{}, op, s.nhv, s.hv_nsm,

@@ -18,11 +18,15 @@
 //     every four slabs as one FP32 sum.
 //   * The epilogue warps collect the weighted sums in 96 bits per output; the
 //     last kernel rounds them once to FP64.
-// So a product's error is one rounding plus about 2^-57 of (largest H in the
-// row) (largest W in the column), below that of a chain of FP64 FMAs: measured
-// against products in 64 bits 1.3-4.9e-16 where the chains had 1.7-8.7e-16.
-// The left and right products go to two planes; the last kernel adds them and
-// the A x B terms (:808-857).
+// So a product's error is one rounding plus about 2^-61 sqrt(K) (largest H in the
+// row) (largest W in the column): relative to the largest elements, where a
+// chain of FP64 FMAs errs relative to the products it adds.  With elements of
+// one size that is less than the chain's error (against sums in FP64 pairs
+// 1.3-4.9e-16 where the chains had 1.7-8.7e-16); with a graded row, or where
+// large elements meet small ones only, it is more.  The solvers need no more:
+// a Krylov vector is accurate relative to its norm.  A product that goes to the
+// caller (nss_hv) has every element checked against sum |H||W| (k_split_size,
+// k_split_terms<true>), and k_hv_fp64 sums the tiles that do not pass.
 //
 // What bounds it: a slab of a 128 x 64 tile is 40 MMAs (digit i of A against
 // digits 0 .. 6-i of B, which lie one after the other in shared memory and land
@@ -50,7 +54,6 @@ namespace {
 
 constexpr int SP_THREADS = 320;            // producer, MMA, 8 epilogue warps
 constexpr int SP_EPI0 = 2, SP_NEPI = 8;
-constexpr int SP_BADEXP = 1 << 20;         // scale exponent of a row with an Inf or NaN
 
 // instruction descriptor, kind::f16: D FP32, A and B bf16, both K-major
 __device__ __forceinline__ constexpr uint32_t idesc_bf16(int n) {
@@ -91,36 +94,11 @@ __device__ __forceinline__ uint32_t digit_bf16(uint64_t u, int q) {
     return __float_as_uint(__uint_as_float(0x4B000000u | f) - 8388864.0f) >> 16;
 }
 
-// (s0 2^42 + r) 2^e rounded to nearest even, in integer arithmetic
-__device__ __forceinline__ double fixed_to_double(int s0, int64_t r, int e) {
-    uint64_t l = ((uint64_t)(int64_t)s0 << 42) + (uint64_t)r;
-    int64_t h = (int64_t)(s0 >> 22) + (r >> 63) + (l < (uint64_t)r ? 1 : 0);
-    const uint64_t sign = (uint64_t)h & 0x8000000000000000ull;
-    if (sign) {
-        l = 0 - l;
-        h = ~h + (l == 0 ? 1 : 0);
-    }
-    if (((uint64_t)h | l) == 0) return 0.0;
-    // normalised: the leading bit at bit 63 of u, the rest below it in l
-    uint64_t u = (uint64_t)h;
-    int lz;
-    if (u) {
-        lz = __clzll((long long)u);                  // at least 36: h has 28 bits
-        u = (u << lz) | (l >> (64 - lz));
-        l <<= lz;
-    } else {
-        const int z = __clzll((long long)l);
-        u = l << z;
-        l = 0;
-        lz = 64 + z;
-    }
-    uint64_t m = u >> 11;
-    const uint32_t low = (uint32_t)u & 0x7ffu;
-    if (low > 0x400u || (low == 0x400u && (l || (m & 1)))) ++m;
-    const int ex = 127 - lz + e + 1023;
-    if (ex <= 0) return __longlong_as_double((long long)sign);          // below the normal range
-    if (ex >= 2047) return __longlong_as_double((long long)(sign | 0x7ff0000000000000ull));
-    return __longlong_as_double((long long)(sign | (((uint64_t)(ex - 1) << 52) + m)));
+// |x| 2^-e as bf16 bits, towards zero (0 from 2^-126 on, and for subnormals)
+__device__ __forceinline__ uint32_t size_bf16(double x, int e) {
+    const uint32_t hi = (uint32_t)__double2hiint(x) & 0x7fffffffu;
+    const int ex = (int)(hi >> 20) - 896 - e;
+    return ex <= 0 || hi < 0x100000u ? 0u : ((uint32_t)ex << 7) | ((hi >> 13) & 0x7fu);
 }
 
 // high word of |x| -> scale exponent e with |x| < 2^e for the largest such word of a row
@@ -152,9 +130,10 @@ __device__ __forceinline__ float trunc32(double x, int e) {
 constexpr int SP_STRIP = 768;
 __global__ void __launch_bounds__(32 * SP_ROWS) k_split_pack(const double *__restrict__ x, const SplitJob *__restrict__ jobs,
                                                              uint32_t *__restrict__ pool, int *__restrict__ exps,
-                                                             float *__restrict__ x32, int *clear, const int *stop) {
+                                                             int *__restrict__ nnzs, float *__restrict__ x32, bool sizes,
+                                                             int *clear, const int *stop) {
     if (stop && *stop) return;
-    if (clear && blockIdx.x == 0 && threadIdx.x == 0) *clear = 0;
+    if (clear && blockIdx.x == 0 && threadIdx.x < SP_REDO_LIST) clear[threadIdx.x] = 0;
     extern __shared__ double strip[];
     const SplitJob J = jobs[blockIdx.x];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -179,17 +158,27 @@ __global__ void __launch_bounds__(32 * SP_ROWS) k_split_pack(const double *__res
         }
     };
     uint32_t m = 0;
+    int cnt = 0;                                     // the row's nonzero elements
     for (int k0 = 0; k0 < J.k; k0 += part) {
         const int kn = min(part, J.k - k0);
         if (k0) __syncthreads();
         load(k0, kn);
         __syncthreads();
         if (on)
-            for (int k = lane; k < kn; k += 32) m = max(m, (uint32_t)__double2hiint(mine[k]) & 0x7fffffffu);
+            for (int k = lane; k < kn; k += 32) {
+                const uint32_t hi = (uint32_t)__double2hiint(mine[k]) & 0x7fffffffu;
+                m = max(m, hi);
+                cnt += (hi | (uint32_t)__double2loint(mine[k])) != 0;
+            }
     }
     m = __reduce_max_sync(0xffffffffu, m);
-    const int e = scale_exp(m);
-    if (on && lane == 0) exps[J.exp + r] = e;
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
+    const int e = cnt ? scale_exp(m) : SP_ZEROEXP;
+    const bool live = e < SP_BADEXP && e > SP_ZEROEXP;   // else the digits are zeros
+    if (on && lane == 0) {
+        exps[J.exp + r] = e;
+        nnzs[J.exp + r] = cnt;
+    }
     for (int c = 0; c < nch; ++c) {
         int k0 = c * SP_KC, kn = min(SP_KC, J.k - k0), at = k0;
         if (J.k > SP_STRIP) {
@@ -201,19 +190,22 @@ __global__ void __launch_bounds__(32 * SP_ROWS) k_split_pack(const double *__res
         if (!on) continue;
         const double a = 2 * lane < kn ? mine[at + 2 * lane] : 0.0, b = 2 * lane + 1 < kn ? mine[at + 2 * lane + 1] : 0.0;
         uint64_t ua = 0, ub = 0;
-        if (e < SP_BADEXP) {
+        if (live) {
             ua = to_fixed(a, e);
             ub = to_fixed(b, e);
         }
+        if (sizes)
+            pool[((int64_t)J.abs + (int64_t)c * J.rows + r) * (SP_KC / 2) + lane] =
+                live ? (size_bf16(a, e) | (size_bf16(b, e) << 16)) : 0u;
         if (x32 && J.kind == 0) {
             float *o = x32 + J.src + (int64_t)r * J.ld + k0 + 2 * lane;
-            if (2 * lane < kn) o[0] = e < SP_BADEXP ? trunc32(a, e) : 0.f;
-            if (2 * lane + 1 < kn) o[1] = e < SP_BADEXP ? trunc32(b, e) : 0.f;
+            if (2 * lane < kn) o[0] = live ? trunc32(a, e) : 0.f;
+            if (2 * lane + 1 < kn) o[1] = live ? trunc32(b, e) : 0.f;
         }
 #pragma unroll
         for (int q = 0; q < SP_D; ++q)
             pool[((int64_t)J.row + (int64_t)(c * SP_D + q) * J.rows + r) * (SP_KC / 2) + lane] =
-                e < SP_BADEXP ? (digit_bf16(ua, q) | (digit_bf16(ub, q) << 16)) : 0u;
+                live ? (digit_bf16(ua, q) | (digit_bf16(ub, q) << 16)) : 0u;
     }
 }
 
@@ -472,6 +464,144 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_sector_split(const __grid_con
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(C::TCOLS));
 }
 
+// sum |H||W| of every output, in units of the operands' scales and a little
+// below (bf16 towards zero, FP32 sums): the products of the absolute values, 128
+// x 256 outputs a tile (an MMA takes ~130 cycles whatever its width).  One lane
+// issues the copies (four slabs of A and B in flight), one the MMAs, four warps
+// store.  Waits are bounded as in k_sector_split.
+namespace {
+constexpr int SZ_THREADS = 192, SZ_STAGES = 4;
+struct SizeCfg {
+    static constexpr int A_BYTES = SP_M * 128, B_BYTES = SP_SN * 128;
+    static constexpr int SMEM = SZ_STAGES * (A_BYTES + B_BYTES) + 1024;
+    static_assert(SMEM <= 232448 - 256, "shared memory plan");
+};
+}  // namespace
+
+__global__ void __launch_bounds__(SZ_THREADS, 1) k_split_size(const __grid_constant__ CUtensorMap map_a,
+                                                               const __grid_constant__ CUtensorMap map_b,
+                                                               const SplitItem *__restrict__ items,
+                                                               const int2 *__restrict__ ranges, float *__restrict__ out,
+                                                               int64_t plane, uint32_t spin, int *err, const int *stop) {
+    using C = SizeCfg;
+    if (stop && *stop) return;   // before any TMEM allocation: uniform exit
+    extern __shared__ uint8_t sp_raw[];
+    uint8_t *smem = (uint8_t *)(((uintptr_t)sp_raw + 1023) & ~(uintptr_t)1023);
+    __shared__ __align__(8) uint64_t full[SZ_STAGES], empty[SZ_STAGES], tfull, tempty, drain;
+    __shared__ uint32_t tmem_base;
+    __shared__ int abort_s;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int2 rg = ranges[blockIdx.x];
+    if (threadIdx.x == 0) {
+        for (int q = 0; q < SZ_STAGES; ++q) {
+            mbar_init(smem_u32(&full[q]), 1);
+            mbar_init(smem_u32(&empty[q]), 1);
+        }
+        mbar_init(smem_u32(&tfull), 1);
+        mbar_init(smem_u32(&tempty), 4);
+        mbar_init(smem_u32(&drain), 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        abort_s = 0;
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
+                     "r"((uint32_t)SP_SN));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tmem_base;
+    volatile int *abort = &abort_s;
+    const uint32_t drain_spin = spin > (1u << 22) ? spin : (1u << 22);
+    auto give_up = [&]() {
+        *abort = 1;
+        atomicExch(err, 1);
+    };
+    auto slabs = [](int k) { return (k + SP_KC - 1) / SP_KC; };
+    auto abox = [&](int st) { return smem_u32(smem + (size_t)st * (C::A_BYTES + C::B_BYTES)); };
+    // columns of an item's tile, a multiple of 16
+    auto width = [](const SplitItem &m) { return min(SP_SN, (m.dr - m.n0 + 15) & ~15); };
+
+    if (warp == 0 && lane == 0) {
+        // ---- TMA producer
+        int it = 0, issued = 0;
+        bool ok = true;
+        for (int i = rg.x; i < rg.y && ok && !*abort; ++i) {
+            const SplitItem m = items[i];
+            for (int c = 0; c < slabs(m.k); ++c, ++it) {
+                const int st = it % SZ_STAGES;
+                if (!mbar_wait(smem_u32(&empty[st]), ((uint32_t)(it / SZ_STAGES) & 1u) ^ 1u, spin, abort)) { give_up(); ok = false; break; }
+                const uint32_t fb = smem_u32(&full[st]);
+                mbar_expect_tx(fb, (uint32_t)(C::A_BYTES + C::B_BYTES));
+                tma_load_2d(abox(st), &map_a, 0, m.a_row + c * m.a_rows + m.m0, fb);
+                tma_load_2d(abox(st) + C::A_BYTES, &map_b, 0, m.b_row + c * m.b_rows + m.n0, fb);
+                ++issued;
+            }
+        }
+        // no copy of this CTA may still be landing when it leaves
+        volatile int never = 0;
+        for (int q = 0; q < SZ_STAGES; ++q) {
+            const int fills = (issued + SZ_STAGES - 1 - q) / SZ_STAGES;
+            if (fills && !mbar_wait(smem_u32(&full[q]), (uint32_t)(fills - 1) & 1u, drain_spin, &never)) atomicExch(err, 1);
+        }
+    } else if (warp == 1 && lane == 0) {
+        // ---- MMA issuer
+        int it = 0;
+        bool issued = false, ok = true;
+        for (int i = rg.x; i < rg.y && ok && !*abort; ++i) {
+            const SplitItem m = items[i];
+            const int nk = slabs(m.k);
+            if (!mbar_wait(smem_u32(&tempty), ((uint32_t)(i - rg.x) & 1u) ^ 1u, spin, abort)) { give_up(); break; }
+            for (int c = 0; c < nk; ++c, ++it) {
+                const int st = it % SZ_STAGES;
+                if (!mbar_wait(smem_u32(&full[st]), (uint32_t)(it / SZ_STAGES) & 1u, spin, abort)) { give_up(); ok = false; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const int ks = min(SP_KC / 16, (m.k - c * SP_KC + 15) / 16);   // K steps with anything in them
+                for (int kk = 0; kk < ks; ++kk)
+                    mma_bf16(tmem, desc_sw128(abox(st) + kk * 32), desc_sw128(abox(st) + C::A_BYTES + kk * 32),
+                             idesc_bf16(width(m)), c > 0 || kk > 0 ? 1u : 0u);
+                issued = true;
+                mma_commit(smem_u32(&empty[st]));
+            }
+            if (ok) mma_commit(smem_u32(&tfull));
+        }
+        if (issued) {   // every MMA of this lane done before the CTA frees its TMEM
+            mma_commit(smem_u32(&drain));
+            volatile int never = 0;
+            if (!mbar_wait(smem_u32(&drain), 0u, drain_spin, &never)) atomicExch(err, 1);
+        }
+    } else if (warp >= 2) {
+        // ---- warp w stores the rows of TMEM lanes 32 (w % 4) .. +31
+        const int qr = warp & 3;
+        for (int i = rg.x; i < rg.y && !*abort; ++i) {
+            const SplitItem m = items[i];
+            bool got = true;
+            if (lane == 0) got = mbar_wait(smem_u32(&tfull), (uint32_t)(i - rg.x) & 1u, spin, abort);
+            if (__shfl_sync(0xffffffffu, got ? 1 : 0, 0) == 0) {
+                if (lane == 0) give_up();
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const int il = m.m0 + 32 * qr + lane;
+            float *o = out + (int64_t)m.plane * plane + m.off + (int64_t)m.n0 * m.dl + il;
+            for (int c0 = 0; c0 < width(m); c0 += 16) {
+                uint32_t r[16];
+                tmem_ld16(tmem + ((uint32_t)(32 * qr) << 16) + (uint32_t)c0, r);
+                if (il < m.dl)
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        if (m.n0 + c0 + j < m.dr) o[(int64_t)(c0 + j) * m.dl] = __uint_as_float(r[j]);
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&tempty));
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)SP_SN));
+}
+
 // hv = plane 0 + plane 1 (rounded to FP64) + sum_t A W_q B^T, one CTA per 8 x
 // 32 outputs of a sector, a warp a row.  Per term A's row and B's columns give
 // their dominant (column, value).  The entries of A's row beside it (below 2^-40
@@ -482,9 +612,20 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_sector_split(const __grid_con
 // operations a term and output, spread over all SMs (in the GEMM's epilogue
 // they would hold one SM's FP64 pipe for 8 us a tile); the chain of dependent
 // loads bounds it, hence the tile and term records.
+//
+// GUARD (a product for the caller): a side of an element passes when the error
+// that the digits leave in it, 2^-61.3 sqrt(nonzero products) 2^e for a row and a
+// column of scale 2^e (the six digit products of i + j = 7 that are dropped, 148
+// rms a digit), is below 2^-53 of the element's sum |H||W| over both sides, one
+// rounding of a sum of that size.  Elements of rows with an Inf or NaN do not
+// pass.  Tiles of 4 x 8 that hold one that does not go to the list of k_hv_fp64,
+// with the sides that it has to sum.
+constexpr float SP_PASS = 0.0032f;               // 2^(53 - 61.3)
 struct SplitTerms {
     const SplitTerm *terms;
-    const int *tcol, *dptr, *dcol, *exps;
+    const int *tcol, *dptr, *dcol, *exps, *nnzs;
+    const float *size;
+    int *redo;
     const double *tval;
     const float *dval;
     const DevTerm *csr;
@@ -492,30 +633,50 @@ struct SplitTerms {
     const double *ab_val;
 };
 
+template <bool GUARD>
 __global__ void __launch_bounds__(256, 4) k_split_terms(const double *__restrict__ v, const float *__restrict__ v32,
                                                      const int64_t *__restrict__ planes,
                                                      const int *__restrict__ planes0, int64_t n, double *__restrict__ hv,
                                                      const SplitTile *__restrict__ tiles, SplitTerms T, const int *stop) {
     if (stop && *stop) return;
     __shared__ double dense[8][33];
+    __shared__ unsigned failed;                      // tiles of k_hv_fp64 with a side that does not pass (left, right << 8)
+    if (GUARD && threadIdx.x == 0) failed = 0;
+    if (GUARD) __syncthreads();
     const SplitTile t = tiles[blockIdx.x];
     {   // the two planes (column-major), eight rows of four columns a warp
         const int r = threadIdx.x & 7, c = threadIdx.x >> 3, il = t.row0 + r, ir = t.col0 + c;
+        const bool in = il < t.dl && ir < t.dr;
         double x = 0.0;
-        if (il < t.dl && ir < t.dr) {
+        if (in) {
             const int64_t e = t.off + (int64_t)ir * t.dl + il;
             const int64_t p0 = planes[e], p1 = planes[n + e];
             const int q0 = planes0[e], q1 = planes0[n + e];
-            // scale exponents: H_L row, W column; W row, H_R row
-            const int x0 = T.exps[t.exp + il], x1 = T.exps[t.exp + 2 * t.dl + t.dr + ir];
-            const int y0 = T.exps[t.exp + t.dl + t.dr + il], y1 = T.exps[t.exp + t.dl + ir];
-            x = (x0 >= SP_BADEXP || x1 >= SP_BADEXP || y0 >= SP_BADEXP || y1 >= SP_BADEXP)
-                    ? __longlong_as_double(0x7ff8000000000000ll)
+            // H_L row, W column; W row, H_R row
+            const int i0 = t.exp + il, i1 = t.exp + 2 * t.dl + t.dr + ir, i2 = t.exp + t.dl + t.dr + il, i3 = t.exp + t.dl + ir;
+            const int x0 = T.exps[i0], x1 = T.exps[i1], y0 = T.exps[i2], y1 = T.exps[i3];
+            const bool bad = x0 >= SP_BADEXP || x1 >= SP_BADEXP || y0 >= SP_BADEXP || y1 >= SP_BADEXP;
+            x = bad ? __longlong_as_double(0x7ff8000000000000ll)
                     : fixed_to_double(q0, p0, x0 + x1 - 56) + fixed_to_double(q1, p1, y0 + y1 - 56);
+            if constexpr (GUARD) {
+                // both sides in units of the larger scale (a row of zeros: nothing)
+                const bool zl = min(x0, x1) == SP_ZEROEXP, zr = min(y0, y1) == SP_ZEROEXP;
+                const int el = zl ? SP_ZEROEXP : x0 + x1, er = zr ? SP_ZEROEXP : y0 + y1, em = max(el, er);
+                auto unit = [&](bool z, int d) { return z || d < -126 ? 0.f : __int_as_float((127 + d) << 23); };
+                const float fl = unit(zl, el - em), fr = unit(zr, er - em);
+                const float sum = fl * T.size[e] + fr * T.size[n + e];
+                const bool left = bad || sum < SP_PASS * fl * sqrtf((float)min(T.nnzs[i0], T.nnzs[i1]));
+                const bool right = bad || sum < SP_PASS * fr * sqrtf((float)min(T.nnzs[i2], T.nnzs[i3]));
+                if (left || right) atomicOr(&failed, (left ? 1u : 0u) << ((r / 4) * 4 + c / 8) | (right ? 0x100u : 0u) << ((r / 4) * 4 + c / 8));
+            }
         }
         dense[r][c] = x;
     }
     __syncthreads();
+    if (GUARD && threadIdx.x < 8) {
+        const int sides = (failed >> threadIdx.x & 1) | (failed >> (threadIdx.x + 8) & 1) << 1;
+        if (sides) T.redo[SP_REDO_LIST + atomicAdd(T.redo + SP_REDO_COUNT, 1)] = (blockIdx.x * 8 + threadIdx.x) * 4 + sides;
+    }
     const int lane = threadIdx.x & 31;
     const int il = t.row0 + (threadIdx.x >> 5), ir = t.col0 + lane;
     if (il >= t.dl) return;                          // whole warps
@@ -615,34 +776,38 @@ void split_layout(const DevSb &s, const std::vector<int> &rowptr, const std::vec
     // pool rows and scale exponents of the four operands of every sector
     int64_t row = 0;
     struct Rows {
-        int hl, hr, w, wt, ehl, ehr, ew, ewt;
+        int hl, hr, w, wt, ehl, ehr, ew, ewt, ahl, ahr, aw, awt;
     };
     std::vector<Rows> rs(s.nsb);
-    auto jobs = [](std::vector<SplitJob> &v, int64_t src, int ld, int rows, int k, int kind, int row0, int exp0) {
-        for (int r = 0; r < rows; r += SP_ROWS) v.push_back(SplitJob{src, ld, rows, k, r, kind, row0, exp0, 0});
+    auto jobs = [](std::vector<SplitJob> &v, int64_t src, int ld, int rows, int k, int kind, int row0, int exp0, int abs0) {
+        for (int r = 0; r < rows; r += SP_ROWS) v.push_back(SplitJob{src, ld, rows, k, r, kind, row0, exp0, abs0});
     };
     int64_t tiles32 = 0;
     for (int k = 0; k < s.nsb; ++k) {
         const int dl = s.dls[k], dr = s.drs[k];
         Rows &R = rs[k];
-        auto take = [&](int rows, int kk) {
+        auto take = [&](int rows, int kk, int boxes = SP_D) {
             const int r0 = (int)row;
-            row += (int64_t)SP_D * slabs(kk) * rows;
+            row += (int64_t)boxes * slabs(kk) * rows;
             return r0;
         };
         R.hl = take(dl, dl);
         R.hr = take(dr, dr);
         R.w = take(dl, dr);
         R.wt = take(dr, dl);
+        R.ahl = take(dl, dl, 1);
+        R.ahr = take(dr, dr, 1);
+        R.aw = take(dl, dr, 1);
+        R.awt = take(dr, dl, 1);
         R.ehl = p.nexp;
         R.ehr = R.ehl + dl;
         R.ew = R.ehr + dr;
         R.ewt = R.ew + dl;
         p.nexp = R.ewt + dr;
-        jobs(p.jobs_hl, s.hl_off[k], dl, dl, dl, 0, R.hl, R.ehl);
-        jobs(p.jobs_hr, s.hr_off[k], dr, dr, dr, 0, R.hr, R.ehr);
-        jobs(p.jobs_w, s.off[k], dr, dl, dr, 0, R.w, R.ew);
-        jobs(p.jobs_w, s.off[k], dr, dr, dl, 1, R.wt, R.ewt);
+        jobs(p.jobs_hl, s.hl_off[k], dl, dl, dl, 0, R.hl, R.ehl, R.ahl);
+        jobs(p.jobs_hr, s.hr_off[k], dr, dr, dr, 0, R.hr, R.ehr, R.ahr);
+        jobs(p.jobs_w, s.off[k], dr, dl, dr, 0, R.w, R.ew, R.aw);
+        jobs(p.jobs_w, s.off[k], dr, dr, dl, 1, R.wt, R.ewt, R.awt);
         tiles32 += 2 * (int64_t)((dl + SP_M - 1) / SP_M) * ((dr + 31) / 32);
         for (int a = 0; a < dl; a += 8)
             for (int b = 0; b < dr; b += 32)
@@ -650,7 +815,7 @@ void split_layout(const DevSb &s, const std::vector<int> &rowptr, const std::vec
                                             s.hl_off[k], s.hr_off[k]});
         p.kmax = std::max({p.kmax, dl, dr});
     }
-    row += SP_M;   // a box that starts near the end of the pool stays inside it
+    row += std::max(SP_M, SP_SN);   // a box that starts near the end of the pool stays inside it
     p.pool_rows = row;
     // the longest packing jobs first
     std::stable_sort(p.jobs_w.begin(), p.jobs_w.end(), [](const SplitJob &a, const SplitJob &b) { return a.k > b.k; });
@@ -667,27 +832,40 @@ void split_layout(const DevSb &s, const std::vector<int> &rowptr, const std::vec
                 p.items.push_back(SplitItem{R.w, R.hr, dl, dr, dr, dl, dr, m0, n0, 1, s.off[k]});
             }
     }
+    for (int k = 0; k < s.nsb; ++k) {
+        const int dl = s.dls[k], dr = s.drs[k];
+        const Rows &R = rs[k];
+        for (int m0 = 0; m0 < dl; m0 += SP_M)
+            for (int n0 = 0; n0 < dr; n0 += SP_SN) {
+                p.sitems.push_back(SplitItem{R.ahl, R.awt, dl, dr, dl, dl, dr, m0, n0, 0, s.off[k]});
+                p.sitems.push_back(SplitItem{R.aw, R.ahr, dl, dr, dr, dl, dr, m0, n0, 1, s.off[k]});
+            }
+    }
     // longest first onto the least loaded CTA (an item costs its slabs plus
     // about one of epilogue)
-    std::stable_sort(p.items.begin(), p.items.end(),
-                     [&](const SplitItem &a, const SplitItem &b) { return slabs(a.k) > slabs(b.k); });
-    const int G = (int)std::min<size_t>(p.items.size(), (size_t)std::max(1, nsm));
-    std::vector<int64_t> load(G, 0);
-    std::vector<std::vector<int>> own(G);
-    for (size_t e = 0; e < p.items.size(); ++e) {
-        const int b = (int)(std::min_element(load.begin(), load.end()) - load.begin());
-        load[b] += slabs(p.items[e].k) + 1;
-        own[b].push_back((int)e);
-    }
-    p.grid = G;
-    std::vector<SplitItem> ordered;
-    ordered.reserve(p.items.size());
-    for (int g = 0; g < G; ++g) {
-        const int start = (int)ordered.size();
-        for (int e : own[g]) ordered.push_back(p.items[e]);
-        p.rng.push_back(make_int2(start, (int)ordered.size()));
-    }
-    p.items.swap(ordered);
+    auto deal = [&](std::vector<SplitItem> &items, std::vector<int2> &rng) {
+        std::stable_sort(items.begin(), items.end(),
+                         [&](const SplitItem &a, const SplitItem &b) { return slabs(a.k) > slabs(b.k); });
+        const int G = (int)std::min<size_t>(items.size(), (size_t)std::max(1, nsm));
+        std::vector<int64_t> load(G, 0);
+        std::vector<std::vector<int>> own(G);
+        for (size_t e = 0; e < items.size(); ++e) {
+            const int b = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+            load[b] += slabs(items[e].k) + 1;
+            own[b].push_back((int)e);
+        }
+        std::vector<SplitItem> ordered;
+        ordered.reserve(items.size());
+        for (int g = 0; g < G; ++g) {
+            const int start = (int)ordered.size();
+            for (int e : own[g]) ordered.push_back(items[e]);
+            rng.push_back(make_int2(start, (int)ordered.size()));
+        }
+        items.swap(ordered);
+        return G;
+    };
+    p.grid = deal(p.items, p.rng);
+    p.sgrid = deal(p.sitems, p.srng);
     // A x B terms: the dominant entry of every row, and the small rest of A's
     constexpr double SMALL = 0x1p-40;
     for (size_t ti = 0; ti < s.terms.size(); ++ti) {
@@ -738,18 +916,20 @@ int split_finish(Ctx &c, const SplitPlan &p) {
     NSS_CUDA_TRY(c, allow_smem((const void *)k_split_pack, smem));
     c.launches += 2;
     k_split_pack<<<(unsigned)p.jobs_hl.size(), 32 * SP_ROWS, smem, c.stream>>>(s.d_hl, s.d_sp_jobs_hl, s.d_sp_pool, s.d_sp_exp,
-                                                                            nullptr, nullptr, nullptr);
+                                                                            s.d_sp_exp + p.nexp, nullptr, true, nullptr, nullptr);
     k_split_pack<<<(unsigned)p.jobs_hr.size(), 32 * SP_ROWS, smem, c.stream>>>(s.d_hr, s.d_sp_jobs_hr, s.d_sp_pool, s.d_sp_exp,
-                                                                            nullptr, nullptr, nullptr);
+                                                                            s.d_sp_exp + p.nexp, nullptr, true, nullptr, nullptr);
     NSS_CUDA_TRY(c, cudaGetLastError());
+    s.sp_nexp = p.nexp;
     s.sp_nitems = (int)p.items.size();
     s.sp_njobs = (int)p.jobs_w.size();
     s.sp_ntiles = (int)p.tiles.size();
     s.sp_bn = p.bn;
     s.sp_grid = p.grid;
-    for (int which = 0; which < 2; ++which)
-        if (int rc = tc_tensor_map(c, which == 0 ? s.sp_map_a : s.sp_map_b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, s.d_sp_pool,
-                                   SP_KC, p.pool_rows, which == 0 ? SP_M : p.bn))
+    s.sp_sgrid = p.sgrid;
+    const std::pair<unsigned char *, int> maps[3] = {{s.sp_map_a, SP_M}, {s.sp_map_b, p.bn}, {s.sp_map_s, SP_SN}};
+    for (const auto &m : maps)
+        if (int rc = tc_tensor_map(c, m.first, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, s.d_sp_pool, SP_KC, p.pool_rows, m.second))
             return rc;
     return NSS_OK;
 }
@@ -768,17 +948,33 @@ int launch_split(Ctx &c, int *err, const int *stop) {
     return NSS_OK;
 }
 
+int launch_size(Ctx &c, int *err, const int *stop) {
+    NSS_CUDA_TRY(c, allow_smem((const void *)k_split_size, SizeCfg::SMEM));
+    DevSb &s = c.sb;
+    alignas(64) CUtensorMap ma, mb;
+    std::memcpy(&ma, s.sp_map_a, sizeof(ma));
+    std::memcpy(&mb, s.sp_map_s, sizeof(mb));
+    c.launches += 1;
+    k_split_size<<<s.sp_sgrid, SZ_THREADS, SizeCfg::SMEM, c.stream>>>(ma, mb, s.d_sp_sitems, s.d_sp_srng, s.d_sp_size, s.n,
+                                                                     wait_limit(), err, stop);
+    return NSS_OK;
+}
+
 }  // namespace
 
-int hv_device_split(Ctx &c, const double *d_v, double *d_hv, const int *stop, int *err, bool clear) {
+int hv_device_split(Ctx &c, const double *d_v, double *d_hv, const int *stop, bool standalone) {
     DevSb &s = c.sb;
+    int *err = standalone ? s.d_sp_redo + SP_REDO_ERR : s.d_tc_err, *nnzs = s.d_sp_exp + s.sp_nexp;
     c.launches += 3;
-    k_split_pack<<<(unsigned)s.sp_njobs, 32 * SP_ROWS, s.sp_pack_smem, c.stream>>>(d_v, s.d_sp_jobs_w, s.d_sp_pool, s.d_sp_exp,
-                                                                              s.d_sp_x32, clear ? err : nullptr, stop);
+    k_split_pack<<<(unsigned)s.sp_njobs, 32 * SP_ROWS, s.sp_pack_smem, c.stream>>>(
+        d_v, s.d_sp_jobs_w, s.d_sp_pool, s.d_sp_exp, nnzs, s.d_sp_x32, standalone, standalone ? s.d_sp_redo : nullptr, stop);
+    if (standalone)
+        if (int rc = launch_size(c, err, stop)) return rc;
     if (int rc = s.sp_bn == 64 ? launch_split<64>(c, err, stop) : launch_split<32>(c, err, stop)) return rc;
-    SplitTerms T{s.d_sp_terms, s.d_sp_tcol, s.d_sp_dptr, s.d_sp_dcol, s.d_sp_exp, s.d_sp_tval, s.d_sp_dval, s.d_terms,
-                 s.d_ab_rowptr, s.d_ab_col, s.d_ab_val};
-    k_split_terms<<<(unsigned)s.sp_ntiles, 256, 0, c.stream>>>(d_v, s.d_sp_x32, s.d_sp_out, s.d_sp_out0, s.n, d_hv, s.d_sp_tiles, T, stop);
+    SplitTerms T{s.d_sp_terms, s.d_sp_tcol, s.d_sp_dptr, s.d_sp_dcol, s.d_sp_exp, nnzs, s.d_sp_size, s.d_sp_redo, s.d_sp_tval,
+                 s.d_sp_dval, s.d_terms, s.d_ab_rowptr, s.d_ab_col, s.d_ab_val};
+    auto terms = standalone ? k_split_terms<true> : k_split_terms<false>;
+    terms<<<(unsigned)s.sp_ntiles, 256, 0, c.stream>>>(d_v, s.d_sp_x32, s.d_sp_out, s.d_sp_out0, s.n, d_hv, s.d_sp_tiles, T, stop);
     NSS_CUDA_TRY(c, cudaGetLastError());
     return NSS_OK;
 }

@@ -1,0 +1,124 @@
+"""FP64 products on the tensor cores, element by element.
+
+The digits of an operand are relative to the largest element of its row, so
+operands with elements of very different size, or products that meet in small
+elements only, are where a product through them could have fewer bits than one
+summed in FP64.  nss_hv promises an FP64 chain's error for every element:
+(Dl + Dr + terms + 8) 2^-53 (|H_L||W| + |W||H_R^T| + |A||W||B^T|), and beside
+it 2^-1074 per operation.  The reference sums in FP64 pairs.
+"""
+import numpy as np
+import pytest
+import scipy.sparse as sp
+
+pytestmark = pytest.mark.gpu
+
+EPS = 2.0 ** -53
+
+
+def _two_sum(a, b):
+    s = a + b
+    t = s - a
+    return s, (a - (s - t)) + (b - t)
+
+
+def _split(a):
+    c = 134217729.0 * a
+    h = c - (c - a)
+    return h, a - h
+
+
+def _matmul(A, B):
+    """A @ B in FP64 pairs (Dekker products, compensated sums)."""
+    hi, lo = np.zeros((A.shape[0], B.shape[1])), np.zeros((A.shape[0], B.shape[1]))
+    for k in range(A.shape[1]):
+        a, b = A[:, k:k + 1], B[k:k + 1]
+        p = a * b
+        (ah, al), (bh, bl) = _split(a), _split(b)
+        hi, r = _two_sum(hi, p)
+        lo += r + (((ah * bh - p) + ah * bl + al * bh) + al * bl)
+    return hi + lo
+
+
+class _Sb:
+    """Sectors (dl, dr) with given dense H and terms (out, in, A, B)."""
+
+    def __init__(self, monkeypatch, dims, hl, hr, terms=(), split="1", **kw):
+        import nssdmrg_gb300 as nss
+        nss.lib()
+        monkeypatch.setenv("NSS_SPLIT64", split)
+        self.dims, self.hl, self.hr, self.terms = dims, hl, hr, list(terms)
+        self.off = np.concatenate([[0], np.cumsum([a * b for a, b in dims])[:-1]]).astype(np.int64)
+        self.s = nss.Superblock(0, **kw)
+        up = [(t, k, q, 0, sp.csr_matrix(A), sp.csr_matrix(B), int(self.off[k]), int(self.off[q]))
+              for t, (k, q, A, B) in enumerate(self.terms)]
+        self.s.upload([a for a, _ in dims], [b for _, b in dims], self.off, [sp.csr_matrix(h) for h in hl],
+                      [sp.csr_matrix(h) for h in hr], up, len(up), sum(a for a, _ in dims), sum(b for _, b in dims))
+        self.n = sum(a * b for a, b in dims)
+
+    def sectors(self, v):
+        return [v[o:o + a * b].reshape(a, b) for o, (a, b) in zip(self.off, self.dims)]
+
+    def check(self, v, scale=1.0):
+        """The product of v * scale (a power of two) against the exact one of v."""
+        got = self.sectors(self.s.spmatvec(v * scale))
+        W = self.sectors(v)
+        for k, (a, b) in enumerate(self.dims):
+            parts = [(_matmul(self.hl[k], W[k]), abs(self.hl[k]) @ abs(W[k]), a),
+                     (_matmul(W[k], self.hr[k].T.copy()), abs(W[k]) @ abs(self.hr[k].T), b)]
+            for ko, q, A, B in self.terms:
+                if ko == k:
+                    parts.append((_matmul(_matmul(A, W[q]), B.T.copy()), abs(A) @ abs(W[q]) @ abs(B.T),
+                                  int((A != 0).sum(1).max()) + int((B != 0).sum(1).max())))
+            want = sum(p[0] for p in parts)
+            mag = sum(p[1] for p in parts)
+            ops = sum(p[2] for p in parts) + 8
+            tol = ops * (EPS * mag * scale + 2.0 ** -1074)
+            err = np.abs(got[k] - want * scale)
+            assert (err <= tol).all(), (k, a, b, float((err / np.maximum(tol, 1e-300)).max()))
+
+
+DIMS = [[(70, 66), (40, 130)], [(200, 180), (33, 5), (1, 300)]]
+
+
+def _operators(kind, dims, rng):
+    def make(d):
+        if kind == "diagonal":
+            return np.diag(rng.standard_normal(d))
+        if kind == "near diagonal":
+            return np.diag(rng.standard_normal(d)) + 1e-11 * rng.standard_normal((d, d))
+        if kind == "graded":
+            i = np.arange(d)
+            return rng.standard_normal((d, d)) * 10.0 ** (-8.0 * abs(i[:, None] - i) / d)
+        if kind == "sparse":
+            return rng.standard_normal((d, d)) * (rng.random((d, d)) < 3.0 / d)
+        return rng.standard_normal((d, d))
+    return [make(a) for a, _ in dims], [make(b) for _, b in dims]
+
+
+def _vector(kind, dims, rng):
+    out = []
+    for a, b in dims:
+        w = rng.standard_normal((a, b))
+        i, j = np.arange(a)[:, None] / a, np.arange(b)[None] / b
+        if kind == "graded":
+            w = w * 10.0 ** (-6.0 * (i + j))
+        if kind == "steep":
+            w = w * 10.0 ** (-20.0 * abs(i - j))
+        if kind == "one element":
+            w = np.zeros((a, b))
+            w[a // 2, b // 3] = 0.7
+        out.append(w.reshape(-1))
+    return np.concatenate(out)
+
+
+@pytest.mark.parametrize("vector", ["normal", "graded", "steep", "one element"])
+@pytest.mark.parametrize("operators", ["diagonal", "near diagonal", "graded", "sparse", "dense"])
+@pytest.mark.parametrize("dims", DIMS, ids=["two", "three"])
+def test_every_element_as_a_chain(monkeypatch, dims, operators, vector):
+    rng = np.random.default_rng(len(operators) * 10 + len(vector))
+    sb = _Sb(monkeypatch, dims, *_operators(operators, dims, rng))
+    v = _vector(vector, dims, rng)
+    sb.check(v)
+    sb.check(v)                                      # the product leaves its scratch as it found it
+    sb.s.close()
