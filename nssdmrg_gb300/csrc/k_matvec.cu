@@ -834,11 +834,13 @@ __global__ void __launch_bounds__(32 * HV_WARPS) k_hv_fp64(const double *__restr
         if constexpr (REDO) {
             part += acc;
             acc = 0.0;
-            if (in && sides != 3) {
-                const int64_t e = t.off + (int64_t)ir * dl + il + (sides & 1 ? redo.n : 0);
-                const int x0 = s.exp + (sides & 1 ? dl + dr + il : il), x1 = s.exp + (sides & 1 ? dl + ir : 2 * dl + dr + ir);
-                part += fixed_to_double(redo.planes0[e], redo.planes[e], redo.exps[x0] + redo.exps[x1] - 56);
-            }
+            if (in)
+                for (int side = 0; side < 2; ++side)
+                    if (!(sides >> side & 1)) {      // left: H_L row, W column; right: W row, H_R row
+                        const int64_t e = t.off + (int64_t)ir * dl + il + side * redo.n;
+                        const int x0 = s.exp + (side ? dl + dr + il : il), x1 = s.exp + (side ? dl + ir : 2 * dl + dr + ir);
+                        part += fixed_to_double(redo.planes0[e], redo.planes[e], redo.exps[x0] + redo.exps[x1] - 56);
+                    }
         }
         if (!t.csr) {
             for (int tb = t.t0; tb < t.t1; tb += 4) {

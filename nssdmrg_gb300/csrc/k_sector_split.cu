@@ -607,7 +607,7 @@ __global__ void __launch_bounds__(SZ_THREADS, 1) k_split_size(const __grid_const
 // their dominant (column, value).  The entries of A's row beside it (below 2^-40
 // of A's largest: rounding left by the renormalisation, up to a block sector's
 // width of them) are summed in FP32 against the FP32 copy of W, which is scaled
-// by its rows' powers of two: an error of 2^-61 of the term.  A lane holds one
+// by its rows' powers of two: an error of 2^-61 of A's largest times W's.  A lane holds one
 // such entry, its gather is broadcast, eight gathers in flight.  Two FP64
 // operations a term and output, spread over all SMs (in the GEMM's epilogue
 // they would hold one SM's FP64 pipe for 8 us a tile); the chain of dependent
@@ -617,9 +617,11 @@ __global__ void __launch_bounds__(SZ_THREADS, 1) k_split_size(const __grid_const
 // that the digits leave in it, 2^-61.3 sqrt(nonzero products) 2^e for a row and a
 // column of scale 2^e (the six digit products of i + j = 7 that are dropped, 148
 // rms a digit), is below 2^-53 of the element's sum |H||W| over both sides, one
-// rounding of a sum of that size.  Elements of rows with an Inf or NaN do not
-// pass.  Tiles of 4 x 8 that hold one that does not go to the list of k_hv_fp64,
-// with the sides that it has to sum.
+// rounding of a sum of that size.  The small entries of A pass when what FP32
+// leaves of them is below 2^-53 of the dominant products' sizes and the dense
+// part.  Elements that rows with an Inf or NaN enter do not pass.  Tiles of 4 x 8
+// that hold one that does not go to the list of k_hv_fp64, which sums the terms
+// and the sides that failed.
 constexpr float SP_PASS = 0.0032f;               // 2^(53 - 61.3)
 struct SplitTerms {
     const SplitTerm *terms;
@@ -640,7 +642,7 @@ __global__ void __launch_bounds__(256, 4) k_split_terms(const double *__restrict
                                                      const SplitTile *__restrict__ tiles, SplitTerms T, const int *stop) {
     if (stop && *stop) return;
     __shared__ double dense[8][33];
-    __shared__ unsigned failed;                      // tiles of k_hv_fp64 with a side that does not pass (left, right << 8)
+    __shared__ unsigned failed;                      // tiles of k_hv_fp64 with something that does not pass (left, right << 8, terms << 16)
     if (GUARD && threadIdx.x == 0) failed = 0;
     if (GUARD) __syncthreads();
     const SplitTile t = tiles[blockIdx.x];
@@ -673,88 +675,119 @@ __global__ void __launch_bounds__(256, 4) k_split_terms(const double *__restrict
         dense[r][c] = x;
     }
     __syncthreads();
-    if (GUARD && threadIdx.x < 8) {
-        const int sides = (failed >> threadIdx.x & 1) | (failed >> (threadIdx.x + 8) & 1) << 1;
-        if (sides) T.redo[SP_REDO_LIST + atomicAdd(T.redo + SP_REDO_COUNT, 1)] = (blockIdx.x * 8 + threadIdx.x) * 4 + sides;
-    }
     const int lane = threadIdx.x & 31;
     const int il = t.row0 + (threadIdx.x >> 5), ir = t.col0 + lane;
-    if (il >= t.dl) return;                          // whole warps
-    const bool in = ir < t.dr;
-    const int64_t e0 = t.off + (int64_t)il * t.dr + ir;
-    double acc = 0.0;
-    bool dusty = false;
-    // the dominant entries, four terms' loads in flight
-    for (int tb = t.t0; tb < t.t1; tb += 4) {
-        SplitTerm tm[4];
-        int aj[4], bj[4];
-        double c[4], w[4];
+    if (il < t.dl) {                                 // whole warps
+        const bool in = ir < t.dr;
+        const int64_t e0 = t.off + (int64_t)il * t.dr + ir;
+        double acc = 0.0;
+        double rest = 0.0, sizes = 0.0;              // error of the small entries' sums; |dominant products|
+        bool dusty = false;
+        // the dominant entries, four terms' loads in flight
+        for (int tb = t.t0; tb < t.t1; tb += 4) {
+            SplitTerm tm[4];
+            int aj[4], bj[4];
+            double c[4], w[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) tm[q] = T.terms[min(tb + q, t.t1 - 1)];
+            for (int q = 0; q < 4; ++q) tm[q] = T.terms[min(tb + q, t.t1 - 1)];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const bool on = tb + q < t.t1 && !tm[q].general;
-            dusty = dusty || tm[q].general || tm[q].dust >= 0;
-            aj[q] = on ? T.tcol[tm[q].a + il] : -1;
-            bj[q] = on && in ? T.tcol[tm[q].b + ir] : -1;
-            c[q] = (on ? T.tval[tm[q].a + il] : 0.0) * (on && in ? T.tval[tm[q].b + ir] : 0.0);
+            for (int q = 0; q < 4; ++q) {
+                const bool on = tb + q < t.t1 && !tm[q].general;
+                dusty = dusty || tm[q].general || tm[q].dust >= 0;
+                aj[q] = on ? T.tcol[tm[q].a + il] : -1;
+                bj[q] = on && in ? T.tcol[tm[q].b + ir] : -1;
+                c[q] = (on ? T.tval[tm[q].a + il] : 0.0) * (on && in ? T.tval[tm[q].b + ir] : 0.0);
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                w[q] = aj[q] >= 0 && bj[q] >= 0 ? v[tm[q].off + (int64_t)aj[q] * tm[q].drq + bj[q]] : 0.0;
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (aj[q] >= 0 && bj[q] >= 0) acc = fma(c[q], w[q], acc);
         }
+        if (dusty)
+            for (int ti = t.t0; ti < t.t1; ++ti) {
+                const SplitTerm tm = T.terms[ti];
+                if (tm.general) {                        // several sizeable entries in a row: the CSR loop
+                    if (!in) continue;
+                    const DevTerm c = T.csr[tm.term];
+                    const double *W = v + tm.off;
+                    for (int ja = T.ab_rp[c.a_rp + il]; ja < T.ab_rp[c.a_rp + il + 1]; ++ja) {
+                        const int64_t row = (int64_t)T.ab_col[ja] * tm.drq;
+                        double cb = 0.0;
+                        for (int jb = T.ab_rp[c.b_rp + ir]; jb < T.ab_rp[c.b_rp + ir + 1]; ++jb)
+                            cb = fma(T.ab_val[jb], W[row + T.ab_col[jb]], cb);
+                        acc = fma(T.ab_val[ja], cb, acc);
+                    }
+                    continue;
+                }
+                const int bj = in ? T.tcol[tm.b + ir] : -1;
+                if (GUARD && bj >= 0 && T.tcol[tm.a + il] >= 0)
+                    sizes = fma(fabs(T.tval[tm.a + il] * T.tval[tm.b + ir]), fabs(v[tm.off + (int64_t)T.tcol[tm.a + il] * tm.drq + bj]), sizes);
+                if (tm.dust < 0) continue;
+                const int p0 = T.dptr[tm.dust + il], p1 = T.dptr[tm.dust + il + 1];   // uniform over the warp
+                const float *W32 = v32 + tm.off + max(bj, 0);
+                for (int p = p0; p < p1; p += 32) {
+                    const int cnt = min(32, p1 - p);
+                    const int dc = lane < cnt ? T.dcol[p + lane] : 0;
+                    const int ex = lane < cnt ? T.exps[tm.ew + dc] : SP_ZEROEXP;
+                    // powers of two of the input rows relative to the largest of them
+                    const int top = __reduce_max_sync(0xffffffffu, ex);
+                    const float dx = lane < cnt ? T.dval[p + lane] : 0.f;
+                    float dv = 0.f;
+                    if (ex - top > -120) dv = dx * __int_as_float((127 + ex - top) << 23);
+                    const int at = dc * tm.drq;
+                    float s = 0.f, size = 0.f;
+                    for (int u = 0; u < cnt; u += 8) {
+                        float g[8];
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-            w[q] = aj[q] >= 0 && bj[q] >= 0 ? v[tm[q].off + (int64_t)aj[q] * tm[q].drq + bj[q]] : 0.0;
+                        for (int q = 0; q < 8; ++q) g[q] = W32[__shfl_sync(0xffffffffu, at, u + q)];
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-            if (aj[q] >= 0 && bj[q] >= 0) acc = fma(c[q], w[q], acc);
+                        for (int q = 0; q < 8; ++q) {
+                            const float a = __shfl_sync(0xffffffffu, dv, u + q);
+                            s = fmaf(a, g[q], s);
+                            if (GUARD) size = fmaf(fabsf(a), fabsf(g[q]), size);
+                        }
+                    }
+                    if (top >= SP_BADEXP) {              // a row with an Inf or NaN
+                        if (bj >= 0) acc = rest = __longlong_as_double(0x7ff8000000000000ll);
+                        continue;
+                    }
+                    if constexpr (GUARD) {
+                        // FP32 sums of 32 truncated elements: 2^-20 of their size; what
+                        // lies 2^-120 below the largest row is left out, and a sum
+                        // below FP32's normal range
+                        const float most = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(dx))));
+                        const float lost = fmaf(0x1p-114f, most, 0x1p-126f);
+                        const double unit = __hiloint2double(min(max(top + 1023, 1), 2046) << 20, 0);
+                        if (bj >= 0 && top > SP_ZEROEXP) rest = fma((double)fmaf(size, 0x1p-20f, lost) * unit, fabs(T.tval[tm.b + ir]), rest);
+                    }
+                    if (bj >= 0 && s != 0.f) {
+                        // s 2^top as a double by its bits (s is normal or negligible)
+                        const uint32_t b = __float_as_uint(s);
+                        const int e = (int)((b >> 23) & 0xff) - 127 + top + 1023;
+                        if (e > 0 && e < 2047 && ((b >> 23) & 0xff))
+                            acc = fma(__hiloint2double((int)((b & 0x80000000u) | ((uint32_t)e << 20) | ((b & 0x7fffffu) >> 3)),
+                                                       (int)(b << 29)),
+                                      T.tval[tm.b + ir], acc);
+                        else if (GUARD && e <= 0)
+                            rest += 0x1p-1022;
+                    }
+                }
+            }
+        if (GUARD && dusty && in && !(rest <= 0x1p-53 * (sizes + fabs(dense[threadIdx.x >> 5][lane]))))
+            atomicOr(&failed, 0x10000u << ((threadIdx.x >> 7) * 4 + lane / 8));
+        if (in) hv[e0] = dense[threadIdx.x >> 5][lane] + acc;
     }
-    if (dusty)
-        for (int ti = t.t0; ti < t.t1; ++ti) {
-            const SplitTerm tm = T.terms[ti];
-            if (tm.general) {                        // several sizeable entries in a row: the CSR loop
-                if (!in) continue;
-                const DevTerm c = T.csr[tm.term];
-                const double *W = v + tm.off;
-                for (int ja = T.ab_rp[c.a_rp + il]; ja < T.ab_rp[c.a_rp + il + 1]; ++ja) {
-                    const int64_t row = (int64_t)T.ab_col[ja] * tm.drq;
-                    double cb = 0.0;
-                    for (int jb = T.ab_rp[c.b_rp + ir]; jb < T.ab_rp[c.b_rp + ir + 1]; ++jb)
-                        cb = fma(T.ab_val[jb], W[row + T.ab_col[jb]], cb);
-                    acc = fma(T.ab_val[ja], cb, acc);
-                }
-                continue;
-            }
-            if (tm.dust < 0) continue;
-            const int p0 = T.dptr[tm.dust + il], p1 = T.dptr[tm.dust + il + 1];   // uniform over the warp
-            const int bj = in ? T.tcol[tm.b + ir] : -1;
-            const float *W32 = v32 + tm.off + max(bj, 0);
-            for (int p = p0; p < p1; p += 32) {
-                const int cnt = min(32, p1 - p);
-                const int dc = lane < cnt ? T.dcol[p + lane] : 0;
-                const int ex = lane < cnt ? T.exps[tm.ew + dc] : -(1 << 20);
-                // powers of two of the input rows relative to the largest of them
-                const int top = __reduce_max_sync(0xffffffffu, ex);
-                float dv = 0.f;
-                if (lane < cnt && ex - top > -120) dv = T.dval[p + lane] * __int_as_float((127 + ex - top) << 23);
-                const int at = dc * tm.drq;
-                float s = 0.f;
-                for (int u = 0; u < cnt; u += 8) {
-                    float g[8];
-#pragma unroll
-                    for (int q = 0; q < 8; ++q) g[q] = W32[__shfl_sync(0xffffffffu, at, u + q)];
-#pragma unroll
-                    for (int q = 0; q < 8; ++q) s = fmaf(__shfl_sync(0xffffffffu, dv, u + q), g[q], s);
-                }
-                if (bj >= 0 && s != 0.f) {
-                    // s 2^top as a double by its bits (s is normal or negligible)
-                    const uint32_t b = __float_as_uint(s);
-                    const int e = (int)((b >> 23) & 0xff) - 127 + top + 1023;
-                    if (e > 0 && e < 2047 && ((b >> 23) & 0xff))
-                        acc = fma(__hiloint2double((int)((b & 0x80000000u) | ((uint32_t)e << 20) | ((b & 0x7fffffu) >> 3)),
-                                                   (int)(b << 29)),
-                                  T.tval[tm.b + ir], acc);
-                }
-            }
+    if constexpr (GUARD) {
+        __syncthreads();
+        if (threadIdx.x < 8) {
+            const unsigned f = failed >> threadIdx.x;
+            if (f & 0x10101u)
+                T.redo[SP_REDO_LIST + atomicAdd(T.redo + SP_REDO_COUNT, 1)] =
+                    (blockIdx.x * 8 + threadIdx.x) * 4 + (f & 1) + (f >> 7 & 2);
         }
-    if (in) hv[e0] = dense[threadIdx.x >> 5][lane] + acc;
+    }
 }
 
 // ---------------------------------------------------------------------------

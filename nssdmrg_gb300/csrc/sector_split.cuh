@@ -127,7 +127,7 @@ int split_finish(Ctx &c, const SplitPlan &p);
 // left to k_hv_fp64 go to sb.d_sp_redo (cleared first); else the former to
 // sb.d_tc_err and the product is accurate relative to the rows' largest elements.
 int hv_device_split(Ctx &c, const double *d_v, double *d_hv, const int *stop, bool standalone);
-// sb.d_sp_redo; the list holds 4 tile + sides (1: H_L W, 2: W H_R^T)
+// sb.d_sp_redo; the list holds 4 tile + sides to sum (1: H_L W, 2: W H_R^T)
 constexpr int SP_REDO_ERR = 0, SP_REDO_COUNT = 1, SP_REDO_LIST = 2;
 
 }  // namespace nss

@@ -122,3 +122,92 @@ def test_every_element_as_a_chain(monkeypatch, dims, operators, vector):
     sb.check(v)
     sb.check(v)                                      # the product leaves its scratch as it found it
     sb.s.close()
+
+
+def _cross(dims, rng, small):
+    """Terms between sectors: +-1 in a shifted diagonal, `small` beside it in half of A."""
+    out = []
+    for k, (a1, b1) in enumerate(dims):
+        q = (k + 1) % len(dims)
+        a0, b0 = dims[q]
+        A = np.zeros((a1, a0))
+        A[np.arange(a1), np.arange(a1) % a0] = rng.choice([-1.0, 1.0], a1)
+        rest = small * rng.standard_normal((a1, a0)) * (rng.random((a1, a0)) < 0.5)
+        A = np.where(A != 0, A, rest)
+        B = np.zeros((b1, b0))
+        B[np.arange(b1), rng.integers(0, b0, b1)] = rng.standard_normal(b1)
+        out.append((k, q, A, B))
+    return out
+
+
+@pytest.mark.parametrize("small", [1e-13, 1e-17])
+def test_small_entries_of_a_alone(monkeypatch, small):
+    """Rows of A whose large entry meets a zero row of the vector, so that only
+    the small entries count; and rows where it meets a tiny one."""
+    dims = [(70, 66), (40, 130), (90, 33)]
+    rng = np.random.default_rng(11)
+    zeros = [np.zeros((a, a)) for a, _ in dims], [np.zeros((b, b)) for _, b in dims]
+    sb = _Sb(monkeypatch, dims, *zeros, _cross(dims, rng, small))
+    for tiny in (0.0, 1e-18):
+        v = rng.standard_normal(sb.n)
+        for w in sb.sectors(v):
+            w[::2] *= tiny
+        sb.check(v)
+    v = _vector("steep", dims, rng)
+    sb.check(v)
+    sb.s.close()
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
+def test_non_finite_elements_as_a_chain(monkeypatch, value):
+    """The elements an Inf or NaN reaches, and how, are those of the FP64 chain;
+    the others keep their value."""
+    dims = [(70, 66), (40, 130), (90, 33)]
+    rng = np.random.default_rng(13)
+    hl, hr = _operators("dense", dims, rng)
+    hl[0][:, 5] = 0.0                                # 0 x Inf
+    terms = _cross(dims, rng, 1e-15)
+    v = rng.standard_normal(sum(a * b for a, b in dims))
+    # in columns that the terms of sectors 2 and 0 read
+    cols = [int(np.nonzero(terms[k][3])[1][3]) for k in (2, 0)]
+    a, b = _Sb(monkeypatch, dims, hl, hr, terms), _Sb(monkeypatch, dims, hl, hr, terms, split="0")
+    for at in (5 * 66 + cols[0], 70 * 66 + 3 * 130 + cols[1]):
+        w = v.copy()
+        w[at] = value
+        got, want = a.s.spmatvec(w), b.s.spmatvec(w)
+        np.testing.assert_array_equal(np.isnan(got), np.isnan(want))
+        inf = np.isinf(want)
+        np.testing.assert_array_equal(np.isinf(got), inf)
+        np.testing.assert_array_equal(got[inf], want[inf])
+        fin = np.isfinite(want)
+        assert 0 < fin.sum() < fin.size
+        # both are chains of at most 300 operations on elements of order one
+        np.testing.assert_allclose(got[fin], want[fin], rtol=0, atol=600 * EPS * 300)
+    a.s.close()
+    b.s.close()
+
+
+def test_a_non_finite_row_among_small_entries(monkeypatch):
+    """An Inf or NaN that the small entries of A reach goes to its own column
+    alone; the other columns keep what the small entries give."""
+    dims = [(70, 66), (40, 130), (90, 33)]
+    rng = np.random.default_rng(14)
+    zeros = [np.zeros((a, a)) for a, _ in dims], [np.zeros((b, b)) for _, b in dims]
+    terms = _cross(dims, rng, 1e-14)
+    col = int(np.nonzero(terms[2][3])[1][3])
+    sb, ref = _Sb(monkeypatch, dims, *zeros, terms), _Sb(monkeypatch, dims, *zeros, terms, split="0")
+    v = rng.standard_normal(sb.n)
+    w = sb.sectors(v)[0]
+    w[::2] = 0.0                                     # sector 2's large entries of A meet zeros
+    for value in (np.nan, np.inf):
+        w[6, col] = value
+        got, want = sb.s.spmatvec(v), ref.s.spmatvec(v)
+        np.testing.assert_array_equal(np.isnan(got), np.isnan(want))
+        fin = np.isfinite(want)
+        np.testing.assert_array_equal(np.isfinite(got), fin)
+        # chains of at most 70 products
+        np.testing.assert_allclose(got[fin], want[fin], rtol=200 * EPS, atol=200 * EPS * 1e-14 * 30)
+        sub = sb.sectors(want)[2][::2]
+        assert not np.isfinite(sub).all() and 0 < np.abs(sub[np.isfinite(sub)]).max() < 1e-10
+    sb.s.close()
+    ref.s.close()
