@@ -623,6 +623,7 @@ __global__ void __launch_bounds__(SZ_THREADS, 1) k_split_size(const __grid_const
 // that hold one that does not go to the list of k_hv_fp64, which sums the terms
 // and the sides that failed.
 constexpr float SP_PASS = 0.0032f;               // 2^(53 - 61.3)
+constexpr int SP_LOWEXP = -960;                  // 2^-61 of it is FP64's smallest normal number
 struct SplitTerms {
     const SplitTerm *terms;
     const int *tcol, *dptr, *dcol, *exps, *nnzs;
@@ -667,8 +668,11 @@ __global__ void __launch_bounds__(256, 4) k_split_terms(const double *__restrict
                 auto unit = [&](bool z, int d) { return z || d < -126 ? 0.f : __int_as_float((127 + d) << 23); };
                 const float fl = unit(zl, el - em), fr = unit(zr, er - em);
                 const float sum = fl * T.size[e] + fr * T.size[n + e];
-                const bool left = bad || sum < SP_PASS * fl * sqrtf((float)min(T.nnzs[i0], T.nnzs[i1]));
-                const bool right = bad || sum < SP_PASS * fr * sqrtf((float)min(T.nnzs[i2], T.nnzs[i3]));
+                // planes of this scale may round to a subnormal, which fixed_to_double
+                // does not give; above it what it drops is below the digits' error
+                const bool low = (!zl && el < SP_LOWEXP) || (!zr && er < SP_LOWEXP);
+                const bool left = bad || low || sum < SP_PASS * fl * sqrtf((float)min(T.nnzs[i0], T.nnzs[i1]));
+                const bool right = bad || low || sum < SP_PASS * fr * sqrtf((float)min(T.nnzs[i2], T.nnzs[i3]));
                 if (left || right) atomicOr(&failed, (left ? 1u : 0u) << ((r / 4) * 4 + c / 8) | (right ? 0x100u : 0u) << ((r / 4) * 4 + c / 8));
             }
         }

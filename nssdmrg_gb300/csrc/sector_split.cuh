@@ -18,7 +18,7 @@ constexpr int SP_KMAX = 4096;  // largest contracted dimension (the 64-bit sums)
 constexpr int SP_BADEXP = 1 << 20;         // scale exponent of a row with an Inf or NaN
 constexpr int SP_ZEROEXP = -(1 << 20);     // ... of a row of zeros
 
-// (s0 2^42 + r) 2^e rounded to nearest even, in integer arithmetic
+// (s0 2^42 + r) 2^e rounded to nearest even, in integer arithmetic; 0 below the normal range
 __device__ __forceinline__ double fixed_to_double(int s0, int64_t r, int e) {
     uint64_t l = ((uint64_t)(int64_t)s0 << 42) + (uint64_t)r;
     int64_t h = (int64_t)(s0 >> 22) + (r >> 63) + (l < (uint64_t)r ? 1 : 0);

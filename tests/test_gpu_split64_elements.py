@@ -5,7 +5,8 @@ operands with elements of very different size, or products that meet in small
 elements only, are where a product through them could have fewer bits than one
 summed in FP64.  nss_hv promises an FP64 chain's error for every element:
 (Dl + Dr + terms + 8) 2^-53 (|H_L||W| + |W||H_R^T| + |A||W||B^T|), and beside
-it 2^-1074 per operation.  The reference sums in FP64 pairs.
+it 2^-1074 per operation where results leave the normal range.  The reference
+sums in FP64 pairs.
 """
 import numpy as np
 import pytest
@@ -155,6 +156,28 @@ def test_small_entries_of_a_alone(monkeypatch, small):
         sb.check(v)
     v = _vector("steep", dims, rng)
     sb.check(v)
+    sb.s.close()
+
+
+@pytest.mark.parametrize("scale", [2.0 ** -1030, 2.0 ** -1050, 2.0 ** -1070])
+def test_results_below_the_normal_range(monkeypatch, scale):
+    dims = [(70, 66), (40, 130)]
+    rng = np.random.default_rng(12)
+    sb = _Sb(monkeypatch, dims, *_operators("dense", dims, rng))
+    v = np.round(rng.standard_normal(sb.n), 0)       # a few bits, so that v * scale is exact
+    sb.check(v, scale)
+    sb.s.close()
+
+
+def test_small_products_of_normal_operands(monkeypatch):
+    """Operators and a vector in the normal range whose products lie below it."""
+    dims = [(70, 66), (40, 130)]
+    rng = np.random.default_rng(15)
+    hl, hr = ([np.round(h) * 2.0 ** -60 for h in x] for x in _operators("dense", dims, rng))
+    sb = _Sb(monkeypatch, dims, hl, hr)
+    v = np.round(rng.standard_normal(sb.n), 0)
+    for scale in (2.0 ** -962, 2.0 ** -985, 2.0 ** -1010):
+        sb.check(v, scale)
     sb.s.close()
 
 
