@@ -101,8 +101,10 @@ struct DevSb {
     alignas(64) unsigned char mma_map_a[128] = {}, mma_map_b[128] = {};
     // FP64 product on the tensor cores (k_sector_split.cu), sections of the
     // arena: digit pool [rows][64] bf16, scale exponents, FP32 copy of the
-    // vector, the two output planes, work items with their per-CTA ranges,
-    // packing jobs, A x B terms and output tiles (sp_nitems = 0: not used)
+    // vector, the two output planes (these in Ctx::sp_mem), work items with their
+    // per-CTA ranges, packing jobs, A x B terms and output tiles.  sp_ntiles = 0:
+    // the superblock does not take this path; sp_nitems = 0: no memory for it, and
+    // k_hv_fp64 runs over its tiles
     uint32_t *d_sp_pool = nullptr;
     int *d_sp_exp = nullptr, *d_sp_tcol = nullptr, *d_sp_dptr = nullptr, *d_sp_dcol = nullptr;
     float *d_sp_x32 = nullptr, *d_sp_dval = nullptr;
@@ -296,6 +298,10 @@ struct Ctx {
     int rdm_max_block = 0;
     char *sb_arena = nullptr, *sb_stage = nullptr;   // superblock pool: device arena, pinned staging
     size_t sb_arena_cap = 0, sb_stage_cap = 0;
+    // digits and planes of the FP64 product on the tensor cores: kept from one
+    // superblock to the next, given up when another allocation finds no room
+    char *sp_mem = nullptr;
+    size_t sp_cap = 0;
     double renorm_phase_ms[3] = {0, 0, 0};
     int refine_passes = 0, refine_cluster = 0;   // mixed refinement of the last solve
     bool last_pair = false;                      // ... needed a near-degenerate partner
@@ -309,13 +315,22 @@ struct Ctx {
     size_t peak_used = 0;                // largest `used` so far
 };
 
-// Allocation through the context budget.
+// Give up the memory of the FP64 product on the tensor cores (its products then
+// run on the CUDA cores); false when there is none
+bool split_drop(Ctx &c);
+
+// Allocation through the context budget.  spare: not worth giving up anything for.
 template <class T>
-cudaError_t ctx_alloc(Ctx &c, T **p, size_t count) {
+cudaError_t ctx_alloc(Ctx &c, T **p, size_t count, bool spare = false) {
     size_t bytes = count * sizeof(T);
     if (bytes == 0) bytes = 16;
-    if (c.budget && c.used + bytes > c.budget) return cudaErrorMemoryAllocation;
+    auto over = [&] { return c.budget && c.used + bytes > c.budget; };
+    if (over() && (spare || !split_drop(c) || over())) return cudaErrorMemoryAllocation;
     cudaError_t e = cudaMalloc((void **)p, bytes);
+    if (e == cudaErrorMemoryAllocation && !spare && split_drop(c)) {
+        cudaGetLastError();
+        e = cudaMalloc((void **)p, bytes);
+    }
     if (e == cudaSuccess) {
         c.used += bytes;
         c.peak_used = c.used > c.peak_used ? c.used : c.peak_used;
@@ -328,7 +343,7 @@ void ctx_free(Ctx &c, void *p);
 // k_matvec.cu
 // trusted: the descriptor comes from this library's own setup (its column
 // indices are not re-checked entry by entry)
-int sb_upload(Ctx &c, const nss_sb_desc *d, bool trusted = false);
+int sb_upload(Ctx &c, const nss_sb_desc *d, bool trusted = false, bool allow_split = true);
 // Drop the pool; free_arena also returns its device arena and pinned
 // staging buffer (otherwise kept for the next upload).
 void sb_release(Ctx &c, bool free_arena);

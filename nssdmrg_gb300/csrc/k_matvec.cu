@@ -68,12 +68,36 @@ void ctx_free(Ctx &c, void *p) {
 void sb_release(Ctx &c, bool free_arena) {
     c.sb = DevSb{};
     if (free_arena) {
+        ctx_free(c, c.sp_mem);
+        c.sp_mem = nullptr;
+        c.sp_cap = 0;
         ctx_free(c, c.sb_arena);
         if (c.sb_stage) cudaFreeHost(c.sb_stage);
         c.sb_arena = nullptr;
         c.sb_stage = nullptr;
         c.sb_arena_cap = c.sb_stage_cap = 0;
     }
+}
+
+namespace {
+
+uint64_t next_gen() {
+    static std::atomic<uint64_t> gen{0};
+    return ++gen;
+}
+
+}  // namespace
+
+bool split_drop(Ctx &c) {
+    if (!c.sp_mem) return false;
+    ctx_free(c, c.sp_mem);           // waits for the device
+    c.sp_mem = nullptr;
+    c.sp_cap = 0;
+    if (c.sb.sp_nitems) {
+        c.sb.sp_nitems = 0;
+        c.sb.gen = next_gen();       // graphs captured with it are void
+    }
+    return true;
 }
 
 namespace {
@@ -253,7 +277,7 @@ bool csr_finite(const nss_csr &m) {
 
 // Validate and copy the operator pool.  Errors mirror the reference's stop
 // conditions (wrong sizes, vecDim != m_sb) as NSS_ERR_INVALID.
-int sb_upload(Ctx &c, const nss_sb_desc *d, bool trusted) {
+int sb_upload(Ctx &c, const nss_sb_desc *d, bool trusted, bool allow_split) {
     if (!d || d->nsb <= 0 || d->tnso < 0 || !d->dls || !d->drs || !d->offset || !d->hleft ||
         !d->hright) {
         c.err = "nss_sb_upload: incomplete descriptor";
@@ -410,7 +434,7 @@ int sb_upload(Ctx &c, const nss_sb_desc *d, bool trusted) {
     s.ntiles = (int)tiles.size();
     // k_hv_fp64's terms, with the first entry of every row, and its tiles,
     // longest first
-    const bool split = split_wanted(s);
+    const bool split = allow_split && split_wanted(s);
     std::vector<HvTerm> hv_terms;
     std::vector<HvRec> hv_recs;
     std::vector<int> ell_col;
@@ -664,15 +688,9 @@ int sb_upload(Ctx &c, const nss_sb_desc *d, bool trusted) {
     sg.add(&s.d_hv_terms, hv_terms);
     sg.add(&s.d_ell_col, ell_col);
     sg.add(&s.d_ell_val, ell_val);
-    sg.add_dev(&s.d_sp_redo, SP_REDO_LIST + HV_SUB * sp.tiles.size());
-    sg.add_dev(&s.d_sp_exp, 2 * (size_t)sp.nexp);
-    sg.add_dev(&s.d_sp_size, split ? 2 * (size_t)s.n : 0);
-    sg.add_dev(&s.d_sp_x32, split ? (size_t)s.n : 0);
-    sg.add_dev(&s.d_sp_out, split ? 2 * (size_t)s.n : 0);
-    sg.add_dev(&s.d_sp_out0, split ? 2 * (size_t)s.n : 0);
-    sg.add_dev(&s.d_sp_pool, (size_t)sp.pool_rows * (SP_KC / 2));
     int rc;
-    if ((rc = stage_commit(c, sg))) return rc;
+    // a superblock that fits without the tensor-core product's tables is taken without
+    if ((rc = stage_commit(c, sg))) return split && rc == NSS_ERR_NOMEM ? sb_upload(c, d, trusted, false) : rc;
     NSS_CUDA_TRY(c, cudaMemsetAsync(s.d_hl, 0, (size_t)hl_tot * sizeof(double), c.stream));
     NSS_CUDA_TRY(c, cudaMemsetAsync(s.d_hr, 0, (size_t)hr_tot * sizeof(double), c.stream));
     {
@@ -688,8 +706,7 @@ int sb_upload(Ctx &c, const nss_sb_desc *d, bool trusted) {
     if ((rc = mma_finish(c, plan))) return rc;
     if ((rc = split_finish(c, sp))) return rc;
     NSS_CUDA_TRY(c, cudaStreamSynchronize(c.stream));
-    static std::atomic<uint64_t> g_gen{0};
-    s.gen = ++g_gen;
+    s.gen = next_gen();
     s.valid = true;
     return NSS_OK;
 }
@@ -734,7 +751,7 @@ struct HvOps {
 };
 
 // What k_hv_fp64 computes of a product on the tensor cores: every tile when
-// that gave up, else those on its list, of which the sides that are good come
+// that gave up or did not run (words null), else those on its list, of which the sides that are good come
 // from the planes of digit sums.  A tile is an eighth of a SplitTile.
 struct HvRedo {
     const SplitTile *tiles;
@@ -751,7 +768,7 @@ __global__ void __launch_bounds__(32 * HV_WARPS) k_hv_fp64(const double *__restr
     if (stop && *stop) return;   // the Lanczos loop has already finished (the same for every CTA)
     bool listed = false;
     if constexpr (REDO) {
-        listed = !redo.words[SP_REDO_ERR];
+        listed = redo.words && !redo.words[SP_REDO_ERR];
         if (listed) ntiles = redo.words[SP_REDO_COUNT];
     }
     constexpr int KC = 32;
@@ -1012,12 +1029,15 @@ int hv_device(Ctx &c, const double *d_v, double *d_hv, const int *stop, bool sta
         return NSS_ERR_STATE;
     }
     const HvOps op{s.d_hl, s.d_hr, s.d_hv_terms, s.d_ell_col, s.d_ell_val, s.d_ab_rowptr, s.d_ab_col, s.d_ab_val};
-    if (s.sp_nitems) {
-        if (int rc = hv_device_split(c, d_v, d_hv, stop, standalone)) return rc;
-        if (!standalone) return NSS_OK;
-        k_hv_fp64<true><<<s.hv_grid, 32 * HV_WARPS, 0, c.stream>>>(d_v, d_hv, nullptr, 
-            HvRedo{s.d_sp_tiles, s.d_sp_redo, s.d_sp_out, s.d_sp_out0, s.d_sp_exp, s.n}, op,
-                                                                   s.sp_ntiles * HV_SUB, s.hv_nsm, stop);
+    if (s.sp_ntiles) {
+        const bool tc = s.sp_nitems > 0;             // else all of it here
+        if (tc)
+            if (int rc = hv_device_split(c, d_v, d_hv, stop, standalone)) return rc;
+        if (tc && !standalone) return NSS_OK;
+        k_hv_fp64<true><<<s.hv_grid, 32 * HV_WARPS, 0, c.stream>>>(
+            d_v, d_hv, nullptr,
+            HvRedo{s.d_sp_tiles, tc ? s.d_sp_redo : nullptr, s.d_sp_out, s.d_sp_out0, s.d_sp_exp, s.n}, op,
+            s.sp_ntiles * HV_SUB, s.hv_nsm, stop);
     } else {
         k_hv_fp64<false><<<s.hv_grid, 32 * HV_WARPS, 0, c.stream>>>(d_v, d_hv, s.d_hv_recs, HvRedo{}, op, s.nhv, s.hv_nsm,
                                                                     stop);

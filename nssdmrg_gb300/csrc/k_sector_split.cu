@@ -947,6 +947,38 @@ void split_layout(const DevSb &s, const std::vector<int> &rowptr, const std::vec
 int split_finish(Ctx &c, const SplitPlan &p) {
     DevSb &s = c.sb;
     if (p.items.empty()) return NSS_OK;
+    s.sp_ntiles = (int)p.tiles.size();
+    // the sections that the device fills, at 256-byte boundaries
+    const std::pair<void **, size_t> want[] = {
+        {(void **)&s.d_sp_redo, sizeof(int) * (SP_REDO_LIST + 8 * p.tiles.size())},
+        {(void **)&s.d_sp_exp, sizeof(int) * 2 * (size_t)p.nexp},
+        {(void **)&s.d_sp_size, sizeof(float) * 2 * (size_t)s.n},
+        {(void **)&s.d_sp_x32, sizeof(float) * (size_t)s.n},
+        {(void **)&s.d_sp_out, sizeof(int64_t) * 2 * (size_t)s.n},
+        {(void **)&s.d_sp_out0, sizeof(int) * 2 * (size_t)s.n},
+        {(void **)&s.d_sp_pool, 2 * SP_KC * (size_t)p.pool_rows}};
+    size_t need = 0;
+    for (const auto &w : want) need += (w.second + 255) & ~(size_t)255;
+    if (need > c.sp_cap) {
+        ctx_free(c, c.sp_mem);
+        c.sp_mem = nullptr;
+        c.sp_cap = 0;
+        // headroom: the size varies from step to step
+        for (size_t cap : {need + need / 4, need}) {
+            if (ctx_alloc(c, &c.sp_mem, cap, true) == cudaSuccess) {
+                c.sp_cap = cap;
+                break;
+            }
+            cudaGetLastError();
+            c.sp_mem = nullptr;
+        }
+        if (!c.sp_mem) return NSS_OK;                // the products stay on the CUDA cores
+    }
+    size_t at = 0;
+    for (const auto &w : want) {
+        *w.first = c.sp_mem + at;
+        at += (w.second + 255) & ~(size_t)255;
+    }
     const int part = p.kmax <= SP_STRIP ? p.kmax : SP_STRIP;   // widest strip of a job
     const size_t smem = (size_t)SP_ROWS * (part | 1) * sizeof(double);
     s.sp_pack_smem = smem;
@@ -960,7 +992,6 @@ int split_finish(Ctx &c, const SplitPlan &p) {
     s.sp_nexp = p.nexp;
     s.sp_nitems = (int)p.items.size();
     s.sp_njobs = (int)p.jobs_w.size();
-    s.sp_ntiles = (int)p.tiles.size();
     s.sp_bn = p.bn;
     s.sp_grid = p.grid;
     s.sp_sgrid = p.sgrid;

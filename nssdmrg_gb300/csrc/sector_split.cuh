@@ -121,7 +121,8 @@ bool split_wanted(const DevSb &s);
 // (csr: HvRec::csr per sector)
 void split_layout(const DevSb &s, const std::vector<int> &rowptr, const std::vector<int> &col,
                   const std::vector<double> &val, const std::vector<int> &csr, int nsm, SplitPlan &p);
-// digits of H_L and H_R and the tensor maps, after the dense blocks are built
+// memory, digits of H_L and H_R and the tensor maps, after the dense blocks are
+// built; without room for them sb.sp_nitems stays 0
 int split_finish(Ctx &c, const SplitPlan &p);
 // hv = H v on c.stream.  standalone: a wait that ran out and the tiles that are
 // left to k_hv_fp64 go to sb.d_sp_redo (cleared first); else the former to
