@@ -122,9 +122,13 @@ void *nss_stream(const nss_ctx *ctx);
  * graded over many decades), and whole products whose bounded waits run out,
  * are computed on the CUDA cores instead. */
 int nss_hv(nss_ctx *ctx, int64_t n, const double *v, double *hv);
-/* Same on device pointers, ordered on the context's stream. */
+/* Same on device pointers, ordered on the context's stream.  Captured from it
+ * into a CUDA graph, a product uses its own vectors and the superblock alone (on
+ * the CUDA cores), so that graphs may be replayed at the same time. */
 int nss_hv_device(nss_ctx *ctx, int64_t n, const double *d_v, double *d_hv);
-/* The FP32 product of the mixed-precision path, on device pointers. */
+/* The FP32 product of the mixed-precision path, on device pointers; its
+ * tensor-core sectors go through planes of the superblock, one product at a
+ * time. */
 int nss_hv_device_f32(nss_ctx *ctx, int64_t n, const float *d_v, float *d_hv);
 
 /* Lowest `neigen` eigenpairs of the uploaded H_sb (replaces sp_eigh at

@@ -350,7 +350,8 @@ void sb_release(Ctx &c, bool free_arena);
 // `stop` (may be null): a device flag; the kernels return at once when set.
 // standalone: a product for a caller that only gets its result.  What the
 // tensor cores do not deliver (a wait that ran out, elements that their digits
-// hold less exactly than a chain of FP64 sums) k_hv_fp64 then computes.
+// hold less exactly than a chain of FP64 sums) k_hv_fp64 then computes; while
+// c.stream is being captured it computes all of it.
 // Solvers pass false and look at sb.d_tc_err with their other results.
 int hv_device(Ctx &c, const double *d_v, double *d_hv, const int *stop = nullptr, bool standalone = false);
 // add_planes false: the tensor-core sectors' part stays in sb.d_mma_out (mma_nplanes planes)

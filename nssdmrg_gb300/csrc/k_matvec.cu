@@ -1030,7 +1030,14 @@ int hv_device(Ctx &c, const double *d_v, double *d_hv, const int *stop, bool sta
     }
     const HvOps op{s.d_hl, s.d_hr, s.d_hv_terms, s.d_ell_col, s.d_ell_val, s.d_ab_rowptr, s.d_ab_col, s.d_ab_val};
     if (s.sp_ntiles) {
-        const bool tc = s.sp_nitems > 0;             // else all of it here
+        bool tc = s.sp_nitems > 0;                   // else all of it here
+        if (tc && standalone) {
+            // a product that is being captured may be replayed beside others: it
+            // keeps to its own vectors
+            cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+            NSS_CUDA_TRY(c, cudaStreamIsCapturing(c.stream, &cap));
+            tc = cap == cudaStreamCaptureStatusNone;
+        }
         if (tc)
             if (int rc = hv_device_split(c, d_v, d_hv, stop, standalone)) return rc;
         if (tc && !standalone) return NSS_OK;

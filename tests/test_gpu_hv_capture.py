@@ -12,7 +12,7 @@ import scipy.sparse as sp
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("split", ["0"])
+@pytest.mark.parametrize("split", ["0", "1"])
 @pytest.mark.parametrize("dims", [[(60, 60)] * 40, [(130, 70), (33, 200)]], ids=lambda d: f"{len(d)}x{d[0]}")
 def test_replays_at_the_same_time(monkeypatch, dims, split):
     import torch
