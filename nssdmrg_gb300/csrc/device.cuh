@@ -178,6 +178,7 @@ struct DevLanczos {
     uint64_t gx_gen = 0;
     int gx_prec = -1, gx_mmax = 0, gx_ndefl = -1, gx_launches = 0;
     uint32_t gx_spin = 0;        // the wait limit the graph's kernels were captured with
+    float gx_delta = 0.f;        // ... and the threshold of their projections
     const void *gx_anc = nullptr;
     bool gx_failed = false;      // capture failed once: this workspace runs without graphs
 };

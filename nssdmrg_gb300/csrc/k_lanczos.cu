@@ -346,6 +346,9 @@ struct OrthArgs {
     // only; null: w is complete)
     const float *tc = nullptr;
     int tcn = 0;
+    // k_orth: an estimate above this makes the step project; every: all steps do
+    float delta = 0.f;
+    int every = 0;
 };
 
 // The omega recurrence's constants per basis type: level after a projection,
@@ -354,9 +357,13 @@ struct OrthArgs {
 // for Ritz values; what a projection takes off a vector (up to beta times the
 // threshold, mostly along a converged Ritz vector) is not in the tridiagonal
 // matrix, though, and enters a wanted vector that has not converged yet.  At
-// 5e-13 that stays below the solver's tolerance (at 1e-8 a 96-state
+// 5e-13 that stays below the solver's default tolerance (at 1e-8 a 96-state
 // superblock's residual was 1e-10 |theta|); it costs two to four more
-// projecting steps a solve.  The FP32 phase's vector is refined afterwards.
+// projecting steps a solve.  For a tolerance below 1e-12 the threshold is half
+// of it, and a threshold within PRO_EVERY levels of a projection (the tolerance
+// of 1e-15 that a caller gets with 0) means a projection at every step: the third
+// of three states had a residual of 4e-15 |E| by estimates of 5e-13 and has
+// 7e-16.  The FP32 phase's vector is refined afterwards.
 template <class T>
 struct Pro;
 template <>
@@ -367,6 +374,8 @@ template <>
 struct Pro<float> {
     static constexpr float EPS1 = 2.4e-7f, NOISE = 1.2e-7f, DELTA = 5e-5f;
 };
+
+constexpr float PRO_EVERY = 8.f;
 
 constexpr int PRO_TAIL = 16;     // floats after the estimates: the int, then two rows of ANC_MAX products
 
@@ -1038,7 +1047,8 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_orth(OrthArgs a) {
         }
     }
     const T beta_m = j > 0 ? (T)__ldcg(a.beta + j - 1) : (T)0;
-    if (!pro_always<T>(m, n, ps)) pro.load(a.pro, ps, a.alpha, a.beta, j);
+    const bool always = a.every || pro_always<T>(m, n, ps);
+    if (!always) pro.load(a.pro, ps, a.alpha, a.beta, j);
     // no exchange here needs a fence: every CTA works on its own rows, and only
     // the values and the last CTA's stop request travel
     T tot[PA_COLS];
@@ -1065,7 +1075,6 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_orth(OrthArgs a) {
         return;
     }
     const T alpha0 = tot[0];
-    const bool always = pro_always<T>(m, n, ps);
     // three-term step (and the anchor projections); ww = w.w, and what is left
     // of w along u and y_k, taken off when w is normalised: alpha v_j and
     // beta v_{j-1} bring back alpha and beta times the rounding-level products
@@ -1126,7 +1135,7 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k_orth(OrthArgs a) {
         // is enough for the estimates)
         if (tid == 0) pro.set(j, (float)alpha0, sqrtf((float)bb[0]));
         __syncthreads();
-        const bool over = pro.template over<T>(j);
+        const bool over = pro.template over<T>(j, a.delta);
         project = over || force;
         if (project) {
             force = over && !force;
@@ -2398,6 +2407,11 @@ int run_lanczos(Ctx &c, T *V, T *w, int neigen, int mmax, double tol, uint64_t s
     oa.spin = wait_limit();
     oa.jdev = nullptr;
     oa.pro = z.pro;
+    oa.delta = Pro<T>::DELTA;
+    if (sizeof(T) == sizeof(double)) {
+        oa.delta = std::min(oa.delta, 0.5f * (float)tol);
+        oa.every = oa.delta < PRO_EVERY * Pro<T>::EPS1;
+    }
     oa.xep = (unsigned *)z.xch;
     oa.xtot = z.xch + 1;
     oa.xcol = oa.xtot + (size_t)XCOLS * (XMAX + 1);
@@ -2478,7 +2492,7 @@ int run_lanczos(Ctx &c, T *V, T *w, int neigen, int mmax, double tol, uint64_t s
         // the graph for the next ones
         const int prec = sizeof(T) == sizeof(float) ? 1 : 0;
         const bool key_ok = z.gx && z.gx_gen == c.sb.gen && z.gx_prec == prec && z.gx_mmax == mmax &&
-                            z.gx_anc == oa.anc_u && z.gx_ndefl == oa.ndefl && z.gx_spin == oa.spin;
+                            z.gx_anc == oa.anc_u && z.gx_ndefl == oa.ndefl && z.gx_spin == oa.spin && z.gx_delta == oa.delta;
         const bool graphable = c.use_graphs && !z.gx_failed && jend - j0 == CHECK && oa.anc_u == nullptr;
         if (graphable && key_ok) {
             if (from_v)
@@ -2541,6 +2555,7 @@ int run_lanczos(Ctx &c, T *V, T *w, int neigen, int mmax, double tol, uint64_t s
                 z.gx_anc = oa.anc_u;
                 z.gx_ndefl = oa.ndefl;
                 z.gx_spin = oa.spin;
+                z.gx_delta = oa.delta;
                 z.gx_launches = (int)(c.launches - l0);
                 ++c.graph_captures;
             } else {
