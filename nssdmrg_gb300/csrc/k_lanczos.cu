@@ -944,7 +944,7 @@ struct ProSmem {
 // exhausting it the estimates' model no longer holds.
 constexpr int64_t PRO_MIN_N = 3072;
 template <class T>
-__device__ __forceinline__ bool pro_always(int m, int64_t n, int ps) {
+__host__ __device__ __forceinline__ bool pro_always(int m, int64_t n, int ps) {
     return ps > PRO_MAX_PS || (sizeof(T) == 8 ? n < PRO_MIN_N : 8 * (int64_t)m > n);
 }
 
@@ -2729,9 +2729,27 @@ int run_lanczos(Ctx &c, T *V, T *w, int neigen, int mmax, double tol, uint64_t s
                                     cudaMemcpyHostToDevice, st));
     ++c.launches;
     k_ritz<T><<<NBLK, 256, (size_t)ne * m_done * sizeof(double), st>>>(V, m_done, n, z.svec, m_done, ne, z.evecs);
+    // a basis kept orthogonal by estimates gives Ritz vectors that are orthogonal
+    // to some m times their threshold (2.5e-13 between three states); projected,
+    // to rounding
+    const bool project = sizeof(T) == sizeof(double) && !oa.every && !pro_always<T>(m_done, n, oa.pstride);
+    const size_t d64_smem = (size_t)(cap + 2) * sizeof(double) + SUB * sizeof(double);
+    if (project && ne > 1) {
+        NSS_CUDA_TRY(c, allow_smem((const void *)k_dots<double>, d64_smem));
+        NSS_CUDA_TRY(c, allow_smem((const void *)k_update<double>, upd_smem));
+        NSS_CUDA_TRY(c, cudaMemsetAsync(z.flags, 0, F_NFLAGS * sizeof(int), st));
+    }
     for (int e = 0; e < ne; ++e) {
+        double *u = z.evecs + (int64_t)e * n;
+        if (project && e > 0) {
+            NSS_CUDA_TRY(c, cudaMemsetAsync(z.scal + S_ALPHA, 0, sizeof(double), st));
+            c.launches += 2;
+            k_dots<double><<<NBLK, 256, d64_smem, st>>>(z.evecs, e, u, n, z.part, h1, z.scal, z.counter, z.flags, 0, 0, z.beta);
+            k_update<double><<<NBLK, 256, upd_smem, st>>>(z.evecs, e, u, n, h1, z.part, z.scal, z.counter, z.flags, rs_alpha,
+                                                          rs_beta, 0);
+        }
         ++c.launches;
-        normalize_dev<double>(z, z.evecs + (int64_t)e * n, n, st, c.launches);
+        normalize_dev<double>(z, u, n, st, c.launches);
     }
     NSS_CUDA_TRY(c, cudaGetLastError());
     // the pageable sources above are consumed before this returns

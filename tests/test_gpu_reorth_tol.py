@@ -1,10 +1,12 @@
-"""Partial reorthogonalisation against the tolerance and the states asked for.
+"""Partial reorthogonalisation against the tolerance and the vectors asked for.
 
 An FP64 solve of 3072 states or more projects by estimate.  A basis of more
 than 4096 columns projects at every step, so nitermax = 4200 gives the solve to
 compare with.  The residual of a returned pair may exceed that solve's by what
 the stopping test (tol |E|) and the estimates' threshold (half of tol, times
-beta) allow: 3 tol |E| + 2 (its residual).
+beta) allow: 3 tol |E| + 2 (its residual).  The vectors of several states are
+orthogonal to the rounding of one projection: an inner product of two unit
+vectors summed in FP64, below 4e-15.
 """
 import numpy as np
 import pytest
@@ -44,3 +46,12 @@ def test_residual_follows_the_tolerance(solver, tol, neigen):
         print(f"N {s.n} states {neigen} tol {tol:g}: residuals / |E| {res / abs(ev[0])} ({n_est} products), "
               f"every step {rres / abs(ev[0])} ({n_all})")
         assert (res <= 3 * tol * abs(ev[0]) + 2 * rres).all()
+
+
+@pytest.mark.parametrize("tol", [1e-12, 1e-14])
+def test_vectors_of_several_states_are_orthogonal(solver, tol):
+    s = solver
+    ev, vec, _ = s.sb_diag(neigen=3, tol=tol)
+    g = np.abs(vec.T @ vec - np.eye(3))
+    print(f"N {s.n} tol {tol:g}: {g.max():.1e}")
+    assert g.max() <= 4e-15
