@@ -38,7 +38,8 @@ extern "C" {
 #define NSS_ERR_NOMEM       -3   /* allocation failed or over the HBM budget */
 #define NSS_ERR_STATE       -4   /* call out of order (e.g. nss_hv before upload) */
 #define NSS_ERR_NOCONV      -5   /* eigensolver hit its iteration cap */
-#define NSS_ERR_ASYMMETRIC  -6   /* rho not symmetric to 1e-12 (DMRG_RDM.f90:159-160) */
+#define NSS_ERR_ASYMMETRIC  -6   /* rho not symmetric to 1e-12 (DMRG_RDM.f90:159-160); not returned any
+                                  * more: both halves of a rho block come from the same sums */
 #define NSS_ERR_NOCUDA      -7   /* no CUDA device */
 
 /* Precision modes for nss_eigh. */

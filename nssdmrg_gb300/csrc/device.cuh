@@ -289,7 +289,7 @@ struct Ctx {
     // below 32 eps, Rayleigh iteration unsettled, Gram-Schmidt remainder,
     // cluster too large
     int64_t rdm_fail_why[5] = {0, 0, 0, 0, 0};
-    // device time of the last nss_rdm's phases: rho build + symmetry check,
+    // device time of the last nss_rdm's phases: rho build,
     // tridiagonal reductions, eigenvalues (+ library blocks), truncation,
     // kept vectors (+ fallbacks), compact U
     double rdm_phase_ms[6] = {0, 0, 0, 0, 0, 0};
@@ -358,7 +358,7 @@ int hv_device(Ctx &c, const double *d_v, double *d_hv, const int *stop = nullptr
 // add_planes false: the tensor-core sectors' part stays in sb.d_mma_out (mma_nplanes planes)
 int hv_device_fp32(Ctx &c, const float *d_v, float *d_hv, const int *stop = nullptr, bool add_planes = true);
 // k_sector_mma.cu: the dense sector products of the routed sectors into the
-// two output planes (the "terms only" tiles of k_hv_fp32 add them)
+// output planes, which k_add_planes or k_orth add to hv
 int hv_device_mma(Ctx &c, const float *d_v, const int *stop = nullptr);
 struct Hv32Ops;
 Hv32Ops hv32_ops(const DevSb &s);

@@ -133,24 +133,16 @@ struct Hv32Ops {
     const int *item_ell;
     const int2 *ell;             // (column, value bits) of A rows / B columns
     const int4 *term_hdr;        // per term: offset of its input sector (lo, hi), its Dr
-    // output planes of the tensor-core sector GEMM (null when it has no
-    // sectors): a "terms only" tile adds them, plane 0 first, to its A x B
-    // terms; tcn planes, tcs floats apart
-    const float *tc;
-    int tcn;
-    int64_t tcs;
 };
 
 // One 32x32 FP32 output tile t = (sector, row0, col0, flags) by 256 threads
 // (lt = thread index in the group), each owning rows {ty, ty+16} x columns
-// {tx, tx+16}.  A "terms only" tile (t.w & 1) skips the two dense products
-// and adds them from the tensor-core output planes op.tc instead.
-// The outputs, multiplied by `scale`, go to hv; returns this thread's share
-// of sum_i v[i] * out[i] * scale^2 over its outputs (the Lanczos alpha of a
-// unit vector v * scale), meaningful for whole tiles (t.w == 0).
+// {tx, tx+16}.  A "terms only" tile (t.w & 1) skips the two dense products:
+// the tensor-core GEMM forms them beside it, and they are added afterwards
+// (k_add_planes, k_orth).
 template <class Sync>
-__device__ __forceinline__ float hv32_tile(int4 t, const float *__restrict__ v, float *__restrict__ hv,
-                                           const Hv32Ops &op, Tile32Smem &sm, int lt, Sync sync, float scale) {
+__device__ __forceinline__ void hv32_tile(int4 t, const float *__restrict__ v, float *__restrict__ hv,
+                                          const Hv32Ops &op, Tile32Smem &sm, int lt, Sync sync) {
     const int k = t.x, row0 = t.y, col0 = t.z;
     const int dl = op.dls[k], dr = op.drs[k];
     const int64_t o = op.off[k];
@@ -231,23 +223,11 @@ __device__ __forceinline__ float hv32_tile(int4 t, const float *__restrict__ v, 
         }
         sync();
     }
-    float part = 0.f;
     for (int rr = 0; rr < 2; ++rr)
         for (int cc = 0; cc < 2; ++cc) {
             const int il = row0 + ty + 16 * rr, ir = col0 + tx + 16 * cc;
-            if (il < dl && ir < dr) {
-                const int64_t idx = (int64_t)il * dr + ir;
-                float y = acc[rr][cc] * scale;
-                if ((t.w & 1) && op.tc) {
-                    float d = op.tc[o + idx];
-                    for (int p = 1; p < op.tcn; ++p) d += op.tc[(int64_t)p * op.tcs + o + idx];
-                    y += d;
-                }
-                hv[o + idx] = y;
-                part = fmaf(W[idx] * scale, y, part);
-            }
+            if (il < dl && ir < dr) hv[o + (int64_t)il * dr + ir] = acc[rr][cc];
         }
-    return part;
 }
 
 }  // namespace nss

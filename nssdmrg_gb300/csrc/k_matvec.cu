@@ -507,7 +507,7 @@ int sb_upload(Ctx &c, const nss_sb_desc *d, bool trusted, bool allow_split) {
     }
     // Sectors on the tensor-core GEMM (k_sector_mma.cu) get their A x B
     // terms from "terms only" CUDA-core tiles (w = 1), listed first, which
-    // k_hv_fp32 runs after the GEMM and which add its two output planes.
+    // k_hv_fp32 runs beside the GEMM; its output planes are added afterwards.
     MmaPlan plan;
     int tc_thr = c.tc_min_dl, tc_bn = c.mma_bn;
     c.tune_cand = -1;
@@ -941,7 +941,7 @@ __global__ void __launch_bounds__(256) k_hv_fp32(const float *__restrict__ v, fl
                                                  const int4 *__restrict__ tiles, Hv32Ops op, const int *stop) {
     if (stop && *stop) return;   // the Lanczos loop has already finished
     __shared__ Tile32Smem sm;
-    hv32_tile(tiles[blockIdx.x], v, hv, op, sm, threadIdx.x, CtaSync{}, 1.0f);
+    hv32_tile(tiles[blockIdx.x], v, hv, op, sm, threadIdx.x, CtaSync{});
 }
 
 Hv32Ops hv32_ops(const DevSb &s) {
@@ -961,9 +961,6 @@ Hv32Ops hv32_ops(const DevSb &s) {
     op.item_ell = s.d_item_ell;
     op.ell = s.d_ell;
     op.term_hdr = s.d_term_hdr;
-    op.tc = s.mma_nitems ? s.d_mma_out : nullptr;
-    op.tcn = s.mma_nitems ? s.mma_nplanes : 0;
-    op.tcs = s.n;
     return op;
 }
 
@@ -1004,9 +1001,7 @@ int hv_device_fp32(Ctx &c, const float *d_v, float *d_hv, const int *stop, bool 
     NSS_CUDA_TRY(c, cudaEventRecord(c.hv_fork, c.stream));
     NSS_CUDA_TRY(c, cudaStreamWaitEvent(c.hv_side, c.hv_fork, 0));
     if (s.ntiles32 > 0) {
-        Hv32Ops op = hv32_ops(s);
-        op.tc = nullptr;   // the planes come afterwards
-        k_hv_fp32<<<s.ntiles32, 256, 0, c.hv_side>>>(d_v, d_hv, s.d_tiles32, op, stop);
+        k_hv_fp32<<<s.ntiles32, 256, 0, c.hv_side>>>(d_v, d_hv, s.d_tiles32, hv32_ops(s), stop);
         c.launches += 1;
     }
     NSS_CUDA_TRY(c, cudaEventRecord(c.hv_join, c.hv_side));

@@ -9,8 +9,8 @@
 // pieces of consecutive slabs, each writing its partial tile to its own
 // output plane (no atomics: every plane element has one writer, and the
 // plane sum is formed in a fixed order).  The A x B terms of these sectors
-// stay on CUDA cores (k_hv_fp32 "terms only" tiles, launched after this
-// kernel), which add the planes.  The pieces are dealt to the CTAs longest
+// stay on CUDA cores (k_hv_fp32 "terms only" tiles, beside this kernel); the
+// planes are added to them afterwards.  The pieces are dealt to the CTAs longest
 // first onto the least loaded CTA, and each CTA runs its own range.
 //
 // Precision: split TF32.  Every FP32 operand x is split into hi = x rounded
@@ -578,8 +578,8 @@ int mma_finish(Ctx &c, const MmaPlan &p) {
 }
 
 // D_k of every routed sector into the output planes (d_mma_out + q n): pack
-// W, then the persistent GEMM.  The caller's "terms only" tiles add the
-// planes to their A x B terms.
+// W, then the persistent GEMM.  The caller adds the planes to its "terms only"
+// tiles.
 int hv_device_mma(Ctx &c, const float *d_v, const int *stop) {
     DevSb &s = c.sb;
     if (s.mma_nitems == 0) return NSS_OK;

@@ -76,8 +76,8 @@ __device__ __forceinline__ double wmax(double v) {
 }
 
 // Householder tridiagonalisation of one block (n <= SYEV_MAX) in shared
-// memory.  rho blocks are row-major and symmetric (checked before).  The
-// block's rows are first reordered so that the connected components of its
+// memory.  rho blocks are row-major and symmetric (k_rho writes both halves
+// from one sum).  The block's rows are first reordered so that the connected components of its
 // exact nonzero pattern are contiguous (perm[new] = old row): the reflectors
 // of one component then never touch another's rows, T splits exactly at
 // the component boundaries, and eigenvectors keep the exact zeros of the
