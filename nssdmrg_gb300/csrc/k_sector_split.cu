@@ -798,12 +798,10 @@ __global__ void __launch_bounds__(256, 4) k_split_terms(const double *__restrict
 // Host side
 
 bool split_wanted(const DevSb &s) {
-    const char *e = std::getenv("NSS_SPLIT64");
-    if (e && std::atoi(e) == 0) return false;
-    if (e) return true;
     for (int k = 0; k < s.nsb; ++k)
         if (s.dls[k] > SP_KMAX || s.drs[k] > SP_KMAX) return false;
-    return s.flops_dense >= 4e7;
+    const char *e = std::getenv("NSS_SPLIT64");
+    return e ? std::atoi(e) != 0 : s.flops_dense >= 4e7;
 }
 
 void split_layout(const DevSb &s, const std::vector<int> &rowptr, const std::vector<int> &col,

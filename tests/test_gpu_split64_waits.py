@@ -53,3 +53,27 @@ def test_product_is_right_when_its_waits_run_out(monkeypatch):
     assert np.abs(s.spmatvec(v1) - want[0]).max() <= 800 * 2.0 ** -53 * np.abs(want[0]).max()
     s.close()
     g.close()
+
+
+@pytest.mark.parametrize("dr,kernels", [(4096, 5), (4097, 1)])
+def test_the_largest_contracted_dimension(monkeypatch, dr, kernels):
+    """The digit sums hold 4096 products; a wider sector keeps its superblock on
+    the CUDA cores, also where the tensor cores are asked for."""
+    import scipy.sparse as sp
+
+    import nssdmrg_gb300 as nss
+    nss.lib()
+    monkeypatch.setenv("NSS_SPLIT64", "1")
+    rng = np.random.default_rng(dr)
+    s = nss.Superblock()
+    d = rng.standard_normal(dr)
+    s.upload([2], [dr], [0], [sp.csr_matrix(np.array([[1.5, 0.25], [0.25, -2.0]]))], [sp.diags(d).tocsr()], [], 0, 2, dr)
+    v = rng.standard_normal(2 * dr)
+    before = s.launches
+    got = s.spmatvec(v).reshape(2, dr)
+    assert s.launches - before == kernels
+    w = v.reshape(2, dr)
+    want = np.array([[1.5, 0.25], [0.25, -2.0]]) @ w + w * d
+    mag = np.array([[1.5, 0.25], [0.25, 2.0]]) @ abs(w) + abs(w * d)
+    assert (abs(got - want) <= 10 * 2.0 ** -53 * mag).all()
+    s.close()
