@@ -751,8 +751,9 @@ struct HvOps {
 };
 
 // What k_hv_fp64 computes of a product on the tensor cores: every tile when
-// that gave up or did not run (words null), else those on its list, of which the sides that are good come
-// from the planes of digit sums.  A tile is an eighth of a SplitTile.
+// that gave up or did not run (words null), else those on its list, of which the
+// sides that are good come from the planes of digit sums.  A tile is an eighth
+// of a SplitTile.
 struct HvRedo {
     const SplitTile *tiles;
     const int *words;            // sb.d_sp_redo
@@ -826,13 +827,14 @@ __global__ void __launch_bounds__(32 * HV_WARPS) k_hv_fp64(const double *__restr
         };
         double acc = 0.0, part = 0.0;                // part (redo): a side's sum, the sides are added
         const int first = REDO && !(sides & 1) ? c0 : 0, last = REDO && !(sides & 2) ? c0 : c0 + c1;
-        if (first < last) load(first);
+        if (!REDO || first < last) load(first);
         for (int c = first; c < last; ++c) {
             const bool left = c < c0;
-            if (REDO && c == c0) {
-                part = acc;
-                acc = 0.0;
-            }
+            if constexpr (REDO)
+                if (c == c0) {
+                    part = acc;
+                    acc = 0.0;
+                }
             const int kn = min(KC, left ? dl - c * KC : dr - (c - c0) * KC);
 #pragma unroll
             for (int q = 0; q < HV_TR; ++q) sa[q][lane] = ra[q];
