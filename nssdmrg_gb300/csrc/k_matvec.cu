@@ -753,7 +753,9 @@ struct HvOps {
 // What k_hv_fp64 computes of a product on the tensor cores: every tile when
 // that gave up or did not run (words null), else those on its list, of which the
 // sides that are good come from the planes of digit sums.  A tile is an eighth
-// of a SplitTile.
+// of a SplitTile.  A listed tile's K loops and terms are shared out over the
+// four warps of a CTA, one on each quarter of its SM: there are few of them as a
+// rule, and a warp by itself takes 16 us for 500 products a side.
 struct HvRedo {
     const SplitTile *tiles;
     const int *words;            // sb.d_sp_redo
@@ -783,7 +785,8 @@ __global__ void __launch_bounds__(32 * HV_WARPS) k_hv_fp64(const double *__restr
     // may be left without one is another in each CTA of an SM.  What is above
     // one tile a warp is dealt backwards, so that the warps with the longest
     // first tile get the shortest second one.
-    const int all = HV_WARPS * grid, mine = (int)((warp + blockIdx.x / nsm) % HV_WARPS) * grid + blockIdx.x;
+    const int all = REDO && listed ? grid : HV_WARPS * grid;
+    const int mine = REDO && listed ? blockIdx.x : (int)((warp + blockIdx.x / nsm) % HV_WARPS) * grid + blockIdx.x;
     for (int r = 0; r * all < ntiles; ++r) {
         const int tile = r * all + (r & 1 ? all - 1 - mine : mine);
         if (tile >= ntiles) continue;
@@ -796,7 +799,12 @@ __global__ void __launch_bounds__(32 * HV_WARPS) k_hv_fp64(const double *__restr
             s = redo.tiles[id / HV_SUB];
             t = HvRec{s.dl, s.dr, s.row0 + HV_TR * (sub / (32 / HV_TC)), s.col0 + HV_TC * (sub % (32 / HV_TC)), s.t0, s.t1, s.csr,
                       0, s.off, s.hlo, s.hro};
-            if (t.row0 >= t.dl || t.col0 >= t.dr) continue;
+            if (t.row0 >= t.dl || t.col0 >= t.dr) continue;   // (not of the list)
+            if (listed) {
+                const int t0 = t.t0, nt = t.t1 - t0;
+                t.t0 = t0 + nt * warp / HV_WARPS;
+                t.t1 = t0 + nt * (warp + 1) / HV_WARPS;
+            }
         } else {
             t = recs[tile];
         }
@@ -826,7 +834,12 @@ __global__ void __launch_bounds__(32 * HV_WARPS) k_hv_fp64(const double *__restr
             }
         };
         double acc = 0.0, part = 0.0;                // part (redo): a side's sum, the sides are added
-        const int first = REDO && !(sides & 1) ? c0 : 0, last = REDO && !(sides & 2) ? c0 : c0 + c1;
+        int first = REDO && !(sides & 1) ? c0 : 0, last = REDO && !(sides & 2) ? c0 : c0 + c1;
+        if (REDO && listed) {
+            const int c = first, nc = last - first;
+            first = c + nc * warp / HV_WARPS;
+            last = c + nc * (warp + 1) / HV_WARPS;
+        }
         if (!REDO || first < last) load(first);
         for (int c = first; c < last; ++c) {
             const bool left = c < c0;
@@ -853,7 +866,7 @@ __global__ void __launch_bounds__(32 * HV_WARPS) k_hv_fp64(const double *__restr
         if constexpr (REDO) {
             part += acc;
             acc = 0.0;
-            if (in)
+            if (in && warp == 0)                     // (sides = 3 where every warp has a tile)
                 for (int side = 0; side < 2; ++side)
                     if (!(sides >> side & 1)) {      // left: H_L row, W column; right: W row, H_R row
                         const int64_t e = t.off + (int64_t)ir * dl + il + side * redo.n;
@@ -932,7 +945,18 @@ __global__ void __launch_bounds__(32 * HV_WARPS) k_hv_fp64(const double *__restr
                 }
             }
         }
-        if (in) hv[t.off + (int64_t)il * dr + ir] = REDO ? part + acc : acc;
+        if constexpr (REDO) {
+            acc += part;
+            if (listed) {
+                __shared__ double shares[HV_WARPS][32];
+                shares[warp][lane] = acc;
+                __syncthreads();
+                acc = (shares[0][lane] + shares[1][lane]) + (shares[2][lane] + shares[3][lane]);
+                __syncthreads();
+                if (warp) continue;
+            }
+        }
+        if (in) hv[t.off + (int64_t)il * dr + ir] = acc;
     }
 }
 

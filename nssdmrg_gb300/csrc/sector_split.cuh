@@ -110,15 +110,23 @@ struct SplitPlan {
 };
 
 // whether the superblock's FP64 products take this path: from 40 MFLOP of
-// dense work.  Measured (us a product, CUDA cores against this): spin-1 N =
-// 25 300 (9 MFLOP) 22.9 / 23.0, 100 200 (62) 74 / 29, 398 000 (480) 455 / 56,
-// 1.18 million (2 430) 2 108 / 154.  Superblocks between 10 and 40 MFLOP would
-// gain up to a factor of two; they stay on the CUDA cores, whose results whole
-// runs at those sizes are pinned to in their last digits.  NSS_SPLIT64 = 0 / 1
-// forces a path (comparisons, tests).
+// dense work.  Measured, us a product, one after another on one stream, CUDA
+// cores / this in a solve / this for a caller (every element checked):
+//   spin-1    25 300 states     9 MFLOP    16.5 / 24 / 38
+//            100 200           62          59.5 / 30 / 48
+//            397 700          480         410   / 58 / 82
+//          1 178 000        2 430       2 008   / 158 / 194
+//   spin-1/2  88 500           70          59.5 / 30 / 48
+//            615 700        1 150         912   / 74 / 119
+//   Hubbard  106 700           48          87   / 40 / 60
+// For a caller's vector graded over twelve decades 88, 329, 1 348 (spin-1), 667
+// and 106.  Superblocks between 15 and 40 MFLOP would gain up to a factor of two
+// in a solve; they stay on the CUDA cores, whose results whole runs at those
+// sizes are pinned to in their last digits.  NSS_SPLIT64 = 0 / 1 forces a path
+// (comparisons, tests).
 bool split_wanted(const DevSb &s);
-// the plan from the superblock's tables and its CSR pool (rowptr, col, val)
-// (csr: HvRec::csr per sector)
+// the plan from the superblock's tables, its CSR pool (rowptr, col, val) and
+// HvRec::csr of the sectors
 void split_layout(const DevSb &s, const std::vector<int> &rowptr, const std::vector<int> &col,
                   const std::vector<double> &val, const std::vector<int> &csr, int nsm, SplitPlan &p);
 // memory, digits of H_L and H_R and the tensor maps, after the dense blocks are
