@@ -119,7 +119,7 @@ struct DevSb {
     float *d_sp_size = nullptr;        // standalone products: sums of |H||W|, two planes
     struct SplitItem *d_sp_sitems = nullptr;   // ... and their work items
     int2 *d_sp_srng = nullptr;
-    int sp_sgrid = 0;
+    int sp_sgrid = 0, sp_sn = 256;
     // a standalone product's words: gave up, tiles of k_hv_fp64 to compute, their list
     int *d_sp_redo = nullptr;
     int sp_nexp = 0;                   // scale exponents; the rows' nonzero counts follow them

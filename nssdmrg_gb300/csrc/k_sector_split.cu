@@ -466,7 +466,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_sector_split(const __grid_con
 
 // sum |H||W| of every output, in units of the operands' scales and a little
 // below (bf16 towards zero, FP32 sums): the products of the absolute values, 128
-// x 256 outputs a tile (an MMA takes ~130 cycles whatever its width).  One lane
+// x sn outputs a tile (an MMA takes ~130 cycles whatever its width).  One lane
 // issues the copies (four slabs of A and B in flight), one the MMAs, four warps
 // store.  Waits are bounded as in k_sector_split.
 namespace {
@@ -482,7 +482,7 @@ __global__ void __launch_bounds__(SZ_THREADS, 1) k_split_size(const __grid_const
                                                                const __grid_constant__ CUtensorMap map_b,
                                                                const SplitItem *__restrict__ items,
                                                                const int2 *__restrict__ ranges, float *__restrict__ out,
-                                                               int64_t plane, uint32_t spin, int *err, const int *stop) {
+                                                               int64_t plane, int sn, uint32_t spin, int *err, const int *stop) {
     using C = SizeCfg;
     if (stop && *stop) return;   // before any TMEM allocation: uniform exit
     extern __shared__ uint8_t sp_raw[];
@@ -520,7 +520,7 @@ __global__ void __launch_bounds__(SZ_THREADS, 1) k_split_size(const __grid_const
     auto slabs = [](int k) { return (k + SP_KC - 1) / SP_KC; };
     auto abox = [&](int st) { return smem_u32(smem + (size_t)st * (C::A_BYTES + C::B_BYTES)); };
     // columns of an item's tile, a multiple of 16
-    auto width = [](const SplitItem &m) { return min(SP_SN, (m.dr - m.n0 + 15) & ~15); };
+    auto width = [&](const SplitItem &m) { return min(sn, (m.dr - m.n0 + 15) & ~15); };
 
     if (warp == 0 && lane == 0) {
         // ---- TMA producer
@@ -532,7 +532,7 @@ __global__ void __launch_bounds__(SZ_THREADS, 1) k_split_size(const __grid_const
                 const int st = it % SZ_STAGES;
                 if (!mbar_wait(smem_u32(&empty[st]), ((uint32_t)(it / SZ_STAGES) & 1u) ^ 1u, spin, abort)) { give_up(); ok = false; break; }
                 const uint32_t fb = smem_u32(&full[st]);
-                mbar_expect_tx(fb, (uint32_t)(C::A_BYTES + C::B_BYTES));
+                mbar_expect_tx(fb, (uint32_t)(C::A_BYTES + sn * 128));
                 tma_load_2d(abox(st), &map_a, 0, m.a_row + c * m.a_rows + m.m0, fb);
                 tma_load_2d(abox(st) + C::A_BYTES, &map_b, 0, m.b_row + c * m.b_rows + m.n0, fb);
                 ++issued;
@@ -867,11 +867,18 @@ void split_layout(const DevSb &s, const std::vector<int> &rowptr, const std::vec
                 p.items.push_back(SplitItem{R.w, R.hr, dl, dr, dr, dl, dr, m0, n0, 1, s.off[k]});
             }
     }
+    // the narrowest tiles of which every CTA gets one at most: what counts is
+    // the time of a tile (loads and stores shrink with it)
+    for (p.sn = 64; p.sn < SP_SN; p.sn *= 2) {
+        int64_t tiles = 0;
+        for (int k = 0; k < s.nsb; ++k) tiles += 2 * (int64_t)((s.dls[k] + SP_M - 1) / SP_M) * ((s.drs[k] + p.sn - 1) / p.sn);
+        if (tiles <= nsm) break;
+    }
     for (int k = 0; k < s.nsb; ++k) {
         const int dl = s.dls[k], dr = s.drs[k];
         const Rows &R = rs[k];
         for (int m0 = 0; m0 < dl; m0 += SP_M)
-            for (int n0 = 0; n0 < dr; n0 += SP_SN) {
+            for (int n0 = 0; n0 < dr; n0 += p.sn) {
                 p.sitems.push_back(SplitItem{R.ahl, R.awt, dl, dr, dl, dl, dr, m0, n0, 0, s.off[k]});
                 p.sitems.push_back(SplitItem{R.aw, R.ahr, dl, dr, dr, dl, dr, m0, n0, 1, s.off[k]});
             }
@@ -993,7 +1000,8 @@ int split_finish(Ctx &c, const SplitPlan &p) {
     s.sp_bn = p.bn;
     s.sp_grid = p.grid;
     s.sp_sgrid = p.sgrid;
-    const std::pair<unsigned char *, int> maps[3] = {{s.sp_map_a, SP_M}, {s.sp_map_b, p.bn}, {s.sp_map_s, SP_SN}};
+    s.sp_sn = p.sn;
+    const std::pair<unsigned char *, int> maps[3] = {{s.sp_map_a, SP_M}, {s.sp_map_b, p.bn}, {s.sp_map_s, p.sn}};
     for (const auto &m : maps)
         if (int rc = tc_tensor_map(c, m.first, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, s.d_sp_pool, SP_KC, p.pool_rows, m.second))
             return rc;
@@ -1022,7 +1030,7 @@ int launch_size(Ctx &c, int *err, const int *stop) {
     std::memcpy(&mb, s.sp_map_s, sizeof(mb));
     c.launches += 1;
     k_split_size<<<s.sp_sgrid, SZ_THREADS, SizeCfg::SMEM, c.stream>>>(ma, mb, s.d_sp_sitems, s.d_sp_srng, s.d_sp_size, s.n,
-                                                                     wait_limit(), err, stop);
+                                                                     s.sp_sn, wait_limit(), err, stop);
     return NSS_OK;
 }
 

@@ -13,7 +13,7 @@ namespace nss {
 constexpr int SP_M = 128;      // UMMA M: rows of il per work item
 constexpr int SP_KC = 64;      // K columns per slab (128 bytes of bf16)
 constexpr int SP_D = 7;        // digits of an operand element
-constexpr int SP_SN = 256;     // tile width of the sums of |H||W|
+constexpr int SP_SN = 256;     // largest tile width of the sums of |H||W|
 constexpr int SP_KMAX = 4096;  // largest contracted dimension (the 64-bit sums)
 constexpr int SP_BADEXP = 1 << 20;         // scale exponent of a row with an Inf or NaN
 constexpr int SP_ZEROEXP = -(1 << 20);     // ... of a row of zeros
@@ -51,7 +51,7 @@ __device__ __forceinline__ double fixed_to_double(int s0, int64_t r, int e) {
 }
 
 // One work item: the product of one 128 x BN tile of one phase, H_L W (output
-// plane 0) or W H_R^T (plane 1), or of their absolute values (128 x SP_SN).
+// plane 0) or W H_R^T (plane 1), or of their absolute values (128 x sn).
 // Row indices address the digit pool.
 struct SplitItem {
     int a_row, b_row;            // slab 0 of the A and B operands (digit 0 or absolute values)
@@ -98,7 +98,8 @@ struct SplitPlan {
     std::vector<SplitJob> jobs_w, jobs_hl, jobs_hr;
     int64_t pool_rows = 0;
     int nexp = 0, bn = 64, grid = 0, kmax = 0;
-    std::vector<SplitItem> sitems;     // sums of |H||W|: 128 x SP_SN tiles
+    std::vector<SplitItem> sitems;     // sums of |H||W|: 128 x sn tiles
+    int sn = SP_SN;
     std::vector<int2> srng;
     int sgrid = 0;
     // A x B terms
@@ -112,15 +113,16 @@ struct SplitPlan {
 // whether the superblock's FP64 products take this path: from 40 MFLOP of
 // dense work.  Measured, us a product, one after another on one stream, CUDA
 // cores / this in a solve / this for a caller (every element checked):
-//   spin-1    25 300 states     9 MFLOP    16.5 / 24 / 38
-//            100 200           62          59.5 / 30 / 48
-//            397 700          480         410   / 58 / 82
+//   spin-1    25 300 states     9 MFLOP    16.5 / 24 / 36
+//            100 200           62          59.5 / 30 / 43
+//            397 700          480         410   / 58 / 76
 //          1 178 000        2 430       2 008   / 158 / 194
-//   spin-1/2  88 500           70          59.5 / 30 / 48
-//            615 700        1 150         912   / 74 / 119
-//   Hubbard  106 700           48          87   / 40 / 60
-// For a caller's vector graded over twelve decades 88, 329, 1 348 (spin-1), 667
-// and 106.  Superblocks between 15 and 40 MFLOP would gain up to a factor of two
+//   spin-1/2  88 500           70          59.5 / 30 / 44
+//            615 700        1 150         910   / 74 / 111
+//   Hubbard  106 700           48          87   / 40 / 57
+// For a caller's vector graded over twelve decades 84, 322, 1 349 (spin-1 from
+// 100 200 states), 85, 656 and 103.  Superblocks between 15 and 40 MFLOP would
+// gain up to a factor of two
 // in a solve; they stay on the CUDA cores, whose results whole runs at those
 // sizes are pinned to in their last digits.  NSS_SPLIT64 = 0 / 1 forces a path
 // (comparisons, tests).
