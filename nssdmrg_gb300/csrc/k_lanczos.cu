@@ -2123,6 +2123,23 @@ __global__ void k_run_reset(float *pro, int ps, float eps1, int *flags, double *
     for (int64_t k = t; k < nslots; k += nt) slots[k] = 0.f;
 }
 
+// Ritz vectors of ne states from the coefficients svec[e * m + l] in shared
+// memory: all states in one pass over the basis, or one after the other where
+// their coefficients do not fit together
+template <class T>
+int launch_ritz(Ctx &c, const T *V, int m, int64_t n, const double *svec, int ne, double *out, cudaStream_t st,
+                int64_t &launches) {
+    const int at_once = (size_t)ne * m * sizeof(double) <= CHUNK_SMEM_MAX ? ne : 1;
+    const size_t smem = (size_t)at_once * m * sizeof(double);
+    NSS_CUDA_TRY(c, allow_smem((const void *)k_ritz<T>, smem));
+    for (int e = 0; e < ne; e += at_once) {
+        ++launches;
+        k_ritz<T><<<NBLK, 256, smem, st>>>(V, m, n, svec + (int64_t)e * m, m, at_once, out + (int64_t)e * n);
+    }
+    NSS_CUDA_TRY(c, cudaGetLastError());
+    return NSS_OK;
+}
+
 // x <- x / ||x|| on stream st (two launches)
 template <class T>
 void normalize_dev(DevLanczos &z, T *x, int64_t n, cudaStream_t st, int64_t &launches) {
@@ -2696,6 +2713,7 @@ int run_lanczos(Ctx &c, T *V, T *w, int neigen, int mmax, double tol, uint64_t s
         }
         NSS_CUDA_TRY(c, cudaMemcpyAsync(z.svec, cvec.data(), cvec.size() * sizeof(double), cudaMemcpyHostToDevice, st));
         c.launches += 2;
+        NSS_CUDA_TRY(c, allow_smem((const void *)k_ritz_anchor<T>, cvec.size() * sizeof(double)));
         k_ritz_anchor<T><<<NBLK, 256, cvec.size() * sizeof(double), st>>>(V, m_done, n, z.svec, anc->u, anc->out);
         normalize_dev<double>(z, anc->out, n, st, c.launches);
         NSS_CUDA_TRY(c, cudaGetLastError());
@@ -2727,8 +2745,7 @@ int run_lanczos(Ctx &c, T *V, T *w, int neigen, int mmax, double tol, uint64_t s
     NSS_CUDA_TRY(c, cudaMemcpyAsync(z.resid, resid.data(), ne * sizeof(double), cudaMemcpyHostToDevice, st));
     NSS_CUDA_TRY(c, cudaMemcpyAsync(z.svec, svec.data(), (size_t)ne * m_done * sizeof(double),
                                     cudaMemcpyHostToDevice, st));
-    ++c.launches;
-    k_ritz<T><<<NBLK, 256, (size_t)ne * m_done * sizeof(double), st>>>(V, m_done, n, z.svec, m_done, ne, z.evecs);
+    if (int rc2 = launch_ritz<T>(c, V, m_done, n, z.svec, ne, z.evecs, st, c.launches)) return rc2;
     // a basis kept orthogonal by estimates gives Ritz vectors that are orthogonal
     // to some m times their threshold (2.5e-13 between three states); projected,
     // to rounding
@@ -3447,8 +3464,8 @@ int engine_step(BatchEngine &E, int max_done, int *ndone, int *ids, double *ener
         const cudaStream_t s = B.c->stream;
         if ((rc = fork(B))) return rc;
         NSS_CUDA_TRY(c0, cudaMemcpyAsync(z.svec, B.svec.data(), (size_t)m * sizeof(double), cudaMemcpyHostToDevice, s));
-        c0.launches += 2;
-        k_ritz<float><<<NBLK, 256, (size_t)m * sizeof(double), s>>>(z.V32, m, B.n, z.svec, m, 1, z.evecs);
+        ++c0.launches;
+        if ((rc = launch_ritz<float>(c0, z.V32, m, B.n, z.svec, 1, z.evecs, s, c0.launches))) return rc;
         normalize_dev<double>(z, z.evecs, B.n, s, c0.launches);
         if ((rc = fp64_energy(B, b, true)) || (rc = join(B, b))) return rc;
     }
@@ -3460,6 +3477,7 @@ int engine_step(BatchEngine &E, int max_done, int *ndone, int *ids, double *ener
         NSS_CUDA_TRY(c0, cudaMemcpyAsync(z.svec, B.cvec.data(), B.cvec.size() * sizeof(double), cudaMemcpyHostToDevice,
                                          s));
         c0.launches += 2;
+        NSS_CUDA_TRY(c0, allow_smem((const void *)k_ritz_anchor<float>, B.cvec.size() * sizeof(double)));
         k_ritz_anchor<float><<<NBLK, 256, B.cvec.size() * sizeof(double), s>>>(z.V32, B.m_done, B.n, z.svec, z.evecs,
                                                                                z.evecs);
         normalize_dev<double>(z, z.evecs, B.n, s, c0.launches);
