@@ -122,10 +122,9 @@ struct SplitPlan {
 //   Hubbard  106 700           48          87   / 40 / 57
 // For a caller's vector graded over twelve decades 84, 322, 1 349 (spin-1 from
 // 100 200 states), 85, 656 and 103.  Superblocks between 15 and 40 MFLOP would
-// gain up to a factor of two
-// in a solve; they stay on the CUDA cores, whose results whole runs at those
-// sizes are pinned to in their last digits.  NSS_SPLIT64 = 0 / 1 forces a path
-// (comparisons, tests).
+// gain up to a factor of two in a solve; they stay on the CUDA cores, whose
+// results whole runs at those sizes are pinned to in their last digits.
+// NSS_SPLIT64 = 0 / 1 forces a path (comparisons, tests).
 bool split_wanted(const DevSb &s);
 // the plan from the superblock's tables, its CSR pool (rowptr, col, val) and
 // HvRec::csr of the sectors
